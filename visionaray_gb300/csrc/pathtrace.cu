@@ -5,14 +5,18 @@
 // visionaray runs the whole path (all bounces, its traversal, shading and shadow
 // ray) in one thread per pixel; threads of a warp diverge as soon as paths end at
 // different bounces or traverse different subtrees.  Here a frame is a sequence of
-// passes, one per sample index; each pass keeps one path per pixel and advances all
-// live paths one bounce at a time through three kernels:
+// passes of several samples per pixel (as many as kPassPaths paths hold, so that a small
+// frame fills the GPU and takes few launches); a pass keeps one path per pixel and sample,
+// the samples of a pixel next to each other, and advances all live paths one bounce at a
+// time through three stages:
 //   extend : closest-hit traversal of the live rays (queue in, hits out)
 //   shade  : surface sampling, emission with MIS, next-event estimation (light
 //            sample + shadow ray), throughput update, Russian roulette; live paths
 //            and shadow rays are appended to compacted queues with one atomic per
 //            warp (ballot + popc)
-//   shadow : any-hit traversal of the shadow queue, unoccluded contributions added
+//   shadow : any-hit traversal of the shadow queue, unoccluded contributions added (over
+//            instances in one launch with the next bounce's extend, which does not depend
+//            on it)
 // so every traversal launch runs over a dense queue of live rays.  The arithmetic is
 // the reference's, operation for operation (this file is compiled with
 // --fmad=false; divisions and square roots are IEEE), and the random numbers are
@@ -23,6 +27,7 @@
 #include "instances.cuh"
 #include "pt_shade.cuh"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -77,7 +82,8 @@ struct frame_buffers
     float4* radiance;
     uint2* rng_flags;   // draw counter, flags
     float4* sum;
-    uint32_t* counts;   // queue 0, queue 1, shadow queue
+    uint32_t* counts;   // per bounce: its ray queue's length, its shadow queue's
+    uint32_t samples;   // samples per pixel of this pass: path p is sample p % samples of pixel p / samples
     // queue order by origin cell (GBRT_TRACE_SORT_RAYS): keys / values and their
     // double buffers, the sort's scratch
     uint32_t* keys;
@@ -110,20 +116,16 @@ __device__ __forceinline__ void store_ray(gbrt_ray* dst, v3 o, v3 d, float tmin,
 }
 
 // Jittered primary rays (detail/sched_common.h:209-233: jitter x drawn before y) through
-// the pinhole camera (detail/pinhole_camera.inl:103-120).
+// the pinhole camera (detail/pinhole_camera.inl:103-120), and the pass's queue lengths.
 __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t width, uint32_t height,
-                                                    uint32_t frame, uint32_t sample, camera_basis cam)
+                                                    uint32_t frame, uint32_t first_sample, uint32_t num_counts,
+                                                    camera_basis cam)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    uint32_t n = width * height;
-    if (i == 0)
-    {
-        fb.counts[0] = n;
-        fb.counts[1] = 0;
-        fb.counts[2] = 0;
-    }
+    const uint32_t n = width * height * fb.samples;
+    for (uint32_t k = i; k < num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
     if (i >= n) return;
-    v3 d = primary_dir(cam, width, height, frame, i, sample);
+    v3 d = primary_dir(cam, width, height, frame, i / fb.samples, first_sample + i % fb.samples);
     store_ray(&fb.rays[0][i], { cam.eye.x, cam.eye.y, cam.eye.z }, d, 0.0f, FLT_MAX);
     fb.path[0][i] = i;
     fb.throughput[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -131,17 +133,21 @@ __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t w
     fb.rng_flags[i] = make_uint2(2u, kLastSpecular);
 }
 
+// The unoccluded contribution of shadow queue entry j.
+__device__ __forceinline__ void add_shadow(frame_buffers const& fb, uint32_t j)
+{
+    const uint32_t p = fb.shadow_path[j];
+    const float4 c = fb.shadow_contrib[j];
+    const float4 r = fb.radiance[p];
+    fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
+}
+
 template <bool Wide>
-__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_extend(frame_buffers fb, int q, bvh_view v,
-                                                                  uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_extend(frame_buffers fb, int q, uint32_t bounce,
+                                                                  bvh_view v, uint32_t* __restrict__ status)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i == 0)
-    {
-        fb.counts[q ^ 1] = 0;   // the shade kernel that follows appends to these
-        fb.counts[2] = 0;
-    }
-    uint32_t n = fb.counts[q];
+    uint32_t n = fb.counts[2 * bounce];
     if (i >= n) return;
     const float4* rp = reinterpret_cast<const float4*>(&fb.rays[q][i]);
     float4 r0 = rp[0], r1 = rp[1];
@@ -176,17 +182,12 @@ __global__ void __launch_bounds__(kBlock) pt_queue_keys(const gbrt_ray* __restri
 
 // pt_extend over the queue in the order perm (thread i traces queue entry perm[i]).
 template <bool Wide>
-__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_extend_sorted(frame_buffers fb, int q,
+__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_extend_sorted(frame_buffers fb, int q, uint32_t bounce,
                                                                          const uint32_t* __restrict__ perm,
                                                                          bvh_view v, uint32_t* __restrict__ status)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i == 0)
-    {
-        fb.counts[q ^ 1] = 0;
-        fb.counts[2] = 0;
-    }
-    uint32_t n = fb.counts[q];
+    uint32_t n = fb.counts[2 * bounce];
     if (i >= n) return;
     uint32_t j = __ldg(&perm[i]);
     if (j >= n)
@@ -212,96 +213,97 @@ struct inst_shade
     int32_t num_instances;
 };
 
-__global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffers fb, int q, shade_params sp,
-                                                   inst_shade is, uint32_t* __restrict__ status)
+// The queue's length is on the device; a fixed grid walks it (blocks of later, shorter
+// queues are not launched for nothing).
+__global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffers fb, int q, uint32_t first_sample,
+                                                                    shade_params sp0, inst_shade is,
+                                                                    uint32_t* __restrict__ status)
 {
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    uint32_t n = fb.counts[q];
-    bool live = i < n;
-
-    vertex_out out;
-    out.cont = false;
-    out.shadow = false;
-    uint32_t p = 0;
-    float tmin = 0.0f, tmax = 0.0f;
-    if (live)
+    const uint32_t n = fb.counts[2 * sp0.bounce];
+    for (uint32_t base = blockIdx.x * kBlock; base < n; base += gridDim.x * kBlock)
     {
-        p = fb.path[q][i];
-        const float4* rp = reinterpret_cast<const float4*>(&fb.rays[q][i]);
-        float4 r0 = rp[0], r1 = rp[1];
-        tmin = r1.z;
-        tmax = r1.w;
-        uint4 hh = fb.hits[i];
-        if (is.views && int(hh.x) >= 0)
+        const uint32_t i = base + threadIdx.x;
+        const bool live = i < n;
+        shade_params sp = sp0;
+        vertex_out out;
+        out.cont = false;
+        out.shadow = false;
+        uint32_t p = 0;
+        float tmin = 0.0f, tmax = 0.0f;
+        if (live)
         {
-            // the hit instance's triangle, carried to world space by shade_vertex
-            const int inst = int(hh.z);
-            if (inst >= 0 && inst < is.num_instances)
+            p = fb.path[q][i];
+            const float4* rp = reinterpret_cast<const float4*>(&fb.rays[q][i]);
+            float4 r0 = rp[0], r1 = rp[1];
+            tmin = r1.z;
+            tmax = r1.w;
+            uint4 hh = fb.hits[i];
+            if (is.views && int(hh.x) >= 0)
             {
-                const bvh_view bv = is.views[inst];
-                sp.tris = bv.tris;
-                sp.num_tris = bv.num_tris;
-                sp.xform = is.forward + 3 * inst;
-                sp.geom_base = is.geom_base[inst];
+                // the hit instance's triangle, carried to world space by shade_vertex
+                const int inst = int(hh.z);
+                if (inst >= 0 && inst < is.num_instances)
+                {
+                    const bvh_view bv = is.views[inst];
+                    sp.tris = bv.tris;
+                    sp.num_tris = bv.num_tris;
+                    sp.xform = is.forward + 3 * inst;
+                    sp.geom_base = is.geom_base[inst];
+                }
+                else
+                {
+                    atomicOr(status, kStatusBadIndex);
+                    hh.x = 0xFFFFFFFFu;
+                }
             }
-            else
-            {
-                atomicOr(status, kStatusBadIndex);
-                hh.x = 0xFFFFFFFFu;
-            }
+            uint2 rf = fb.rng_flags[p];
+            path_state st{ xyz(fb.throughput[p]), xyz(fb.radiance[p]), rf.x, rf.y };
+            sp.sample = first_sample + p % fb.samples;
+            shade_vertex(sp, p / fb.samples, sp.bounce, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w,
+                         int(hh.x), __uint_as_float(hh.y), st, out, status);
+            fb.throughput[p] = make_float4(st.thr.x, st.thr.y, st.thr.z, 0.0f);
+            fb.radiance[p] = make_float4(st.rad.x, st.rad.y, st.rad.z, 0.0f);
+            fb.rng_flags[p] = make_uint2(st.k, st.flags);
         }
-        uint2 rf = fb.rng_flags[p];
-        path_state st{ xyz(fb.throughput[p]), xyz(fb.radiance[p]), rf.x, rf.y };
-        shade_vertex(sp, p, sp.bounce, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w, int(hh.x),
-                     __uint_as_float(hh.y), st, out, status);
-        fb.throughput[p] = make_float4(st.thr.x, st.thr.y, st.thr.z, 0.0f);
-        fb.radiance[p] = make_float4(st.rad.x, st.rad.y, st.rad.z, 0.0f);
-        fb.rng_flags[p] = make_uint2(st.k, st.flags);
-    }
 
-    uint32_t slot = warp_append(out.cont, &fb.counts[q ^ 1]);
-    if (out.cont)
-    {
-        store_ray(&fb.rays[q ^ 1][slot], out.next_o, out.next_d, tmin, tmax);
-        fb.path[q ^ 1][slot] = p;
-    }
-    uint32_t sslot = warp_append(out.shadow, &fb.counts[2]);
-    if (out.shadow)
-    {
-        store_ray(&fb.shadow_rays[sslot], out.sh_o, out.sh_d, sp.epsilon, out.sh_tmax);
-        fb.shadow_path[sslot] = p;
-        fb.shadow_contrib[sslot] = make_float4(out.contrib.x, out.contrib.y, out.contrib.z, 0.0f);
+        uint32_t slot = warp_append(out.cont, &fb.counts[2 * sp.bounce + 2]);
+        if (out.cont)
+        {
+            store_ray(&fb.rays[q ^ 1][slot], out.next_o, out.next_d, tmin, tmax);
+            fb.path[q ^ 1][slot] = p;
+        }
+        uint32_t sslot = warp_append(out.shadow, &fb.counts[2 * sp.bounce + 1]);
+        if (out.shadow)
+        {
+            store_ray(&fb.shadow_rays[sslot], out.sh_o, out.sh_d, sp.epsilon, out.sh_tmax);
+            fb.shadow_path[sslot] = p;
+            fb.shadow_contrib[sslot] = make_float4(out.contrib.x, out.contrib.y, out.contrib.z, 0.0f);
+        }
     }
 }
 
 template <bool Wide>
-__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow(frame_buffers fb, bvh_view v,
+__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow(frame_buffers fb, uint32_t bounce, bvh_view v,
                                                                   uint32_t* __restrict__ status)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    uint32_t n = fb.counts[2];
+    uint32_t n = fb.counts[2 * bounce + 1];
     if (i >= n) return;
     const float4* rp = reinterpret_cast<const float4*>(&fb.shadow_rays[i]);
     float4 r0 = rp[0], r1 = rp[1];
     trace_result h = traverse_view_shared<true, Wide, kBlock, kPtSharedStack>(v, { r0.x, r0.y, r0.z },
                                                                              { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    if (h.tri < 0)
-    {
-        uint32_t p = fb.shadow_path[i];
-        float4 c = fb.shadow_contrib[i];
-        float4 r = fb.radiance[p];
-        fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
-    }
+    if (h.tri < 0) add_shadow(fb, i);
 }
 
 // pt_shadow over the shadow queue in the order perm.
 template <bool Wide>
-__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow_sorted(frame_buffers fb,
+__global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow_sorted(frame_buffers fb, uint32_t bounce,
                                                                          const uint32_t* __restrict__ perm,
                                                                          bvh_view v, uint32_t* __restrict__ status)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    uint32_t n = fb.counts[2];
+    uint32_t n = fb.counts[2 * bounce + 1];
     if (i >= n) return;
     uint32_t j = __ldg(&perm[i]);
     if (j >= n)
@@ -313,13 +315,7 @@ __global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow_sorted(frame_b
     float4 r0 = rp[0], r1 = rp[1];
     trace_result h = traverse_view_shared<true, Wide, kBlock, kPtSharedStack>(v, { r0.x, r0.y, r0.z },
                                                                              { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    if (h.tri < 0)
-    {
-        uint32_t p = fb.shadow_path[j];
-        float4 c = fb.shadow_contrib[j];
-        float4 r = fb.radiance[p];
-        fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
-    }
+    if (h.tri < 0) add_shadow(fb, j);
 }
 
 // Bottom-level stack entries of the two-level queries held in shared memory (0: the
@@ -344,71 +340,56 @@ __device__ __forceinline__ tlas_result trace_tlas(tlas_view const& tv, f3 o, f3 
         return traverse_tlas<AnyHit>(tv, o, d, tmin, tmax, status);
 }
 
-// pt_extend and pt_shadow over a two-level tree: hits carry the instance in z.
-__global__ void __launch_bounds__(kBlock, kPtTlasMinBlocks) pt_extend_tlas(frame_buffers fb, int q, tlas_view tv,
-                                                                       uint32_t* __restrict__ status)
+// The traversal of one bounce over a two-level tree: the closest hits of its ray queue
+// (grid row 0 when extend is set; hits carry the instance in z) and the shadow rays of the
+// bounce before (the other row).
+__global__ void __launch_bounds__(kBlock, kPtTlasMinBlocks) pt_trace_tlas(frame_buffers fb, int q, uint32_t bounce,
+                                                                          uint32_t extend, tlas_view tv,
+                                                                          uint32_t* __restrict__ status)
 {
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i == 0)
-    {
-        fb.counts[q ^ 1] = 0;   // the shade kernel that follows appends to these
-        fb.counts[2] = 0;
-    }
-    uint32_t n = fb.counts[q];
+    const bool closest = extend != 0 && blockIdx.y == 0;
+    const uint32_t n = closest ? fb.counts[2 * bounce] : fb.counts[2 * bounce - 1];
+    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
-    const float4* rp = reinterpret_cast<const float4*>(&fb.rays[q][i]);
-    float4 r0 = rp[0], r1 = rp[1];
-    tlas_result h = trace_tlas<false>(tv, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    fb.hits[i] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), uint32_t(h.inst), 0u);
-}
-
-__global__ void __launch_bounds__(kBlock, kPtTlasMinBlocks) pt_shadow_tlas(frame_buffers fb, tlas_view tv,
-                                                                       uint32_t* __restrict__ status)
-{
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    uint32_t n = fb.counts[2];
-    if (i >= n) return;
-    const float4* rp = reinterpret_cast<const float4*>(&fb.shadow_rays[i]);
-    float4 r0 = rp[0], r1 = rp[1];
-    tlas_result h = trace_tlas<true>(tv, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    if (h.tri < 0)
+    const float4* rp = reinterpret_cast<const float4*>(closest ? &fb.rays[q][i] : &fb.shadow_rays[i]);
+    const float4 r0 = rp[0], r1 = rp[1];
+    const f3 o = { r0.x, r0.y, r0.z }, d = { r0.w, r1.x, r1.y };
+    if (closest)
     {
-        uint32_t p = fb.shadow_path[i];
-        float4 c = fb.shadow_contrib[i];
-        float4 r = fb.radiance[p];
-        fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
-    }
-}
-
-// rr.color += result.color over the samples (sched_common.h:452-470): the path's
-// radiance with alpha 1 if the camera ray hit, else the background.
-__global__ void __launch_bounds__(kBlock) pt_accumulate(frame_buffers fb, uint32_t n, uint32_t sample, float4 bg)
-{
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= n) return;
-    float4 c = (fb.rng_flags[i].y & kFirstHit) ? make_float4(fb.radiance[i].x, fb.radiance[i].y, fb.radiance[i].z, 1.0f)
-                                               : bg;
-    if (sample == 0)
-    {
-        float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        fb.sum[i] = make_float4(z.x + c.x, z.y + c.y, z.z + c.z, z.w + c.w);
+        const tlas_result h = trace_tlas<false>(tv, o, d, r1.z, r1.w, status);
+        fb.hits[i] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), uint32_t(h.inst), 0u);
     }
     else
     {
-        float4 s = fb.sum[i];
-        fb.sum[i] = make_float4(s.x + c.x, s.y + c.y, s.z + c.z, s.w + c.w);
+        const tlas_result h = trace_tlas<true>(tv, o, d, r1.z, r1.w, status);
+        if (h.tri < 0) add_shadow(fb, i);
     }
 }
 
-// rr.color /= spp; accum = src * sfactor + dst * dfactor; color = accum
-// (sched_common.h:472-511, pixel_access.h:1040-1043).
-__global__ void __launch_bounds__(kBlock) pt_blend(frame_buffers fb, uint32_t n, float spp, float sfactor,
-                                                   float dfactor, float4* __restrict__ accum,
-                                                   float4* __restrict__ color)
+// rr.color += result.color over the samples, in sample order (sched_common.h:452-470):
+// each path's radiance with alpha 1 if the camera ray hit, else the background.  The last
+// pass then takes rr.color /= spp; accum = src * sfactor + dst * dfactor; color = accum
+// (sched_common.h:472-511, pixel_access.h:1040-1043); the others keep the sum.
+__global__ void __launch_bounds__(kBlock) pt_accumulate(frame_buffers fb, uint32_t n, uint32_t first_sample,
+                                                        uint32_t last, float4 bg, float spp, float sfactor,
+                                                        float dfactor, float4* __restrict__ accum,
+                                                        float4* __restrict__ color)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
-    float4 s = fb.sum[i];
+    float4 s = first_sample == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : fb.sum[i];
+    for (uint32_t k = 0; k < fb.samples; ++k)
+    {
+        const uint64_t p = uint64_t(i) * fb.samples + k;
+        const float4 r = fb.radiance[p];
+        const float4 c = (fb.rng_flags[p].y & kFirstHit) ? make_float4(r.x, r.y, r.z, 1.0f) : bg;
+        s = make_float4(s.x + c.x, s.y + c.y, s.z + c.z, s.w + c.w);
+    }
+    if (!last)
+    {
+        fb.sum[i] = s;
+        return;
+    }
     float4 a = make_float4(s.x / spp, s.y / spp, s.z / spp, s.w / spp);
     // dfactor == 0 overwrites: the previous contents (possibly never written) are not read
     float4 d = dfactor != 0.0f ? accum[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -478,7 +459,7 @@ __global__ void __launch_bounds__(kBlock, kMegaMinBlocks) pt_megakernel(bvh_view
         float4 c = (st.flags & kFirstHit) ? make_float4(st.rad.x, st.rad.y, st.rad.z, 1.0f) : bg;
         sum = make_float4(sum.x + c.x, sum.y + c.y, sum.z + c.z, sum.w + c.w);
     }
-    // pt_blend's arithmetic
+    // pt_accumulate's arithmetic
     const float n = float(spp);
     float4 a = make_float4(sum.x / n, sum.y / n, sum.z / n, sum.w / n);
     float4 dst = dfactor != 0.0f ? accum[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -703,12 +684,31 @@ __global__ void __launch_bounds__(kBlock, kAdjointMinBlocks) pt_adjoint(bvh_view
 
 inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
-gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t n, frame_buffers& fb)
+// Paths of a pass: 2^22 (0.8 GB of path state).  One sample per pixel and pass left a
+// small frame's launches short of the GPU and every bounce's tail idle.  Measured against
+// that: 641x479x4 over instances 8.30 -> 4.70 ms (its extend and shadow in one launch too),
+// 512x512x16 forward frame 30.1 -> 19.7 ms, 1920x1080x8 box 76.0 -> 63.5 ms.
+constexpr uint64_t kPassPaths = 1ull << 22;
+
+// Samples per pixel and pass of a frame of npix pixels: as many as kPassPaths allow, evenly
+// over the passes.
+uint32_t pass_samples(uint32_t npix, uint32_t spp)
 {
+    const uint64_t most = std::max<uint64_t>(1, std::min<uint64_t>(spp, kPassPaths / npix));
+    const uint64_t passes = (spp + most - 1) / most;
+    return uint32_t((spp + passes - 1) / passes);
+}
+
+// The buffers of a pass of n paths over npix pixels with num_counts queue lengths; sort: with
+// the queue order's keys.
+gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint32_t num_counts, bool sort,
+                              frame_buffers& fb)
+{
+    const size_t key = sort ? size_t(n) * 4 : 0;
     size_t sizes[] = { size_t(n) * 32, size_t(n) * 32, size_t(n) * 4, size_t(n) * 4, size_t(n) * 16,
                        size_t(n) * 32, size_t(n) * 4,  size_t(n) * 16, size_t(n) * 16, size_t(n) * 16,
-                       size_t(n) * 8,  size_t(n) * 16, 64, size_t(n) * 4, size_t(n) * 4, size_t(n) * 4,
-                       size_t(n) * 4, radix_sort_scratch_bytes(n) };
+                       size_t(n) * 8,  size_t(npix) * 16, size_t(num_counts) * 4, key, key, key,
+                       key, sort ? radix_sort_scratch_bytes(n) : 0 };
     constexpr int kParts = int(sizeof(sizes) / sizeof(sizes[0]));
     size_t total = 0;
     for (size_t s : sizes) total += align256(s);
@@ -1120,14 +1120,60 @@ shade_params shade_params_for(gbrt_context const* ctx, gbrt_pt_scene const* scen
     return sp;
 }
 
-// The frame's average blended into accum and written to color (cuda_sched's blend).
-gbrt_status finish_frame(gbrt_context* ctx, frame_buffers const& fb, gbrt_pt_params const& p, uint32_t blocks,
-                         float* d_accum, float* d_color)
+// The launch that ends a pass of pass_samples(...) samples from first_sample on.
+gbrt_status end_pass(gbrt_context* ctx, frame_buffers const& fb, gbrt_pt_params const& p, uint32_t first_sample, float4 bg,
+                     float* d_accum, float* d_color)
 {
     const uint32_t n = p.width * p.height;
-    pt_blend<<<blocks, kBlock, 0, ctx->stream>>>(fb, n, float(p.spp), p.sfactor, p.dfactor,
-                                                 reinterpret_cast<float4*>(d_accum), reinterpret_cast<float4*>(d_color));
-    GBRT_LAUNCH_CHECK(ctx, "pt_blend");
+    const uint32_t last = first_sample + fb.samples >= p.spp ? 1u : 0u;
+    pt_accumulate<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
+        fb, n, first_sample, last, bg, float(p.spp), p.sfactor, p.dfactor, reinterpret_cast<float4*>(d_accum),
+        reinterpret_cast<float4*>(d_color));
+    GBRT_LAUNCH_CHECK(ctx, "pt_accumulate");
+    return GBRT_OK;
+}
+
+// A wavefront frame whose traversal launches are trace(fb, q, bounce, extend, shadow):
+// the closest hits of bounce's ray queue q if extend, the shadow rays of the bounce before
+// if shadow.
+template <class Trace>
+gbrt_status render_passes(gbrt_context* ctx, camera_basis const& cam, gbrt_pt_params const& p, shade_params sp,
+                          inst_shade const& is, uint32_t num_lights, bool empty, bool sort, float4 bg, float* d_accum,
+                          float* d_color, Trace trace)
+{
+    const uint32_t npix = p.width * p.height;
+    const uint32_t samples = pass_samples(npix, p.spp);
+    const uint32_t n = npix * samples;
+    const uint32_t num_counts = 2 * (p.num_bounces + 1);
+    cudaStream_t s = ctx->stream;
+    frame_buffers fb;
+    gbrt_status st = frame_buffers_for(ctx, npix, n, num_counts, sort, fb);
+    if (st != GBRT_OK) return st;
+    const uint32_t blocks = (n + kBlock - 1) / kBlock;
+    const uint32_t shade_blocks = std::min(blocks, uint32_t(ctx->num_sms) * kShadeMinBlocks * 4);
+    for (uint32_t smp = 0; smp < p.spp; smp += fb.samples)
+    {
+        fb.samples = std::min(samples, p.spp - smp);
+        pt_raygen<<<blocks, kBlock, 0, s>>>(fb, p.width, p.height, p.frame_id, smp, num_counts, cam);
+        GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
+        int q = 0;
+        for (uint32_t b = 0; b < p.num_bounces && !empty; ++b)
+        {
+            sp.bounce = b;
+            st = trace(fb, q, b, true, b > 0 && num_lights > 0);
+            if (st != GBRT_OK) return st;
+            pt_shade<<<shade_blocks, kBlock, 0, s>>>(fb, q, smp, sp, is, ctx->d_status);
+            GBRT_LAUNCH_CHECK(ctx, "pt_shade");
+            q ^= 1;
+        }
+        if (p.num_bounces > 0 && !empty && num_lights > 0)
+        {
+            st = trace(fb, q, p.num_bounces, false, true);
+            if (st != GBRT_OK) return st;
+        }
+        st = end_pass(ctx, fb, p, smp, bg, d_accum, d_color);
+        if (st != GBRT_OK) return st;
+    }
     return GBRT_OK;
 }
 
@@ -1135,44 +1181,23 @@ gbrt_status finish_frame(gbrt_context* ctx, frame_buffers const& fb, gbrt_pt_par
 // top-level tree and the instances' trees (traverse_tlas), each hit shaded with its
 // instance's triangle carried to world space and its instance's material slots.
 gbrt_status render_frame_instanced(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam,
-                                   gbrt_pt_params const& p, shade_params sp, float4 bg, uint32_t blocks,
-                                   float* d_accum, float* d_color)
+                                   gbrt_pt_params const& p, shade_params sp, float4 bg, float* d_accum, float* d_color)
 {
     if (p.flags & (GBRT_PT_MEGAKERNEL | GBRT_PT_SORT_QUEUES))
         return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace: the megakernel and sorted queues take a single tree");
-    const uint32_t n = p.width * p.height;
-    cudaStream_t s = ctx->stream;
     gbrt_tlas const* t = scene->tlas;
     const tlas_view tv{ t->nodes, t->records, t->views, t->num_instances > 0 ? t->root : kEmptyLink,
                         int32_t(t->num_inner), int32_t(t->num_instances) };
     const inst_shade is{ t->views, t->forward, scene->inst_geom, int32_t(t->num_instances) };
-    frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, n, fb);
-    if (st != GBRT_OK) return st;
-    for (uint32_t smp = 0; smp < p.spp; ++smp)
-    {
-        sp.sample = smp;
-        pt_raygen<<<blocks, kBlock, 0, s>>>(fb, p.width, p.height, p.frame_id, smp, cam);
-        GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
-        int q = 0;
-        for (uint32_t b = 0; b < p.num_bounces && t->num_instances > 0; ++b)
-        {
-            sp.bounce = b;
-            pt_extend_tlas<<<blocks, kBlock, 0, s>>>(fb, q, tv, ctx->d_status);
-            GBRT_LAUNCH_CHECK(ctx, "pt_extend_tlas");
-            pt_shade<<<blocks, kBlock, 0, s>>>(fb, q, sp, is, ctx->d_status);
-            GBRT_LAUNCH_CHECK(ctx, "pt_shade");
-            if (scene->num_lights > 0)
-            {
-                pt_shadow_tlas<<<blocks, kBlock, 0, s>>>(fb, tv, ctx->d_status);
-                GBRT_LAUNCH_CHECK(ctx, "pt_shadow_tlas");
-            }
-            q ^= 1;
-        }
-        pt_accumulate<<<blocks, kBlock, 0, s>>>(fb, n, smp, bg);
-        GBRT_LAUNCH_CHECK(ctx, "pt_accumulate");
-    }
-    return finish_frame(ctx, fb, p, blocks, d_accum, d_color);
+    auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
+        const uint32_t blocks = (p.width * p.height * fb.samples + kBlock - 1) / kBlock;
+        pt_trace_tlas<<<dim3(blocks, extend && shadow ? 2 : 1), kBlock, 0, ctx->stream>>>(fb, q, b, extend ? 1u : 0u,
+                                                                                          tv, ctx->d_status);
+        GBRT_LAUNCH_CHECK(ctx, "pt_trace_tlas");
+        return GBRT_OK;
+    };
+    return render_passes(ctx, cam, p, sp, is, scene->num_lights, t->num_instances == 0, false, bg, d_accum, d_color,
+                         trace);
 }
 
 // One frame of the wavefront path tracer into accum (blended) and color.
@@ -1195,7 +1220,7 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
     const uint32_t blocks = (n + kBlock - 1) / kBlock;
     cudaStream_t s = ctx->stream;
     if (scene->tlas)
-        return render_frame_instanced(ctx, scene, cam, p, sp, bg, blocks, d_accum, d_color);
+        return render_frame_instanced(ctx, scene, cam, p, sp, bg, d_accum, d_color);
     const bvh_view v = view_of(bvh);
     const bool wide = bvh->nodes4 != nullptr && (ctx->trace_flags & GBRT_TRACE_WIDE_NODES);
     if (p.flags & GBRT_PT_MEGAKERNEL)
@@ -1209,9 +1234,7 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
         GBRT_LAUNCH_CHECK(ctx, "pt_megakernel");
         return GBRT_OK;
     }
-    frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, n, fb);
-    if (st != GBRT_OK) return st;
+    const inst_shade no_instances{ nullptr, nullptr, nullptr, 0 };
     // GBRT_PT_SORT_QUEUES: each bounce's ray and shadow queues ordered by origin cell of
     // the scene box before they are traced (as the ray queries order their rays).
     // Measured slower on the box scene (1920x1080x64: 847 vs 703 ms per frame; a sort of
@@ -1222,73 +1245,51 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
     float ext[3] = { bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2] };
     const float3 scale = make_float3(ext[0] > 0.0f ? 256.0f / ext[0] : 0.0f, ext[1] > 0.0f ? 256.0f / ext[1] : 0.0f,
                                      ext[2] > 0.0f ? 256.0f / ext[2] : 0.0f);
-    for (uint32_t smp = 0; smp < p.spp; ++smp)
-    {
-        sp.sample = smp;
-        pt_raygen<<<blocks, kBlock, 0, s>>>(fb, p.width, p.height, p.frame_id, smp, cam);
-        GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
-        int q = 0;
-        if (bvh->num_prims > 0)
+    auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
+        const uint32_t paths = n * fb.samples;
+        const uint32_t blocks = (paths + kBlock - 1) / kBlock;
+        auto order = [&](const gbrt_ray* rays, const uint32_t* count) -> gbrt_status {
+            pt_queue_keys<<<blocks, kBlock, 0, s>>>(rays, count, paths, lo, scale, fb.keys, fb.vals);
+            GBRT_LAUNCH_CHECK(ctx, "pt_queue_keys");
+            return radix_sort_pairs(ctx, fb.keys, fb.vals, fb.keys_alt, fb.vals_alt, paths, 24, fb.sort_scratch, s);
+        };
+        if (shadow)
         {
-            for (uint32_t b = 0; b < p.num_bounces; ++b)
+            if (sort)
             {
-                sp.bounce = b;
-                // camera rays are coherent in pixel order; later queues are ordered by origin
-                if (sort && b > 0)
-                {
-                    pt_queue_keys<<<blocks, kBlock, 0, s>>>(fb.rays[q], fb.counts + q, n, lo, scale, fb.keys, fb.vals);
-                    GBRT_LAUNCH_CHECK(ctx, "pt_queue_keys");
-                    st = radix_sort_pairs(ctx, fb.keys, fb.vals, fb.keys_alt, fb.vals_alt, n, 24, fb.sort_scratch, s);
-                    if (st != GBRT_OK) return st;
-                    if (wide)
-                        pt_extend_sorted<true><<<blocks, kBlock, 0, s>>>(fb, q, fb.vals, v, ctx->d_status);
-                    else
-                        pt_extend_sorted<false><<<blocks, kBlock, 0, s>>>(fb, q, fb.vals, v, ctx->d_status);
-                }
-                else if (wide)
-                {
-                    pt_extend<true><<<blocks, kBlock, 0, s>>>(fb, q, v, ctx->d_status);
-                }
-                else
-                {
-                    pt_extend<false><<<blocks, kBlock, 0, s>>>(fb, q, v, ctx->d_status);
-                }
-                GBRT_LAUNCH_CHECK(ctx, "pt_extend");
-                pt_shade<<<blocks, kBlock, 0, s>>>(fb, q, sp, inst_shade{ nullptr, nullptr, nullptr, 0 },
-                                                   ctx->d_status);
-                GBRT_LAUNCH_CHECK(ctx, "pt_shade");
-                if (scene->num_lights > 0)
-                {
-                    if (sort)
-                    {
-                        pt_queue_keys<<<blocks, kBlock, 0, s>>>(fb.shadow_rays, fb.counts + 2, n, lo, scale, fb.keys,
-                                                                fb.vals);
-                        GBRT_LAUNCH_CHECK(ctx, "pt_queue_keys");
-                        st = radix_sort_pairs(ctx, fb.keys, fb.vals, fb.keys_alt, fb.vals_alt, n, 24, fb.sort_scratch,
-                                              s);
-                        if (st != GBRT_OK) return st;
-                        if (wide)
-                            pt_shadow_sorted<true><<<blocks, kBlock, 0, s>>>(fb, fb.vals, v, ctx->d_status);
-                        else
-                            pt_shadow_sorted<false><<<blocks, kBlock, 0, s>>>(fb, fb.vals, v, ctx->d_status);
-                    }
-                    else if (wide)
-                    {
-                        pt_shadow<true><<<blocks, kBlock, 0, s>>>(fb, v, ctx->d_status);
-                    }
-                    else
-                    {
-                        pt_shadow<false><<<blocks, kBlock, 0, s>>>(fb, v, ctx->d_status);
-                    }
-                    GBRT_LAUNCH_CHECK(ctx, "pt_shadow");
-                }
-                q ^= 1;
+                gbrt_status st = order(fb.shadow_rays, fb.counts + 2 * b - 1);
+                if (st != GBRT_OK) return st;
+                wide ? pt_shadow_sorted<true><<<blocks, kBlock, 0, s>>>(fb, b - 1, fb.vals, v, ctx->d_status)
+                     : pt_shadow_sorted<false><<<blocks, kBlock, 0, s>>>(fb, b - 1, fb.vals, v, ctx->d_status);
             }
+            else
+            {
+                wide ? pt_shadow<true><<<blocks, kBlock, 0, s>>>(fb, b - 1, v, ctx->d_status)
+                     : pt_shadow<false><<<blocks, kBlock, 0, s>>>(fb, b - 1, v, ctx->d_status);
+            }
+            GBRT_LAUNCH_CHECK(ctx, "pt_shadow");
         }
-        pt_accumulate<<<blocks, kBlock, 0, s>>>(fb, n, smp, bg);
-        GBRT_LAUNCH_CHECK(ctx, "pt_accumulate");
-    }
-    return finish_frame(ctx, fb, p, blocks, d_accum, d_color);
+        if (extend)
+        {
+            // camera rays are coherent in pixel order; later queues are ordered by origin
+            if (sort && b > 0)
+            {
+                gbrt_status st = order(fb.rays[q], fb.counts + 2 * b);
+                if (st != GBRT_OK) return st;
+                wide ? pt_extend_sorted<true><<<blocks, kBlock, 0, s>>>(fb, q, b, fb.vals, v, ctx->d_status)
+                     : pt_extend_sorted<false><<<blocks, kBlock, 0, s>>>(fb, q, b, fb.vals, v, ctx->d_status);
+            }
+            else
+            {
+                wide ? pt_extend<true><<<blocks, kBlock, 0, s>>>(fb, q, b, v, ctx->d_status)
+                     : pt_extend<false><<<blocks, kBlock, 0, s>>>(fb, q, b, v, ctx->d_status);
+            }
+            GBRT_LAUNCH_CHECK(ctx, "pt_extend");
+        }
+        return GBRT_OK;
+    };
+    return render_passes(ctx, cam, p, sp, no_instances, scene->num_lights, bvh->num_prims == 0, sort, bg, d_accum,
+                         d_color, trace);
 }
 
 } // namespace
