@@ -269,7 +269,7 @@ gbrt_status upload_bvh2(gbrt_context* ctx, gbrt_bvh_node const* nodes, uint32_t 
 // chunks); build_lbvh_in_scratch re-checks it at run time.
 struct lbvh_scratch_layout
 {
-    size_t centroids, keys, vals, keys_alt, vals_alt, leaf_parent, arrivals, nodes, tris, words, sort, total;
+    size_t centroids, keys, vals, keys_alt, vals_alt, flags, waiting, slots, nodes, tris, words, sort, total;
 };
 
 constexpr size_t scratch_align(size_t v) { return (v + 255) & ~size_t(255); }
@@ -283,8 +283,9 @@ constexpr lbvh_scratch_layout lbvh_scratch_layout_for(uint32_t n)
     l.vals = o;        o = scratch_align(o + size_t(n) * 4);
     l.keys_alt = o;    o = scratch_align(o + size_t(n) * 4);
     l.vals_alt = o;    o = scratch_align(o + size_t(n) * 4);
-    l.leaf_parent = o; o = scratch_align(o + size_t(n) * 4);
-    l.arrivals = o;    o = scratch_align(o + size_t(n) * 4);
+    l.flags = o;       o = scratch_align(o + size_t(n) * 4);
+    l.waiting = o;     o = scratch_align(o + (size_t(n) / 512 + 1) * 514 * 4);   // agg_waiting_words
+    l.slots = o;       o = scratch_align(o + size_t(n) * 64);   // agg_slot (agglomerate.cuh)
     l.nodes = o;       o = scratch_align(o + size_t(n) * 64);
     l.tris = o;        o = scratch_align(o + size_t(n) * 48);
     l.words = o;       o = scratch_align(o + 8 * 4);

@@ -11,15 +11,15 @@
 //                     scene build computes
 //   two stable radix sorts: by code, then by scene, giving (scene, code, index) order,
 //                     i.e. every scene's segment sorted as its own build sorts it
-//   batch_hierarchy : Karras splits inside each segment, links in arena indices
-//   batch_refit     : the bottom-up refit of refit_and_emit over all segments
+//   agglomerate     : hierarchy, boxes and leaf triangles of every segment from below, links
+//                     in arena indices (agglomerate.cuh)
 // so each scene's tree equals gbrt_bvh_build_lbvh's for that scene: same codes, same
 // order, same topology and boxes, hence bit-identical hits.  No stage allocates or
 // synchronises: a build can be captured in a CUDA graph.
 
-#include "collapse.cuh"
-#include "lbvh_device.cuh"
 #include "traverse_core.cuh"
+#include "agglomerate.cuh"
+#include "collapse.cuh"
 
 #include <algorithm>
 #include <new>
@@ -81,10 +81,12 @@ __global__ void __launch_bounds__(kBlock) batch_centroids(gbrt_triangle const* _
 __global__ void __launch_bounds__(kBlock) batch_morton(const float4* __restrict__ centroids,
                                                        const uint32_t* __restrict__ prim_scene, uint32_t total,
                                                        const int* __restrict__ bounds, uint32_t* __restrict__ codes_in,
-                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ values)
+                                                       uint32_t* __restrict__ keys, uint32_t* __restrict__ values,
+                                                       uint32_t* __restrict__ flags)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= total) return;
+    flags[i] = 0;   // agglomerate's
     const int* cbo = bounds + 6 * prim_scene[i];
     box3 cb;
     cb.lo = { ordered_to_float(cbo[0]), ordered_to_float(cbo[1]), ordered_to_float(cbo[2]) };
@@ -127,53 +129,6 @@ __global__ void __launch_bounds__(kBlock) gather_codes(const uint32_t* __restric
     if (i < total) sorted_codes[i] = codes_in[values[i]];
 }
 
-// Inner node g of the arena: Karras split inside its scene's segment, links translated
-// to arena indices (inner: inner_offsets[s] + c, leaf: ~(offsets[s] + j)).
-__global__ void __launch_bounds__(kBlock) batch_hierarchy(const uint32_t* __restrict__ sorted_codes,
-                                                          const uint32_t* __restrict__ offsets,
-                                                          const uint32_t* __restrict__ inner_offsets,
-                                                          uint32_t num_scenes, uint32_t total_inner,
-                                                          bvh2_node* __restrict__ nodes, int* __restrict__ leaf_parent,
-                                                          int2* __restrict__ ranges)
-{
-    uint32_t g = blockIdx.x * kBlock + threadIdx.x;
-    if (g >= total_inner) return;
-    uint32_t s = upper_segment(inner_offsets, num_scenes, g);
-    int base_leaf = int(offsets[s]);
-    int base_inner = int(inner_offsets[s]);
-    int n = int(offsets[s + 1]) - base_leaf;
-    int i = int(g) - base_inner;
-    int first, last, split;
-    karras_node(sorted_codes + base_leaf, n, i, first, last, split);
-    int left = split, right = split + 1;
-    int cl, cr;
-    int gi = int(g);
-    if (left == first)
-    {
-        cl = ~(base_leaf + left);
-        leaf_parent[base_leaf + left] = (gi << 1) | 0;
-    }
-    else
-    {
-        cl = base_inner + left;
-        nodes[base_inner + left].link.w = (gi << 1) | 0;
-    }
-    if (right == last)
-    {
-        cr = ~(base_leaf + right);
-        leaf_parent[base_leaf + right] = (gi << 1) | 1;
-    }
-    else
-    {
-        cr = base_inner + right;
-        nodes[base_inner + right].link.w = (gi << 1) | 1;
-    }
-    nodes[g].link.x = cl;
-    nodes[g].link.y = cr;
-    if (i == 0) nodes[g].link.w = -1;
-    ranges[g] = make_int2(base_leaf + first, base_leaf + last);
-}
-
 // Level 0 of the arena's wide collapse: scene s with an inner root gets wide node s.
 __global__ void __launch_bounds__(kBlock) batch_collapse_seed(const int32_t* __restrict__ roots, uint32_t num_scenes,
                                                               int2* __restrict__ q, uint32_t* __restrict__ count,
@@ -183,60 +138,6 @@ __global__ void __launch_bounds__(kBlock) batch_collapse_seed(const int32_t* __r
     if (s == 0) *node_counter = num_scenes;
     if (s >= num_scenes || roots[s] < 0) return;
     q[atomicAdd(count, 1u)] = make_int2(roots[s], int(s));
-}
-
-// refit_and_emit over all segments: a leaf without a parent (a one-triangle scene) only
-// emits its triangle; every root records its height into *height (max over scenes).
-__global__ void __launch_bounds__(kBlock) batch_refit(gbrt_triangle const* __restrict__ tris_in,
-                                                      const uint32_t* __restrict__ sorted_ids, uint32_t total,
-                                                      uint32_t total_inner, const int* __restrict__ leaf_parent,
-                                                      bvh2_node* __restrict__ nodes, uint32_t* __restrict__ arrivals,
-                                                      tri48* __restrict__ tris_out, uint32_t* __restrict__ height_out,
-                                                      uint32_t* __restrict__ status)
-{
-    uint32_t j = blockIdx.x * kBlock + threadIdx.x;
-    if (j >= total) return;
-    uint32_t id = __ldg(&sorted_ids[j]);
-    if (id >= total)
-    {
-        atomicOr(status, kStatusBadIndex);
-        return;
-    }
-    tri_in t = load_tri(tris_in, id);
-    tri48 o;
-    o.t0 = make_float4(t.v1.x, t.v1.y, t.v1.z, __uint_as_float(t.prim_id));
-    o.t1 = make_float4(t.e1.x, t.e1.y, t.e1.z, __uint_as_float(t.geom_id));
-    o.t2 = make_float4(t.e2.x, t.e2.y, t.e2.z, __uint_as_float(kLastInLeaf));
-    tris_out[j] = o;
-    int link = leaf_parent[j];
-    if (link == -1) return;   // one-triangle scene: the leaf is the root
-    box3 b = tri_box(t);
-    int height = 0;
-    for (uint32_t step = 0; step < total; ++step)
-    {
-        if (link < 0 || uint32_t(link >> 1) >= total_inner)
-        {
-            atomicOr(status, kStatusBadIndex);
-            return;
-        }
-        int node = link >> 1, side = link & 1;
-        bvh2_node* nd = &nodes[node];
-        store_child_box(nd, side, b);
-        atomicMax(&nd->link.z, height + 1);
-        __threadfence();
-        if (atomicAdd(&arrivals[node], 1u) == 0) return;
-        __threadfence();
-        b = load_union_cg(nd);
-        height = __ldcg(&nd->link.z);
-        int up = __ldcg(&nd->link.w);
-        if (up < 0)
-        {
-            atomicMax(height_out, uint32_t(height));
-            return;
-        }
-        link = up;
-    }
-    atomicOr(status, kStatusBadIndex);
 }
 
 // closest_hit of every scene's rays: ray r belongs to the scene whose ray range holds it.
@@ -312,7 +213,7 @@ inline size_t align_up(size_t v) { return (v + 255) & ~size_t(255); }
 
 struct batch_scratch
 {
-    size_t centroids, prim_scene, bounds, codes_in, keys_alt, vals_alt, scene_keys, leaf_parent, arrivals, sort, total;
+    size_t centroids, prim_scene, bounds, codes_in, keys_alt, vals_alt, scene_keys, flags, waiting, slots, sort, total;
 };
 
 batch_scratch scratch_layout(uint32_t total, uint32_t num_scenes)
@@ -326,8 +227,9 @@ batch_scratch scratch_layout(uint32_t total, uint32_t num_scenes)
     l.keys_alt = o;    o = align_up(o + size_t(total) * 4);
     l.vals_alt = o;    o = align_up(o + size_t(total) * 4);
     l.scene_keys = o;  o = align_up(o + size_t(total) * 4);
-    l.leaf_parent = o; o = align_up(o + size_t(total) * 4);
-    l.arrivals = o;    o = align_up(o + size_t(total) * 4);
+    l.flags = o;       o = align_up(o + size_t(total) * 4);
+    l.waiting = o;     o = align_up(o + agg_waiting_words(total) * 4);
+    l.slots = o;       o = align_up(o + size_t(total) * sizeof(agg_slot));
     l.sort = o;        o = align_up(o + radix_sort_scratch_bytes(total));
     l.total = o;
     return l;
@@ -375,8 +277,9 @@ gbrt_status batch_build(gbrt_context* ctx, gbrt_batch* b, gbrt_triangle const* d
     uint32_t* keys_alt = reinterpret_cast<uint32_t*>(base + l.keys_alt);
     uint32_t* vals_alt = reinterpret_cast<uint32_t*>(base + l.vals_alt);
     uint32_t* scene_keys = reinterpret_cast<uint32_t*>(base + l.scene_keys);
-    int* leaf_parent = reinterpret_cast<int*>(base + l.leaf_parent);
-    uint32_t* arrivals = reinterpret_cast<uint32_t*>(base + l.arrivals);
+    uint32_t* flags = reinterpret_cast<uint32_t*>(base + l.flags);
+    uint32_t* waiting = reinterpret_cast<uint32_t*>(base + l.waiting);
+    agg_slot* slots = reinterpret_cast<agg_slot*>(base + l.slots);
     const uint32_t n = b->total;
 
     batch_init_bounds<<<blocks_for(uint64_t(b->num_scenes) * 6), kBlock, 0, s>>>(bounds, b->num_scenes);
@@ -385,7 +288,7 @@ gbrt_status batch_build(gbrt_context* ctx, gbrt_batch* b, gbrt_triangle const* d
                                                       bounds);
     GBRT_LAUNCH_CHECK(ctx, "batch_centroids");
     batch_morton<<<blocks_for(n), kBlock, 0, s>>>(centroids, prim_scene, n, bounds, codes_in, b->sorted_codes,
-                                                   b->sorted_ids);
+                                                   b->sorted_ids, flags);
     GBRT_LAUNCH_CHECK(ctx, "batch_morton");
     gbrt_status st = radix_sort_pairs(ctx, b->sorted_codes, b->sorted_ids, keys_alt, vals_alt, n, 30, base + l.sort, s);
     if (st != GBRT_OK) return st;
@@ -400,20 +303,12 @@ gbrt_status batch_build(gbrt_context* ctx, gbrt_batch* b, gbrt_triangle const* d
         gather_codes<<<blocks_for(n), kBlock, 0, s>>>(b->sorted_ids, codes_in, n, b->sorted_codes);
         GBRT_LAUNCH_CHECK(ctx, "gather_codes");
     }
-    GBRT_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, size_t(n) * 4, s));
-    GBRT_CUDA(ctx, cudaMemsetAsync(arrivals, 0, size_t(n) * 4, s));
     GBRT_CUDA(ctx, cudaMemsetAsync(b->d_height, 0, 4, s));
-    if (b->total_inner > 0)
-    {
-        GBRT_CUDA(ctx, cudaMemsetAsync(b->nodes, 0, size_t(b->total_inner) * sizeof(bvh2_node), s));
-        batch_hierarchy<<<blocks_for(b->total_inner), kBlock, 0, s>>>(b->sorted_codes, b->d_offsets, b->d_inner_offsets,
-                                                                      b->num_scenes, b->total_inner, b->nodes,
-                                                                      leaf_parent, b->ranges);
-        GBRT_LAUNCH_CHECK(ctx, "batch_hierarchy");
-    }
-    batch_refit<<<blocks_for(n), kBlock, 0, s>>>(d_tris, b->sorted_ids, n, b->total_inner, leaf_parent, b->nodes,
-                                                 arrivals, b->tris, b->d_height, ctx->d_status);
-    GBRT_LAUNCH_CHECK(ctx, "batch_refit");
+    const agg_args args{ d_tris, b->sorted_ids, b->sorted_codes, n, b->d_offsets, b->d_inner_offsets, b->num_scenes,
+                         b->nodes, b->ranges, slots, flags, waiting, waiting + agg_blocks(n) * (kAggBlock + 1), b->tris,
+                         b->d_height, ctx->d_status };
+    st = agglomerate<true>(ctx, args, s);
+    if (st != GBRT_OK) return st;
     ++b->build_gen;
     return GBRT_OK;
 }

@@ -9,8 +9,9 @@
 //     z01  = (c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z)
 //     link = (child0, child1, height, parent)
 // child >= 0 is an inner node index; child < 0 is a leaf whose first triangle is
-// ~child.  height is the subtree height (leaves 0); parent is the parent inner
-// node (-1 for the root) -- both are build-time fields, unused by traversal.
+// ~child.  height is the subtree height (leaves 0); parent is (parent inner node << 1) |
+// side in a PLOC tree (-1 for the root; its refit climbs them), -1 in the others -- both
+// are unused by traversal.
 //
 // Triangles: 48 bytes, three float4, stored in leaf order so that a leaf is a
 // contiguous run; the last triangle of a leaf carries kLastInLeaf.

@@ -9,18 +9,15 @@
 //                         address).
 //   2. morton_codes     : centroid quantised op-for-op as lbvh.h:253-267.
 //   3. radix sort       : stable, by the 30-bit code (radix_sort.cu).
-//   4. build_hierarchy  : Karras split per inner node (lbvh.h:120-185, 281-330).
-//   5. refit_and_emit   : one thread per leaf writes the triangle in leaf order and its
-//                         box into the parent's child slot, then climbs; at each node
-//                         the SECOND arriving thread continues (an atomic counter per
-//                         node) so every node is combined once -- the reference walks
-//                         every leaf to the root with 6 CAS loops per level
-//                         (lbvh.h:332-372).
+//   4. agglomerate      : Karras' tree (lbvh.h:120-185, 281-330) from below, with the
+//                         boxes and the leaf triangles, in one kernel (agglomerate.cuh);
+//                         the reference walks every leaf to the root with 6 CAS loops per
+//                         level (lbvh.h:332-372).
 // Topology and boxes equal the reference's for identical Morton codes; the node-pair
 // layout is gbrt::bvh2_node (bvh_layout.cuh).
 
+#include "agglomerate.cuh"
 #include "collapse.cuh"
-#include "lbvh_device.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -82,10 +79,12 @@ __global__ void __launch_bounds__(kBlock) centroid_bounds(gbrt_triangle const* _
 __global__ void __launch_bounds__(kBlock) morton_codes(const float4* __restrict__ centroids, uint32_t n,
                                                        const int* __restrict__ cb_ordered,
                                                        uint32_t* __restrict__ keys,
-                                                       uint32_t* __restrict__ values)
+                                                       uint32_t* __restrict__ values,
+                                                       uint32_t* __restrict__ flags)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
+    if (flags) flags[i] = 0;   // agglomerate's, cleared here instead of by a memset
     box3 cb;
     cb.lo = { ordered_to_float(cb_ordered[0]), ordered_to_float(cb_ordered[1]), ordered_to_float(cb_ordered[2]) };
     cb.hi = { ordered_to_float(cb_ordered[3]), ordered_to_float(cb_ordered[4]), ordered_to_float(cb_ordered[5]) };
@@ -111,47 +110,9 @@ __global__ void __launch_bounds__(kBlock) morton_codes(const float4* __restrict_
     values[i] = i;
 }
 
-// Inner node i of n-1: children into nodes[i].link.{x,y} (inner index, or ~leaf for a
-// leaf), parent links for inner children in nodes[c].link.w = (i << 1) | side, for
-// leaves in leaf_parent[j].
-__global__ void __launch_bounds__(kBlock) build_hierarchy(const uint32_t* __restrict__ codes, int n,
-                                                          bvh2_node* __restrict__ nodes,
-                                                          int* __restrict__ leaf_parent,
-                                                          int2* __restrict__ ranges)
-{
-    int i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= n - 1) return;
-    int first, last, split;
-    karras_node(codes, n, i, first, last, split);
-    if (ranges) ranges[i] = make_int2(first, last);   // the sorted primitives under node i
-
-    int left = split, right = split + 1;
-    int cl, cr;
-    if (left == first)
-    {
-        cl = ~left;
-        leaf_parent[left] = (i << 1) | 0;
-    }
-    else
-    {
-        cl = left;
-        nodes[left].link.w = (i << 1) | 0;
-    }
-    if (right == last)
-    {
-        cr = ~right;
-        leaf_parent[right] = (i << 1) | 1;
-    }
-    else
-    {
-        cr = right;
-        nodes[right].link.w = (i << 1) | 1;
-    }
-    nodes[i].link.x = cl;
-    nodes[i].link.y = cr;
-    if (i == 0) nodes[0].link.w = -1;
-}
-
+// The refit of a PLOC tree, whose topology is in its links: one thread per leaf writes the
+// triangle in leaf order and its box into the parent's child slot, then climbs; at each
+// node the second arriving thread continues (an atomic counter per node).
 __global__ void __launch_bounds__(kBlock) refit_and_emit(gbrt_triangle const* __restrict__ tris_in,
                                                          const uint32_t* __restrict__ sorted_ids, int n,
                                                          const int* __restrict__ leaf_parent,
@@ -279,43 +240,35 @@ __global__ void collapse_root(int2* __restrict__ q, uint32_t* __restrict__ count
 
 // lbvh::collapse (lbvh.h:374-451): nodes of the cuda_index_bvh layout -- root at 0, the
 // children of inner node i at 1+2i and 2+2i, one primitive per leaf with first_prim =
-// the original index.
+// the original index -- and the index list 0, 1, 2, ... (lbvh.h:453).  A node's two
+// 32-byte children are adjacent and 16-byte aligned: four 128-bit stores per thread.
+// Scalar stores of the same bytes took 688 us for 8.4 M triangles, bound by the store
+// instructions.
 __global__ void __launch_bounds__(kBlock) export_collapse(const bvh2_node* __restrict__ nodes, int num_inner,
                                                           const uint32_t* __restrict__ sorted_ids,
-                                                          gbrt_bvh_node* __restrict__ out)
+                                                          gbrt_bvh_node* __restrict__ out,
+                                                          uint32_t* __restrict__ indices)
 {
     int i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= num_inner) return;
-    bvh2_node nd = nodes[i];
-    box3 cbox[2];
-    cbox[0].lo = { nd.xy0.x, nd.xy0.z, nd.z01.x };
-    cbox[0].hi = { nd.xy0.y, nd.xy0.w, nd.z01.y };
-    cbox[1].lo = { nd.xy1.x, nd.xy1.z, nd.z01.z };
-    cbox[1].hi = { nd.xy1.y, nd.xy1.w, nd.z01.w };
-    int child[2] = { nd.link.x, nd.link.y };
-    auto put = [&](gbrt_bvh_node& d, box3 const& b, uint32_t first, uint16_t count) {
-        d.bbox_min[0] = b.lo.x;
-        d.bbox_min[1] = b.lo.y;
-        d.bbox_min[2] = b.lo.z;
-        d.bbox_max[0] = b.hi.x;
-        d.bbox_max[1] = b.hi.y;
-        d.bbox_max[2] = b.hi.z;
-        d.first_child_or_prim = first;
-        d.num_prims = count;
-        d.ordered_traversal_axis = 0;
-        d.ordered_traversal_sign = 0;
-    };
-    for (int s = 0; s < 2; ++s)
-    {
-        gbrt_bvh_node& d = out[1 + 2 * i + s];
-        if (child[s] < 0)
-            put(d, cbox[s], __ldg(&sorted_ids[~child[s]]), 1);
-        else
-            put(d, cbox[s], uint32_t(1 + 2 * child[s]), 0);
-    }
+    const bvh2_node nd = nodes[i];
+    // first_child_or_prim, then num_prims | axis | sign in one word (0 for the last two)
+    auto first = [&](int c) { return c < 0 ? __ldg(&sorted_ids[~c]) : uint32_t(1 + 2 * c); };
+    auto count = [](int c) { return c < 0 ? 1u : 0u; };
+    float4* o = reinterpret_cast<float4*>(out + 1 + 2 * i);
+    o[0] = make_float4(nd.xy0.x, nd.xy0.z, nd.z01.x, nd.xy0.y);
+    o[1] = make_float4(nd.xy0.w, nd.z01.y, __uint_as_float(first(nd.link.x)), __uint_as_float(count(nd.link.x)));
+    o[2] = make_float4(nd.xy1.x, nd.xy1.z, nd.z01.z, nd.xy1.y);
+    o[3] = make_float4(nd.xy1.w, nd.z01.w, __uint_as_float(first(nd.link.y)), __uint_as_float(count(nd.link.y)));
+    indices[i] = uint32_t(i);
+    if (i == num_inner - 1) indices[i + 1] = uint32_t(i + 1);
     if (i == 0)
     {
-        put(out[0], box_union_cas(cbox[0], cbox[1]), 1u, 0);
+        const box3 b = box_union_cas({ { nd.xy0.x, nd.xy0.z, nd.z01.x }, { nd.xy0.y, nd.xy0.w, nd.z01.y } },
+                                     { { nd.xy1.x, nd.xy1.z, nd.z01.z }, { nd.xy1.y, nd.xy1.w, nd.z01.w } });
+        float4* r = reinterpret_cast<float4*>(out);
+        r[0] = make_float4(b.lo.x, b.lo.y, b.lo.z, b.hi.x);
+        r[1] = make_float4(b.hi.y, b.hi.z, __uint_as_float(1u), __uint_as_float(0u));
     }
 }
 
@@ -372,12 +325,6 @@ __global__ void emit_single(gbrt_triangle const* __restrict__ tris_in, tri48* __
     o.t1 = make_float4(t.e1.x, t.e1.y, t.e1.z, __uint_as_float(t.geom_id));
     o.t2 = make_float4(t.e2.x, t.e2.y, t.e2.z, __uint_as_float(kLastInLeaf));
     tris_out[0] = o;
-}
-
-__global__ void __launch_bounds__(kBlock) iota(uint32_t* __restrict__ out, uint32_t n)
-{
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i < n) out[i] = i;
 }
 
 __global__ void __launch_bounds__(kBlock) scatter_codes(const uint32_t* __restrict__ sorted_codes,
@@ -459,64 +406,53 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
         free_wide_nodes(bvh);
     }
 
-    // scratch: centroids | keys_alt | vals_alt | leaf_parent | arrivals | cb(6) | height | sort
+    // scratch: centroids | keys_alt | vals_alt | flags | cb(6) | height | sort | slots, then
+    // the wide collapse, if one is asked for
     size_t off_centroids = 0;
     size_t off_keys_alt = align_up(off_centroids + size_t(n) * 16);
     size_t off_vals_alt = align_up(off_keys_alt + size_t(n) * 4);
-    size_t off_parent = align_up(off_vals_alt + size_t(n) * 4);
-    size_t off_arrivals = align_up(off_parent + size_t(n) * 4);
-    size_t off_cb = align_up(off_arrivals + size_t(n) * 4);
+    size_t off_flags = align_up(off_vals_alt + size_t(n) * 4);
+    size_t off_cb = align_up(off_flags + size_t(n) * 4);
     size_t off_sort = align_up(off_cb + 8 * 4);
+    size_t off_waiting = align_up(off_sort + radix_sort_scratch_bytes(n));
+    size_t off_slots = align_up(off_waiting + agg_waiting_words(n) * 4);
     // wide collapse: node ranges, two level queues, per-level counts, node counter and
     // the nodes themselves (a tree with n leaves has at most 2n / (L + 1) nodes above L
     // leaves, the bound on the wide node count for leaves of at most L triangles)
     const int leaf_max = kLeafMax4;
     const uint32_t cap4 = uint32_t(2ull * n / (leaf_max + 1) + 2);
     const size_t wide_bytes = (ctx->trace_flags & GBRT_TRACE_WIDE8_NODES) ? sizeof(bvh8_node) : sizeof(bvh4_node);
-    size_t off_ranges = align_up(off_sort + radix_sort_scratch_bytes(n));
+    const bool want_wide = (ctx->trace_flags & (GBRT_TRACE_WIDE_NODES | GBRT_TRACE_COMPRESSED_NODES |
+                                                GBRT_TRACE_WIDE8_NODES)) != 0;
+    size_t off_ranges = align_up(off_slots + size_t(n) * sizeof(agg_slot));
     size_t off_q0 = align_up(off_ranges + size_t(n) * 8);
     size_t off_q1 = align_up(off_q0 + size_t(cap4) * 8);
     size_t off_counts = align_up(off_q1 + size_t(cap4) * 8);
     size_t off_nodes4 = align_up(off_counts + 256 * 4);
-    size_t total = off_nodes4 + size_t(cap4) * wide_bytes;
+    size_t total = want_wide ? off_nodes4 + size_t(cap4) * wide_bytes : off_ranges;
     gbrt_status st = ensure_scratch(ctx, total);
     if (st != GBRT_OK) return st;
     char* base = static_cast<char*>(ctx->scratch);
     float4* centroids = reinterpret_cast<float4*>(base + off_centroids);
     uint32_t* keys_alt = reinterpret_cast<uint32_t*>(base + off_keys_alt);
     uint32_t* vals_alt = reinterpret_cast<uint32_t*>(base + off_vals_alt);
-    int* leaf_parent = reinterpret_cast<int*>(base + off_parent);
-    uint32_t* arrivals = reinterpret_cast<uint32_t*>(base + off_arrivals);
+    uint32_t* flags = reinterpret_cast<uint32_t*>(base + off_flags);
     int* cb = reinterpret_cast<int*>(base + off_cb);
     uint32_t* root_height = reinterpret_cast<uint32_t*>(cb + 6);
-    int2* ranges = reinterpret_cast<int2*>(base + off_ranges);
+    uint32_t* waiting = reinterpret_cast<uint32_t*>(base + off_waiting);
+    agg_slot* slots = reinterpret_cast<agg_slot*>(base + off_slots);
+    int2* ranges = want_wide ? reinterpret_cast<int2*>(base + off_ranges) : nullptr;
     int2* queue[2] = { reinterpret_cast<int2*>(base + off_q0), reinterpret_cast<int2*>(base + off_q1) };
     uint32_t* level_counts = reinterpret_cast<uint32_t*>(base + off_counts);   // [0..254]
     uint32_t* node4_counter = level_counts + 255;
     void* wide_tmp = base + off_nodes4;
 
-    // cb = (+FLT_MAX x3, -FLT_MAX x3) as ordered ints; root height 1 by default
-    int init[8];
-    {
-        float lo = FLT_MAX, hi = -FLT_MAX;
-        int li, hi_i;
-        memcpy(&li, &lo, 4);
-        memcpy(&hi_i, &hi, 4);
-        hi_i = hi_i ^ 0x7FFFFFFF;   // negative float -> ordered int
-        for (int a = 0; a < 3; ++a)
-        {
-            init[a] = li;
-            init[3 + a] = hi_i;
-        }
-        init[6] = 1;
-        init[7] = 0;
-    }
-    GBRT_CUDA(ctx, cudaMemcpyAsync(cb, init, sizeof(init), cudaMemcpyHostToDevice, s));
-
+    init_build_words<<<1, 8, 0, s>>>(cb);
+    GBRT_LAUNCH_CHECK(ctx, "init_build_words");
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
     GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
-    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, bvh->sorted_codes, bvh->sorted_ids);
+    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, bvh->sorted_codes, bvh->sorted_ids, flags);
     GBRT_LAUNCH_CHECK(ctx, "morton_codes");
     st = radix_sort_pairs(ctx, bvh->sorted_codes, bvh->sorted_ids, keys_alt, vals_alt, n, 30,
                           base + off_sort);
@@ -524,15 +460,11 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
 
     if (n > 1)
     {
-        GBRT_CUDA(ctx, cudaMemsetAsync(bvh->nodes, 0, size_t(bvh->num_inner) * sizeof(bvh2_node), s));
-        GBRT_CUDA(ctx, cudaMemsetAsync(arrivals, 0, size_t(n) * 4, s));
-        GBRT_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, size_t(n) * 4, s));
-        build_hierarchy<<<blocks_for(n - 1), kBlock, 0, s>>>(bvh->sorted_codes, int(n), bvh->nodes, leaf_parent,
-                                                             ranges);
-        GBRT_LAUNCH_CHECK(ctx, "build_hierarchy");
-        refit_and_emit<<<blocks_for(n), kBlock, 0, s>>>(d_tris, bvh->sorted_ids, int(n), leaf_parent, bvh->nodes,
-                                                        arrivals, bvh->tris, root_height, ctx->d_status);
-        GBRT_LAUNCH_CHECK(ctx, "refit_and_emit");
+        const agg_args args{ d_tris, bvh->sorted_ids, bvh->sorted_codes, n, nullptr, nullptr, 0, bvh->nodes, ranges,
+                             slots, flags, waiting, waiting + agg_blocks(n) * (kAggBlock + 1), bvh->tris, root_height,
+                             ctx->d_status };
+        st = agglomerate<false>(ctx, args, s);
+        if (st != GBRT_OK) return st;
         uint32_t h = 0;
         bvh2_node root;
         GBRT_CUDA(ctx, cudaMemcpyAsync(&h, root_height, 4, cudaMemcpyDeviceToHost, s));
@@ -613,8 +545,10 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
 
 // bvh_refitter::refit (detail/bvh/refit.h:25-117) on the GPU: the tree keeps its
 // topology and leaf order; the leaf triangles are re-emitted from the new positions and
-// every node's boxes recomputed bottom-up by the build's refit kernel (second arrival
-// continues).  The 4-wide collapse, if any, is dropped (queries fall back to the pairs).
+// every node's boxes recomputed bottom-up: an LBVH by the build's own kernel from the
+// sorted codes it keeps (the same codes give the same topology), a PLOC tree along its
+// parent links (second arrival continues).  The wide collapse, if any, is dropped (queries
+// fall back to the pairs).
 gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_tris)
 {
     const uint32_t n = bvh->num_prims;
@@ -631,21 +565,42 @@ gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_
         GBRT_LAUNCH_CHECK(ctx, "emit_single");
         return set_single_box(ctx, bvh, d_tris);
     }
-    const size_t off_parent = 0, off_arrivals = align_up(size_t(n) * 4), off_height = align_up(off_arrivals + size_t(n) * 4);
-    gbrt_status st = ensure_scratch(ctx, off_height + 256);
-    if (st != GBRT_OK) return st;
-    char* base = static_cast<char*>(ctx->scratch);
-    int* leaf_parent = reinterpret_cast<int*>(base + off_parent);
-    uint32_t* arrivals = reinterpret_cast<uint32_t*>(base + off_arrivals);
-    uint32_t* root_height = reinterpret_cast<uint32_t*>(base + off_height);
-    GBRT_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, size_t(n) * 4, s));
-    GBRT_CUDA(ctx, cudaMemsetAsync(arrivals, 0, size_t(n) * 4, s));
-    leaf_parents_of<<<blocks_for(bvh->num_inner), kBlock, 0, s>>>(bvh->nodes, int(bvh->num_inner), int(n),
-                                                                  leaf_parent, ctx->d_status);
-    GBRT_LAUNCH_CHECK(ctx, "leaf_parents_of");
-    refit_and_emit<<<blocks_for(n), kBlock, 0, s>>>(d_tris, bvh->sorted_ids, int(n), leaf_parent, bvh->nodes, arrivals,
-                                                    bvh->tris, root_height, ctx->d_status);
-    GBRT_LAUNCH_CHECK(ctx, "refit_and_emit");
+    if (bvh->kind == bvh_kind::lbvh)
+    {
+        const size_t off_waiting = align_up(size_t(n) * 4), off_slots = align_up(off_waiting + agg_waiting_words(n) * 4),
+                     off_height = align_up(off_slots + size_t(n) * sizeof(agg_slot));
+        gbrt_status st = ensure_scratch(ctx, off_height + 256);
+        if (st != GBRT_OK) return st;
+        char* base = static_cast<char*>(ctx->scratch);
+        uint32_t* flags = reinterpret_cast<uint32_t*>(base);
+        uint32_t* waiting = reinterpret_cast<uint32_t*>(base + off_waiting);
+        GBRT_CUDA(ctx, cudaMemsetAsync(flags, 0, size_t(n) * 4, s));
+        const agg_args args{ d_tris, bvh->sorted_ids, bvh->sorted_codes, n, nullptr, nullptr, 0, bvh->nodes, nullptr,
+                             reinterpret_cast<agg_slot*>(base + off_slots), flags, waiting,
+                             waiting + agg_blocks(n) * (kAggBlock + 1), bvh->tris,
+                             reinterpret_cast<uint32_t*>(base + off_height), ctx->d_status };
+        st = agglomerate<false>(ctx, args, s);
+        if (st != GBRT_OK) return st;
+    }
+    else
+    {
+        const size_t off_parent = 0, off_arrivals = align_up(size_t(n) * 4),
+                     off_height = align_up(off_arrivals + size_t(n) * 4);
+        gbrt_status st = ensure_scratch(ctx, off_height + 256);
+        if (st != GBRT_OK) return st;
+        char* base = static_cast<char*>(ctx->scratch);
+        int* leaf_parent = reinterpret_cast<int*>(base + off_parent);
+        uint32_t* arrivals = reinterpret_cast<uint32_t*>(base + off_arrivals);
+        uint32_t* root_height = reinterpret_cast<uint32_t*>(base + off_height);
+        GBRT_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, size_t(n) * 4, s));
+        GBRT_CUDA(ctx, cudaMemsetAsync(arrivals, 0, size_t(n) * 4, s));
+        leaf_parents_of<<<blocks_for(bvh->num_inner), kBlock, 0, s>>>(bvh->nodes, int(bvh->num_inner), int(n),
+                                                                      leaf_parent, ctx->d_status);
+        GBRT_LAUNCH_CHECK(ctx, "leaf_parents_of");
+        refit_and_emit<<<blocks_for(n), kBlock, 0, s>>>(d_tris, bvh->sorted_ids, int(n), leaf_parent, bvh->nodes,
+                                                        arrivals, bvh->tris, root_height, ctx->d_status);
+        GBRT_LAUNCH_CHECK(ctx, "refit_and_emit");
+    }
     bvh2_node root;
     GBRT_CUDA(ctx, cudaMemcpyAsync(&root, bvh->nodes + (bvh->root > 0 ? bvh->root : 0), sizeof(root),
                                    cudaMemcpyDeviceToHost, s));
@@ -677,7 +632,7 @@ gbrt_status morton_order(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
     GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
-    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, codes_out, ids_out);
+    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, codes_out, ids_out, nullptr);
     GBRT_LAUNCH_CHECK(ctx, "morton_codes");
     return radix_sort_pairs(ctx, codes_out, ids_out, reinterpret_cast<uint32_t*>(base + off_keys_alt),
                             reinterpret_cast<uint32_t*>(base + off_vals_alt), n, 30, base + off_sort);
@@ -697,10 +652,8 @@ gbrt_status export_bvh2(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_bvh_node* d
         return GBRT_OK;
     }
     export_collapse<<<blocks_for(bvh->num_inner), kBlock, 0, s>>>(bvh->nodes, int(bvh->num_inner), bvh->sorted_ids,
-                                                                  d_nodes);
+                                                                  d_nodes, d_indices);
     GBRT_LAUNCH_CHECK(ctx, "export_collapse");
-    iota<<<blocks_for(n), kBlock, 0, s>>>(d_indices, n);
-    GBRT_LAUNCH_CHECK(ctx, "iota");
     return GBRT_OK;
 }
 
@@ -720,7 +673,8 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
 {
     if (n == 0) return GBRT_OK;
     const lbvh_scratch_layout l = lbvh_scratch_layout_for(n);
-    if (l.total > scratch_bytes || radix_sort_scratch_bytes(n) > l.total - l.sort)
+    if (l.total > scratch_bytes || radix_sort_scratch_bytes(n) > l.total - l.sort ||
+        agg_waiting_words(n) * 4 > l.slots - l.waiting)
         return fail(ctx, GBRT_ERR_TOO_LARGE, "LBVH build: scratch region too small for this many triangles");
     char* base = static_cast<char*>(scratch);
     float4* centroids = reinterpret_cast<float4*>(base + l.centroids);
@@ -728,8 +682,9 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
     uint32_t* vals = reinterpret_cast<uint32_t*>(base + l.vals);
     uint32_t* keys_alt = reinterpret_cast<uint32_t*>(base + l.keys_alt);
     uint32_t* vals_alt = reinterpret_cast<uint32_t*>(base + l.vals_alt);
-    int* leaf_parent = reinterpret_cast<int*>(base + l.leaf_parent);
-    uint32_t* arrivals = reinterpret_cast<uint32_t*>(base + l.arrivals);
+    uint32_t* flags = reinterpret_cast<uint32_t*>(base + l.flags);
+    uint32_t* waiting = reinterpret_cast<uint32_t*>(base + l.waiting);
+    agg_slot* slots = reinterpret_cast<agg_slot*>(base + l.slots);
     bvh2_node* nodes = reinterpret_cast<bvh2_node*>(base + l.nodes);
     tri48* tris = reinterpret_cast<tri48*>(base + l.tris);
     int* words = reinterpret_cast<int*>(base + l.words);
@@ -741,7 +696,7 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, words);
     GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
-    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, words, keys, vals);
+    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, words, keys, vals, flags);
     GBRT_LAUNCH_CHECK(ctx, "morton_codes");
     gbrt_status st = radix_sort_pairs(ctx, keys, vals, keys_alt, vals_alt, n, 30, base + l.sort);
     if (st != GBRT_OK) return st;
@@ -754,20 +709,14 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
         GBRT_LAUNCH_CHECK(ctx, "export_single_leaf");
         return GBRT_OK;
     }
-    // every call starts from cleared nodes, arrival counters and parent links: the
-    // region keeps whatever the previous build left in it
-    GBRT_CUDA(ctx, cudaMemsetAsync(nodes, 0, size_t(n - 1) * sizeof(bvh2_node), s));
-    GBRT_CUDA(ctx, cudaMemsetAsync(arrivals, 0, size_t(n) * 4, s));
-    GBRT_CUDA(ctx, cudaMemsetAsync(leaf_parent, 0xFF, size_t(n) * 4, s));
-    build_hierarchy<<<blocks_for(n - 1), kBlock, 0, s>>>(keys, int(n), nodes, leaf_parent, nullptr);
-    GBRT_LAUNCH_CHECK(ctx, "build_hierarchy");
-    refit_and_emit<<<blocks_for(n), kBlock, 0, s>>>(d_tris, vals, int(n), leaf_parent, nodes, arrivals, tris,
-                                                    root_height, ctx->d_status);
-    GBRT_LAUNCH_CHECK(ctx, "refit_and_emit");
-    export_collapse<<<blocks_for(n - 1), kBlock, 0, s>>>(nodes, int(n - 1), vals, d_nodes);
+    // every record of the tree is written whole and the flags were cleared with the codes:
+    // nothing of the previous build in the region is read
+    const agg_args args{ d_tris, vals, keys, n, nullptr, nullptr, 0, nodes, nullptr, slots, flags, waiting,
+                         waiting + agg_blocks(n) * (kAggBlock + 1), tris, root_height, ctx->d_status };
+    st = agglomerate<false>(ctx, args, s);
+    if (st != GBRT_OK) return st;
+    export_collapse<<<blocks_for(n - 1), kBlock, 0, s>>>(nodes, int(n - 1), vals, d_nodes, d_indices);
     GBRT_LAUNCH_CHECK(ctx, "export_collapse");
-    iota<<<blocks_for(n), kBlock, 0, s>>>(d_indices, n);
-    GBRT_LAUNCH_CHECK(ctx, "iota");
     return GBRT_OK;
 }
 

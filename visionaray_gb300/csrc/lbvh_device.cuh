@@ -1,6 +1,6 @@
 // Device helpers of the LBVH builders (lbvh.cu: one scene; batch.cu: many scenes in
-// one pass): triangle loads and bounds in the reference's arithmetic, Karras splits,
-// and the child-box slots of the node pairs used by the bottom-up refit.
+// one pass): triangle loads and bounds in the reference's arithmetic, and the child-box
+// slots of the node pairs used by the PLOC refit.
 #pragma once
 
 #include "api_internal.h"
@@ -65,42 +65,6 @@ __device__ __forceinline__ float warp_max(float v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = ref_max(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
     return v;
-}
-
-// Karras delta: common-prefix length of sorted keys i and j, with the index as a
-// tie-break for equal keys, -1 outside [0, n).
-__device__ __forceinline__ int kdelta(const uint32_t* __restrict__ codes, int n, int i, uint32_t ci, int j)
-{
-    if (j < 0 || j >= n) return -1;
-    uint32_t x = ci ^ __ldg(&codes[j]);
-    return x == 0 ? 32 + __clz(uint32_t(i) ^ uint32_t(j)) : __clz(x);
-}
-
-// Karras node i of the n sorted keys (lbvh.h:120-185): its key range [first, last] and
-// split position (left child covers [first, split], right [split + 1, last]).
-__device__ __forceinline__ void karras_node(const uint32_t* __restrict__ codes, int n, int i, int& first, int& last,
-                                            int& split)
-{
-    uint32_t ci = __ldg(&codes[i]);
-    int d = kdelta(codes, n, i, ci, i + 1) >= kdelta(codes, n, i, ci, i - 1) ? 1 : -1;
-    int dmin = kdelta(codes, n, i, ci, i - d);
-    int lmax = 2;
-    while (kdelta(codes, n, i, ci, i + lmax * d) > dmin) lmax <<= 1;
-    int l = 0;
-    for (int t = lmax >> 1; t >= 1; t >>= 1)
-        if (kdelta(codes, n, i, ci, i + (l + t) * d) > dmin) l += t;
-    int j = i + l * d;
-    int dnode = kdelta(codes, n, i, ci, j);
-    int s = 0;
-    int t = l;
-    do
-    {
-        t = (t + 1) >> 1;
-        if (kdelta(codes, n, i, ci, i + (s + t) * d) > dnode) s += t;
-    } while (t > 1);
-    split = i + s * d + min(d, 0);
-    first = min(i, j);
-    last = max(i, j);
 }
 
 __device__ __forceinline__ void store_child_box(bvh2_node* node, int side, box3 const& b)

@@ -14,10 +14,10 @@
 // Limits and sharing:
 //   - at most kNoAllocMaxPrims (65,536) triangles; larger inputs are rejected with
 //     GBRT_ERR_TOO_LARGE before any GPU work;
-//   - the array holds about 10 MB per device;
+//   - the array holds about 14 MB per device;
 //   - every call on a device uses the same array and leaves its contents behind; the
-//     build clears what must start at zero (node records, arrival counters, parent
-//     links, bounds words) itself, so calls that follow one another on a stream are
+//     build clears what must start at zero (flags, bounds words) itself, so calls that
+//     follow one another on a stream are
 //     independent, but calls whose executions overlap on the GPU (two streams, two
 //     host threads) race on the array and give wrong trees;
 //   - the first call on a device looks up the array's device address
