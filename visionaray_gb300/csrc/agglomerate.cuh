@@ -1,5 +1,5 @@
-// Bottom-up LBVH construction from sorted Morton codes in one kernel: hierarchy, boxes,
-// node records and leaf triangles (lbvh.cu: one scene; batch.cu: many scenes in one
+// Bottom-up LBVH construction from sorted Morton codes: hierarchy, boxes, node records and
+// leaf triangles in one pass (lbvh.cu: one scene; batch.cu: many scenes in one
 // arena).
 //
 // The tree is Karras' (lbvh.h:120-185, 281-330) but found from below, after Apetrei,
@@ -18,6 +18,11 @@
 // the split's flag; the second arrival reads the other side's).  No thread waits for
 // another one.  In one kernel, each block's few climbing threads held its registers and
 // shared memory through a chain of fences and atomics: 1,151 us for 8.4 M triangles.
+//
+// Measured on 8,388,608 triangles (heightfield 2048^2): in-place rebuild 1.76 -> 1.11 ms;
+// a refit (these two kernels and a memset of the flags) 0.67 ms.  Bound by the load/store
+// pipe (56 %: the triangle gather, 112 B of stores per triangle, the mail in shared memory)
+// and by the divergence of the climb (9 of 32 lanes, issue slots 44 %).
 #pragma once
 
 #include "lbvh_device.cuh"

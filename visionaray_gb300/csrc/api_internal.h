@@ -19,6 +19,14 @@ enum : uint32_t
     kStatusBadIndex      = 1u << 2,   // a node/triangle index outside its array was skipped
 };
 
+namespace gbrt {
+struct build_result
+{
+    float lo[3], hi[3];   // the root's box
+    uint32_t height;
+};
+} // namespace gbrt
+
 struct gbrt_context
 {
     int device = 0;
@@ -28,6 +36,14 @@ struct gbrt_context
     uint64_t launches = 0;
 
     uint32_t* d_status = nullptr;     // one word of status bits
+
+    // Device memory of the trees this context builds: a pool that keeps up to kPoolKeep
+    // bytes of freed trees for the next ones (api.cu, alloc_tree), made at the first build.
+    static constexpr uint64_t kPoolKeep = 4ull << 30;
+    cudaMemPool_t pool = nullptr;
+    // What a build reports to the host, written by its last kernels straight into mapped
+    // pinned memory: one synchronisation and no copies at the end of a build.
+    gbrt::build_result* h_result = nullptr;
 
     // Reusable scratch for builds (grown on demand, freed with the context).
     void* scratch = nullptr;
@@ -105,6 +121,9 @@ struct gbrt_bvh
     uint32_t num_inner = 0;      // inner nodes (records in `nodes`)
     int32_t root = 0;            // >= 0 inner node, < 0 leaf (~first triangle)
     uint32_t height = 0;         // levels of inner nodes on the longest root-leaf path
+    // GPU-built trees: one allocation that holds nodes, tris, sorted_codes and sorted_ids;
+    // null for uploaded trees, which own nodes and tris themselves
+    void* arena = nullptr;
     gbrt::bvh2_node* nodes = nullptr;
     gbrt::tri48* tris = nullptr; // leaf order
     // LBVH only: sorted Morton codes and, per sorted position, the input index.
@@ -240,6 +259,11 @@ struct device_guard
 gbrt_status fail(gbrt_context* ctx, gbrt_status st, std::string const& what);
 // Maps a CUDA error to a status, recording `where`.
 gbrt_status check_cuda(gbrt_context* ctx, cudaError_t err, const char* where);
+// The arrays of a tree of n > 0 triangles (nothing to do if it has them already): one
+// allocation from the context's pool.
+gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n);
+// The host and device address of the context's build_result (allocated once).
+gbrt_status ensure_result(gbrt_context* ctx, build_result** device);
 // Grows the context scratch to at least `bytes`.
 gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes);
 

@@ -345,6 +345,21 @@ __global__ void init_build_words(int* __restrict__ words)
     else if (t < 8) words[t] = t == 6 ? 1 : 0;
 }
 
+// The root's box -- the union of its two child boxes with the reference's min / max (x < y ?
+// x : y) -- and the tree's height (height may be null), for the host.
+__global__ void report_build(const bvh2_node* __restrict__ root, const uint32_t* __restrict__ height,
+                             build_result* __restrict__ out)
+{
+    const bvh2_node r = *root;
+    out->lo[0] = ref_min(r.xy0.x, r.xy1.x);
+    out->hi[0] = ref_max(r.xy0.y, r.xy1.y);
+    out->lo[1] = ref_min(r.xy0.z, r.xy1.z);
+    out->hi[1] = ref_max(r.xy0.w, r.xy1.w);
+    out->lo[2] = ref_min(r.z01.x, r.z01.z);
+    out->hi[2] = ref_max(r.z01.y, r.z01.w);
+    if (height) out->height = *height;
+}
+
 inline uint32_t blocks_for(uint64_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
 
 inline size_t align_up(size_t v) { return (v + 255) & ~size_t(255); }
@@ -369,18 +384,14 @@ gbrt_status set_single_box(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const
     return GBRT_OK;
 }
 
-// The scene box: the union of the root's two child boxes with the reference's min / max
-// (x < y ? x : y), as the exported root node holds it.
-void set_scene_box(gbrt_bvh* bvh, bvh2_node const& root)
+// The scene box: the root's, as the exported root node holds it.
+void set_scene_box(gbrt_bvh* bvh, build_result const& r)
 {
-    auto mn = [](float a, float b) { return a < b ? a : b; };
-    auto mx = [](float a, float b) { return a < b ? b : a; };
-    bvh->lo[0] = mn(root.xy0.x, root.xy1.x);
-    bvh->hi[0] = mx(root.xy0.y, root.xy1.y);
-    bvh->lo[1] = mn(root.xy0.z, root.xy1.z);
-    bvh->hi[1] = mx(root.xy0.w, root.xy1.w);
-    bvh->lo[2] = mn(root.z01.x, root.z01.z);
-    bvh->hi[2] = mx(root.z01.y, root.z01.w);
+    for (int a = 0; a < 3; ++a)
+    {
+        bvh->lo[a] = r.lo[a];
+        bvh->hi[a] = r.hi[a];
+    }
 }
 
 gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t n, gbrt_bvh* bvh)
@@ -394,11 +405,11 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
 
     cudaStream_t s = ctx->stream;
     // a rebuild (gbrt_bvh_rebuild_lbvh) of a tree of the same size writes into its arrays
-    if (!bvh->tris) GBRT_CUDA(ctx, cudaMalloc(&bvh->tris, size_t(n) * sizeof(tri48)));
-    if (!bvh->sorted_codes) GBRT_CUDA(ctx, cudaMalloc(&bvh->sorted_codes, size_t(n) * 4));
-    if (!bvh->sorted_ids) GBRT_CUDA(ctx, cudaMalloc(&bvh->sorted_ids, size_t(n) * 4));
-    if (bvh->num_inner > 0 && !bvh->nodes)
-        GBRT_CUDA(ctx, cudaMalloc(&bvh->nodes, size_t(bvh->num_inner) * sizeof(bvh2_node)));
+    gbrt_status st = alloc_tree(ctx, bvh, n);
+    if (st != GBRT_OK) return st;
+    build_result* result = nullptr;
+    st = ensure_result(ctx, &result);
+    if (st != GBRT_OK) return st;
     if (bvh->nodes4 || bvh->nodes8)
     {
         // a rebuild with a wide collapse from the previous build: its size may change
@@ -430,7 +441,7 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     size_t off_counts = align_up(off_q1 + size_t(cap4) * 8);
     size_t off_nodes4 = align_up(off_counts + 256 * 4);
     size_t total = want_wide ? off_nodes4 + size_t(cap4) * wide_bytes : off_ranges;
-    gbrt_status st = ensure_scratch(ctx, total);
+    st = ensure_scratch(ctx, total);
     if (st != GBRT_OK) return st;
     char* base = static_cast<char*>(ctx->scratch);
     float4* centroids = reinterpret_cast<float4*>(base + off_centroids);
@@ -465,14 +476,12 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
                              ctx->d_status };
         st = agglomerate<false>(ctx, args, s);
         if (st != GBRT_OK) return st;
-        uint32_t h = 0;
-        bvh2_node root;
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&h, root_height, 4, cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&root, bvh->nodes, sizeof(root), cudaMemcpyDeviceToHost, s));
+        report_build<<<1, 1, 0, s>>>(bvh->nodes, root_height, result);
+        GBRT_LAUNCH_CHECK(ctx, "report_build");
         GBRT_CUDA(ctx, cudaStreamSynchronize(s));
+        const uint32_t h = ctx->h_result->height;
         bvh->height = h;
-        // scene bounds: the union of the root's two child boxes
-        set_scene_box(bvh, root);
+        set_scene_box(bvh, *ctx->h_result);
 
         // collapse into wide nodes (on request), one level per launch; the pair tree has
         // h inner levels, so h levels drain every queue
@@ -601,11 +610,13 @@ gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_
                                                         arrivals, bvh->tris, root_height, ctx->d_status);
         GBRT_LAUNCH_CHECK(ctx, "refit_and_emit");
     }
-    bvh2_node root;
-    GBRT_CUDA(ctx, cudaMemcpyAsync(&root, bvh->nodes + (bvh->root > 0 ? bvh->root : 0), sizeof(root),
-                                   cudaMemcpyDeviceToHost, s));
+    build_result* result = nullptr;
+    gbrt_status st = ensure_result(ctx, &result);
+    if (st != GBRT_OK) return st;
+    report_build<<<1, 1, 0, s>>>(bvh->nodes + (bvh->root > 0 ? bvh->root : 0), nullptr, result);
+    GBRT_LAUNCH_CHECK(ctx, "report_build");
     GBRT_CUDA(ctx, cudaStreamSynchronize(s));
-    set_scene_box(bvh, root);
+    set_scene_box(bvh, *ctx->h_result);
     return GBRT_OK;
 }
 

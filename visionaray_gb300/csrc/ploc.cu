@@ -260,11 +260,9 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     bvh->height = 0;
     if (n == 0) return GBRT_OK;
     cudaStream_t s = ctx->stream;
-    GBRT_CUDA(ctx, cudaMalloc(&bvh->tris, size_t(n) * sizeof(tri48)));
-    GBRT_CUDA(ctx, cudaMalloc(&bvh->sorted_codes, size_t(n) * 4));
-    GBRT_CUDA(ctx, cudaMalloc(&bvh->sorted_ids, size_t(n) * 4));
-    if (bvh->num_inner > 0) GBRT_CUDA(ctx, cudaMalloc(&bvh->nodes, size_t(bvh->num_inner) * sizeof(bvh2_node)));
-    gbrt_status st = morton_order(ctx, d_tris, n, bvh->sorted_codes, bvh->sorted_ids);
+    gbrt_status st = alloc_tree(ctx, bvh, n);
+    if (st != GBRT_OK) return st;
+    st = morton_order(ctx, d_tris, n, bvh->sorted_codes, bvh->sorted_ids);
     if (st != GBRT_OK) return st;
 
     // scratch (after the sort): clusters twice, neighbours, flags, prefix, scan levels
