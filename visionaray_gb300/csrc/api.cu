@@ -60,15 +60,18 @@ gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
     }
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t nodes = up(size_t(n - 1) * sizeof(bvh2_node)), tris = up(size_t(n) * sizeof(tri48)),
-                 words = up(size_t(n) * 4);
+                 words = up(size_t(n) * 4), quads = up(size_t(n) * sizeof(quad_node));
     void* p = nullptr;
-    GBRT_CUDA(ctx, cudaMallocFromPoolAsync(&p, nodes + tris + 2 * words, ctx->pool, ctx->stream));
+    GBRT_CUDA(ctx, cudaMallocFromPoolAsync(&p, nodes + quads + tris + 2 * words, ctx->pool, ctx->stream));
     char* base = static_cast<char*>(p);
     bvh->arena = p;
     bvh->nodes = n > 1 ? reinterpret_cast<bvh2_node*>(base) : nullptr;
-    bvh->tris = reinterpret_cast<tri48*>(base + nodes);
-    bvh->sorted_codes = reinterpret_cast<uint32_t*>(base + nodes + tris);
-    bvh->sorted_ids = reinterpret_cast<uint32_t*>(base + nodes + tris + words);
+    base += nodes;
+    bvh->quads = n > 1 ? reinterpret_cast<quad_node*>(base) : nullptr;
+    base += quads;
+    bvh->tris = reinterpret_cast<tri48*>(base);
+    bvh->sorted_codes = reinterpret_cast<uint32_t*>(base + tris);
+    bvh->sorted_ids = reinterpret_cast<uint32_t*>(base + tris + words);
     return GBRT_OK;
 }
 
@@ -102,6 +105,7 @@ void free_bvh_arrays(gbrt_bvh* b)
         cudaFree(b->tris);
     }
     b->nodes = nullptr;
+    b->quads = nullptr;
     b->tris = nullptr;
     b->sorted_codes = nullptr;
     b->sorted_ids = nullptr;

@@ -24,6 +24,7 @@ struct build_result
 {
     float lo[3], hi[3];   // the root's box
     uint32_t height;
+    uint32_t quads_bad;   // some box is outside what the quad nodes cover
 };
 } // namespace gbrt
 
@@ -121,8 +122,8 @@ struct gbrt_bvh
     uint32_t num_inner = 0;      // inner nodes (records in `nodes`)
     int32_t root = 0;            // >= 0 inner node, < 0 leaf (~first triangle)
     uint32_t height = 0;         // levels of inner nodes on the longest root-leaf path
-    // GPU-built trees: one allocation that holds nodes, tris, sorted_codes and sorted_ids;
-    // null for uploaded trees, which own nodes and tris themselves
+    // GPU-built trees: one allocation that holds nodes, quads, tris, sorted_codes and
+    // sorted_ids; null for uploaded trees, which own nodes and tris themselves
     void* arena = nullptr;
     gbrt::bvh2_node* nodes = nullptr;
     gbrt::tri48* tris = nullptr; // leaf order
@@ -140,6 +141,10 @@ struct gbrt_bvh
     gbrt::bvh4q_node* nodes4q = nullptr;   // the same nodes quantised (GBRT_TRACE_COMPRESSED_NODES)
     gbrt::bvh8_node* nodes8 = nullptr;     // 8-wide collapse (GBRT_TRACE_WIDE8_NODES)
     uint32_t num_nodes8 = 0;
+    // Quad nodes (num_inner + 1 records in the arena; GPU-built trees of two triangles or
+    // more) and whether queries may use them: every box inside the quantisation's range.
+    gbrt::quad_node* quads = nullptr;
+    bool quads_ok = false;
 };
 
 namespace gbrt {
@@ -328,6 +333,12 @@ constexpr lbvh_scratch_layout lbvh_scratch_layout_for(uint32_t n)
 // not synchronise; stream-ordered on ctx->stream.
 gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t n, void* scratch,
                                   size_t scratch_bytes, gbrt_bvh_node* d_nodes, uint32_t* d_indices);
+
+// quads.cu: the quad nodes of num_inner > 0 node pairs on `stream` (quads holds num_inner + 1
+// records, the last one's org[0] cleared before); enqueue only.  host_bad (may be null): a
+// word that is set if the tree must not be traversed through them.
+gbrt_status make_quads(gbrt_context* ctx, bvh2_node const* nodes, uint32_t num_inner, quad_node* quads,
+                       uint32_t* host_bad, cudaStream_t stream);
 
 // radix_sort.cu: stable LSD sort of (key, value) pairs by the low `key_bits` bits.
 // Result lands in (keys, values); keys_alt/values_alt are same-sized scratch.  With

@@ -44,6 +44,27 @@ static_assert(sizeof(tri48) == 48, "triangle is 48 bytes");
 constexpr uint32_t kLastInLeaf = 1u;
 constexpr int kStackSize = 64;   // traversal stack entries (tree height must stay below)
 
+// Quad node (64 bytes = two 256-bit loads): the up to four grandchildren of one node
+// pair, their boxes quantised outward to 8 bits per plane.  Record i of the quad array
+// belongs to node pair i: slots 0 and 1 are the children of the pair's child 0, slots 2
+// and 3 those of child 1; a child that is a leaf takes both slots of its half, the second
+// with an empty box (low planes 255, high planes 0).  So a depth-first walk of the quads
+// in slot order meets the leaves in the order of a walk of the pairs.  A plane q of axis a
+// stands at org[a] + q * cell[a]; scale holds 2^15 * cell, which is what the decoded
+// plane values 1 + q * 2^-15 are multiplied with (quad_trace.cuh).  link: as a node
+// pair's (>= 0 node pair / quad index, < 0 leaf ~triangle).  The array holds one record
+// more than there are node pairs: org[0] of the last one is 0 when every box was finite
+// and within the range the quantisation covers, else 1.
+struct __align__(64) quad_node
+{
+    float org[3];
+    float scale_x;
+    int32_t link[4];
+    uint32_t lox, hix, loy, hiy, loz, hiz;   // slot k in byte k
+    float scale_y, scale_z;
+};
+static_assert(sizeof(quad_node) == 64, "quad node is one 64-byte record");
+
 // 4-wide node (128 bytes = eight 128-bit loads), collapsed from the node pairs: the
 // six box planes of the four children in SoA form, so one float4 per plane serves all
 // four slab tests.  count[k] > 0: leaf of count[k] contiguous triangles starting at

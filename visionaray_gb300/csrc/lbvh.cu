@@ -335,11 +335,13 @@ __global__ void __launch_bounds__(kBlock) scatter_codes(const uint32_t* __restri
     if (j < n) out[sorted_ids[j]] = sorted_codes[j];
 }
 
-// Centroid-bounds words (+FLT_MAX x3, -FLT_MAX x3 as ordered ints) and the root
-// height word, set on the device so a build needs no host-side staging.
-__global__ void init_build_words(int* __restrict__ words)
+// Centroid-bounds words (+FLT_MAX x3, -FLT_MAX x3 as ordered ints), the root height word
+// and the quads' validity word (may be null), set on the device so a build needs no
+// host-side staging.
+__global__ void init_build_words(int* __restrict__ words, float* __restrict__ quads_bad)
 {
     int t = threadIdx.x;
+    if (t == 0 && quads_bad) *quads_bad = 0.0f;
     if (t < 3) words[t] = float_to_ordered(FLT_MAX);
     else if (t < 6) words[t] = float_to_ordered(-FLT_MAX);
     else if (t < 8) words[t] = t == 6 ? 1 : 0;
@@ -458,7 +460,7 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     uint32_t* node4_counter = level_counts + 255;
     void* wide_tmp = base + off_nodes4;
 
-    init_build_words<<<1, 8, 0, s>>>(cb);
+    init_build_words<<<1, 8, 0, s>>>(cb, bvh->quads ? &bvh->quads[bvh->num_inner].org[0] : nullptr);
     GBRT_LAUNCH_CHECK(ctx, "init_build_words");
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
@@ -476,11 +478,15 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
                              ctx->d_status };
         st = agglomerate<false>(ctx, args, s);
         if (st != GBRT_OK) return st;
+        ctx->h_result->quads_bad = 0;
+        st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+        if (st != GBRT_OK) return st;
         report_build<<<1, 1, 0, s>>>(bvh->nodes, root_height, result);
         GBRT_LAUNCH_CHECK(ctx, "report_build");
         GBRT_CUDA(ctx, cudaStreamSynchronize(s));
         const uint32_t h = ctx->h_result->height;
         bvh->height = h;
+        bvh->quads_ok = ctx->h_result->quads_bad == 0;
         set_scene_box(bvh, *ctx->h_result);
 
         // collapse into wide nodes (on request), one level per launch; the pair tree has
@@ -613,9 +619,14 @@ gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_
     build_result* result = nullptr;
     gbrt_status st = ensure_result(ctx, &result);
     if (st != GBRT_OK) return st;
+    GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
+    ctx->h_result->quads_bad = 0;
+    st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+    if (st != GBRT_OK) return st;
     report_build<<<1, 1, 0, s>>>(bvh->nodes + (bvh->root > 0 ? bvh->root : 0), nullptr, result);
     GBRT_LAUNCH_CHECK(ctx, "report_build");
     GBRT_CUDA(ctx, cudaStreamSynchronize(s));
+    bvh->quads_ok = ctx->h_result->quads_bad == 0;
     set_scene_box(bvh, *ctx->h_result);
     return GBRT_OK;
 }
@@ -638,7 +649,7 @@ gbrt_status morton_order(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_
     char* base = static_cast<char*>(ctx->scratch);
     float4* centroids = reinterpret_cast<float4*>(base + off_centroids);
     int* cb = reinterpret_cast<int*>(base + off_cb);
-    init_build_words<<<1, 8, 0, s>>>(cb);
+    init_build_words<<<1, 8, 0, s>>>(cb, nullptr);
     GBRT_LAUNCH_CHECK(ctx, "init_build_words");
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
@@ -702,7 +713,7 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
     uint32_t* root_height = reinterpret_cast<uint32_t*>(words + 6);
     cudaStream_t s = ctx->stream;
 
-    init_build_words<<<1, 32, 0, s>>>(words);
+    init_build_words<<<1, 32, 0, s>>>(words, nullptr);
     GBRT_LAUNCH_CHECK(ctx, "init_build_words");
     uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
     centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, words);

@@ -14,9 +14,8 @@
 //            sample + shadow ray), throughput update, Russian roulette; live paths
 //            and shadow rays are appended to compacted queues with one atomic per
 //            warp (ballot + popc)
-//   shadow : any-hit traversal of the shadow queue, unoccluded contributions added (over
-//            instances in one launch with the next bounce's extend, which does not depend
-//            on it)
+//   shadow : any-hit traversal of the shadow queue, unoccluded contributions added; it
+//            shares a launch with the next bounce's extend, which does not depend on it
 // so every traversal launch runs over a dense queue of live rays.  The arithmetic is
 // the reference's, operation for operation (this file is compiled with
 // --fmad=false; divisions and square roots are IEEE), and the random numbers are
@@ -26,6 +25,7 @@
 
 #include "instances.cuh"
 #include "pt_shade.cuh"
+#include "quad_trace.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -140,6 +140,35 @@ __device__ __forceinline__ void add_shadow(frame_buffers const& fb, uint32_t j)
     const float4 c = fb.shadow_contrib[j];
     const float4 r = fb.radiance[p];
     fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
+}
+
+// The traversal of one bounce over the quad nodes: the closest hits of its ray queue
+// (blocks of row 0 when extend is set) and the shadow rays of the bounce before (the other
+// row).  Both queues' lengths are on the device; the grid holds the most warps that any
+// length takes, each warp finds its span from the length.
+__global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(frame_buffers fb, int q, uint32_t bounce,
+                                                                             uint32_t extend, bvh_view v,
+                                                                             uint32_t resident,
+                                                                             uint32_t* __restrict__ status)
+{
+    __shared__ int stack_mem[kQuadStack * kQuadBlock];
+    const bool closest = extend != 0 && blockIdx.y == 0;
+    const uint32_t n = closest ? fb.counts[2 * bounce] : fb.counts[2 * bounce - 1];
+    const uint32_t span = quad_span(n, resident);
+    const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
+    if (first >= n) return;
+    const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
+    auto index = [](uint32_t k) { return k; };
+    if (closest)
+        quad_trace<false, true>(stack_mem, v, fb.rays[q], n, next, end, status, index,
+                                [&](uint32_t j, trace_result const& h) {
+                                    fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
+                                });
+    else
+        quad_trace<true, true>(stack_mem, v, fb.shadow_rays, n, next, end, status, index,
+                               [&](uint32_t j, trace_result const& h) {
+                                   if (h.tri < 0) add_shadow(fb, j);
+                               });
 }
 
 template <bool Wide>
@@ -1241,6 +1270,20 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
     // the full queue per bounce and per shadow pass, for little coherence among diffuse
     // bounces), so it is an option.
     const bool sort = (p.flags & GBRT_PT_SORT_QUEUES) && bvh->num_prims > 0;
+    if (bvh->quads_ok && !wide && !sort)
+    {
+        const uint32_t resident = uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32);
+        auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
+            const uint32_t warps = quad_max_warps(n * fb.samples, resident);
+            const uint32_t grid = (warps + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+            pt_trace_quads<<<dim3(grid, extend && shadow ? 2 : 1), kQuadBlock, 0, s>>>(fb, q, b, extend ? 1u : 0u, v,
+                                                                                       resident, ctx->d_status);
+            GBRT_LAUNCH_CHECK(ctx, "pt_trace_quads");
+            return GBRT_OK;
+        };
+        return render_passes(ctx, cam, p, sp, no_instances, scene->num_lights, false, false, bg, d_accum, d_color,
+                             trace);
+    }
     const float3 lo = make_float3(bvh->lo[0], bvh->lo[1], bvh->lo[2]);
     float ext[3] = { bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2] };
     const float3 scale = make_float3(ext[0] > 0.0f ? 256.0f / ext[0] : 0.0f, ext[1] > 0.0f ? 256.0f / ext[1] : 0.0f,

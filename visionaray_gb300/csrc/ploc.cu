@@ -311,9 +311,17 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     {
         if (node_base != n - 1) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: wrong node count");
         float4 root_lo, root_hi;
+        build_result* result = nullptr;
+        st = ensure_result(ctx, &result);
+        if (st != GBRT_OK) return st;
+        ctx->h_result->quads_bad = 0;
+        GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
+        st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+        if (st != GBRT_OK) return st;
         GBRT_CUDA(ctx, cudaMemcpyAsync(&root_lo, lo[cur], sizeof(root_lo), cudaMemcpyDeviceToHost, s));
         GBRT_CUDA(ctx, cudaMemcpyAsync(&root_hi, hi[cur], sizeof(root_hi), cudaMemcpyDeviceToHost, s));
         GBRT_CUDA(ctx, cudaStreamSynchronize(s));
+        bvh->quads_ok = ctx->h_result->quads_bad == 0;
         int root = 0, height = 0;
         memcpy(&root, &root_lo.w, 4);
         memcpy(&height, &root_hi.w, 4);

@@ -1,0 +1,327 @@
+// Warp-stepped traversal of the quad nodes (bvh_layout.cuh, quads.cu), shared by the ray
+// queries (traverse.cu) and the path tracer (pathtrace.cu).
+//
+// What bounded the node-pair loop (traverse_core.cuh): a warp of incoherent rays ran it
+// with 7.9 of 32 lanes active, since lanes that reach a leaf wait for the lanes still
+// descending and ended rays wait for the warp's longest one, and its 64-byte node fetches
+// kept the load/store pipe 62 % busy (two wavefronts per lane and visit).  Here
+//   - a node visit tests four grandchildren out of one 64-byte record, so a ray takes half
+//     the visits (and half the wavefronts);
+//   - every iteration advances each busy lane by one node (two per vote round) and runs
+//     the leaf tests once enough lanes wait at one, so no lane waits for a whole descent;
+//   - a warp owns a span of rays and refills its idle lanes from it.
+// Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
+// query 3.36 -> 2.38 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.66 ms.  What
+// bounds it now: issue slots (64 %), the ALU pipe (63 %) and the load/store pipe (60 %)
+// about equally.
+//
+// The answers are the node-pair loop's, bit for bit, although the visits differ:
+//   - Boxes only get larger (quantised outward, and the distances below carry a margin
+//     for every rounding), so each leaf whose own box the pair loop's slab test accepts is
+//     reached, and triangles are tested with the same arithmetic.
+//   - The pair loop returns some triangle T that hits within [tmin, tmax] and whose leaf
+//     box the ray hits (the boxes of a tree are nested and the slab test is monotone, so
+//     an accepted leaf box implies accepted ancestors).  Among those let T* be the one of
+//     smallest t.  The pair loop can return another one only if it dropped T* for a triangle
+//     with t <= the entry distance of T*'s leaf box, or met an equal t first.  So if no
+//     other hit has t <= max(t*, entry distance of T*'s leaf box), T* is its answer;
+//     otherwise (a ray through a shared edge, coincident triangles) the ray is traced
+//     again by the pair loop.  Nodes are culled 1/256 beyond the best t, so such a second
+//     hit is met whatever the order.
+//   - Any hit, unordered: the pair loop reports the first hit of a depth-first walk in
+//     child order, and the quads' slots are in that order.  Any hit, near first (shadow
+//     rays): only whether there is a hit is used.
+//   - A ray with non-finite or extreme components, and one whose walk needs more than the
+//     shared stack, is traced by the pair loop too.
+#pragma once
+
+#include "traverse_core.cuh"
+
+namespace gbrt {
+
+// Threads of a block and shared stack entries per thread of every kernel that runs
+// quad_trace: 24 x 128 x 4 B = 12 KB per block.  A visit pushes up to three entries; 16
+// entries sent 125 of the 4.2 M heightfield rays to the pair loop, 24 none.
+constexpr int kQuadBlock = 128;
+constexpr int kQuadStack = 24;
+// Resident blocks the register allocation must allow: 9 (36 warps, 56 registers, no
+// spills).  Heightfield closest hit 2.38 ms; 2.43 at 10 blocks (48 registers, spilling),
+// 2.61 at 12, 2.75 at 8 without the second node step per round.
+constexpr int kQuadMinBlocks = 9;
+// Idle lanes of a warp that trigger a refill, and lanes waiting at a leaf that trigger the
+// leaf tests (or no lane left at a node).
+constexpr int kQuadRefill = 8;
+constexpr int kQuadLeafLanes = 4;
+
+// Rays per warp for n rays on a GPU that holds `resident` warps of the kernel: few rays
+// are spread over all resident warps (a warp's time is its slowest chain of dependent node
+// loads, and rays of other warps do not lengthen it: 1,023 rays over a 4,099-triangle
+// soup take 31 us one per warp, 47 us eight per warp); many rays go in about three waves
+// of spans of up to 256, which the block scheduler balances.
+__host__ __device__ __forceinline__ uint32_t quad_span(uint32_t n, uint32_t resident)
+{
+    const uint32_t one = (n + resident - 1) / resident;
+    if (one <= 8) return one > 0 ? one : 1;
+    const uint32_t three = (n + 3 * resident - 1) / (3 * resident);
+    return three < 8 ? 8 : (three > 256 ? 256 : three);
+}
+
+// The most warps that any ray count up to n takes at quad_span of that count.
+__host__ __forceinline__ uint32_t quad_max_warps(uint32_t n, uint32_t resident)
+{
+    const uint64_t waves = uint64_t(n) / 256 + 1;
+    const uint64_t cap = waves > 3ull * resident ? waves : 3ull * resident;
+    return uint32_t(n < cap ? n : cap);
+}
+
+__device__ __forceinline__ float max3f(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3f(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// A triangle's own leaf box (tri_box in lbvh_device.cuh, for finite input) against a ray
+// by the pair loop's slab test: whether it is hit, and its entry distance.
+__device__ __forceinline__ bool leaf_box_hit(f3 o, f3 id, float tmin, float tmax, f3 v, f3 e1, f3 e2, float& tn)
+{
+    const f3 p = { __fadd_rn(v.x, e1.x), __fadd_rn(v.y, e1.y), __fadd_rn(v.z, e1.z) };
+    const f3 q = { __fadd_rn(v.x, e2.x), __fadd_rn(v.y, e2.y), __fadd_rn(v.z, e2.z) };
+    const float lx = (ref_min(ref_min(v.x, p.x), q.x) - o.x) * id.x, hx = (ref_max(ref_max(v.x, p.x), q.x) - o.x) * id.x;
+    const float ly = (ref_min(ref_min(v.y, p.y), q.y) - o.y) * id.y, hy = (ref_max(ref_max(v.y, p.y), q.y) - o.y) * id.y;
+    const float lz = (ref_min(ref_min(v.z, p.z), q.z) - o.z) * id.z, hz = (ref_max(ref_max(v.z, p.z), q.z) - o.z) * id.z;
+    tn = fmaxf(tmin, fmaxf(fminf(lx, hx), fmaxf(fminf(ly, hy), fminf(lz, hz))));
+    return fminf(tmax, fminf(fmaxf(lx, hx), fminf(fmaxf(ly, hy), fmaxf(lz, hz)))) >= tn;
+}
+
+// Whether the quads' conservative arithmetic covers a ray: components finite and
+// moderate, each direction component zero or not below 2^-40 of the largest.  Within
+// these bounds 1 / d clamped to 2^64 and the products with it stay normal floats.
+__device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d)
+{
+    const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
+    const float md = fmaxf(fmaxf(ax, ay), az), low = md * 9.094947017729282e-13f;
+    const float mo = fabsf(o.x) + fabsf(o.y) + fabsf(o.z);
+    return md >= 9.094947017729282e-13f && md <= 1.099511627776e12f && mo <= 1.152921504606847e18f &&
+           (ax >= low || ax == 0.0f) && (ay >= low || ay == 0.0f) && (az >= low || az == 0.0f);
+}
+
+// Traces the rays index(next .. end - 1) of `rays` with the calling warp (every lane must
+// call it with the same next and end) and calls done(ray, result) for each, in any order
+// and from any lane.  index(k) below n is a ray; v.quads must be valid for v.nodes.
+// stack_mem: kQuadStack * kQuadBlock shared words of the block.
+template <bool AnyHit, bool NearFirst, class Index, class Done>
+__device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, const gbrt_ray* __restrict__ rays,
+                                           uint32_t n, uint32_t next, const uint32_t end,
+                                           uint32_t* __restrict__ status, Index index, Done done)
+{
+    constexpr int kDeep = INT32_MAX;   // best_tri of a ray that the pair loop answers
+    const uint32_t full = 0xFFFFFFFFu, none = 0xFFFFFFFFu;
+    const uint32_t lane_bit = 1u << (threadIdx.x & 31u);
+    // the lane's stack column as shared-memory addresses; the entry at col ends the walk
+    const uint32_t col = uint32_t(__cvta_generic_to_shared(stack_mem)) + 4u * threadIdx.x;
+    const uint32_t top_limit = col + 4u * kQuadBlock * (kQuadStack - 4);
+    uint32_t ray = none, top = col;
+    int node = kEmptyLink, best_tri = -1;
+    f3 o = { 0.0f, 0.0f, 0.0f }, d = { 0.0f, 0.0f, 0.0f }, id = { 0.0f, 0.0f, 0.0f };
+    float tmin = 0.0f, tmax = 0.0f, limit = 0.0f, best_t = 0.0f, second_t = 0.0f;
+
+    // One quad: the nearest (or first) hit child becomes `node`, the others are pushed; with
+    // no hit the stack is popped.
+    auto step = [&]() {
+        float a[8], b[8];
+        ld8(v.quads + node, a);
+        ld8(reinterpret_cast<const char*>(v.quads + node) + 32, b);
+        // the distance to plane value f = 1 + q 2^-15 of an axis is f * S + O with S =
+        // 2^15 cell / d and O = (org - o) / d - S; the margin 2^-21 (|org - o| / |d| + |S|)
+        // is more than the roundings here and those of the pair loop's test together
+        const float k21 = 4.76837158203125e-07f;
+        const float Sx = a[3] * id.x, Sy = b[6] * id.y, Sz = b[7] * id.z;
+        const float Ax = (a[0] - o.x) * id.x, Ay = (a[1] - o.y) * id.y, Az = (a[2] - o.z) * id.z;
+        const float Ox = Ax - Sx, Oy = Ay - Sy, Oz = Az - Sz;
+        const float mx = fabsf(Ax) + fabsf(Sx), my = fabsf(Ay) + fabsf(Sy), mz = fabsf(Az) + fabsf(Sz);
+        const float nxo = __fmaf_rn(-k21, mx, Ox), fxo = __fmaf_rn(k21, mx, Ox);
+        const float nyo = __fmaf_rn(-k21, my, Oy), fyo = __fmaf_rn(k21, my, Oy);
+        const float nzo = __fmaf_rn(-k21, mz, Oz), fzo = __fmaf_rn(k21, mz, Oz);
+        // near and far planes by the direction's sign: one select per four planes
+        const bool sx = id.x < 0.0f, sy = id.y < 0.0f, sz = id.z < 0.0f;
+        const uint32_t nx4 = __float_as_uint(sx ? b[1] : b[0]), fx4 = __float_as_uint(sx ? b[0] : b[1]);
+        const uint32_t ny4 = __float_as_uint(sy ? b[3] : b[2]), fy4 = __float_as_uint(sy ? b[2] : b[3]);
+        const uint32_t nz4 = __float_as_uint(sz ? b[5] : b[4]), fz4 = __float_as_uint(sz ? b[4] : b[5]);
+        float tn[4], tf[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+        {
+            // byte k of the planes into bits 8..15 of 1.0f: the float 1 + q 2^-15
+            const uint32_t sel = 0x7604u | (k << 4);
+            auto plane = [&](uint32_t q) { return __uint_as_float(__byte_perm(q, 0x3F800000u, sel)); };
+            const float nx = __fmaf_rn(plane(nx4), Sx, nxo), fx = __fmaf_rn(plane(fx4), Sx, fxo);
+            const float ny = __fmaf_rn(plane(ny4), Sy, nyo), fy = __fmaf_rn(plane(fy4), Sy, fyo);
+            const float nz = __fmaf_rn(plane(nz4), Sz, nzo), fz = __fmaf_rn(plane(fz4), Sz, fzo);
+            tn[k] = max3f(fmaxf(nx, ny), nz, tmin);
+            tf[k] = min3f(fminf(fx, fy), fz, limit);
+        }
+        // Selection, pushes and pop as predicated PTX: as C++ they became branches that
+        // split the warp (401 -> 361 instructions per ray).  Only the nearest child is
+        // chosen; the others keep slot order (sorting them saves 1 % of the visits).  A
+        // child equal to the chosen one (the empty slot of a leaf's half, if its inverted
+        // box passes) is not pushed.
+        if constexpr (NearFirst)
+            asm volatile(
+                "{\n\t.reg .pred h0,h1,h2,h3,p,q;\n\t.reg .f32 t0,t1,t2,t3,ta,tb;\n\t.reg .b32 la,lb;\n\t"
+                "setp.le.f32 h0, %2, %6;\n\tsetp.le.f32 h1, %3, %7;\n\t"
+                "setp.le.f32 h2, %4, %8;\n\tsetp.le.f32 h3, %5, %9;\n\t"
+                "selp.f32 t0, %2, 0f7F800000, h0;\n\tselp.f32 t1, %3, 0f7F800000, h1;\n\t"
+                "selp.f32 t2, %4, 0f7F800000, h2;\n\tselp.f32 t3, %5, 0f7F800000, h3;\n\t"
+                "setp.lt.f32 p, t1, t0;\n\tselp.b32 la, %11, %10, p;\n\tmin.f32 ta, t0, t1;\n\t"
+                "setp.lt.f32 q, t3, t2;\n\tselp.b32 lb, %13, %12, q;\n\tmin.f32 tb, t2, t3;\n\t"
+                "setp.lt.f32 p, tb, ta;\n\tselp.b32 %0, lb, la, p;\n\tmin.f32 ta, ta, tb;\n\t"
+                "setp.ne.and.s32 q, %13, %0, h3;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %13;\n\t"
+                "setp.ne.and.s32 q, %12, %0, h2;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %12;\n\t"
+                "setp.ne.and.s32 q, %11, %0, h1;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %11;\n\t"
+                "setp.ne.and.s32 q, %10, %0, h0;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %10;\n\t"
+                "setp.eq.f32 p, ta, 0f7F800000;\n\t@p ld.shared.b32 %0, [%1];\n\t@p sub.u32 %1, %1, %14;\n\t}"
+                : "=&r"(node), "+r"(top)
+                : "f"(tn[0]), "f"(tn[1]), "f"(tn[2]), "f"(tn[3]), "f"(tf[0]), "f"(tf[1]), "f"(tf[2]), "f"(tf[3]),
+                  "r"(__float_as_int(a[4])), "r"(__float_as_int(a[5])), "r"(__float_as_int(a[6])),
+                  "r"(__float_as_int(a[7])), "n"(4 * kQuadBlock)
+                : "memory");
+        else
+            asm volatile(
+                "{\n\t.reg .pred h0,h1,h2,h3,p,q;\n\t"
+                "setp.le.f32 h0, %2, %6;\n\tsetp.le.f32 h1, %3, %7;\n\t"
+                "setp.le.f32 h2, %4, %8;\n\tsetp.le.f32 h3, %5, %9;\n\t"
+                "selp.b32 %0, %12, %13, h2;\n\tselp.b32 %0, %11, %0, h1;\n\tselp.b32 %0, %10, %0, h0;\n\t"
+                "setp.ne.and.s32 q, %13, %0, h3;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %13;\n\t"
+                "setp.ne.and.s32 q, %12, %0, h2;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %12;\n\t"
+                "setp.ne.and.s32 q, %11, %0, h1;\n\t@q add.u32 %1, %1, %14;\n\t@q st.shared.b32 [%1], %11;\n\t"
+                "or.pred p, h0, h1;\n\tor.pred q, h2, h3;\n\tor.pred p, p, q;\n\t"
+                "@!p ld.shared.b32 %0, [%1];\n\t@!p sub.u32 %1, %1, %14;\n\t}"
+                : "=&r"(node), "+r"(top)
+                : "f"(tn[0]), "f"(tn[1]), "f"(tn[2]), "f"(tn[3]), "f"(tf[0]), "f"(tf[1]), "f"(tf[2]), "f"(tf[3]),
+                  "r"(__float_as_int(a[4])), "r"(__float_as_int(a[5])), "r"(__float_as_int(a[6])),
+                  "r"(__float_as_int(a[7])), "n"(4 * kQuadBlock)
+                : "memory");
+        const bool deep = top > top_limit;   // at least one free entry short of a visit's three
+        node = deep ? kEmptyLink : node;
+        best_tri = deep ? kDeep : best_tri;
+    };
+
+    for (;;)
+    {
+        // a link outside both ranges (the end of a walk, or a corrupt one) leaves a lane idle
+        const uint32_t nodes = __ballot_sync(full, uint32_t(node) < uint32_t(v.num_inner));
+        const bool leaf = uint32_t(~node) < uint32_t(v.num_tris);
+        const uint32_t leaves = __ballot_sync(full, leaf);
+        const uint32_t busy = nodes | leaves;
+        if (busy == 0 || (next < end && 32 - __popc(busy) >= kQuadRefill))
+        {
+            if (!(busy & lane_bit))
+            {
+                if (ray != none)
+                {
+                    if (node != kEmptyLink) atomicOr(status, kStatusBadIndex);
+                    trace_result res{ best_tri, best_t, 0.0f, 0.0f };
+                    bool exact = best_tri == kDeep;
+                    if (best_tri >= 0 && !exact)
+                    {
+                        const tri48* tp = v.tris + best_tri;
+                        const float4 t0 = ldg4(&tp->t0), t1 = ldg4(&tp->t1), t2 = ldg4(&tp->t2);
+                        const f3 v1 = { t0.x, t0.y, t0.z }, e1 = { t1.x, t1.y, t1.z }, e2 = { t2.x, t2.y, t2.z };
+                        float tn;
+                        const bool in_box = leaf_box_hit(o, { safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z) }, tmin, tmax,
+                                                         v1, e1, e2, tn);
+                        exact = !in_box || (!AnyHit && second_t <= fmaxf(best_t, tn));
+                        // u and v by the same test on the same inputs: the same values
+                        const tri_hit h = intersect_triangle(o, d, v1, e1, e2);
+                        res.u = h.u;
+                        res.v = h.v;
+                    }
+                    if (exact)
+                    {
+                        local_stack<kStackSize> stack;
+                        res = traverse_bvh_with<AnyHit, decltype(stack), NearFirst>(
+                            stack, v.nodes, v.tris, v.root, v.num_inner, v.num_tris, o, d, tmin, tmax, status);
+                    }
+                    done(ray, res);
+                    ray = none;
+                }
+                node = kEmptyLink;
+                const uint32_t k = next + __popc(~busy & (lane_bit - 1u));
+                if (k < end)
+                {
+                    ray = index(k);
+                    if (ray < n)
+                    {
+                        const float4 r0 = ldg4(&rays[ray]);
+                        const float4 r1 = ldg4(reinterpret_cast<const float4*>(&rays[ray]) + 1);
+                        const float big = 1.8446744073709552e19f;   // 2^64
+                        o = { r0.x, r0.y, r0.z };
+                        d = { r0.w, r1.x, r1.y };
+                        id = { fminf(fmaxf(safe_rcp(d.x), -big), big), fminf(fmaxf(safe_rcp(d.y), -big), big),
+                               fminf(fmaxf(safe_rcp(d.z), -big), big) };
+                        tmin = r1.z;
+                        limit = tmax = r1.w;
+                        best_t = second_t = FLT_MAX;
+                        top = col;
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(top), "r"(kEmptyLink) : "memory");
+                        const bool ok = quad_ray_ok(o, d);
+                        node = ok ? v.root : kEmptyLink;
+                        best_tri = ok ? -1 : kDeep;
+                    }
+                    else
+                    {
+                        atomicOr(status, kStatusBadIndex);
+                        ray = none;
+                    }
+                }
+            }
+            const bool last = busy == 0 && next >= end;
+            next = min(end, next + __popc(~busy));
+            if (last) break;
+            continue;
+        }
+        if (leaves != 0 && (nodes == 0 || __popc(leaves) >= kQuadLeafLanes))
+        {
+            if (leaf)
+            {
+                const int t = ~node;
+                const tri48* tp = v.tris + t;
+                const float4 t0 = ldg4(&tp->t0), t1 = ldg4(&tp->t1), t2 = ldg4(&tp->t2);
+                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(node) : "r"(top) : "memory");
+                top -= 4u * kQuadBlock;
+                const tri_hit h = intersect_triangle(o, d, { t0.x, t0.y, t0.z }, { t1.x, t1.y, t1.z },
+                                                     { t2.x, t2.y, t2.z });
+                if (h.hit && h.t >= tmin && h.t <= tmax)
+                {
+                    if (AnyHit)
+                    {
+                        best_tri = t;
+                        best_t = h.t;
+                        node = kEmptyLink;
+                    }
+                    else
+                    {
+                        second_t = fminf(second_t, fmaxf(h.t, best_t));
+                        best_tri = h.t < best_t ? t : best_tri;
+                        best_t = fminf(h.t, best_t);
+                        limit = fminf(tmax, best_t + fabsf(best_t) * (1.0f / 256.0f));
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (uint32_t(node) < uint32_t(v.num_inner)) step();
+        __syncwarp();
+        if (uint32_t(node) < uint32_t(v.num_inner)) step();
+        __syncwarp();
+    }
+}
+
+} // namespace gbrt

@@ -7,7 +7,7 @@
 // 32 rays of a warp start in one region of the scene and share its upper tree path.
 // Each ray is still traced independently: the hits are identical bit for bit.
 
-#include "traverse_core.cuh"
+#include "quad_trace.cuh"
 
 namespace gbrt {
 namespace {
@@ -86,6 +86,28 @@ __global__ void __launch_bounds__(kTraceBlock, AnyHit ? kMinBlocksAny : kMinBloc
     uint32_t prim = h.tri >= 0 ? __float_as_uint(ldg4(&v.tris[h.tri].t0).w) : GBRT_NO_HIT;
     reinterpret_cast<uint4*>(hits)[j] =
         make_uint4(prim, __float_as_uint(h.t), __float_as_uint(h.u), __float_as_uint(h.v));
+}
+
+// The ray queries over the quad nodes: warp w of the grid traces the span [w span, (w + 1)
+// span) of the rays, in the order perm if there is one.
+template <bool AnyHit>
+__global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_view v, const gbrt_ray* __restrict__ rays,
+                                                                          uint32_t n, uint32_t span,
+                                                                          const uint32_t* __restrict__ perm,
+                                                                          gbrt_hit* __restrict__ hits,
+                                                                          uint32_t* __restrict__ status)
+{
+    __shared__ int stack_mem[kQuadStack * kQuadBlock];
+    const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
+    if (first >= n) return;
+    const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
+    quad_trace<AnyHit, !AnyHit>(
+        stack_mem, v, rays, n, next, end, status, [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
+        [&](uint32_t j, trace_result const& h) {
+            const uint32_t prim = h.tri >= 0 ? __float_as_uint(ldg4(&v.tris[h.tri].t0).w) : GBRT_NO_HIT;
+            reinterpret_cast<uint4*>(hits)[j] =
+                make_uint4(prim, __float_as_uint(h.t), __float_as_uint(h.u), __float_as_uint(h.v));
+        });
 }
 
 // Persistent traversal with per-lane refill (Aila & Laine 2009, "persistent
@@ -323,6 +345,18 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
     const bool wide = !wide8 && !compressed && bvh->nodes4 != nullptr && (ctx->trace_flags & GBRT_TRACE_WIDE_NODES);
     const bool have_scratch = scratch && scratch_bytes >= trace_scratch_bytes(n);
     const bool persistent = (ctx->trace_flags & GBRT_TRACE_PERSISTENT) && !wide && !compressed && !wide8 && have_scratch;
+    // GPU-built trees go through their quad nodes; the pairs stay for uploaded trees, trees
+    // of one triangle and trees whose boxes the quads do not cover
+    const bool quads = bvh->quads_ok && !wide && !compressed && !wide8 && !persistent;
+    auto launch_quads = [&](const uint32_t* order) -> gbrt_status {
+        const uint32_t span = quad_span(n, uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32));
+        const uint32_t grid = (uint32_t((uint64_t(n) + span - 1) / span) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+        kernel_timer timer(ctx, stream);
+        auto kernel = any_hit ? trace_quads<true> : trace_quads<false>;
+        kernel<<<grid, kQuadBlock, 0, stream>>>(v, d_rays, n, span, order, d_hits, ctx->d_status);
+        GBRT_LAUNCH_CHECK(ctx, "trace_quads");
+        return GBRT_OK;
+    };
     const uint32_t* perm = nullptr;
     if ((ctx->trace_flags & GBRT_TRACE_SORT_RAYS) && n >= kSortMinRays && have_scratch)
     {
@@ -346,6 +380,7 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
                                           &sorted);
         if (st != GBRT_OK) return st;
         perm = sorted;   // vals or vals_alt, wherever the last pass left the order
+        if (quads) return launch_quads(perm);
         if (!persistent)
         {
             kernel_timer timer(ctx, stream);
@@ -380,6 +415,7 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
         GBRT_LAUNCH_CHECK(ctx, "trace_rays_dynamic");
         return GBRT_OK;
     }
+    if (quads) return launch_quads(nullptr);
     kernel_timer timer(ctx, stream);
     auto launch = [&](auto kernel) { kernel<<<blocks, kTraceBlock, 0, stream>>>(v, d_rays, n, d_hits, ctx->d_status); };
     if (wide8)

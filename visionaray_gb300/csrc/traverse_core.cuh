@@ -444,13 +444,14 @@ struct bvh_view
     const bvh4_node* nodes4;
     const bvh4q_node* nodes4q;
     const bvh8_node* nodes8;
+    const quad_node* quads;   // null: the node pairs only
     const tri48* tris;
     int32_t root, num_inner, num_nodes4, num_tris, num_nodes8;
 };
 
 inline bvh_view view_of(gbrt_bvh const* b)
 {
-    return { b->nodes, b->nodes4, b->nodes4q, b->nodes8, b->tris, b->root, int32_t(b->num_inner),
+    return { b->nodes, b->nodes4, b->nodes4q, b->nodes8, b->quads, b->tris, b->root, int32_t(b->num_inner),
              int32_t(b->num_nodes4), int32_t(b->num_prims), int32_t(b->num_nodes8) };
 }
 
