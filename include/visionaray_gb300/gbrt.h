@@ -480,7 +480,8 @@ gbrt_status gbrt_pathtrace_forward(gbrt_context* ctx, gbrt_pt_scene const* scene
  * (RGBA32F, alpha ignored) into d_grad_albedo and d_grad_emission (3 floats per slot,
  * ADDED to; zero them first).  Each (pixel, sample) path is re-traced from its random
  * numbers -- the same shading code as the forward frame, so the same path -- and its
- * vertices swept backwards; nothing of the forward frame is stored (memory O(pixels)).
+ * vertices swept backwards; nothing of the forward frame is stored.  Paths are replayed in
+ * passes whose state and vertex records take at most about 3 GB of context-owned memory.
  * Gradients are accumulated with warp-reduced FP32 atomics.  Geometry, visibility and
  * roulette decisions are not differentiated.  num_bounces <= 16.  A scene over
  * instances (gbrt_pt_scene_create_instanced) replays through the same two-level tree;

@@ -59,13 +59,6 @@ constexpr int kBlock = 128;
 // 16 blocks (32 registers, spilling) 666 with 16 entries, 671 with 8.
 constexpr int kPtSharedStack = 16;
 constexpr int kPtMinBlocks = 12;
-// The adjoint's replay kernel: resident blocks its registers must allow -- 16 blocks
-// (64 warps, 32 registers; the vertex records live in local memory anyway): backward
-// 15.4 -> 13.0 ms per inverse-rendering step (8 blocks 13.4, 12 blocks 14.3).  Its
-// traversal keeps the whole stack in local memory: a shared-memory top of 8 / 16
-// entries took the 512x512x16 replay from 46.2 to 55.1 / 65.6 ms (the shared carve-out
-// takes the L1 that the local vertex records use).
-constexpr int kAdjointMinBlocks = 16;
 // The shading kernel: 8 resident blocks (32 warps, at most 64 registers), the occupancy
 // it has without the out-of-line material samplers' call overhead.
 constexpr int kShadeMinBlocks = 8;
@@ -83,7 +76,14 @@ struct frame_buffers
     uint2* rng_flags;   // draw counter, flags
     float4* sum;
     uint32_t* counts;   // per bounce: its ray queue's length, its shadow queue's
-    uint32_t samples;   // samples per pixel of this pass: path p is sample p % samples of pixel p / samples
+    // path p of the pass is sample first_sample + p % samples of pixel first_pixel + p / samples
+    uint32_t first_pixel, samples, first_sample;
+    // the adjoint's replay: per bounce and path a vertex_rec in kRecWords float4
+    // (rec[(bounce * paths + p) * kRecWords]), and each path's number of vertices; null for
+    // a frame
+    float4* rec;
+    uint32_t* num_rec;
+    uint32_t paths;
     // queue order by origin cell (GBRT_TRACE_SORT_RAYS): keys / values and their
     // double buffers, the sort's scratch
     uint32_t* keys;
@@ -92,6 +92,14 @@ struct frame_buffers
     uint32_t* vals_alt;
     void* sort_scratch;
 };
+
+constexpr int kRecWords = 5;
+
+// The pixel and sample of path p of a pass.
+__device__ __forceinline__ uint2 path_sample(frame_buffers const& fb, uint32_t p)
+{
+    return make_uint2(fb.first_pixel + p / fb.samples, fb.first_sample + p % fb.samples);
+}
 
 // Appends the lanes with `take` to a queue: one atomic per warp.  Every lane of the
 // warp must call it.
@@ -117,15 +125,15 @@ __device__ __forceinline__ void store_ray(gbrt_ray* dst, v3 o, v3 d, float tmin,
 
 // Jittered primary rays (detail/sched_common.h:209-233: jitter x drawn before y) through
 // the pinhole camera (detail/pinhole_camera.inl:103-120), and the pass's queue lengths.
-__global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t width, uint32_t height,
-                                                    uint32_t frame, uint32_t first_sample, uint32_t num_counts,
+__global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t n, uint32_t width,
+                                                    uint32_t height, uint32_t frame, uint32_t num_counts,
                                                     camera_basis cam)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    const uint32_t n = width * height * fb.samples;
     for (uint32_t k = i; k < num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
     if (i >= n) return;
-    v3 d = primary_dir(cam, width, height, frame, i / fb.samples, first_sample + i % fb.samples);
+    const uint2 ps = path_sample(fb, i);
+    v3 d = primary_dir(cam, width, height, frame, ps.x, ps.y);
     store_ray(&fb.rays[0][i], { cam.eye.x, cam.eye.y, cam.eye.z }, d, 0.0f, FLT_MAX);
     fb.path[0][i] = i;
     fb.throughput[i] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
@@ -133,13 +141,56 @@ __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t w
     fb.rng_flags[i] = make_uint2(2u, kLastSpecular);
 }
 
-// The unoccluded contribution of shadow queue entry j.
-__device__ __forceinline__ void add_shadow(frame_buffers const& fb, uint32_t j)
+// The answer of shadow queue entry j of a bounce: an unoccluded contribution is added to
+// its path's radiance; in a replay an occluded one is taken out of its vertex record.
+__device__ __forceinline__ void finish_shadow(frame_buffers const& fb, uint32_t j, uint32_t bounce, bool occluded)
 {
+    if (fb.rec)
+    {
+        if (occluded)
+        {
+            float* kind = &fb.rec[(uint64_t(bounce) * fb.paths + fb.shadow_path[j]) * kRecWords].x;
+            *kind = __uint_as_float(__float_as_uint(*kind) & 0xFFu);
+        }
+        return;
+    }
+    if (occluded) return;
     const uint32_t p = fb.shadow_path[j];
     const float4 c = fb.shadow_contrib[j];
     const float4 r = fb.radiance[p];
     fb.radiance[p] = make_float4(r.x + c.x, r.y + c.y, r.z + c.z, 0.0f);
+}
+
+// vertex_rec in kRecWords float4 (the kind and the next-event flag share a word).
+__device__ __forceinline__ void store_rec(frame_buffers const& fb, uint32_t bounce, uint32_t p, vertex_rec const& r)
+{
+    float4* o = fb.rec + (uint64_t(bounce) * fb.paths + p) * kRecWords;
+    o[0] = make_float4(__uint_as_float(r.kind | r.nee << 8), __uint_as_float(r.geom), __uint_as_float(r.lgeom), r.rr);
+    o[1] = make_float4(r.thr.x, r.thr.y, r.thr.z, r.w);
+    o[2] = make_float4(r.x, r.b0, r.kl, r.lint.x);
+    o[3] = make_float4(r.lint.y, r.lint.z, r.gnee.x, r.gnee.y);
+    o[4] = make_float4(r.gnee.z, r.f.spec.x, r.f.spec.y, r.f.spec.z);
+}
+
+__device__ __forceinline__ vertex_rec load_rec(frame_buffers const& fb, uint32_t bounce, uint32_t p)
+{
+    const float4* o = fb.rec + (uint64_t(bounce) * fb.paths + p) * kRecWords;
+    const float4 a = o[0], b = o[1], c = o[2], d = o[3], e = o[4];
+    vertex_rec r;
+    r.kind = __float_as_uint(a.x) & 0xFFu;
+    r.nee = __float_as_uint(a.x) >> 8;
+    r.geom = __float_as_uint(a.y);
+    r.lgeom = __float_as_uint(a.z);
+    r.rr = a.w;
+    r.thr = { b.x, b.y, b.z };
+    r.w = b.w;
+    r.x = c.x;
+    r.b0 = c.y;
+    r.kl = c.z;
+    r.lint = { c.w, d.x, d.y };
+    r.gnee = { d.z, d.w, e.x };
+    r.f.spec = { e.y, e.z, e.w };
+    return r;
 }
 
 // The traversal of one bounce over the quad nodes: the closest hits of its ray queue
@@ -167,7 +218,7 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(fra
     else
         quad_trace<true, true>(stack_mem, v, fb.shadow_rays, n, next, end, status, index,
                                [&](uint32_t j, trace_result const& h) {
-                                   if (h.tri < 0) add_shadow(fb, j);
+                                   finish_shadow(fb, j, bounce - 1, h.tri >= 0);
                                });
 }
 
@@ -244,9 +295,12 @@ struct inst_shade
 
 // The queue's length is on the device; a fixed grid walks it (blocks of later, shorter
 // queues are not launched for nothing).
-__global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffers fb, int q, uint32_t first_sample,
-                                                                    shade_params sp0, inst_shade is,
-                                                                    uint32_t* __restrict__ status)
+// Extended, Env: shade_vertex's (a scene of matte and emissive slots without an environment
+// light takes the kernel without those branches).  Record: the adjoint's replay, which
+// keeps every vertex and no radiance.
+template <bool Extended, bool Env, bool Record>
+__global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffers fb, int q, shade_params sp0,
+                                                                    inst_shade is, uint32_t* __restrict__ status)
 {
     const uint32_t n = fb.counts[2 * sp0.bounce];
     for (uint32_t base = blockIdx.x * kBlock; base < n; base += gridDim.x * kBlock)
@@ -286,13 +340,19 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffer
                 }
             }
             uint2 rf = fb.rng_flags[p];
-            path_state st{ xyz(fb.throughput[p]), xyz(fb.radiance[p]), rf.x, rf.y };
-            sp.sample = first_sample + p % fb.samples;
-            shade_vertex(sp, p / fb.samples, sp.bounce, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w,
-                         int(hh.x), __uint_as_float(hh.y), st, out, status);
+            path_state st{ xyz(fb.throughput[p]), Record ? v3{ 0.0f, 0.0f, 0.0f } : xyz(fb.radiance[p]), rf.x, rf.y };
+            const uint2 ps = path_sample(fb, p);
+            sp.sample = ps.y;
+            shade_vertex<Extended, Env>(sp, ps.x, sp.bounce, { r0.x, r0.y, r0.z }, { r0.w, r1.x, r1.y }, r1.z, r1.w,
+                                        int(hh.x), __uint_as_float(hh.y), st, out, status);
             fb.throughput[p] = make_float4(st.thr.x, st.thr.y, st.thr.z, 0.0f);
-            fb.radiance[p] = make_float4(st.rad.x, st.rad.y, st.rad.z, 0.0f);
+            if (!Record) fb.radiance[p] = make_float4(st.rad.x, st.rad.y, st.rad.z, 0.0f);
             fb.rng_flags[p] = make_uint2(st.k, st.flags);
+            if (Record)
+            {
+                store_rec(fb, sp.bounce, p, out.rec);
+                fb.num_rec[p] = sp.bounce + 1;
+            }
         }
 
         uint32_t slot = warp_append(out.cont, &fb.counts[2 * sp.bounce + 2]);
@@ -306,7 +366,8 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) pt_shade(frame_buffer
         {
             store_ray(&fb.shadow_rays[sslot], out.sh_o, out.sh_d, sp.epsilon, out.sh_tmax);
             fb.shadow_path[sslot] = p;
-            fb.shadow_contrib[sslot] = make_float4(out.contrib.x, out.contrib.y, out.contrib.z, 0.0f);
+            if (!Record)
+                fb.shadow_contrib[sslot] = make_float4(out.contrib.x, out.contrib.y, out.contrib.z, 0.0f);
         }
     }
 }
@@ -322,7 +383,7 @@ __global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow(frame_buffers 
     float4 r0 = rp[0], r1 = rp[1];
     trace_result h = traverse_view_shared<true, Wide, kBlock, kPtSharedStack>(v, { r0.x, r0.y, r0.z },
                                                                              { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    if (h.tri < 0) add_shadow(fb, i);
+    finish_shadow(fb, i, bounce, h.tri >= 0);
 }
 
 // pt_shadow over the shadow queue in the order perm.
@@ -344,7 +405,7 @@ __global__ void __launch_bounds__(kBlock, kPtMinBlocks) pt_shadow_sorted(frame_b
     float4 r0 = rp[0], r1 = rp[1];
     trace_result h = traverse_view_shared<true, Wide, kBlock, kPtSharedStack>(v, { r0.x, r0.y, r0.z },
                                                                              { r0.w, r1.x, r1.y }, r1.z, r1.w, status);
-    if (h.tri < 0) add_shadow(fb, j);
+    finish_shadow(fb, j, bounce, h.tri >= 0);
 }
 
 // Bottom-level stack entries of the two-level queries held in shared memory (0: the
@@ -391,7 +452,7 @@ __global__ void __launch_bounds__(kBlock, kPtTlasMinBlocks) pt_trace_tlas(frame_
     else
     {
         const tlas_result h = trace_tlas<true>(tv, o, d, r1.z, r1.w, status);
-        if (h.tri < 0) add_shadow(fb, i);
+        finish_shadow(fb, i, bounce - 1, h.tri >= 0);
     }
 }
 
@@ -399,14 +460,13 @@ __global__ void __launch_bounds__(kBlock, kPtTlasMinBlocks) pt_trace_tlas(frame_
 // each path's radiance with alpha 1 if the camera ray hit, else the background.  The last
 // pass then takes rr.color /= spp; accum = src * sfactor + dst * dfactor; color = accum
 // (sched_common.h:472-511, pixel_access.h:1040-1043); the others keep the sum.
-__global__ void __launch_bounds__(kBlock) pt_accumulate(frame_buffers fb, uint32_t n, uint32_t first_sample,
-                                                        uint32_t last, float4 bg, float spp, float sfactor,
-                                                        float dfactor, float4* __restrict__ accum,
-                                                        float4* __restrict__ color)
+__global__ void __launch_bounds__(kBlock) pt_accumulate(frame_buffers fb, uint32_t n, uint32_t last, float4 bg,
+                                                        float spp, float sfactor, float dfactor,
+                                                        float4* __restrict__ accum, float4* __restrict__ color)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= n) return;
-    float4 s = first_sample == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : fb.sum[i];
+    float4 s = fb.first_sample == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : fb.sum[i];
     for (uint32_t k = 0; k < fb.samples; ++k)
     {
         const uint64_t p = uint64_t(i) * fb.samples + k;
@@ -556,81 +616,36 @@ __device__ __forceinline__ v3 nee_throughput_adjoint(vertex_rec const& r, v3 adj
     return tb;
 }
 
-// Path-replay backpropagation (Vicini, Speierer & Jakob 2021): one thread per
-// (pixel, sample) re-traces its path from its random-number counter -- the same
-// shade_vertex, so the replay is bit-identical to the forward frame -- keeping only
-// this path's vertices, then sweeps them backwards to turn the pixel's adjoint
-// dL/dI / spp into gradients w.r.t. the albedo of every matte vertex and the emission
-// of every emissive vertex and sampled light.  Memory stays O(pixels): nothing of the
-// forward frame is stored.  Geometry, visibility and the Russian-roulette decision are
-// not differentiated (the roulette's 1 / p weight is).  Inst: the scene is a two-level
-// tree (tv, is; v unused): each hit binds its instance's triangles, rows and material
-// slots before it is shaded, as the wavefront shade kernel does.
-template <bool Wide, bool Extended, bool Env, bool Inst>
-__global__ void __launch_bounds__(kBlock, kAdjointMinBlocks) pt_adjoint(bvh_view v, tlas_view tv, inst_shade is,
-                                                     shade_params sp, camera_basis cam, uint32_t width,
-                                                     uint32_t height, uint32_t spp, uint32_t num_bounces,
-                                                     const float4* __restrict__ img_adj, float* __restrict__ grad_albedo,
-                                                     float* __restrict__ grad_emission, uint32_t* __restrict__ status)
+// The reverse sweep of path-replay backpropagation (Vicini, Speierer & Jakob 2021).  A
+// backward call re-traces every (pixel, sample) path from its random-number counter -- the
+// frame's own stages, so the replay is bit-identical to the forward frame -- keeping the
+// vertices of one bounded pass of paths at a time, and this kernel sweeps a path's vertices
+// backwards to turn the pixel's adjoint dL/dI / spp into gradients w.r.t. the albedo of
+// every matte vertex and the emission of every emissive vertex and sampled light.  Nothing
+// of the forward frame is stored.  Geometry, visibility and the Russian-roulette decision
+// are not differentiated (the roulette's 1 / p weight is).
+// One kernel that replayed and swept a path per thread (records in local memory) took
+// 46.2 ms for 512x512x16 paths of 6 bounces at 4,094 triangles, its traversal diverging
+// across paths and bounces; the passes take 21.3 ms, 7.2 of them this kernel, bound by the
+// atomics on the few slots that most vertices share (walls and light).
+__global__ void __launch_bounds__(kBlock) pt_sweep(frame_buffers fb, uint32_t n, uint32_t num_bounces, float inv_spp,
+                                                   shade_params sp, const float4* __restrict__ img_adj,
+                                                   float* __restrict__ grad_albedo, float* __restrict__ grad_emission)
 {
-    // one query of the replay: the scene's tree, or the two-level tree with the hit
-    // instance bound into sp (closest-hit queries only; a shadow query binds nothing)
-    auto query = [&](auto any_hit, v3 o, v3 d, float tmin, float tmax) -> trace_result {
-        constexpr bool kAny = decltype(any_hit)::value;
-        if constexpr (Inst)
-        {
-            tlas_result h = traverse_tlas<kAny>(tv, { o.x, o.y, o.z }, { d.x, d.y, d.z }, tmin, tmax, status);
-            if (!kAny && h.tri >= 0)
-            {
-                const bvh_view bv = is.views[h.inst];
-                sp.tris = bv.tris;
-                sp.num_tris = bv.num_tris;
-                sp.xform = is.forward + 3 * h.inst;
-                sp.geom_base = is.geom_base[h.inst];
-            }
-            return trace_result{ h.tri, h.t, h.u, h.v };
-        }
-        else
-        {
-            return traverse_view<kAny, Wide>(v, { o.x, o.y, o.z }, { d.x, d.y, d.z }, tmin, tmax, status);
-        }
-    };
     const uint32_t full = 0xFFFFFFFFu;
-    const uint32_t npix = width * height;
-    const uint64_t gid = uint64_t(blockIdx.x) * kBlock + threadIdx.x;
-    const bool active = gid < uint64_t(npix) * spp;
-    const uint32_t pixel = active ? uint32_t(gid % npix) : 0u;
-    const uint32_t sample = active ? uint32_t(gid / npix) : 0u;
-    vertex_rec recs[kMaxReplay];
-    int nrec = 0;
+    // consecutive threads take consecutive pixels of one sample (the replay's queues hold a
+    // pixel's samples together): what a warp adds at once, and so the rounding of the sums,
+    // does not depend on the replay's order of paths
+    const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
+    const uint32_t pixels = n / fb.samples;
+    const bool active = t < n;
+    const uint32_t p = active ? t % pixels * fb.samples + t / pixels : 0;
+    const int nrec = active ? int(min(fb.num_rec[p], num_bounces)) : 0;
     v3 adj = { 0.0f, 0.0f, 0.0f };
-    if (active)
+    if (active && (fb.rng_flags[p].y & kFirstHit))
     {
-        sp.sample = sample;
-        v3 d = primary_dir(cam, width, height, sp.frame, pixel, sample);
-        v3 o = { cam.eye.x, cam.eye.y, cam.eye.z };
-        path_state st{ { 1.0f, 1.0f, 1.0f }, { 0.0f, 0.0f, 0.0f }, 2u, kLastSpecular };
-        for (uint32_t bounce = 0; bounce < num_bounces && bounce < uint32_t(kMaxReplay); ++bounce)
-        {
-            trace_result h = query(std::false_type{}, o, d, 0.0f, FLT_MAX);
-            vertex_out out;
-            shade_vertex<Extended, Env>(sp, pixel, bounce, o, d, 0.0f, FLT_MAX, h.tri, h.t, st, out, status);
-            if (out.shadow)
-            {
-                trace_result sh = query(std::true_type{}, out.sh_o, out.sh_d, sp.epsilon, out.sh_tmax);
-                if (sh.tri >= 0) out.rec.nee = 0;   // occluded: no contribution to differentiate
-            }
-            recs[nrec++] = out.rec;
-            if (!out.cont) break;
-            o = out.next_o;
-            d = out.next_d;
-        }
-        if (st.flags & kFirstHit)
-        {
-            float4 a4 = img_adj[pixel];
-            float inv = 1.0f / float(spp);
-            adj = { a4.x * inv, a4.y * inv, a4.z * inv };
-        }
+        const float4 a4 = img_adj[path_sample(fb, p).x];
+        adj = { a4.x * inv_spp, a4.y * inv_spp, a4.z * inv_spp };
     }
     // reverse sweep, warp-uniform so the gradient adds can be reduced per warp
     int kmax = __reduce_max_sync(full, nrec);
@@ -643,12 +658,12 @@ __global__ void __launch_bounds__(kBlock, kAdjointMinBlocks) pt_adjoint(bvh_view
         bool add_a = false, add_e = false, add_l = false;
         if (here)
         {
-            vertex_rec const& r = recs[k];
+            const vertex_rec r = load_rec(fb, uint32_t(k), p);
             geom = r.geom;
             if (r.kind == kVertexMiss)
             {
                 // the ambient or environment light the ray left into
-                tbar = adj * (Env ? r.f.spec : v3{ sp.ambient.x, sp.ambient.y, sp.ambient.z });
+                tbar = adj * (sp.env ? r.f.spec : v3{ sp.ambient.x, sp.ambient.y, sp.ambient.z });
             }
             else if (r.kind == kVertexEnd)
             {
@@ -729,15 +744,16 @@ uint32_t pass_samples(uint32_t npix, uint32_t spp)
 }
 
 // The buffers of a pass of n paths over npix pixels with num_counts queue lengths; sort: with
-// the queue order's keys.
+// the queue order's keys; record_bounces: with the vertex records of that many bounces.
 gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint32_t num_counts, bool sort,
-                              frame_buffers& fb)
+                              uint32_t record_bounces, frame_buffers& fb)
 {
     const size_t key = sort ? size_t(n) * 4 : 0;
     size_t sizes[] = { size_t(n) * 32, size_t(n) * 32, size_t(n) * 4, size_t(n) * 4, size_t(n) * 16,
                        size_t(n) * 32, size_t(n) * 4,  size_t(n) * 16, size_t(n) * 16, size_t(n) * 16,
                        size_t(n) * 8,  size_t(npix) * 16, size_t(num_counts) * 4, key, key, key,
-                       key, sort ? radix_sort_scratch_bytes(n) : 0 };
+                       key, sort ? radix_sort_scratch_bytes(n) : 0,
+                       size_t(n) * record_bounces * kRecWords * 16, record_bounces ? size_t(n) * 4 : 0 };
     constexpr int kParts = int(sizeof(sizes) / sizeof(sizes[0]));
     size_t total = 0;
     for (size_t s : sizes) total += align256(s);
@@ -779,6 +795,11 @@ gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint
     fb.keys_alt = static_cast<uint32_t*>(ptr[15]);
     fb.vals_alt = static_cast<uint32_t*>(ptr[16]);
     fb.sort_scratch = ptr[17];
+    fb.rec = record_bounces ? static_cast<float4*>(ptr[18]) : nullptr;
+    fb.num_rec = static_cast<uint32_t*>(ptr[19]);
+    fb.paths = n;
+    fb.first_pixel = 0;
+    fb.first_sample = 0;
     return GBRT_OK;
 }
 
@@ -1149,120 +1170,137 @@ shade_params shade_params_for(gbrt_context const* ctx, gbrt_pt_scene const* scen
     return sp;
 }
 
-// The launch that ends a pass of pass_samples(...) samples from first_sample on.
-gbrt_status end_pass(gbrt_context* ctx, frame_buffers const& fb, gbrt_pt_params const& p, uint32_t first_sample, float4 bg,
-                     float* d_accum, float* d_color)
+// The shading kernel of a scene.
+using shade_kernel = void (*)(frame_buffers, int, shade_params, inst_shade, uint32_t*);
+shade_kernel pick_shade(gbrt_pt_scene const* scene, bool record)
 {
-    const uint32_t n = p.width * p.height;
-    const uint32_t last = first_sample + fb.samples >= p.spp ? 1u : 0u;
-    pt_accumulate<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
-        fb, n, first_sample, last, bg, float(p.spp), p.sfactor, p.dfactor, reinterpret_cast<float4*>(d_accum),
-        reinterpret_cast<float4*>(d_color));
-    GBRT_LAUNCH_CHECK(ctx, "pt_accumulate");
+    if (scene->env) return record ? pt_shade<true, true, true> : pt_shade<true, true, false>;
+    if (scene->extended) return record ? pt_shade<true, false, true> : pt_shade<true, false, false>;
+    return record ? pt_shade<false, false, true> : pt_shade<false, false, false>;
+}
+
+// One pass of n paths: camera rays, then per bounce traversal and shading.  trace(fb, q,
+// bounce, n, extend, shadow) launches the closest hits of the bounce's ray queue q if
+// extend, the shadow rays of the bounce before if shadow.
+template <class Trace>
+gbrt_status run_pass(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam, gbrt_pt_params const& p,
+                     shade_params sp, inst_shade const& is, bool empty, frame_buffers const& fb, uint32_t n,
+                     uint32_t num_counts, Trace const& trace)
+{
+    cudaStream_t s = ctx->stream;
+    const uint32_t blocks = (n + kBlock - 1) / kBlock;
+    const uint32_t shade_blocks = std::min(blocks, uint32_t(ctx->num_sms) * kShadeMinBlocks * 4);
+    const shade_kernel shade = pick_shade(scene, fb.rec != nullptr);
+    const bool lights = scene->num_lights > 0;
+    pt_raygen<<<blocks, kBlock, 0, s>>>(fb, n, p.width, p.height, p.frame_id, num_counts, cam);
+    GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
+    int q = 0;
+    for (uint32_t b = 0; b < p.num_bounces && !empty; ++b)
+    {
+        sp.bounce = b;
+        gbrt_status st = trace(fb, q, b, n, true, b > 0 && lights);
+        if (st != GBRT_OK) return st;
+        shade<<<shade_blocks, kBlock, 0, s>>>(fb, q, sp, is, ctx->d_status);
+        GBRT_LAUNCH_CHECK(ctx, "pt_shade");
+        q ^= 1;
+    }
+    if (p.num_bounces > 0 && !empty && lights) return trace(fb, q, p.num_bounces, n, false, true);
     return GBRT_OK;
 }
 
-// A wavefront frame whose traversal launches are trace(fb, q, bounce, extend, shadow):
-// the closest hits of bounce's ray queue q if extend, the shadow rays of the bounce before
-// if shadow.
+// A wavefront frame: passes of several samples per pixel, the last one blended into accum
+// and written to color.
 template <class Trace>
-gbrt_status render_passes(gbrt_context* ctx, camera_basis const& cam, gbrt_pt_params const& p, shade_params sp,
-                          inst_shade const& is, uint32_t num_lights, bool empty, bool sort, float4 bg, float* d_accum,
-                          float* d_color, Trace trace)
+gbrt_status render_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam,
+                          gbrt_pt_params const& p, shade_params const& sp, inst_shade const& is, bool empty, bool sort,
+                          float4 bg, float* d_accum, float* d_color, Trace const& trace)
 {
     const uint32_t npix = p.width * p.height;
     const uint32_t samples = pass_samples(npix, p.spp);
-    const uint32_t n = npix * samples;
     const uint32_t num_counts = 2 * (p.num_bounces + 1);
-    cudaStream_t s = ctx->stream;
     frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, npix, n, num_counts, sort, fb);
+    gbrt_status st = frame_buffers_for(ctx, npix, npix * samples, num_counts, sort, 0, fb);
     if (st != GBRT_OK) return st;
-    const uint32_t blocks = (n + kBlock - 1) / kBlock;
-    const uint32_t shade_blocks = std::min(blocks, uint32_t(ctx->num_sms) * kShadeMinBlocks * 4);
     for (uint32_t smp = 0; smp < p.spp; smp += fb.samples)
     {
+        fb.first_sample = smp;
         fb.samples = std::min(samples, p.spp - smp);
-        pt_raygen<<<blocks, kBlock, 0, s>>>(fb, p.width, p.height, p.frame_id, smp, num_counts, cam);
-        GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
-        int q = 0;
-        for (uint32_t b = 0; b < p.num_bounces && !empty; ++b)
-        {
-            sp.bounce = b;
-            st = trace(fb, q, b, true, b > 0 && num_lights > 0);
-            if (st != GBRT_OK) return st;
-            pt_shade<<<shade_blocks, kBlock, 0, s>>>(fb, q, smp, sp, is, ctx->d_status);
-            GBRT_LAUNCH_CHECK(ctx, "pt_shade");
-            q ^= 1;
-        }
-        if (p.num_bounces > 0 && !empty && num_lights > 0)
-        {
-            st = trace(fb, q, p.num_bounces, false, true);
-            if (st != GBRT_OK) return st;
-        }
-        st = end_pass(ctx, fb, p, smp, bg, d_accum, d_color);
+        st = run_pass(ctx, scene, cam, p, sp, is, empty, fb, npix * fb.samples, num_counts, trace);
         if (st != GBRT_OK) return st;
+        pt_accumulate<<<(npix + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
+            fb, npix, smp + fb.samples >= p.spp ? 1u : 0u, bg, float(p.spp), p.sfactor, p.dfactor,
+            reinterpret_cast<float4*>(d_accum), reinterpret_cast<float4*>(d_color));
+        GBRT_LAUNCH_CHECK(ctx, "pt_accumulate");
     }
     return GBRT_OK;
 }
 
-// The wavefront frame of a scene over a two-level tree: each queue traced through the
-// top-level tree and the instances' trees (traverse_tlas), each hit shaded with its
-// instance's triangle carried to world space and its instance's material slots.
-gbrt_status render_frame_instanced(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam,
-                                   gbrt_pt_params const& p, shade_params sp, float4 bg, float* d_accum, float* d_color)
+// Bytes of vertex records that a backward pass may hold (its paths: at most kPassPaths).
+constexpr uint64_t kRecordBytes = 2ull << 30;
+
+// Path-replay backpropagation in passes of a range of pixels and samples: each pass replayed
+// by the frame's stages with records, then swept.
+template <class Trace>
+gbrt_status replay_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam,
+                          gbrt_pt_params const& p, shade_params const& sp, inst_shade const& is, bool sort,
+                          const float* d_image_adjoint, float* d_grad_albedo, float* d_grad_emission,
+                          Trace const& trace)
 {
-    if (p.flags & (GBRT_PT_MEGAKERNEL | GBRT_PT_SORT_QUEUES))
-        return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace: the megakernel and sorted queues take a single tree");
-    gbrt_tlas const* t = scene->tlas;
-    const tlas_view tv{ t->nodes, t->records, t->views, t->num_instances > 0 ? t->root : kEmptyLink,
-                        int32_t(t->num_inner), int32_t(t->num_instances) };
-    const inst_shade is{ t->views, t->forward, scene->inst_geom, int32_t(t->num_instances) };
-    auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
-        const uint32_t blocks = (p.width * p.height * fb.samples + kBlock - 1) / kBlock;
-        pt_trace_tlas<<<dim3(blocks, extend && shadow ? 2 : 1), kBlock, 0, ctx->stream>>>(fb, q, b, extend ? 1u : 0u,
-                                                                                          tv, ctx->d_status);
-        GBRT_LAUNCH_CHECK(ctx, "pt_trace_tlas");
-        return GBRT_OK;
-    };
-    return render_passes(ctx, cam, p, sp, is, scene->num_lights, t->num_instances == 0, false, bg, d_accum, d_color,
-                         trace);
+    if (p.num_bounces == 0) return GBRT_OK;   // paths without vertices
+    const uint32_t npix = p.width * p.height;
+    const uint64_t most = std::min(kPassPaths, kRecordBytes / (uint64_t(p.num_bounces) * kRecWords * 16));
+    const uint32_t pixels = uint32_t(std::min<uint64_t>(npix, most));
+    const uint32_t samples = uint32_t(std::min<uint64_t>(p.spp, most / pixels));
+    const uint32_t num_counts = 2 * (p.num_bounces + 1);
+    frame_buffers fb;
+    gbrt_status st = frame_buffers_for(ctx, 0, pixels * samples, num_counts, sort, p.num_bounces, fb);
+    if (st != GBRT_OK) return st;
+    for (uint32_t smp = 0; smp < p.spp; smp += samples)
+    {
+        fb.first_sample = smp;
+        fb.samples = std::min(samples, p.spp - smp);
+        for (uint32_t px = 0; px < npix; px += pixels)
+        {
+            fb.first_pixel = px;
+            const uint32_t n = std::min(pixels, npix - px) * fb.samples;
+            st = run_pass(ctx, scene, cam, p, sp, is, false, fb, n, num_counts, trace);
+            if (st != GBRT_OK) return st;
+            pt_sweep<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
+                fb, n, p.num_bounces, 1.0f / float(p.spp), sp, reinterpret_cast<const float4*>(d_image_adjoint),
+                d_grad_albedo, d_grad_emission);
+            GBRT_LAUNCH_CHECK(ctx, "pt_sweep");
+        }
+    }
+    return GBRT_OK;
 }
 
-// One frame of the wavefront path tracer into accum (blended) and color.
-gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_camera const& camera,
-                         gbrt_pt_params const& p, const float* albedo, const float* emission, float* d_accum,
-                         float* d_color)
+// Calls run(trace, instances, sort) with the scene's traversal launches (run_pass's trace),
+// its instances' shading data (null views for a single tree) and whether the queues are
+// sorted.
+template <class Run>
+gbrt_status with_tracer(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_pt_params const& p, Run run)
 {
-    if ((reinterpret_cast<uintptr_t>(d_accum) & 15u) || (reinterpret_cast<uintptr_t>(d_color) & 15u))
-        return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace: images must be 16-byte aligned");
-    const uint32_t n = p.width * p.height;
-    camera_basis cam = camera_for(camera, p.width, p.height);
-    gbrt_bvh const* bvh = scene->bvh;
-    gbrt_status tst = ensure_trig_table(ctx);   // a no-op unless the scene came from another context
-    if (tst != GBRT_OK) return tst;
-    shade_params sp = shade_params_for(ctx, scene, p, albedo, emission);
-    // background: ambient_light(bg.xyz, bg.w).intensity with alpha 1 (kernels.h:172-174,
-    // pathtracing.inl:62)
-    float4 bg = make_float4(p.background[0] * p.background[3], p.background[1] * p.background[3],
-                            p.background[2] * p.background[3], 1.0f);
-    const uint32_t blocks = (n + kBlock - 1) / kBlock;
     cudaStream_t s = ctx->stream;
-    if (scene->tlas)
-        return render_frame_instanced(ctx, scene, cam, p, sp, bg, d_accum, d_color);
+    if (gbrt_tlas const* t = scene->tlas)
+    {
+        // a scene over a two-level tree: each queue traced through the top-level tree and the
+        // instances' trees (traverse_tlas), each hit shaded with its instance's triangle
+        // carried to world space and its instance's material slots
+        const tlas_view tv{ t->nodes, t->records, t->views, t->num_instances > 0 ? t->root : kEmptyLink,
+                            int32_t(t->num_inner), int32_t(t->num_instances) };
+        const inst_shade is{ t->views, t->forward, scene->inst_geom, int32_t(t->num_instances) };
+        auto trace = [&](frame_buffers const& fb, int q, uint32_t b, uint32_t n, bool extend,
+                         bool shadow) -> gbrt_status {
+            pt_trace_tlas<<<dim3((n + kBlock - 1) / kBlock, extend && shadow ? 2 : 1), kBlock, 0, s>>>(
+                fb, q, b, extend ? 1u : 0u, tv, ctx->d_status);
+            GBRT_LAUNCH_CHECK(ctx, "pt_trace_tlas");
+            return GBRT_OK;
+        };
+        return run(trace, is, false);
+    }
+    gbrt_bvh const* bvh = scene->bvh;
     const bvh_view v = view_of(bvh);
     const bool wide = bvh->nodes4 != nullptr && (ctx->trace_flags & GBRT_TRACE_WIDE_NODES);
-    if (p.flags & GBRT_PT_MEGAKERNEL)
-    {
-        auto launch = [&](auto kernel) {
-            kernel<<<blocks, kBlock, 0, s>>>(v, sp, cam, p.width, p.height, p.spp, p.num_bounces, bg, p.sfactor,
-                                             p.dfactor, reinterpret_cast<float4*>(d_accum),
-                                             reinterpret_cast<float4*>(d_color), ctx->d_status);
-        };
-        wide ? launch(pt_megakernel<true>) : launch(pt_megakernel<false>);
-        GBRT_LAUNCH_CHECK(ctx, "pt_megakernel");
-        return GBRT_OK;
-    }
     const inst_shade no_instances{ nullptr, nullptr, nullptr, 0 };
     // GBRT_PT_SORT_QUEUES: each bounce's ray and shadow queues ordered by origin cell of
     // the scene box before they are traced (as the ray queries order their rays).
@@ -1273,28 +1311,26 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
     if (bvh->quads_ok && !wide && !sort)
     {
         const uint32_t resident = uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32);
-        auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
-            const uint32_t warps = quad_max_warps(n * fb.samples, resident);
-            const uint32_t grid = (warps + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+        auto trace = [&](frame_buffers const& fb, int q, uint32_t b, uint32_t n, bool extend,
+                         bool shadow) -> gbrt_status {
+            const uint32_t grid = (quad_max_warps(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
             pt_trace_quads<<<dim3(grid, extend && shadow ? 2 : 1), kQuadBlock, 0, s>>>(fb, q, b, extend ? 1u : 0u, v,
                                                                                        resident, ctx->d_status);
             GBRT_LAUNCH_CHECK(ctx, "pt_trace_quads");
             return GBRT_OK;
         };
-        return render_passes(ctx, cam, p, sp, no_instances, scene->num_lights, false, false, bg, d_accum, d_color,
-                             trace);
+        return run(trace, no_instances, false);
     }
     const float3 lo = make_float3(bvh->lo[0], bvh->lo[1], bvh->lo[2]);
     float ext[3] = { bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2] };
     const float3 scale = make_float3(ext[0] > 0.0f ? 256.0f / ext[0] : 0.0f, ext[1] > 0.0f ? 256.0f / ext[1] : 0.0f,
                                      ext[2] > 0.0f ? 256.0f / ext[2] : 0.0f);
-    auto trace = [&](frame_buffers const& fb, int q, uint32_t b, bool extend, bool shadow) -> gbrt_status {
-        const uint32_t paths = n * fb.samples;
-        const uint32_t blocks = (paths + kBlock - 1) / kBlock;
+    auto trace = [&](frame_buffers const& fb, int q, uint32_t b, uint32_t n, bool extend, bool shadow) -> gbrt_status {
+        const uint32_t blocks = (n + kBlock - 1) / kBlock;
         auto order = [&](const gbrt_ray* rays, const uint32_t* count) -> gbrt_status {
-            pt_queue_keys<<<blocks, kBlock, 0, s>>>(rays, count, paths, lo, scale, fb.keys, fb.vals);
+            pt_queue_keys<<<blocks, kBlock, 0, s>>>(rays, count, n, lo, scale, fb.keys, fb.vals);
             GBRT_LAUNCH_CHECK(ctx, "pt_queue_keys");
-            return radix_sort_pairs(ctx, fb.keys, fb.vals, fb.keys_alt, fb.vals_alt, paths, 24, fb.sort_scratch, s);
+            return radix_sort_pairs(ctx, fb.keys, fb.vals, fb.keys_alt, fb.vals_alt, n, 24, fb.sort_scratch, s);
         };
         if (shadow)
         {
@@ -1331,8 +1367,45 @@ gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_cam
         }
         return GBRT_OK;
     };
-    return render_passes(ctx, cam, p, sp, no_instances, scene->num_lights, bvh->num_prims == 0, sort, bg, d_accum,
-                         d_color, trace);
+    return run(trace, no_instances, sort);
+}
+
+// One frame of the path tracer into accum (blended) and color.
+gbrt_status render_frame(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_camera const& camera,
+                         gbrt_pt_params const& p, const float* albedo, const float* emission, float* d_accum,
+                         float* d_color)
+{
+    if ((reinterpret_cast<uintptr_t>(d_accum) & 15u) || (reinterpret_cast<uintptr_t>(d_color) & 15u))
+        return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace: images must be 16-byte aligned");
+    const uint32_t n = p.width * p.height;
+    camera_basis cam = camera_for(camera, p.width, p.height);
+    gbrt_bvh const* bvh = scene->bvh;
+    gbrt_status tst = ensure_trig_table(ctx);   // a no-op unless the scene came from another context
+    if (tst != GBRT_OK) return tst;
+    shade_params sp = shade_params_for(ctx, scene, p, albedo, emission);
+    // background: ambient_light(bg.xyz, bg.w).intensity with alpha 1 (kernels.h:172-174,
+    // pathtracing.inl:62)
+    float4 bg = make_float4(p.background[0] * p.background[3], p.background[1] * p.background[3],
+                            p.background[2] * p.background[3], 1.0f);
+    if (scene->tlas && (p.flags & (GBRT_PT_MEGAKERNEL | GBRT_PT_SORT_QUEUES)))
+        return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace: the megakernel and sorted queues take a single tree");
+    if (p.flags & GBRT_PT_MEGAKERNEL)
+    {
+        const bvh_view v = view_of(bvh);
+        const bool wide = bvh->nodes4 != nullptr && (ctx->trace_flags & GBRT_TRACE_WIDE_NODES);
+        auto launch = [&](auto kernel) {
+            kernel<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
+                v, sp, cam, p.width, p.height, p.spp, p.num_bounces, bg, p.sfactor, p.dfactor,
+                reinterpret_cast<float4*>(d_accum), reinterpret_cast<float4*>(d_color), ctx->d_status);
+        };
+        wide ? launch(pt_megakernel<true>) : launch(pt_megakernel<false>);
+        GBRT_LAUNCH_CHECK(ctx, "pt_megakernel");
+        return GBRT_OK;
+    }
+    const bool empty = scene->tlas ? scene->tlas->num_instances == 0 : bvh->num_prims == 0;
+    return with_tracer(ctx, scene, p, [&](auto const& trace, inst_shade const& is, bool sort) {
+        return render_passes(ctx, scene, cam, p, sp, is, empty, sort, bg, d_accum, d_color, trace);
+    });
 }
 
 } // namespace
@@ -1375,7 +1448,8 @@ extern "C" gbrt_status gbrt_pathtrace_backward(gbrt_context* ctx, gbrt_pt_scene 
         return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace_backward: null parameter or gradient array");
     if (reinterpret_cast<uintptr_t>(d_image_adjoint) & 15u)
         return fail(ctx, GBRT_ERR_INVALID_ARG, "pathtrace_backward: adjoint image must be 16-byte aligned");
-    gbrt_pt_params const& p = *params;
+    gbrt_pt_params p = *params;
+    p.flags &= ~GBRT_PT_SORT_QUEUES;   // scheduling only; the replay keeps the queues' order
     if (p.num_bounces > uint32_t(kMaxReplay))
         return fail(ctx, GBRT_ERR_TOO_LARGE, "pathtrace_backward: at most 16 bounces");
     gbrt_tlas const* t = scene->tlas;
@@ -1389,33 +1463,7 @@ extern "C" gbrt_status gbrt_pathtrace_backward(gbrt_context* ctx, gbrt_pt_scene 
     shade_params sp = shade_params_for(ctx, scene, p, d_albedo, d_emission);
     const uint64_t paths = uint64_t(p.width) * p.height * p.spp;
     if (paths > (1ull << 31)) return fail(ctx, GBRT_ERR_TOO_LARGE, "pathtrace_backward: more than 2^31 paths");
-    const uint32_t blocks = uint32_t((paths + kBlock - 1) / kBlock);
-    bvh_view v{};
-    tlas_view tv{};
-    inst_shade is{ nullptr, nullptr, nullptr, 0 };
-    bool wide = false;
-    if (t)
-    {
-        tv = tlas_view{ t->nodes, t->records, t->views, t->root, int32_t(t->num_inner), int32_t(t->num_instances) };
-        is = inst_shade{ t->views, t->forward, scene->inst_geom, int32_t(t->num_instances) };
-    }
-    else
-    {
-        v = view_of(bvh);
-        wide = bvh->nodes4 != nullptr && (ctx->trace_flags & GBRT_TRACE_WIDE_NODES);
-    }
-    // matte / emissive scenes get the replay without the other materials' branches
-    // (an environment light takes the full replay)
-    auto kernel = t ? (scene->env        ? pt_adjoint<false, true, true, true>
-                       : scene->extended ? pt_adjoint<false, true, false, true>
-                                         : pt_adjoint<false, false, false, true>)
-                  : scene->env ? (wide ? pt_adjoint<true, true, true, false> : pt_adjoint<false, true, true, false>)
-                  : wide ? (scene->extended ? pt_adjoint<true, true, false, false> : pt_adjoint<true, false, false, false>)
-                         : (scene->extended ? pt_adjoint<false, true, false, false>
-                                            : pt_adjoint<false, false, false, false>);
-    kernel<<<blocks, kBlock, 0, ctx->stream>>>(v, tv, is, sp, cam, p.width, p.height, p.spp, p.num_bounces,
-                                               reinterpret_cast<const float4*>(d_image_adjoint), d_grad_albedo,
-                                               d_grad_emission, ctx->d_status);
-    GBRT_LAUNCH_CHECK(ctx, "pt_adjoint");
-    return GBRT_OK;
+    return with_tracer(ctx, scene, p, [&](auto const& trace, inst_shade const& is, bool sort) {
+        return replay_passes(ctx, scene, cam, p, sp, is, sort, d_image_adjoint, d_grad_albedo, d_grad_emission, trace);
+    });
 }
