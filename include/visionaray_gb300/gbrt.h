@@ -577,7 +577,8 @@ gbrt_status gbrt_batch_set_frames(gbrt_context* ctx, gbrt_batch* batch, gbrt_cam
                                   gbrt_pt_params const* h_params, gbrt_material const* h_materials,
                                   uint32_t num_materials);
 
-/* Launch shape of gbrt_batch_pathtrace (the autotuner's search space).            */
+/* Launch shape of gbrt_batch_pathtrace (the autotuner's search space).  Shapes with a
+ * 64-entry stack on the unsorted node pairs differ in the pixel order only.        */
 #define GBRT_BATCH_ORDER_ROWS 0u    /* a warp's pixels are consecutive in a row       */
 #define GBRT_BATCH_ORDER_BLOCKS 1u  /* a warp's 32 pixels are an 8x4 screen block
                                        (scenes with width % 8 == 0, height % 4 == 0;
@@ -605,10 +606,12 @@ gbrt_status gbrt_batch_get_launch(gbrt_batch const* batch, gbrt_batch_launch* ou
  * synchronises the context stream.                                                 */
 gbrt_status gbrt_batch_height(gbrt_context* ctx, gbrt_batch const* batch, uint32_t* out);
 
-/* One frame of every scene in a single persistent launch: warps take tiles of pixels of
- * any scene from one atomic work queue and run the path tracer (the same shading as
- * gbrt_pathtrace_frame, so scene s's image equals the one gbrt_pathtrace_frame
- * renders with its camera, params and lights).  d_images: RGBA32F, 16-byte aligned,
+/* One frame of every scene (the same shading as gbrt_pathtrace_frame, so scene s's image
+ * equals the one gbrt_pathtrace_frame renders with its camera, params and lights).  With
+ * the full 64-entry stack, width 2 and no sorting (the default) the frame goes through the
+ * queues of the wavefront renderer, all scenes' paths together, and the block and tile of
+ * the launch shape do not matter; otherwise through a single persistent launch whose warps
+ * take tiles of pixels of any scene from one atomic work queue.  d_images: RGBA32F, 16-byte aligned,
  * scene s at pixel offset sum_{t<s} width_t * height_t.  Enqueue only.              */
 gbrt_status gbrt_batch_pathtrace(gbrt_context* ctx, gbrt_batch* batch, float* d_images);
 

@@ -228,6 +228,13 @@ struct gbrt_batch
     uint32_t* sort_buf = nullptr;
     void* sort_scratch = nullptr;
     uint32_t sort_capacity = 0;
+    // the wavefront frame (batch_wf.cu; allocated on first use): the arena's quad nodes
+    // (total_inner + 1), the build they were made from, and one pass's path state
+    gbrt::quad_node* quads = nullptr;
+    uint64_t quads_gen = 0;
+    void* path_buf = nullptr;
+    size_t path_bytes = 0;
+    uint32_t max_spp = 0, max_bounces = 0;   // over the scenes' frames
     // lights (gbrt_batch_set_lights): 4 float4 per light, scene s's lights at
     // [light_offsets[s], light_offsets[s + 1])
     float4* d_lights = nullptr;
@@ -377,6 +384,12 @@ gbrt_status batch_collapse(gbrt_context* ctx, gbrt_batch* b, uint32_t width, cud
 // last build's collapse at this width is current.
 gbrt_status batch_frame_stage(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t stream,
                               bool force_collapse);
+// batch_wf.cu: whether the launch's frames go through the wavefront renderer, its buffers
+// (allocated outside a capture), and the frame (enqueue only; force_quads re-makes the quad
+// nodes even when the last build's are current).
+bool batch_wavefront_applies(gbrt_batch const* b);
+gbrt_status ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b);
+gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t s, bool force_quads);
 
 } // namespace gbrt
 

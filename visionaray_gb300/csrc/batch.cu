@@ -261,6 +261,8 @@ void free_batch(gbrt_batch* b)
     cudaFree(b->wide_counts);
     cudaFree(b->sort_buf);
     cudaFree(b->sort_scratch);
+    cudaFree(b->quads);
+    cudaFree(b->path_buf);
 }
 
 } // namespace

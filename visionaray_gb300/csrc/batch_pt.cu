@@ -131,6 +131,7 @@ gbrt_status ensure_batch_extras(gbrt_context* ctx, gbrt_batch* b)
         if (st != GBRT_OK) return st;
     }
     if (b->launch.sort) return ensure_batch_sort(ctx, b);
+    if (batch_wavefront_applies(b)) return ensure_batch_wavefront(ctx, b);
     return GBRT_OK;
 }
 
@@ -148,6 +149,11 @@ gbrt_status batch_frame_stage(gbrt_context* ctx, gbrt_batch* b, float* d_images,
         return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: wide nodes not allocated");
     if (b->launch.sort && (!b->sort_buf || b->sort_capacity < b->total_pixels))
         return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: sort buffers not allocated");
+    if (batch_wavefront_applies(b))
+    {
+        if (!ctx->d_trig) return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: frames not set on this context");
+        return batch_wavefront(ctx, b, d_images, stream, force_collapse);
+    }
     int per_sm = 0;
     GBRT_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, int(b->launch.block), 0));
     if (per_sm < 1) per_sm = 1;
@@ -281,6 +287,12 @@ extern "C" gbrt_status gbrt_batch_set_frames(gbrt_context* ctx, gbrt_batch* batc
             kind == GBRT_MATERIAL_MIRROR || kind == GBRT_MATERIAL_GLASS || kind == GBRT_MATERIAL_PLASTIC;
     }
     batch->total_pixels = uint32_t(total);
+    batch->max_spp = batch->max_bounces = 0;
+    for (uint32_t s = 0; s < ns; ++s)
+    {
+        batch->max_spp = std::max(batch->max_spp, h_params[s].spp);
+        batch->max_bounces = std::max(batch->max_bounces, h_params[s].num_bounces);
+    }
     batch->frames_set = ns;
     batch->graph_dirty = true;
     return GBRT_OK;

@@ -114,12 +114,15 @@ __device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d)
 
 // Traces the rays index(next .. end - 1) of `rays` with the calling warp (every lane must
 // call it with the same next and end) and calls done(ray, result) for each, in any order
-// and from any lane.  index(k) below n is a ray; v.quads must be valid for v.nodes.
-// stack_mem: kQuadStack * kQuadBlock shared words of the block.
-template <bool AnyHit, bool NearFirst, class Index, class Done>
-__device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, const gbrt_ray* __restrict__ rays,
-                                           uint32_t n, uint32_t next, const uint32_t end,
-                                           uint32_t* __restrict__ status, Index index, Done done)
+// and from any lane.  index(k) below n is a ray, root(ray) the link its walk starts from.
+// stack_mem: kQuadStack * kQuadBlock shared words of the block.  bad: null when the host
+// knows the quads valid, else their validity word (the last record's org[0]): when it is
+// set every ray takes the pair loop.
+template <bool AnyHit, bool NearFirst, class Root, class Index, class Done>
+__device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, const float* __restrict__ bad,
+                                           const gbrt_ray* __restrict__ rays, uint32_t n, uint32_t next,
+                                           const uint32_t end, uint32_t* __restrict__ status, Root root, Index index,
+                                           Done done)
 {
     constexpr int kDeep = INT32_MAX;   // best_tri of a ray that the pair loop answers
     const uint32_t full = 0xFFFFFFFFu, none = 0xFFFFFFFFu;
@@ -247,7 +250,7 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
                     {
                         local_stack<kStackSize> stack;
                         res = traverse_bvh_with<AnyHit, decltype(stack), NearFirst>(
-                            stack, v.nodes, v.tris, v.root, v.num_inner, v.num_tris, o, d, tmin, tmax, status);
+                            stack, v.nodes, v.tris, root(ray), v.num_inner, v.num_tris, o, d, tmin, tmax, status);
                     }
                     done(ray, res);
                     ray = none;
@@ -271,8 +274,8 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
                         best_t = second_t = FLT_MAX;
                         top = col;
                         asm volatile("st.shared.b32 [%0], %1;" ::"r"(top), "r"(kEmptyLink) : "memory");
-                        const bool ok = quad_ray_ok(o, d);
-                        node = ok ? v.root : kEmptyLink;
+                        const bool ok = quad_ray_ok(o, d) && !(bad && *bad != 0.0f);
+                        node = ok ? root(ray) : kEmptyLink;
                         best_tri = ok ? -1 : kDeep;
                     }
                     else

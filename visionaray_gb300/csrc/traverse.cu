@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_vi
     if (first >= n) return;
     const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
     quad_trace<AnyHit, !AnyHit>(
-        stack_mem, v, rays, n, next, end, status, [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
+        stack_mem, v, nullptr, rays, n, next, end, status, [&](uint32_t) { return v.root; },
+        [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
         [&](uint32_t j, trace_result const& h) {
             const uint32_t prim = h.tri >= 0 ? __float_as_uint(ldg4(&v.tris[h.tri].t0).w) : GBRT_NO_HIT;
             reinterpret_cast<uint4*>(hits)[j] =
