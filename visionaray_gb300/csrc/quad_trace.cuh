@@ -53,24 +53,35 @@ constexpr int kQuadMinBlocks = 9;
 constexpr int kQuadRefill = 8;
 constexpr int kQuadLeafLanes = 4;
 
-// Rays per warp for n rays on a GPU that holds `resident` warps of the kernel: few rays
-// are spread over all resident warps (a warp's time is its slowest chain of dependent node
-// loads, and rays of other warps do not lengthen it: 1,023 rays over a 4,099-triangle
-// soup take 31 us one per warp, 47 us eight per warp); many rays go in about three waves
-// of spans of up to 256, which the block scheduler balances.
+// Rays per warp for n rays on a GPU that holds `resident` warps of the kernel (5,472 on 152
+// SMs).  As many warps as rays while they fit: a warp's time is its slowest chain of
+// dependent node loads, and rays of other warps do not lengthen it (4,096 camera rays over
+// 65,536 triangles 65 us one per warp, 87 us four per warp).  Beyond that, lanes that
+// advance together pay more than warps (16,384 rays: 88 us sixteen per warp, 100 three per
+// warp; 65,536: 104 us 32 per warp, 132 twelve): about 3/4 of the resident warps, at least
+// half to fully occupied ones.  Long queries go in up to 2 1/4 waves of spans of 128 to
+// 256, which the block scheduler balances (1,048,576 secondary rays: 637 us at 128, 684 at
+// 64, 687 at 256; 4.2 M: 2.60 ms at 128, 2.49 at 256).
 __host__ __device__ __forceinline__ uint32_t quad_span(uint32_t n, uint32_t resident)
 {
-    const uint32_t one = (n + resident - 1) / resident;
-    if (one <= 8) return one > 0 ? one : 1;
-    const uint32_t three = (n + 3 * resident - 1) / (3 * resident);
-    return three < 8 ? 8 : (three > 256 ? 256 : three);
+    if (n <= resident) return 1;
+    const uint32_t full = resident * 3 / 4, sparse = resident * 3 / 16, waves = resident * 9 / 4;
+    const uint32_t one = (n + full - 1) / full;
+    if (one <= 128)
+    {
+        const uint32_t lanes = (n + sparse - 1) / sparse;
+        const uint32_t least = lanes < 32 ? lanes : 32;
+        return one > least ? one : least;
+    }
+    const uint32_t many = (n + waves - 1) / waves;
+    return many < 128 ? 128 : (many > 256 ? 256 : many);
 }
 
 // The most warps that any ray count up to n takes at quad_span of that count.
 __host__ __forceinline__ uint32_t quad_max_warps(uint32_t n, uint32_t resident)
 {
-    const uint64_t waves = uint64_t(n) / 256 + 1;
-    const uint64_t cap = waves > 3ull * resident ? waves : 3ull * resident;
+    const uint64_t long_spans = uint64_t(n) / 256 + 1, waves = uint64_t(resident) * 9 / 4 + 1;
+    const uint64_t cap = long_spans > waves ? long_spans : waves;
     return uint32_t(n < cap ? n : cap);
 }
 
