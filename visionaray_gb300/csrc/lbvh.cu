@@ -76,6 +76,27 @@ __global__ void __launch_bounds__(kBlock) centroid_bounds(gbrt_triangle const* _
     }
 }
 
+// The Morton code of a centroid in the centroid bounds: centroid -= center; centroid =
+// (centroid + size * 0.5) / size; centroid = min(max(centroid * 1024, 0), 1023)
+// (lbvh.h:253-267).
+__device__ __forceinline__ uint32_t morton_code(f3 centroid, box3 const& cb)
+{
+    const f3 center = box_center(cb);
+    const float c[3] = { centroid.x, centroid.y, centroid.z }, cc[3] = { center.x, center.y, center.z };
+    const float cs[3] = { __fsub_rn(cb.hi.x, cb.lo.x), __fsub_rn(cb.hi.y, cb.lo.y), __fsub_rn(cb.hi.z, cb.lo.z) };
+    uint32_t q[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        float v = __fsub_rn(c[a], cc[a]);
+        v = __fdiv_rn(__fadd_rn(v, __fmul_rn(cs[a], 0.5f)), cs[a]);
+        v = __fmul_rn(v, 1024.0f);
+        v = ref_min(ref_max(v, 0.0f), 1023.0f);
+        q[a] = static_cast<uint32_t>(v);
+    }
+    return morton3(q[0], q[1], q[2]);
+}
+
 __global__ void __launch_bounds__(kBlock) morton_codes(const float4* __restrict__ centroids, uint32_t n,
                                                        const int* __restrict__ cb_ordered,
                                                        uint32_t* __restrict__ keys,
@@ -88,25 +109,8 @@ __global__ void __launch_bounds__(kBlock) morton_codes(const float4* __restrict_
     box3 cb;
     cb.lo = { ordered_to_float(cb_ordered[0]), ordered_to_float(cb_ordered[1]), ordered_to_float(cb_ordered[2]) };
     cb.hi = { ordered_to_float(cb_ordered[3]), ordered_to_float(cb_ordered[4]), ordered_to_float(cb_ordered[5]) };
-    f3 center = box_center(cb);
-    f3 size = { __fsub_rn(cb.hi.x, cb.lo.x), __fsub_rn(cb.hi.y, cb.lo.y), __fsub_rn(cb.hi.z, cb.lo.z) };
-    float4 c4 = centroids[i];
-    float c[3] = { c4.x, c4.y, c4.z };
-    float cc[3] = { center.x, center.y, center.z };
-    float cs[3] = { size.x, size.y, size.z };
-    uint32_t q[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-        // centroid -= center; centroid = (centroid + size * 0.5) / size;
-        // centroid = min(max(centroid * 1024, 0), 1023)       (lbvh.h:256-263)
-        float v = __fsub_rn(c[a], cc[a]);
-        v = __fdiv_rn(__fadd_rn(v, __fmul_rn(cs[a], 0.5f)), cs[a]);
-        v = __fmul_rn(v, 1024.0f);
-        v = ref_min(ref_max(v, 0.0f), 1023.0f);
-        q[a] = static_cast<uint32_t>(v);
-    }
-    keys[i] = morton3(q[0], q[1], q[2]);
+    const float4 c = centroids[i];
+    keys[i] = morton_code({ c.x, c.y, c.z }, cb);
     values[i] = i;
 }
 
@@ -161,6 +165,171 @@ __global__ void __launch_bounds__(kBlock) refit_and_emit(gbrt_triangle const* __
         link = up;
     }
     atomicOr(status, kStatusBadIndex);
+}
+
+// The Morton order of up to kSmallOrder triangles in one block: centroid bounds, codes and
+// the stable sort (four 8-bit passes in shared memory), Items triangles per thread.  At
+// these sizes the separate kernels are bound by their eleven launches, this one by its
+// barriers and one SM's issue.  Rebuilds, separate kernels -> this: 300 triangles 84 -> 34
+// us, 1,024 106 -> 56, 4,096 122 -> 85, 8,192 134 -> 110; 16 triangles per thread would not
+// fit its 64 registers, and the difference shrinks.  Also clears flags (may be null), the root height word (to 1) and
+// the quads' validity word (may be null).
+constexpr uint32_t kSmallOrder = 8192;
+constexpr int kSmallThreads = 1024, kSmallWarps = kSmallThreads / 32;
+constexpr size_t small_order_bytes(int items) { return size_t(2 * items * kSmallThreads + kSmallWarps * 256) * 4; }
+
+template <int Items>
+__global__ void __launch_bounds__(kSmallThreads) small_order(gbrt_triangle const* __restrict__ tris, uint32_t n,
+                                                             uint32_t* __restrict__ codes, uint32_t* __restrict__ ids,
+                                                             uint32_t* __restrict__ flags,
+                                                             uint32_t* __restrict__ root_height,
+                                                             float* __restrict__ quads_bad)
+{
+    extern __shared__ uint32_t small_mem[];
+    uint32_t* skeys = small_mem;
+    uint32_t* svals = skeys + Items * kSmallThreads;
+    uint32_t* hist = svals + Items * kSmallThreads;   // [warp][digit]
+    __shared__ float red[kSmallWarps][6];
+    __shared__ uint32_t digit_base[256];
+    __shared__ uint32_t ws[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t lanes_below = (1u << lane) - 1u;
+    if (tid == 0)
+    {
+        if (root_height) *root_height = 1;
+        if (quads_bad) *quads_bad = 0.0f;
+    }
+    // item k of a lane is triangle warp * 32 Items + 32 k + lane: a warp holds consecutive ones
+    auto item = [&](int k) { return uint32_t(warp * 32 * Items + 32 * k + lane); };
+    float c[Items][3];
+    float mn[3] = { FLT_MAX, FLT_MAX, FLT_MAX }, mx[3] = { -FLT_MAX, -FLT_MAX, -FLT_MAX };
+#pragma unroll
+    for (int k = 0; k < Items; ++k)
+    {
+        const uint32_t i = item(k);
+        if (i >= n) continue;
+        if (flags) flags[i] = 0;
+        const f3 x = box_center(tri_box(load_tri(tris, i)));
+        c[k][0] = x.x, c[k][1] = x.y, c[k][2] = x.z;
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+        {
+            mn[a] = ref_min(mn[a], cas_lo(c[k][a]));
+            mx[a] = ref_max(mx[a], cas_hi(c[k][a]));
+        }
+    }
+    for (int a = 0; a < 3; ++a)
+    {
+        mn[a] = warp_min(mn[a]);
+        mx[a] = warp_max(mx[a]);
+        if (lane == 0)
+        {
+            red[warp][a] = mn[a];
+            red[warp][3 + a] = mx[a];
+        }
+    }
+    __syncthreads();
+    box3 cb;
+    {
+        float b[6];
+        for (int a = 0; a < 6; ++a)
+        {
+            const float v = red[lane][a];   // kSmallWarps == 32
+            b[a] = a < 3 ? warp_min(v) : warp_max(v);
+        }
+        cb = { { b[0], b[1], b[2] }, { b[3], b[4], b[5] } };
+    }
+    uint32_t key[Items], val[Items];
+#pragma unroll
+    for (int k = 0; k < Items; ++k)
+    {
+        // past the end: a key above every 30-bit code, so it stays behind them
+        key[k] = item(k) < n ? morton_code({ c[k][0], c[k][1], c[k][2] }, cb) : 0xFFFFFFFFu;
+        val[k] = item(k);
+    }
+    for (int shift = 0; shift < 32; shift += 8)
+    {
+        for (int j = tid; j < kSmallWarps * 256; j += kSmallThreads) hist[j] = 0;
+        __syncthreads();
+        uint32_t rank[Items];
+        uint32_t* mine = hist + warp * 256;
+#pragma unroll
+        for (int k = 0; k < Items; ++k)
+        {
+            const uint32_t d = (key[k] >> shift) & 255u;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+            const uint32_t before = mine[d];
+            __syncwarp();
+            if ((peers & lanes_below) == 0) mine[d] = before + __popc(peers);
+            __syncwarp();
+            rank[k] = before + __popc(peers & lanes_below);
+        }
+        __syncthreads();
+        uint32_t total = 0, x = 0;
+        if (tid < 256)
+        {
+            for (int w = 0; w < kSmallWarps; ++w)
+            {
+                const uint32_t h = hist[w * 256 + tid];
+                hist[w * 256 + tid] = total;
+                total += h;
+            }
+            x = total;
+            for (int o = 1; o < 32; o <<= 1)
+            {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) ws[warp] = x;
+        }
+        __syncthreads();
+        if (tid < 256)
+        {
+            uint32_t base = 0;
+            for (int w = 0; w < warp; ++w) base += ws[w];
+            digit_base[tid] = base + x - total;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < Items; ++k)
+        {
+            const uint32_t d = (key[k] >> shift) & 255u;
+            const uint32_t pos = digit_base[d] + mine[d] + rank[k];
+            skeys[pos] = key[k];
+            svals[pos] = val[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < Items; ++k)
+        {
+            key[k] = skeys[item(k)];
+            val[k] = svals[item(k)];
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < Items; ++k)
+        if (item(k) < n)
+        {
+            codes[item(k)] = key[k];
+            ids[item(k)] = val[k];
+        }
+}
+
+gbrt_status launch_small_order(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t n, uint32_t* codes,
+                               uint32_t* ids, uint32_t* flags, uint32_t* root_height, float* quads_bad)
+{
+    auto go = [&](auto kernel, int items) -> gbrt_status {
+        const size_t bytes = small_order_bytes(items);
+        GBRT_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+        kernel<<<1, kSmallThreads, bytes, ctx->stream>>>(d_tris, n, codes, ids, flags, root_height, quads_bad);
+        GBRT_LAUNCH_CHECK(ctx, "small_order");
+        return GBRT_OK;
+    };
+    if (n <= 1024) return go(small_order<1>, 1);
+    if (n <= 2048) return go(small_order<2>, 2);
+    if (n <= 4096) return go(small_order<4>, 4);
+    return go(small_order<8>, 8);
 }
 
 // bvh_compressed_node<4>::init (bvh.h:350-393) on the GPU, rounding outward: origin =
@@ -460,16 +629,25 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     uint32_t* node4_counter = level_counts + 255;
     void* wide_tmp = base + off_nodes4;
 
-    init_build_words<<<1, 8, 0, s>>>(cb, bvh->quads ? &bvh->quads[bvh->num_inner].org[0] : nullptr);
-    GBRT_LAUNCH_CHECK(ctx, "init_build_words");
-    uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
-    centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
-    GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
-    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, bvh->sorted_codes, bvh->sorted_ids, flags);
-    GBRT_LAUNCH_CHECK(ctx, "morton_codes");
-    st = radix_sort_pairs(ctx, bvh->sorted_codes, bvh->sorted_ids, keys_alt, vals_alt, n, 30,
-                          base + off_sort);
-    if (st != GBRT_OK) return st;
+    float* quads_bad = bvh->quads ? &bvh->quads[bvh->num_inner].org[0] : nullptr;
+    if (n <= kSmallOrder)
+    {
+        st = launch_small_order(ctx, d_tris, n, bvh->sorted_codes, bvh->sorted_ids, flags, root_height, quads_bad);
+        if (st != GBRT_OK) return st;
+    }
+    else
+    {
+        init_build_words<<<1, 8, 0, s>>>(cb, quads_bad);
+        GBRT_LAUNCH_CHECK(ctx, "init_build_words");
+        uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
+        centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, cb);
+        GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
+        morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, cb, bvh->sorted_codes, bvh->sorted_ids, flags);
+        GBRT_LAUNCH_CHECK(ctx, "morton_codes");
+        st = radix_sort_pairs(ctx, bvh->sorted_codes, bvh->sorted_ids, keys_alt, vals_alt, n, 30,
+                              base + off_sort);
+        if (st != GBRT_OK) return st;
+    }
 
     if (n > 1)
     {
@@ -638,6 +816,7 @@ gbrt_status morton_order(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_
                          uint32_t* ids_out)
 {
     if (n == 0) return GBRT_OK;
+    if (n <= kSmallOrder) return launch_small_order(ctx, d_tris, n, codes_out, ids_out, nullptr, nullptr, nullptr);
     cudaStream_t s = ctx->stream;
     size_t off_centroids = 0;
     size_t off_keys_alt = align_up(off_centroids + size_t(n) * 16);
@@ -713,15 +892,24 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
     uint32_t* root_height = reinterpret_cast<uint32_t*>(words + 6);
     cudaStream_t s = ctx->stream;
 
-    init_build_words<<<1, 32, 0, s>>>(words, nullptr);
-    GBRT_LAUNCH_CHECK(ctx, "init_build_words");
-    uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
-    centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, words);
-    GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
-    morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, words, keys, vals, flags);
-    GBRT_LAUNCH_CHECK(ctx, "morton_codes");
-    gbrt_status st = radix_sort_pairs(ctx, keys, vals, keys_alt, vals_alt, n, 30, base + l.sort);
-    if (st != GBRT_OK) return st;
+    gbrt_status st = GBRT_OK;
+    if (n <= kSmallOrder)
+    {
+        st = launch_small_order(ctx, d_tris, n, keys, vals, flags, root_height, nullptr);
+        if (st != GBRT_OK) return st;
+    }
+    else
+    {
+        init_build_words<<<1, 32, 0, s>>>(words, nullptr);
+        GBRT_LAUNCH_CHECK(ctx, "init_build_words");
+        uint32_t grid = std::min<uint32_t>(blocks_for(n), uint32_t(ctx->num_sms) * 8);
+        centroid_bounds<<<grid, kBlock, 0, s>>>(d_tris, n, centroids, words);
+        GBRT_LAUNCH_CHECK(ctx, "centroid_bounds");
+        morton_codes<<<blocks_for(n), kBlock, 0, s>>>(centroids, n, words, keys, vals, flags);
+        GBRT_LAUNCH_CHECK(ctx, "morton_codes");
+        st = radix_sort_pairs(ctx, keys, vals, keys_alt, vals_alt, n, 30, base + l.sort);
+        if (st != GBRT_OK) return st;
+    }
 
     if (n == 1)
     {
