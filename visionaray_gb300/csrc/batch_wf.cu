@@ -93,14 +93,14 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) bp_trace_quads(bat
     const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
     auto index = [](uint32_t k) { return k; };
     if (closest)
-        quad_trace<false, true>(
+        quad_trace<false, true, kQuadPathSteps>(
             stack_mem, v, bad, fb.rays[q], n, next, end, status,
             [&](uint32_t j) { return a.frames[a.scene[fb.path[q][j]]].root; }, index,
             [&](uint32_t j, trace_result const& h) {
                 fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
             });
     else
-        quad_trace<true, true>(
+        quad_trace<true, true, kQuadPathSteps>(
             stack_mem, v, bad, fb.shadow_rays, n, next, end, status,
             [&](uint32_t j) { return a.frames[a.scene[fb.shadow_path[j]]].root; }, index,
             [&](uint32_t j, trace_result const& h) { finish_shadow(fb, j, bounce - 1, h.tri >= 0); });

@@ -99,12 +99,12 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(fra
     auto index = [](uint32_t k) { return k; };
     auto root = [&](uint32_t) { return v.root; };
     if (closest)
-        quad_trace<false, true>(stack_mem, v, nullptr, fb.rays[q], n, next, end, status, root, index,
+        quad_trace<false, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.rays[q], n, next, end, status, root, index,
                                 [&](uint32_t j, trace_result const& h) {
                                     fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
                                 });
     else
-        quad_trace<true, true>(stack_mem, v, nullptr, fb.shadow_rays, n, next, end, status, root, index,
+        quad_trace<true, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.shadow_rays, n, next, end, status, root, index,
                                [&](uint32_t j, trace_result const& h) {
                                    finish_shadow(fb, j, bounce - 1, h.tri >= 0);
                                });

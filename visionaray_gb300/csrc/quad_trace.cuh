@@ -7,11 +7,11 @@
 // kept the load/store pipe 62 % busy (two wavefronts per lane and visit).  Here
 //   - a node visit tests four grandchildren out of one 64-byte record, so a ray takes half
 //     the visits (and half the wavefronts);
-//   - every iteration advances each busy lane by one node (two per vote round) and runs
-//     the leaf tests once enough lanes wait at one, so no lane waits for a whole descent;
+//   - every round runs the leaf tests of the lanes that stand at a leaf, then advances each
+//     busy lane by two or three nodes, so no lane waits for a whole descent;
 //   - a warp owns a span of rays and refills its idle lanes from it.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 2.38 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.66 ms.  What
+// query 3.36 -> 2.27 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.60 ms.  What
 // bounds it now: issue slots (64 %), the ALU pipe (63 %) and the load/store pipe (60 %)
 // about equally.
 //
@@ -40,18 +40,26 @@
 namespace gbrt {
 
 // Threads of a block and shared stack entries per thread of every kernel that runs
-// quad_trace: 24 x 128 x 4 B = 12 KB per block.  A visit pushes up to three entries; 16
-// entries sent 125 of the 4.2 M heightfield rays to the pair loop, 24 none.
+// quad_trace: 32 x 128 x 4 B = 16 KB per block.  A visit pushes up to three entries; 16
+// entries sent 125 of the 4.2 M heightfield rays to the pair loop, 24 none, but a path
+// tracer's long tails wait for such rays (high-definition frame 60.2 ms at 20 entries, 49.7
+// at 24, 49.0 at 32).
 constexpr int kQuadBlock = 128;
-constexpr int kQuadStack = 24;
+constexpr int kQuadStack = 32;
 // Resident blocks the register allocation must allow: 9 (36 warps, 56 registers, no
-// spills).  Heightfield closest hit 2.38 ms; 2.43 at 10 blocks (48 registers, spilling),
-// 2.61 at 12, 2.75 at 8 without the second node step per round.
+// spills).  With two steps per round, heightfield closest hit 2.38 ms; 2.43 at 10 blocks
+// (48 registers, spilling), 2.61 at 12.
 constexpr int kQuadMinBlocks = 9;
-// Idle lanes of a warp that trigger a refill, and lanes waiting at a leaf that trigger the
-// leaf tests (or no lane left at a node).
+// Idle lanes of a warp that trigger a refill (6 and 10 within 1 %, 4 and 12 slower).
 constexpr int kQuadRefill = 8;
-constexpr int kQuadLeafLanes = 4;
+// Node steps per round, after the leaf tests of the lanes that stand at one (waiting for
+// several such lanes costs more than it saves: any 48.8 ms per high-definition frame, two
+// 49.0, four 49.7).  Ray queries take three (heightfield closest hit 2.32 -> 2.26 ms, camera
+// rays 354 -> 341 us; four 2.25 ms, but 8.4 M ambient-occlusion rays 2.60 -> 2.63 ms), the
+// path tracer two (three: high-definition frame the same, forward and backward 35.0 -> 36.3
+// ms).
+constexpr int kQuadQuerySteps = 3;
+constexpr int kQuadPathSteps = 2;
 
 // Rays per warp for n rays on a GPU that holds `resident` warps of the kernel (5,472 on 152
 // SMs).  As many warps as rays while they fit: a warp's time is its slowest chain of
@@ -129,7 +137,7 @@ __device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d)
 // stack_mem: kQuadStack * kQuadBlock shared words of the block.  bad: null when the host
 // knows the quads valid, else their validity word (the last record's org[0]): when it is
 // set every ray takes the pair loop.
-template <bool AnyHit, bool NearFirst, class Root, class Index, class Done>
+template <bool AnyHit, bool NearFirst, int Steps, class Root, class Index, class Done>
 __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, const float* __restrict__ bad,
                                            const gbrt_ray* __restrict__ rays, uint32_t n, uint32_t next,
                                            const uint32_t end, uint32_t* __restrict__ status, Root root, Index index,
@@ -230,10 +238,9 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
     for (;;)
     {
         // a link outside both ranges (the end of a walk, or a corrupt one) leaves a lane idle
-        const uint32_t nodes = __ballot_sync(full, uint32_t(node) < uint32_t(v.num_inner));
         const bool leaf = uint32_t(~node) < uint32_t(v.num_tris);
         const uint32_t leaves = __ballot_sync(full, leaf);
-        const uint32_t busy = nodes | leaves;
+        const uint32_t busy = __ballot_sync(full, leaf || uint32_t(node) < uint32_t(v.num_inner));
         if (busy == 0 || (next < end && 32 - __popc(busy) >= kQuadRefill))
         {
             if (!(busy & lane_bit))
@@ -301,17 +308,23 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
             if (last) break;
             continue;
         }
-        if (leaves != 0 && (nodes == 0 || __popc(leaves) >= kQuadLeafLanes))
+        if (leaves != 0)
         {
             if (leaf)
             {
                 const int t = ~node;
                 const tri48* tp = v.tris + t;
-                const float4 t0 = ldg4(&tp->t0), t1 = ldg4(&tp->t1), t2 = ldg4(&tp->t2);
+                // the record's aligned 32 bytes and the other 16: two loads per lane, not three
+                const bool odd = reinterpret_cast<uintptr_t>(tp) & 16;
+                float w[8];
+                ld8(reinterpret_cast<const char*>(tp) + (odd ? 16 : 0), w);
+                const float4 x4 = ldg4(reinterpret_cast<const float4*>(tp) + (odd ? 0 : 2));
+                const f3 t0 = { odd ? x4.x : w[0], odd ? x4.y : w[1], odd ? x4.z : w[2] };
+                const f3 t1 = { odd ? w[0] : w[4], odd ? w[1] : w[5], odd ? w[2] : w[6] };
+                const f3 t2 = { odd ? w[4] : x4.x, odd ? w[5] : x4.y, odd ? w[6] : x4.z };
                 asm volatile("ld.shared.b32 %0, [%1];" : "=r"(node) : "r"(top) : "memory");
                 top -= 4u * kQuadBlock;
-                const tri_hit h = intersect_triangle(o, d, { t0.x, t0.y, t0.z }, { t1.x, t1.y, t1.z },
-                                                     { t2.x, t2.y, t2.z });
+                const tri_hit h = intersect_triangle(o, d, t0, t1, t2);
                 if (h.hit && h.t >= tmin && h.t <= tmax)
                 {
                     if (AnyHit)
@@ -331,10 +344,12 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
             }
             __syncwarp();
         }
-        if (uint32_t(node) < uint32_t(v.num_inner)) step();
-        __syncwarp();
-        if (uint32_t(node) < uint32_t(v.num_inner)) step();
-        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < Steps; ++k)
+        {
+            if (uint32_t(node) < uint32_t(v.num_inner)) step();
+            __syncwarp();
+        }
     }
 }
 

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_vi
     const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
     if (first >= n) return;
     const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
-    quad_trace<AnyHit, !AnyHit>(
+    quad_trace<AnyHit, !AnyHit, kQuadQuerySteps>(
         stack_mem, v, nullptr, rays, n, next, end, status, [&](uint32_t) { return v.root; },
         [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
         [&](uint32_t j, trace_result const& h) {
