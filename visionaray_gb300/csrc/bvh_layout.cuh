@@ -44,10 +44,10 @@ static_assert(sizeof(tri48) == 48, "triangle is 48 bytes");
 constexpr uint32_t kLastInLeaf = 1u;
 constexpr int kStackSize = 64;   // traversal stack entries (tree height must stay below)
 
-// Quad node (64 bytes = two 256-bit loads): the up to four grandchildren of one node
-// pair, their boxes quantised outward to 8 bits per plane.  Record i of the quad array
-// belongs to node pair i: slots 0 and 1 are the children of the pair's child 0, slots 2
-// and 3 those of child 1; a child that is a leaf takes both slots of its half, the second
+// Quad node (64 bytes = two 256-bit loads): up to four descendants of one node pair, their
+// boxes quantised outward to 8 bits per plane.  Record i of the quad array belongs to node
+// pair i: its two children, of which inner ones are replaced in place by their own two
+// children until four slots are full (quads.cu); an empty slot repeats the link before it
 // with an empty box (low planes 255, high planes 0).  So a depth-first walk of the quads
 // in slot order meets the leaves in the order of a walk of the pairs.  A plane q of axis a
 // stands at org[a] + q * cell[a]; scale holds 2^15 * cell, which is what the decoded

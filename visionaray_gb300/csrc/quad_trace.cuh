@@ -5,13 +5,13 @@
 // with 7.9 of 32 lanes active, since lanes that reach a leaf wait for the lanes still
 // descending and ended rays wait for the warp's longest one, and its 64-byte node fetches
 // kept the load/store pipe 62 % busy (two wavefronts per lane and visit).  Here
-//   - a node visit tests four grandchildren out of one 64-byte record, so a ray takes half
+//   - a node visit tests four descendants out of one 64-byte record, so a ray takes half
 //     the visits (and half the wavefronts);
 //   - every round runs the leaf tests of the lanes that stand at a leaf, then advances each
 //     busy lane by two or three nodes, so no lane waits for a whole descent;
 //   - a warp owns a span of rays and refills its idle lanes from it.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 2.27 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.60 ms.  What
+// query 3.36 -> 2.18 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.51 ms.  What
 // bounds it now: issue slots (64 %), the ALU pipe (63 %) and the load/store pipe (60 %)
 // about equally.
 //
@@ -192,8 +192,8 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
         // Selection, pushes and pop as predicated PTX: as C++ they became branches that
         // split the warp (401 -> 361 instructions per ray).  Only the nearest child is
         // chosen; the others keep slot order (sorting them saves 1 % of the visits).  A
-        // child equal to the chosen one (the empty slot of a leaf's half, if its inverted
-        // box passes) is not pushed.
+        // child equal to the chosen one (an empty slot repeats the last link, if its
+        // inverted box passes) is not pushed.
         if constexpr (NearFirst)
             asm volatile(
                 "{\n\t.reg .pred h0,h1,h2,h3,p,q;\n\t.reg .f32 t0,t1,t2,t3,ta,tb;\n\t.reg .b32 la,lb;\n\t"

@@ -1,13 +1,19 @@
-// Quad nodes: two levels of the node pairs in one 64-byte record with outward quantised
-// boxes (layout in bvh_layout.cuh), made from a finished tree in one pass.  The ray
-// queries and the path tracer traverse them (quad_trace.cuh).
+// Quad nodes: up to four descendants of a node pair in one 64-byte record with outward
+// quantised boxes (layout in bvh_layout.cuh), made from a finished tree in one pass.  The
+// ray queries and the path tracer traverse them (quad_trace.cuh).
 //
-// One thread per node pair reads its own record and its two inner children's and writes
-// one record: no queue, no compaction, no level-by-level launches, and a quad has its
-// node pair's index, so the pairs' links serve unchanged.  Every pair gets a quad although
-// a walk from the root meets every second level only: which levels those are is not known
-// bottom-up, and the pass is bound by HBM traffic either way (64 B read and 64 B written
-// per pair).
+// One thread per node pair starts from its two children and twice opens the inner one of
+// the largest box area, in place, so the slots stay in depth-first order (which any-hit
+// queries depend on).  A quad is then full wherever its subtree has four leaves, and the
+// boxes most likely to be hit are the ones replaced.  Against opening both children
+// always: sorted secondary rays over a 2048^2 heightfield 2.27 -> 2.18 ms, ambient
+// occlusion 2.61 -> 2.51, preview frame 237 -> 217 us, high-definition frame 48.2 -> 46.8
+// ms, at the same build time.
+//
+// No queue, no compaction, no level-by-level launches, and a quad has its node pair's
+// index, so the pairs' links serve unchanged.  Every pair gets a quad although a walk from
+// the root meets fewer: which ones those are is not known bottom-up, and the pass is bound
+// by HBM traffic either way (64 B read and 64 B written per pair).
 
 #include "api_internal.h"
 #include "device_math.cuh"
@@ -21,6 +27,33 @@ constexpr int kBlock = 256;
 // keep the node pairs.
 constexpr float kQuadMaxCoord = 1.152921504606847e18f;   // 2^60
 
+struct slot
+{
+    float lo[3], hi[3];
+    int link;
+};
+
+__device__ __forceinline__ slot child(bvh2_node const& p, int s)
+{
+    return s ? slot{ { p.xy1.x, p.xy1.z, p.z01.z }, { p.xy1.y, p.xy1.w, p.z01.w }, p.link.y }
+             : slot{ { p.xy0.x, p.xy0.z, p.z01.x }, { p.xy0.y, p.xy0.w, p.z01.y }, p.link.x };
+}
+
+__device__ __forceinline__ slot pick(bool first, slot const& a, slot const& b)
+{
+    return { { first ? a.lo[0] : b.lo[0], first ? a.lo[1] : b.lo[1], first ? a.lo[2] : b.lo[2] },
+             { first ? a.hi[0] : b.hi[0], first ? a.hi[1] : b.hi[1], first ? a.hi[2] : b.hi[2] },
+             first ? a.link : b.link };
+}
+
+// Half the surface of an inner slot's box (at most FLT_MAX, 0 for a NaN), -1 for a leaf.
+__device__ __forceinline__ float open_area(slot const& s, uint32_t num_inner)
+{
+    const float x = s.hi[0] - s.lo[0], y = s.hi[1] - s.lo[1], z = s.hi[2] - s.lo[2];
+    const float area = x * y + y * z + z * x;
+    return uint32_t(s.link) < num_inner ? fminf(fmaxf(area, 0.0f), FLT_MAX) : -1.0f;
+}
+
 __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __restrict__ nodes, uint32_t num_inner,
                                                           quad_node* __restrict__ quads,
                                                           uint32_t* __restrict__ host_bad)
@@ -28,34 +61,38 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= num_inner) return;
     const bvh2_node p = nodes[i];
-    float lo[3][4], hi[3][4];
-    int link[4];
-    uint32_t empty = 0;
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
+    // named values: an array indexed by the choice goes to local memory (0.28 -> 0.70 ms for
+    // 8.4 M triangles)
+    slot s0 = child(p, 0), s1 = child(p, 1), s2 = s1, s3;
+    const float blo[3] = { fminf(s0.lo[0], s1.lo[0]), fminf(s0.lo[1], s1.lo[1]), fminf(s0.lo[2], s1.lo[2]) };
+    const float bhi[3] = { fmaxf(s0.hi[0], s1.hi[0]), fmaxf(s0.hi[1], s1.hi[1]), fmaxf(s0.hi[2], s1.hi[2]) };
+    int count = 2;
+    const float a0 = open_area(s0, num_inner), a1 = open_area(s1, num_inner);
+    if (a0 >= 0.0f || a1 >= 0.0f)
     {
-        const int c = s ? p.link.y : p.link.x;
-        if (c >= 0 && uint32_t(c) < num_inner)
-        {
-            const bvh2_node q = nodes[c];
-            lo[0][2 * s] = q.xy0.x, hi[0][2 * s] = q.xy0.y, lo[1][2 * s] = q.xy0.z, hi[1][2 * s] = q.xy0.w;
-            lo[2][2 * s] = q.z01.x, hi[2][2 * s] = q.z01.y;
-            lo[0][2 * s + 1] = q.xy1.x, hi[0][2 * s + 1] = q.xy1.y, lo[1][2 * s + 1] = q.xy1.z;
-            hi[1][2 * s + 1] = q.xy1.w, lo[2][2 * s + 1] = q.z01.z, hi[2][2 * s + 1] = q.z01.w;
-            link[2 * s] = q.link.x;
-            link[2 * s + 1] = q.link.y;
-        }
-        else
-        {
-            const float4 xy = s ? p.xy1 : p.xy0;
-            lo[0][2 * s] = xy.x, hi[0][2 * s] = xy.y, lo[1][2 * s] = xy.z, hi[1][2 * s] = xy.w;
-            lo[2][2 * s] = s ? p.z01.z : p.z01.x, hi[2][2 * s] = s ? p.z01.w : p.z01.y;
-            link[2 * s] = link[2 * s + 1] = c;
-            empty |= 2u << (2 * s);
-        }
+        const bool left = a0 >= a1;
+        const bvh2_node q = nodes[left ? s0.link : s1.link];
+        const slot f = child(q, 0), l = child(q, 1);
+        s2 = pick(left, s1, l);
+        s1 = pick(left, l, f);
+        s0 = pick(left, f, s0);
+        count = 3;
     }
-    const float blo[3] = { fminf(p.xy0.x, p.xy1.x), fminf(p.xy0.z, p.xy1.z), fminf(p.z01.x, p.z01.z) };
-    const float bhi[3] = { fmaxf(p.xy0.y, p.xy1.y), fmaxf(p.xy0.w, p.xy1.w), fmaxf(p.z01.y, p.z01.w) };
+    s3 = s2;
+    const float b0 = open_area(s0, num_inner), b1 = open_area(s1, num_inner);
+    const float b2 = count == 3 ? open_area(s2, num_inner) : -1.0f;
+    if (b0 >= 0.0f || b1 >= 0.0f || b2 >= 0.0f)
+    {
+        const bool first = b0 >= b1 && b0 >= b2, last = !first && b2 > b1;
+        const bvh2_node q = nodes[first ? s0.link : (last ? s2.link : s1.link)];
+        const slot f = child(q, 0), l = child(q, 1);
+        s3 = pick(last, l, s2);
+        s2 = pick(first, s1, pick(last, f, l));
+        s1 = pick(first, l, pick(last, s1, f));
+        s0 = pick(first, f, s0);
+        count = 4;
+    }
+    const slot c[4] = { s0, s1, s2, s3 };
     uint32_t qlo[3], qhi[3], scale[3];
     float org[3];
     bool fits = true;
@@ -78,13 +115,13 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
         for (int k = 0; k < 4; ++k)
         {
             float l = 255.0f, h = 0.0f;
-            if (!(empty >> k & 1u))
+            if (k < count)
             {
-                l = floorf(__fsub_rd(lo[a][k], org[a]) * inv);
-                h = ceilf(__fsub_ru(hi[a][k], org[a]) * inv);
+                l = floorf(__fsub_rd(c[k].lo[a], org[a]) * inv);
+                h = ceilf(__fsub_ru(c[k].hi[a], org[a]) * inv);
                 // every box of the record is finite and moderate, or the tree is not
                 // traversed through its quads (fminf / fmaxf above would hide a NaN)
-                fits = fits && fabsf(lo[a][k]) <= kQuadMaxCoord && fabsf(hi[a][k]) <= kQuadMaxCoord && l >= 0.0f &&
+                fits = fits && fabsf(c[k].lo[a]) <= kQuadMaxCoord && fabsf(c[k].hi[a]) <= kQuadMaxCoord && l >= 0.0f &&
                        h <= 255.0f;
             }
             qlo[a] |= uint32_t(fminf(fmaxf(l, 0.0f), 255.0f)) << (8 * k);
@@ -93,7 +130,7 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
     }
     uint4* w = reinterpret_cast<uint4*>(quads + i);
     w[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]), scale[0]);
-    w[1] = make_uint4(link[0], link[1], link[2], link[3]);
+    w[1] = make_uint4(c[0].link, c[1].link, c[2].link, c[3].link);
     w[2] = make_uint4(qlo[0], qhi[0], qlo[1], qhi[1]);
     w[3] = make_uint4(qlo[2], qhi[2], scale[1], scale[2]);
     if (!fits)
