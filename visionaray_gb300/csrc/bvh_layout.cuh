@@ -50,8 +50,8 @@ constexpr int kStackSize = 64;   // traversal stack entries (tree height must st
 // children until four slots are full (quads.cu); an empty slot repeats the link before it
 // with an empty box (low planes 255, high planes 0).  So a depth-first walk of the quads
 // in slot order meets the leaves in the order of a walk of the pairs.  A plane q of axis a
-// stands at org[a] + q * cell[a]; scale holds 2^15 * cell, which is what the decoded
-// plane values 1 + q * 2^-15 are multiplied with (quad_trace.cuh).  link: as a node
+// stands at org[a] + q * cell[a]; scale holds 2^16 * cell, which is what the decoded
+// plane values 1 + q * 2^-16 are multiplied with (quad_trace.cuh).  link: as a node
 // pair's (>= 0 node pair / quad index, < 0 leaf ~triangle).  The array holds one record
 // more than there are node pairs: org[0] of the last one is 0 when every box was finite
 // and within the range the quantisation covers, else 1.

@@ -11,9 +11,9 @@
 //     busy lane by two or three nodes, so no lane waits for a whole descent;
 //   - a warp owns a span of rays and refills its idle lanes from it.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 2.18 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.51 ms.  What
-// bounds it now: issue slots (64 %), the ALU pipe (63 %) and the load/store pipe (60 %)
-// about equally.
+// query 3.36 -> 2.10 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.31 ms.  What
+// bounds it now (a bounce of a 1920 x 1080 path-traced frame): the load/store pipe's
+// wavefronts (80 %), two per lane and node, then issue slots (72 %).
 //
 // The answers are the node-pair loop's, bit for bit, although the visits differ:
 //   - Boxes only get larger (quantised outward, and the distances below carry a margin
@@ -47,17 +47,15 @@ namespace gbrt {
 constexpr int kQuadBlock = 128;
 constexpr int kQuadStack = 32;
 // Resident blocks the register allocation must allow: 9 (36 warps, 56 registers, no
-// spills).  With two steps per round, heightfield closest hit 2.38 ms; 2.43 at 10 blocks
-// (48 registers, spilling), 2.61 at 12.
+// spills).  Heightfield closest hit 2.10 ms; 2.18 at 10 blocks (48 registers, spilling).
 constexpr int kQuadMinBlocks = 9;
 // Idle lanes of a warp that trigger a refill (6 and 10 within 1 %, 4 and 12 slower).
 constexpr int kQuadRefill = 8;
 // Node steps per round, after the leaf tests of the lanes that stand at one (waiting for
-// several such lanes costs more than it saves: any 48.8 ms per high-definition frame, two
-// 49.0, four 49.7).  Ray queries take three (heightfield closest hit 2.32 -> 2.26 ms, camera
-// rays 354 -> 341 us; four 2.25 ms, but 8.4 M ambient-occlusion rays 2.60 -> 2.63 ms), the
-// path tracer two (three: high-definition frame the same, forward and backward 35.0 -> 36.3
-// ms).
+// several such lanes costs more than it saves: any 44.4 ms per high-definition frame, two
+// 44.6, three 44.9).  Ray queries take three (heightfield closest hit 2.15 ms at two, 2.10 at
+// three, 2.09 at four; 8.4 M ambient-occlusion rays 2.35, 2.31, 2.33), the path tracer two
+// (three: high-definition frame 44.4 -> 44.1 ms, forward and backward 32.3 -> 33.0).
 constexpr int kQuadQuerySteps = 3;
 constexpr int kQuadPathSteps = 2;
 
@@ -160,8 +158,8 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
         float a[8], b[8];
         ld8(v.quads + node, a);
         ld8(reinterpret_cast<const char*>(v.quads + node) + 32, b);
-        // the distance to plane value f = 1 + q 2^-15 of an axis is f * S + O with S =
-        // 2^15 cell / d and O = (org - o) / d - S; the margin 2^-21 (|org - o| / |d| + |S|)
+        // the distance to plane value f = 1 + q 2^-16 of an axis is f * S + O with S =
+        // 2^16 cell / d and O = (org - o) / d - S; the margin 2^-21 (|org - o| / |d| + |S|)
         // is more than the roundings here and those of the pair loop's test together
         const float k21 = 4.76837158203125e-07f;
         const float Sx = a[3] * id.x, Sy = b[6] * id.y, Sz = b[7] * id.z;
@@ -180,9 +178,12 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
 #pragma unroll
         for (int k = 0; k < 4; ++k)
         {
-            // byte k of the planes into bits 8..15 of 1.0f: the float 1 + q 2^-15
-            const uint32_t sel = 0x7604u | (k << 4);
-            auto plane = [&](uint32_t q) { return __uint_as_float(__byte_perm(q, 0x3F800000u, sel)); };
+            // byte k of the planes into bits 7..14 of 1.0f: the float 1 + q 2^-16.  The
+            // dot product runs on the FMA pipe; a byte permute, as the rest of the visit
+            // (selects, minima, compares), on the ALU pipe, which was the narrowest one (camera
+            // rays 337 -> 306 us, ambient occlusion 2.51 -> 2.30 ms, high-definition frame
+            // 47.1 -> 44.3).
+            auto plane = [&](uint32_t q) { return __uint_as_float(__dp4a(q, 0x80u << (8 * k), 0x3F800000u)); };
             const float nx = __fmaf_rn(plane(nx4), Sx, nxo), fx = __fmaf_rn(plane(fx4), Sx, fxo);
             const float ny = __fmaf_rn(plane(ny4), Sy, nyo), fy = __fmaf_rn(plane(fy4), Sy, fyo);
             const float nz = __fmaf_rn(plane(nz4), Sz, nzo), fz = __fmaf_rn(plane(fz4), Sz, fzo);

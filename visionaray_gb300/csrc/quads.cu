@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
         const int e = int((__float_as_uint(t) + 0x7FFFFFu) >> 23) - 127;
         const float cell = __int_as_float((e + 127) << 23);
         const float inv = __int_as_float((127 - e) << 23);   // exact
-        scale[a] = uint32_t(e + 127 + 15) << 23;
+        scale[a] = uint32_t(e + 127 + 16) << 23;
         org[a] = __fsub_rd(blo[a], cell);
         qlo[a] = qhi[a] = 0;
 #pragma unroll
