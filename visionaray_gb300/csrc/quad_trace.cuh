@@ -259,7 +259,9 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
                         float tn;
                         const bool in_box = leaf_box_hit(o, { safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z) }, tmin, tmax,
                                                          v1, e1, e2, tn);
-                        exact = !in_box || (!AnyHit && second_t <= fmaxf(best_t, tn));
+                        // a box entered beyond the culling distance (a sliver's t is far off)
+                        // may have hidden such a second hit
+                        exact = !in_box || (!AnyHit && (tn > limit || second_t <= fmaxf(best_t, tn)));
                         // u and v by the same test on the same inputs: the same values
                         const tri_hit h = intersect_triangle(o, d, v1, e1, e2);
                         res.u = h.u;
