@@ -1,4 +1,4 @@
-"""The Morton order of a build at the edges of its sizes: one block holds up to 8,192
+"""The Morton order of a build, alone and in a batch, at the edges of its sizes: one block holds up to 8,192
 triangles (1, 2, 4 or 8 per thread), and the radix sort scans its digit table inside the
 scatter for up to 256 tiles of 4,096 keys.  Codes and trees equal the oracle's, which sorts
 with std::stable_sort; equal codes keep their input order, and triangles that are not
@@ -55,3 +55,21 @@ def test_triangles_that_are_not_finite(oracle, n):
     tris["v1"][n - 1] = (0, 0, np.nan)
     bvh = vg.lbvh_builder().build(vg.as_device_bytes(tris))
     assert np.array_equal(bvh.morton_codes(), oracle.morton_codes(tris))
+
+
+@pytest.mark.parametrize("sizes", [[256, 256], [31, 1, 224, 1, 255], [255, 0, 2, 512, 33], [1] * 70, [8192, 3, 300]])
+def test_batches_across_runs_of_triangles(oracle, sizes):
+    # a warp folds the centroid bounds of 256 triangles, 32 at a time
+    parts = [make(n, "soup") for n in sizes]
+    for k, p in enumerate(parts):
+        p["v1"] += np.float32(k)
+    batch = vg.Batch(np.concatenate([[0], np.cumsum(sizes)]))
+    batch.build(vg.as_device_bytes(np.concatenate(parts)))
+    for s, tris in enumerate(parts):
+        if not len(tris):
+            continue
+        nodes, _ = batch.export_bvh2(s)
+        want = oracle.build_karras(tris)
+        assert np.array_equal(nodes["first"], want.nodes["first"])
+        assert (nodes["bbox_min"] == want.nodes["bbox_min"]).all()
+        assert (nodes["bbox_max"] == want.nodes["bbox_max"]).all()

@@ -4,9 +4,8 @@
 // 226-246); hundreds of small scenes then cost hundreds of launches, allocations and
 // synchronisations each.  Here all scenes' triangles are one array and every stage is
 // one launch over all of them:
-//   batch_centroids : per-triangle bounds and centroid, per-scene centroid bounds (lanes
-//                     of one scene reduced in the warp, one set of atomics per scene
-//                     and warp)
+//   batch_centroids : per-triangle centroid, per-scene centroid bounds (reduced over runs
+//                     of a warp's triangles in one scene, one set of atomics per run)
 //   batch_morton    : each scene's codes against its own bounds -- the codes a single-
 //                     scene build computes
 //   two stable radix sorts: by code, then by scene, giving (scene, code, index) order,
@@ -36,45 +35,87 @@ __global__ void __launch_bounds__(kBlock) batch_init_bounds(int* __restrict__ bo
     bounds[i] = (i % 6) < 3 ? float_to_ordered(FLT_MAX) : float_to_ordered(-FLT_MAX);
 }
 
+// A warp takes kCentroidRun consecutive triangles.  While they lie in one scene, as all but
+// a few do, each lane folds its own and the warp reduces once per run; only the 32 triangles
+// across a boundary go lane group by lane group.  Bound by HBM traffic (48 B read, 20 B
+// written per triangle); with a search and a shuffle loop per triangle, and atomics for
+// every 32 of them, 9.6 M triangles of 64 scenes took 1.11 ms, now 0.17.
+constexpr uint32_t kCentroidRun = 256;
+
 __global__ void __launch_bounds__(kBlock) batch_centroids(gbrt_triangle const* __restrict__ tris, uint32_t total,
                                                           const uint32_t* __restrict__ offsets, uint32_t num_scenes,
                                                           float4* __restrict__ centroids,
                                                           uint32_t* __restrict__ prim_scene, int* __restrict__ bounds)
 {
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    bool active = i < total;
-    uint32_t s = 0;
-    f3 c = { 0.0f, 0.0f, 0.0f };
-    if (active)
-    {
-        s = upper_segment(offsets, num_scenes, i);
-        c = box_center(tri_box(load_tri(tris, i)));
-        centroids[i] = make_float4(c.x, c.y, c.z, 0.0f);
-        prim_scene[i] = s;
-    }
-    uint32_t mask = __ballot_sync(0xFFFFFFFFu, active);
-    if (!active) return;
-    uint32_t peers = __match_any_sync(mask, s);
-    // the reference's atomic fold (lbvh.h:233-238) skips NaN and outward infinities
-    float mn[3] = { cas_lo(c.x), cas_lo(c.y), cas_lo(c.z) }, mx[3] = { cas_hi(c.x), cas_hi(c.y), cas_hi(c.z) };
-    for (uint32_t m = peers; m; m &= m - 1)
-    {
-        int src = __ffs(m) - 1;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t first = (uint64_t(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5)) * kCentroidRun;
+    if (first >= total) return;
+    const uint32_t last = uint32_t(first + kCentroidRun < total ? first + kCentroidRun : total);
+    // this lane's minima and maxima, as ordered integers
+    int mn[3], mx[3];
+    auto clear = [&]() {
         for (int a = 0; a < 3; ++a)
         {
-            float v = __shfl_sync(peers, a == 0 ? c.x : (a == 1 ? c.y : c.z), src);
-            mn[a] = ref_min(mn[a], cas_lo(v));
-            mx[a] = ref_max(mx[a], cas_hi(v));
+            mn[a] = float_to_ordered(FLT_MAX);
+            mx[a] = float_to_ordered(-FLT_MAX);
         }
-    }
-    if ((threadIdx.x & 31) == __ffs(peers) - 1)
-    {
+    };
+    auto reduce = [&](uint32_t lanes, uint32_t s) {
+        const uint32_t rank = __popc(lanes & ((1u << lane) - 1u));
         for (int a = 0; a < 3; ++a)
         {
-            atomicMin(&bounds[6 * s + a], float_to_ordered(mn[a]));
-            atomicMax(&bounds[6 * s + 3 + a], float_to_ordered(mx[a]));
+            const int l = __reduce_min_sync(lanes, mn[a]), h = __reduce_max_sync(lanes, mx[a]);
+            if (rank == 0)
+            {
+                atomicMin(&bounds[6 * s + a], l);
+                atomicMax(&bounds[6 * s + 3 + a], h);
+            }
         }
+        clear();
+    };
+    uint32_t s = upper_segment(offsets, num_scenes, uint32_t(first));
+    uint32_t end = offsets[s + 1];
+    bool open = false;   // mn and mx hold triangles of scene s
+    clear();
+    for (uint32_t i0 = uint32_t(first); i0 < last; i0 += 32)
+    {
+        const uint32_t i = i0 + lane;
+        const bool active = i < last;
+        const uint32_t lanes = __ballot_sync(0xFFFFFFFFu, active);
+        const uint32_t top = last - i0 < 32 ? last : i0 + 32;
+        uint32_t mine = s;
+        const bool one_scene = top <= end;
+        if (!one_scene)
+        {
+            if (open) reduce(0xFFFFFFFFu, s);
+            open = false;
+            if (active) mine = upper_segment(offsets, num_scenes, i);
+        }
+        if (active)
+        {
+            const f3 c = box_center(tri_box(load_tri(tris, i)));
+            centroids[i] = make_float4(c.x, c.y, c.z, 0.0f);
+            prim_scene[i] = mine;
+            // the reference's atomic fold (lbvh.h:233-238) skips NaN and outward infinities
+            const float v[3] = { c.x, c.y, c.z };
+            for (int a = 0; a < 3; ++a)
+            {
+                mn[a] = min(mn[a], float_to_ordered(cas_lo(v[a])));
+                mx[a] = max(mx[a], float_to_ordered(cas_hi(v[a])));
+            }
+        }
+        if (one_scene)
+        {
+            open = true;
+            continue;
+        }
+        if (active) reduce(__match_any_sync(lanes, mine), mine);
+        __syncwarp();
+        // the next triangles continue the last one's scene or start another
+        s = upper_segment(offsets, num_scenes, top < total ? top : total - 1);
+        end = offsets[s + 1];
     }
+    if (open) reduce(0xFFFFFFFFu, s);
 }
 
 // lbvh.h:253-267 against the triangle's own scene's centroid bounds.
@@ -286,8 +327,9 @@ gbrt_status batch_build(gbrt_context* ctx, gbrt_batch* b, gbrt_triangle const* d
 
     batch_init_bounds<<<blocks_for(uint64_t(b->num_scenes) * 6), kBlock, 0, s>>>(bounds, b->num_scenes);
     GBRT_LAUNCH_CHECK(ctx, "batch_init_bounds");
-    batch_centroids<<<blocks_for(n), kBlock, 0, s>>>(d_tris, n, b->d_offsets, b->num_scenes, centroids, prim_scene,
-                                                      bounds);
+    const uint64_t runs = (uint64_t(n) + kCentroidRun - 1) / kCentroidRun;
+    batch_centroids<<<blocks_for(runs * 32), kBlock, 0, s>>>(d_tris, n, b->d_offsets, b->num_scenes, centroids,
+                                                             prim_scene, bounds);
     GBRT_LAUNCH_CHECK(ctx, "batch_centroids");
     batch_morton<<<blocks_for(n), kBlock, 0, s>>>(centroids, prim_scene, n, bounds, codes_in, b->sorted_codes,
                                                    b->sorted_ids, flags);
