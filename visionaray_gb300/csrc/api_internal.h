@@ -25,6 +25,9 @@ struct build_result
     float lo[3], hi[3];   // the root's box
     uint32_t height;
     uint32_t quads_bad;   // some box is outside what the quad nodes cover
+    // the PLOC build's: clusters left, node pairs made, a step without a merge, the root
+    uint32_t clusters, made, stuck;
+    int32_t root;
 };
 } // namespace gbrt
 

@@ -13,6 +13,12 @@
 // cluster -- the root -- is left.  Node pairs carry both children's boxes, parent links
 // and subtree heights, so refits and every traversal kernel apply unchanged; the leaf
 // triangles are the Morton-ordered tri48 records of the LBVH.
+//
+// An iteration is two launches (ploc_nearest, ploc_merge); how many clusters are left stays
+// on the device, and the host looks at it two iterations late, while the next ones run.
+// The last kTail clusters take more than half of the iterations: one block does them all in
+// shared memory (ploc_tail).  982,802 heightfield triangles: 55 iterations of 5 or 7
+// launches and a synchronisation each took 2.1 ms, bound by the host, now 0.6 ms.
 
 #include "lbvh_device.cuh"
 
@@ -25,21 +31,52 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kRadius = 16;   // neighbours searched on each side
-constexpr int kScanItems = 4; // items per thread of the scan
-constexpr int kScanTile = kBlock * kScanItems;
+
+// Clusters per tile of an iteration.  A ploc_nearest block searches its tile and kRadius
+// positions on each side, so that it knows which of its own pairs are mutual, four adjacent
+// clusters per thread: they share most of their 36 neighbours' boxes, whose reads from
+// shared memory bounded the search (982,802 clusters: one per thread 60.8 us, two 36.7, four
+// 29.4; 10,000 are 2 us faster with two, which does not show beside the launches).
+constexpr int kTile = 608;
+constexpr int kSearch = kTile + 2 * kRadius;
+constexpr int kItems = 4;
+constexpr int kSearchThreads = kSearch / kItems;
+constexpr int kStage = kTile + 4 * kRadius;
+// Tiles per group of the prefix sum: a ploc_merge block adds up the groups before its own
+// and the tiles before it in the group.
+constexpr uint32_t kGroup = 64;
+// Clusters that one block finishes, two per thread while there are more than threads.  Its
+// first iteration is about as long as two launches.
+constexpr int kTail = 2048;
+constexpr int kTailThreads = 1024;
+
+// Where the clustering stands, read by an iteration and written for the next one.
+struct ploc_state
+{
+    uint32_t clusters, nodes;   // left, made
+    uint32_t stuck;             // an iteration merged nothing
+};
+
+// Elements of a staged box array, padded so that lanes four (or two) apart read different
+// banks.
+__host__ __device__ constexpr int padded(int e) { return e + (e >> 3); }
 
 inline uint32_t blocks_for(uint64_t n) { return uint32_t((n + kBlock - 1) / kBlock); }
 inline size_t align_up(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Leaf clusters: the box of the j-th triangle in Morton order (id ~j, height 0), and
-// that triangle's tri48 record.
+// that triangle's tri48 record.  Also starts the state and clears the groups' sums.
 __global__ void __launch_bounds__(kBlock) ploc_leaves(gbrt_triangle const* __restrict__ tris_in,
                                                       const uint32_t* __restrict__ sorted_ids, uint32_t n,
                                                       float4* __restrict__ lo, float4* __restrict__ hi,
-                                                      tri48* __restrict__ tris_out, uint32_t* __restrict__ status)
+                                                      tri48* __restrict__ tris_out, ploc_state* __restrict__ state,
+                                                      unsigned long long* __restrict__ groups, uint32_t num_groups,
+                                                      uint32_t* __restrict__ status)
 {
     uint32_t j = blockIdx.x * kBlock + threadIdx.x;
     if (j >= n) return;
+    if (j == 0) *state = { n, 0, 0 };
+    if (j < num_groups) groups[j] = 0;
     uint32_t id = __ldg(&sorted_ids[j]);
     if (id >= n)
     {
@@ -65,189 +102,388 @@ __device__ __forceinline__ float union_area(float4 alo, float4 ahi, float4 blo, 
     return dx * dy + dy * dz + dz * dx;
 }
 
-// Nearest neighbour of every cluster within kRadius positions (smallest union area, ties
-// to the lower index); the block's clusters and their halo are staged in shared memory.
-__global__ void __launch_bounds__(kBlock) ploc_nearest(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                       uint32_t m, int* __restrict__ nn)
+// The kItems adjacent clusters from stage element e0, each against its neighbours in
+// ascending order (a tie keeps the lower one): the stage elements of the nearest, -1 for none.
+// Elements outside the clusters are boxes from -inf to inf, which are nobody's nearest.
+template <int Items>
+__device__ __forceinline__ void nearest_of(const float4* __restrict__ slo, const float4* __restrict__ shi, int e0,
+                                           int nearest[Items])
 {
-    __shared__ float4 slo[kBlock + 2 * kRadius];
-    __shared__ float4 shi[kBlock + 2 * kRadius];
-    const int64_t b0 = int64_t(blockIdx.x) * kBlock;
-    for (int k = threadIdx.x; k < kBlock + 2 * kRadius; k += kBlock)
+    float4 alo[Items], ahi[Items];
+    float best[Items];
+#pragma unroll
+    for (int r = 0; r < Items; ++r)
     {
-        int64_t g = b0 - kRadius + k;
-        if (g >= 0 && g < int64_t(m))
+        alo[r] = slo[padded(e0 + r)];
+        ahi[r] = shi[padded(e0 + r)];
+        best[r] = FLT_MAX;
+        nearest[r] = -1;
+    }
+    auto against = [&](int r, int e, float4 const& blo, float4 const& bhi) {
+        const float a = union_area(alo[r], ahi[r], blo, bhi);
+        if (a < best[r])
         {
-            slo[k] = lo[g];
-            shi[k] = hi[g];
+            best[r] = a;
+            nearest[r] = e;
         }
+    };
+#pragma unroll
+    for (int k = 0; k < Items - 1; ++k)   // neighbours of the first items only
+    {
+        const int e = e0 - kRadius + k;
+        const float4 blo = slo[padded(e)], bhi = shi[padded(e)];
+#pragma unroll
+        for (int r = 0; r <= k; ++r) against(r, e, blo, bhi);
+    }
+    for (int e = e0 + Items - 1 - kRadius; e < e0; ++e)
+    {
+        const float4 blo = slo[padded(e)], bhi = shi[padded(e)];
+#pragma unroll
+        for (int r = 0; r < Items; ++r) against(r, e, blo, bhi);
+    }
+#pragma unroll
+    for (int k = 0; k < Items; ++k)
+    {
+#pragma unroll
+        for (int r = 0; r < Items; ++r)
+            if (r != k) against(r, e0 + k, alo[k], ahi[k]);
+    }
+    for (int e = e0 + Items; e <= e0 + kRadius; ++e)
+    {
+        const float4 blo = slo[padded(e)], bhi = shi[padded(e)];
+#pragma unroll
+        for (int r = 0; r < Items; ++r) against(r, e, blo, bhi);
+    }
+#pragma unroll
+    for (int k = 1; k < Items; ++k)   // of the last items only
+    {
+        const int e = e0 + kRadius + k;
+        const float4 blo = slo[padded(e)], bhi = shi[padded(e)];
+#pragma unroll
+        for (int r = k; r < Items; ++r) against(r, e, blo, bhi);
+    }
+}
+
+__device__ __forceinline__ void stage_outside(float4& lo, float4& hi)
+{
+    const float inf = __int_as_float(0x7F800000);
+    lo = make_float4(-inf, -inf, -inf, 0.0f);
+    hi = make_float4(inf, inf, inf, 0.0f);
+}
+
+// Nearest neighbour of every cluster within kRadius positions (smallest union area), and
+// the merges (high half) and surviving clusters (low half) of every tile and group of
+// tiles.  A cluster merges (and owns the new node) when its nearest neighbour is mutual
+// and lies after it; it disappears when the mutual neighbour lies before it.
+__global__ void __launch_bounds__(kSearchThreads) ploc_nearest(const float4* __restrict__ lo,
+                                                               const float4* __restrict__ hi,
+                                                               const ploc_state* __restrict__ state,
+                                                               int* __restrict__ nn,
+                                                               unsigned long long* __restrict__ tiles,
+                                                               unsigned long long* __restrict__ groups)
+{
+    __shared__ float4 slo[padded(kStage)];
+    __shared__ float4 shi[padded(kStage)];
+    __shared__ int snn[kSearch];
+    __shared__ uint32_t counts[2];
+    const int64_t m = state->clusters;
+    const int64_t b0 = int64_t(blockIdx.x) * kTile;
+    if (b0 >= m || m <= kTail) return;
+    if (threadIdx.x < 2) counts[threadIdx.x] = 0;
+    for (int e = threadIdx.x; e < kStage; e += kSearchThreads)
+    {
+        const int64_t g = b0 - 2 * kRadius + e;
+        float4 l, h;
+        stage_outside(l, h);
+        if (g >= 0 && g < m)
+        {
+            l = lo[g];
+            h = hi[g];
+        }
+        slo[padded(e)] = l;
+        shi[padded(e)] = h;
     }
     __syncthreads();
+    {
+        // element x of snn is cluster b0 - kRadius + x, stage element x + kRadius
+        const int x = int(threadIdx.x) * kItems;
+        int nearest[kItems];
+        nearest_of<kItems>(slo, shi, x + kRadius, nearest);
+#pragma unroll
+        for (int r = 0; r < kItems; ++r) snn[x + r] = nearest[r] >= 0 ? nearest[r] - kRadius : -1;
+    }
+    __syncthreads();
+    uint32_t merges = 0, keeps = 0;
+    for (int k = threadIdx.x; k < kTile && b0 + k < m; k += kSearchThreads)
+    {
+        const int x = k + kRadius, j = snn[x];
+        const bool mutual = j >= 0 && snn[j] == x;
+        nn[b0 + k] = j >= 0 ? int(b0 + j - kRadius) : -1;
+        merges += mutual && x < j;
+        keeps += !(mutual && x > j);
+    }
+    merges = __reduce_add_sync(0xFFFFFFFFu, merges);
+    keeps = __reduce_add_sync(0xFFFFFFFFu, keeps);
+    if ((threadIdx.x & 31) == 0)
+    {
+        atomicAdd(&counts[0], merges);
+        atomicAdd(&counts[1], keeps);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        const unsigned long long sum = (static_cast<unsigned long long>(counts[0]) << 32) | counts[1];
+        tiles[blockIdx.x] = sum;
+        atomicAdd(&groups[blockIdx.x / kGroup], sum);
+    }
+}
+
+// The node pair of clusters a and b (boxes with the id in lo.w and the height in hi.w); a
+// becomes the merged cluster.
+__device__ __forceinline__ bool make_pair(float4& alo, float4& ahi, float4 const& blo, float4 const& bhi, uint32_t node,
+                                          uint32_t num_inner, bvh2_node* __restrict__ nodes,
+                                          uint32_t* __restrict__ status)
+{
+    const int ca = __float_as_int(alo.w), cb = __float_as_int(blo.w);
+    if (node >= num_inner || ca >= int(node) || cb >= int(node))   // children were made in earlier steps
+    {
+        atomicOr(status, kStatusBadIndex);
+        return false;
+    }
+    const int height = max(__float_as_int(ahi.w), __float_as_int(bhi.w)) + 1;
+    bvh2_node nd;
+    nd.xy0 = make_float4(alo.x, ahi.x, alo.y, ahi.y);
+    nd.xy1 = make_float4(blo.x, bhi.x, blo.y, bhi.y);
+    nd.z01 = make_float4(alo.z, ahi.z, blo.z, bhi.z);
+    nd.link = make_int4(ca, cb, height, -1);
+    nodes[node] = nd;
+    if (ca >= 0) nodes[ca].link.w = int(node << 1) | 0;
+    if (cb >= 0) nodes[cb].link.w = int(node << 1) | 1;
+    // merged as the LBVH merges (NaN and outward infinities of a leaf box skipped)
+    alo = make_float4(ref_min(cas_lo(alo.x), cas_lo(blo.x)), ref_min(cas_lo(alo.y), cas_lo(blo.y)),
+                      ref_min(cas_lo(alo.z), cas_lo(blo.z)), __int_as_float(int(node)));
+    ahi = make_float4(ref_max(cas_hi(ahi.x), cas_hi(bhi.x)), ref_max(cas_hi(ahi.y), cas_hi(bhi.y)),
+                      ref_max(cas_hi(ahi.z), cas_hi(bhi.z)), __int_as_float(height));
+    return true;
+}
+
+// One clustering step: merging clusters create the next node pairs in order, survivors are
+// compacted in order into (out_lo, out_hi).  With kTail clusters or fewer left the step
+// only copies them, since the host may launch a few steps too many.  The block of the last
+// tile writes the next state, for the host too; block 0 clears the next step's group sums.
+__global__ void __launch_bounds__(kTile) ploc_merge(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                    const int* __restrict__ nn, const ploc_state* __restrict__ state,
+                                                    ploc_state* __restrict__ next,
+                                                    const unsigned long long* __restrict__ tiles,
+                                                    const unsigned long long* __restrict__ groups,
+                                                    unsigned long long* __restrict__ next_groups, uint32_t num_groups,
+                                                    uint32_t num_inner, bvh2_node* __restrict__ nodes,
+                                                    float4* __restrict__ out_lo, float4* __restrict__ out_hi,
+                                                    uint32_t* __restrict__ host_clusters,
+                                                    uint32_t* __restrict__ status)
+{
+    __shared__ unsigned long long warp_before[kTile / 32];
+    __shared__ uint32_t warp_own[kTile / 32];
+    const ploc_state now = *state;
+    const int64_t m = now.clusters;
+    const int64_t b0 = int64_t(blockIdx.x) * kTile;
+    if (blockIdx.x == 0)
+        for (uint32_t k = threadIdx.x; k < num_groups; k += kTile) next_groups[k] = 0;
     const int64_t i = b0 + threadIdx.x;
-    if (i >= int64_t(m)) return;
-    const int li = threadIdx.x + kRadius;
-    const float4 alo = slo[li], ahi = shi[li];
-    float best = FLT_MAX;
-    int best_j = -1;
-    const int64_t first = i - kRadius > 0 ? i - kRadius : 0;
-    const int64_t last = i + kRadius < int64_t(m) - 1 ? i + kRadius : int64_t(m) - 1;
-    for (int64_t j = first; j <= last; ++j)
+    if (m <= kTail)
     {
-        if (j == i) continue;
-        int lj = int(j - b0) + kRadius;
-        float a = union_area(alo, ahi, slo[lj], shi[lj]);
-        if (a < best)   // ascending j: ties keep the lower index
+        if (i < m)
         {
-            best = a;
-            best_j = int(j);
+            out_lo[i] = lo[i];
+            out_hi[i] = hi[i];
         }
+        if (i == 0) *next = now;
+        return;
     }
-    nn[i] = best_j;
-}
-
-// Merge and keep flags: a cluster merges (and owns the new node) when its nearest
-// neighbour is mutual and lies after it; it disappears when the mutual neighbour lies
-// before it.  Packed as (merge << 32) | keep for one prefix sum of both.
-__global__ void __launch_bounds__(kBlock) ploc_flags(const int* __restrict__ nn, uint32_t m,
-                                                     unsigned long long* __restrict__ flags)
-{
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= m) return;
-    int j = nn[i];
-    bool mutual = j >= 0 && uint32_t(j) < m && nn[j] == int(i);
-    bool merge = mutual && int(i) < j;
-    bool removed = mutual && int(i) > j;
-    flags[i] = (static_cast<unsigned long long>(merge) << 32) | static_cast<unsigned long long>(!removed);
-}
-
-// Exclusive scan of 64-bit values, tile by tile (kScanTile per block), with the tile
-// totals written to sums.
-__global__ void __launch_bounds__(kBlock) scan_tiles(const unsigned long long* __restrict__ in, uint64_t m,
-                                                     unsigned long long* __restrict__ out,
-                                                     unsigned long long* __restrict__ sums)
-{
-    __shared__ unsigned long long warp_tot[kBlock / 32];
-    const uint64_t base = uint64_t(blockIdx.x) * kScanTile + uint64_t(threadIdx.x) * kScanItems;
-    unsigned long long v[kScanItems];
-    unsigned long long run = 0;
-    for (int k = 0; k < kScanItems; ++k)
-    {
-        v[k] = base + k < m ? in[base + k] : 0ull;
-        unsigned long long x = v[k];
-        v[k] = run;   // exclusive within the thread
-        run += x;
-    }
+    if (b0 >= m) return;
+    const int j = i < m ? nn[i] : -1;
+    const bool mutual = j >= 0 && j < m && nn[j] == int(i);
+    const bool merges = mutual && i < j, keeps = i < m && !(mutual && i > j);
+    // (merges << 32 | survivors) of the tiles before this one
+    unsigned long long before = 0;
+    const uint32_t group = blockIdx.x / kGroup;
+    for (uint32_t g = threadIdx.x; g < group; g += kTile) before += groups[g];
+    if (group * kGroup + threadIdx.x < blockIdx.x) before += tiles[group * kGroup + threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long incl = run;
-    for (int o = 1; o < 32; o <<= 1)
+    const uint32_t lanes_below = (1u << lane) - 1u;
+    const uint32_t mm = __ballot_sync(0xFFFFFFFFu, merges), kk = __ballot_sync(0xFFFFFFFFu, keeps);
+    if (lane == 0)
     {
-        unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
+        warp_before[warp] = before;
+        warp_own[warp] = uint32_t(__popc(mm)) << 16 | uint32_t(__popc(kk));
     }
-    if (lane == 31) warp_tot[warp] = incl;
     __syncthreads();
-    unsigned long long warp_base = 0;
-    for (int w = 0; w < warp; ++w) warp_base += warp_tot[w];
-    const unsigned long long thread_base = warp_base + incl - run;
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < m) out[base + k] = thread_base + v[k];
-    if (threadIdx.x == kBlock - 1) sums[blockIdx.x] = warp_base + incl;
-}
-
-__global__ void __launch_bounds__(kBlock) scan_add(unsigned long long* __restrict__ data, uint64_t m,
-                                                   const unsigned long long* __restrict__ offsets)
-{
-    const uint64_t base = uint64_t(blockIdx.x) * kScanTile;
-    const unsigned long long add = offsets[blockIdx.x];
-    for (int k = threadIdx.x; k < kScanTile; k += kBlock)
-        if (base + k < m) data[base + k] += add;
-}
-
-// Exclusive scan of data[0..m) into out; the total goes to *total.  Scratch holds the
-// per-level tile totals (scan_scratch_words(m) 64-bit words).
-size_t scan_scratch_words(uint64_t m)
-{
-    size_t words = 0;
-    while (m > 1)
+    before = 0;
+    uint32_t own = 0, all = 0;
+    for (int w = 0; w < kTile / 32; ++w)
     {
-        m = (m + kScanTile - 1) / kScanTile;
-        words += 2 * m + 64;
+        before += warp_before[w];
+        all += warp_own[w];
+        if (w < warp) own += warp_own[w];
     }
-    return words + 64;
-}
-
-gbrt_status scan_u64(gbrt_context* ctx, const unsigned long long* in, unsigned long long* out, uint64_t m,
-                     unsigned long long* scratch, unsigned long long* total, cudaStream_t s)
-{
-    if (m == 0) return GBRT_OK;
-    const uint64_t tiles = (m + kScanTile - 1) / kScanTile;
-    unsigned long long* sums = scratch;
-    unsigned long long* sums_scan = scratch + tiles + 32;
-    scan_tiles<<<uint32_t(tiles), kBlock, 0, s>>>(in, m, out, sums);
-    GBRT_LAUNCH_CHECK(ctx, "scan_tiles");
-    if (tiles == 1)
+    if (threadIdx.x == 0 && b0 + kTile >= m)
     {
-        GBRT_CUDA(ctx, cudaMemcpyAsync(total, sums, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
-        return GBRT_OK;
+        const uint32_t made = uint32_t(before >> 32) + (all >> 16), left = uint32_t(before) + (all & 0xFFFFu);
+        *next = { made ? left : 0u, now.nodes + made, made ? 0u : 1u };
+        *host_clusters = made ? left : 0u;
     }
-    gbrt_status st = scan_u64(ctx, sums, sums_scan, tiles, sums_scan + tiles + 32, total, s);
-    if (st != GBRT_OK) return st;
-    scan_add<<<uint32_t(tiles), kBlock, 0, s>>>(out, m, sums_scan);
-    GBRT_LAUNCH_CHECK(ctx, "scan_add");
-    return GBRT_OK;
-}
-
-// One clustering step: merging clusters create node pairs [node_base, ...) in order,
-// survivors are compacted in order into (out_lo, out_hi).
-__global__ void __launch_bounds__(kBlock) ploc_merge(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                     const int* __restrict__ nn, uint32_t m,
-                                                     const unsigned long long* __restrict__ flags,
-                                                     const unsigned long long* __restrict__ pre, uint32_t node_base,
-                                                     uint32_t num_inner, bvh2_node* __restrict__ nodes,
-                                                     float4* __restrict__ out_lo, float4* __restrict__ out_hi,
-                                                     uint32_t* __restrict__ status)
-{
-    uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= m) return;
-    const unsigned long long f = flags[i];
-    if (!(f & 1ull)) return;
-    const unsigned long long p = pre[i];
-    const uint32_t dst = uint32_t(p & 0xFFFFFFFFull);
+    if (!keeps) return;
     float4 alo = lo[i], ahi = hi[i];
-    if (f >> 32)
+    if (merges)
     {
-        const int j = nn[i];
-        const uint32_t node = node_base + uint32_t(p >> 32);
-        if (node >= num_inner || j < 0 || uint32_t(j) >= m)
-        {
-            atomicOr(status, kStatusBadIndex);
-            return;
-        }
-        const float4 blo = lo[j], bhi = hi[j];
-        const int ca = __float_as_int(alo.w), cb = __float_as_int(blo.w);
-        if (ca >= int(node) || cb >= int(node))   // children were made in earlier steps
-        {
-            atomicOr(status, kStatusBadIndex);
-            return;
-        }
-        const int height = max(__float_as_int(ahi.w), __float_as_int(bhi.w)) + 1;
-        bvh2_node nd;
-        nd.xy0 = make_float4(alo.x, ahi.x, alo.y, ahi.y);
-        nd.xy1 = make_float4(blo.x, bhi.x, blo.y, bhi.y);
-        nd.z01 = make_float4(alo.z, ahi.z, blo.z, bhi.z);
-        nd.link = make_int4(ca, cb, height, -1);
-        nodes[node] = nd;
-        if (ca >= 0) nodes[ca].link.w = int(node << 1) | 0;
-        if (cb >= 0) nodes[cb].link.w = int(node << 1) | 1;
-        // merged as the LBVH merges (NaN and outward infinities of a leaf box skipped)
-        alo = make_float4(ref_min(cas_lo(alo.x), cas_lo(blo.x)), ref_min(cas_lo(alo.y), cas_lo(blo.y)),
-                          ref_min(cas_lo(alo.z), cas_lo(blo.z)), __int_as_float(int(node)));
-        ahi = make_float4(ref_max(cas_hi(ahi.x), cas_hi(bhi.x)), ref_max(cas_hi(ahi.y), cas_hi(bhi.y)),
-                          ref_max(cas_hi(ahi.z), cas_hi(bhi.z)), __int_as_float(height));
+        const uint32_t node = now.nodes + uint32_t(before >> 32) + (own >> 16) + uint32_t(__popc(mm & lanes_below));
+        if (!make_pair(alo, ahi, lo[j], hi[j], node, num_inner, nodes, status)) return;
     }
+    const uint32_t dst = uint32_t(before) + (own & 0xFFFFu) + uint32_t(__popc(kk & lanes_below));
     out_lo[dst] = alo;
     out_hi[dst] = ahi;
 }
+
+// One step of m clusters in shared memory (cluster k at element k + kRadius), Items per
+// thread.  Returns (merges << 16 | survivors).
+template <int Items>
+__device__ __forceinline__ uint32_t tail_step(float4* slo, float4* shi, int* snn, uint32_t* warp_own, int m,
+                                              uint32_t made, uint32_t num_inner, bvh2_node* __restrict__ nodes,
+                                              uint32_t* __restrict__ status)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k0 = int(threadIdx.x) * Items;
+    if (k0 < m)
+    {
+        int nearest[Items];
+        nearest_of<Items>(slo, shi, k0 + kRadius, nearest);
+#pragma unroll
+        for (int r = 0; r < Items; ++r) snn[k0 + r] = nearest[r] >= 0 ? nearest[r] - kRadius : -1;
+    }
+    __syncthreads();
+    int other[Items];
+    uint32_t what[Items], mine = 0;   // as the return value, of one cluster
+#pragma unroll
+    for (int r = 0; r < Items; ++r)
+    {
+        const int k = k0 + r;
+        other[r] = k < m ? snn[k] : -1;
+        const bool mutual = other[r] >= 0 && snn[other[r]] == k;
+        what[r] = (mutual && k < other[r] ? 1u << 16 : 0u) + (k < m && !(mutual && k > other[r]) ? 1u : 0u);
+        mine += what[r];
+    }
+    uint32_t incl = mine;
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) warp_own[warp] = incl;
+    __syncthreads();
+    const uint32_t of_lane = warp_own[lane];   // kTailThreads / 32 == 32 warps
+    const uint32_t all = __reduce_add_sync(0xFFFFFFFFu, of_lane);
+    uint32_t at = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? of_lane : 0u) + incl - mine;
+    float4 alo[Items], ahi[Items];
+    uint32_t dst[Items];
+#pragma unroll
+    for (int r = 0; r < Items; ++r)
+    {
+        dst[r] = at & 0xFFFFu;
+        if (what[r] & 1u)
+        {
+            alo[r] = slo[padded(k0 + r + kRadius)];
+            ahi[r] = shi[padded(k0 + r + kRadius)];
+            if (what[r] >> 16)
+                make_pair(alo[r], ahi[r], slo[padded(other[r] + kRadius)], shi[padded(other[r] + kRadius)],
+                          made + (at >> 16), num_inner, nodes, status);
+        }
+        at += what[r];
+    }
+    __syncthreads();
+    const int left = int(all & 0xFFFFu);
+#pragma unroll
+    for (int r = 0; r < Items; ++r)
+    {
+        const int k = k0 + r;
+        if (what[r] & 1u)
+        {
+            slo[padded(int(dst[r]) + kRadius)] = alo[r];
+            shi[padded(int(dst[r]) + kRadius)] = ahi[r];
+        }
+        if (k >= left && k < m) stage_outside(slo[padded(k + kRadius)], shi[padded(k + kRadius)]);
+    }
+    __syncthreads();
+    return all;
+}
+
+// Every step from kTail or fewer clusters to the root, in one block, and the report.
+constexpr size_t kTailBytes = 2 * size_t(padded(kTail + 2 * kRadius)) * sizeof(float4);
+
+__global__ void __launch_bounds__(kTailThreads) ploc_tail(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                          const ploc_state* __restrict__ state, uint32_t num_inner,
+                                                          bvh2_node* __restrict__ nodes,
+                                                          build_result* __restrict__ report,
+                                                          uint32_t* __restrict__ status)
+{
+    extern __shared__ float4 tail_mem[];
+    float4* slo = tail_mem;
+    float4* shi = tail_mem + padded(kTail + 2 * kRadius);
+    __shared__ int snn[kTail];
+    __shared__ uint32_t warp_own[kTailThreads / 32];
+    int m = int(state->clusters);
+    uint32_t made = state->nodes;
+    bool stuck = state->stuck != 0 || m > kTail;
+    for (int e = threadIdx.x; e < kTail + 2 * kRadius; e += kTailThreads)
+    {
+        float4 l, h;
+        stage_outside(l, h);
+        if (!stuck && e >= kRadius && e - kRadius < m)
+        {
+            l = lo[e - kRadius];
+            h = hi[e - kRadius];
+        }
+        slo[padded(e)] = l;
+        shi[padded(e)] = h;
+    }
+    __syncthreads();
+    while (!stuck && m > 1)
+    {
+        const uint32_t step = m > kTailThreads ? tail_step<2>(slo, shi, snn, warp_own, m, made, num_inner, nodes, status)
+                                               : tail_step<1>(slo, shi, snn, warp_own, m, made, num_inner, nodes, status);
+        made += step >> 16;
+        stuck = step >> 16 == 0;
+        m = int(step & 0xFFFFu);
+    }
+    if (threadIdx.x == 0)
+    {
+        const float4 l = slo[padded(kRadius)], h = shi[padded(kRadius)];
+        report->lo[0] = l.x, report->lo[1] = l.y, report->lo[2] = l.z;
+        report->hi[0] = h.x, report->hi[1] = h.y, report->hi[2] = h.z;
+        report->root = __float_as_int(l.w);
+        report->height = uint32_t(__float_as_int(h.w));
+        report->made = made;
+        report->stuck = stuck ? 1u : 0u;
+    }
+}
+
+// Steps between a launch and the host's look at the cluster count: the GPU has two queued
+// while it looks, and at most that many run on kTail clusters for nothing.
+constexpr uint32_t kLate = 2;
+
+struct event_ring
+{
+    cudaEvent_t events[kLate + 1] = {};
+    ~event_ring()
+    {
+        for (cudaEvent_t e : events)
+            if (e) cudaEventDestroy(e);
+    }
+    cudaError_t at(uint32_t i, cudaEvent_t** out)
+    {
+        *out = &events[i % (kLate + 1)];
+        return **out ? cudaSuccess : cudaEventCreateWithFlags(*out, cudaEventDisableTiming);
+    }
+};
 
 } // namespace
 
@@ -265,88 +501,75 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     st = morton_order(ctx, d_tris, n, bvh->sorted_codes, bvh->sorted_ids);
     if (st != GBRT_OK) return st;
 
-    // scratch (after the sort): clusters twice, neighbours, flags, prefix, scan levels
+    // scratch (after the sort): clusters twice, neighbours, tile and group sums, states
+    const uint32_t max_tiles = (n + kTile - 1) / kTile, num_groups = max_tiles / kGroup + 1;
     size_t off_lo0 = 0, off_hi0 = align_up(size_t(n) * 16), off_lo1 = off_hi0 + align_up(size_t(n) * 16);
     size_t off_hi1 = off_lo1 + align_up(size_t(n) * 16), off_nn = off_hi1 + align_up(size_t(n) * 16);
-    size_t off_flags = off_nn + align_up(size_t(n) * 4), off_pre = off_flags + align_up(size_t(n) * 8);
-    size_t off_scan = off_pre + align_up(size_t(n) * 8), off_total = off_scan + align_up(scan_scratch_words(n) * 8);
-    st = ensure_scratch(ctx, off_total + 256);
+    size_t off_tiles = off_nn + align_up(size_t(n) * 4), off_groups = off_tiles + align_up(size_t(max_tiles) * 8);
+    size_t off_state = off_groups + align_up(size_t(num_groups) * 16);
+    st = ensure_scratch(ctx, off_state + 256);
+    if (st != GBRT_OK) return st;
+    build_result* result = nullptr;
+    st = ensure_result(ctx, &result);
     if (st != GBRT_OK) return st;
     char* base = static_cast<char*>(ctx->scratch);
     float4* lo[2] = { reinterpret_cast<float4*>(base + off_lo0), reinterpret_cast<float4*>(base + off_lo1) };
     float4* hi[2] = { reinterpret_cast<float4*>(base + off_hi0), reinterpret_cast<float4*>(base + off_hi1) };
     int* nn = reinterpret_cast<int*>(base + off_nn);
-    auto* flags = reinterpret_cast<unsigned long long*>(base + off_flags);
-    auto* pre = reinterpret_cast<unsigned long long*>(base + off_pre);
-    auto* scan_scratch = reinterpret_cast<unsigned long long*>(base + off_scan);
-    auto* total = reinterpret_cast<unsigned long long*>(base + off_total);
+    auto* tiles = reinterpret_cast<unsigned long long*>(base + off_tiles);
+    auto* group_mem = reinterpret_cast<unsigned long long*>(base + off_groups);
+    unsigned long long* groups[2] = { group_mem, group_mem + num_groups };
+    auto* state = reinterpret_cast<ploc_state*>(base + off_state);
 
-    ploc_leaves<<<blocks_for(n), kBlock, 0, s>>>(d_tris, bvh->sorted_ids, n, lo[0], hi[0], bvh->tris, ctx->d_status);
+    ploc_leaves<<<blocks_for(n), kBlock, 0, s>>>(d_tris, bvh->sorted_ids, n, lo[0], hi[0], bvh->tris, state, groups[0],
+                                                 num_groups, ctx->d_status);
     GBRT_LAUNCH_CHECK(ctx, "ploc_leaves");
-    uint32_t m = n, node_base = 0;
-    int cur = 0;
-    for (uint32_t iter = 0; m > 1; ++iter)
+    auto* host = const_cast<volatile build_result*>(ctx->h_result);
+    host->clusters = n;
+    host->quads_bad = 0;
+    event_ring done;
+    uint32_t iter = 0;
+    for (uint32_t clusters = n; clusters > uint32_t(kTail); ++iter)
     {
-        if (iter >= n) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: no progress");
-        ploc_nearest<<<blocks_for(m), kBlock, 0, s>>>(lo[cur], hi[cur], m, nn);
+        const int cur = int(iter & 1);
+        const uint32_t grid = (clusters + kTile - 1) / kTile;
+        ploc_nearest<<<grid, kSearchThreads, 0, s>>>(lo[cur], hi[cur], state + cur, nn, tiles, groups[cur]);
         GBRT_LAUNCH_CHECK(ctx, "ploc_nearest");
-        ploc_flags<<<blocks_for(m), kBlock, 0, s>>>(nn, m, flags);
-        GBRT_LAUNCH_CHECK(ctx, "ploc_flags");
-        st = scan_u64(ctx, flags, pre, m, scan_scratch, total, s);
-        if (st != GBRT_OK) return st;
-        ploc_merge<<<blocks_for(m), kBlock, 0, s>>>(lo[cur], hi[cur], nn, m, flags, pre, node_base, bvh->num_inner,
-                                                    bvh->nodes, lo[cur ^ 1], hi[cur ^ 1], ctx->d_status);
+        ploc_merge<<<grid, kTile, 0, s>>>(lo[cur], hi[cur], nn, state + cur, state + (cur ^ 1), tiles, groups[cur],
+                                          groups[cur ^ 1], num_groups, bvh->num_inner, bvh->nodes, lo[cur ^ 1],
+                                          hi[cur ^ 1], &result->clusters, ctx->d_status);
         GBRT_LAUNCH_CHECK(ctx, "ploc_merge");
-        unsigned long long t = 0;
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&t, total, sizeof(t), cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaStreamSynchronize(s));
-        const uint32_t merges = uint32_t(t >> 32), keeps = uint32_t(t & 0xFFFFFFFFull);
-        if (merges == 0 || keeps != m - merges)
-            return fail(ctx, GBRT_ERR_CUDA, "PLOC build: inconsistent merge step");
-        node_base += merges;
-        m = keeps;
-        cur ^= 1;
+        cudaEvent_t* mark = nullptr;
+        GBRT_CUDA(ctx, done.at(iter, &mark));
+        GBRT_CUDA(ctx, cudaEventRecord(*mark, s));
+        if (iter >= kLate)
+        {
+            GBRT_CUDA(ctx, done.at(iter - kLate, &mark));
+            GBRT_CUDA(ctx, cudaEventSynchronize(*mark));
+            clusters = host->clusters;
+        }
     }
+    GBRT_CUDA(ctx, cudaFuncSetAttribute(ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTailBytes)));
+    ploc_tail<<<1, kTailThreads, kTailBytes, s>>>(lo[iter & 1], hi[iter & 1], state + (iter & 1), bvh->num_inner,
+                                                  bvh->nodes, result, ctx->d_status);
+    GBRT_LAUNCH_CHECK(ctx, "ploc_tail");
     if (n > 1)
     {
-        if (node_base != n - 1) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: wrong node count");
-        float4 root_lo, root_hi;
-        build_result* result = nullptr;
-        st = ensure_result(ctx, &result);
-        if (st != GBRT_OK) return st;
-        ctx->h_result->quads_bad = 0;
         GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
         st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
         if (st != GBRT_OK) return st;
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&root_lo, lo[cur], sizeof(root_lo), cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&root_hi, hi[cur], sizeof(root_hi), cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaStreamSynchronize(s));
-        bvh->quads_ok = ctx->h_result->quads_bad == 0;
-        int root = 0, height = 0;
-        memcpy(&root, &root_lo.w, 4);
-        memcpy(&height, &root_hi.w, 4);
-        if (root != int(n - 2)) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: unexpected root");
-        bvh->root = root;
-        bvh->height = uint32_t(height);
-        bvh->lo[0] = root_lo.x;
-        bvh->lo[1] = root_lo.y;
-        bvh->lo[2] = root_lo.z;
-        bvh->hi[0] = root_hi.x;
-        bvh->hi[1] = root_hi.y;
-        bvh->hi[2] = root_hi.z;
     }
-    else
+    GBRT_CUDA(ctx, cudaStreamSynchronize(s));
+    const build_result r = *ctx->h_result;
+    if (r.stuck) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: inconsistent merge step");
+    if (r.made != n - 1) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: wrong node count");
+    if (r.root != bvh->root) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: unexpected root");
+    bvh->quads_ok = n > 1 && r.quads_bad == 0;
+    bvh->height = r.height;
+    for (int a = 0; a < 3; ++a)
     {
-        float4 l, h;
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&l, lo[0], sizeof(l), cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaMemcpyAsync(&h, hi[0], sizeof(h), cudaMemcpyDeviceToHost, s));
-        GBRT_CUDA(ctx, cudaStreamSynchronize(s));
-        bvh->lo[0] = l.x;
-        bvh->lo[1] = l.y;
-        bvh->lo[2] = l.z;
-        bvh->hi[0] = h.x;
-        bvh->hi[1] = h.y;
-        bvh->hi[2] = h.z;
+        bvh->lo[a] = r.lo[a];
+        bvh->hi[a] = r.hi[a];
     }
     if (bvh->height + 1 > uint32_t(kStackSize))
         return fail(ctx, GBRT_ERR_STACK_OVERFLOW, "PLOC tree height exceeds the traversal stack");
