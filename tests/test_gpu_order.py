@@ -31,7 +31,7 @@ def check(bvh, tris, oracle):
 
 
 @pytest.mark.parametrize("kind", ["soup", "few", "flat"])
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 1023, 1024, 1025, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 12289])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 255, 256, 257, 287, 1023, 1024, 1025, 2048, 2049, 4096, 4097, 8191, 8192, 8193, 12289])
 def test_one_block_and_few_tiles(oracle, n, kind):
     tris = make(n, kind)
     d = vg.as_device_bytes(tris)

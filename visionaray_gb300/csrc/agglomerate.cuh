@@ -10,19 +10,24 @@
 // the tree: a left child has index r, a right child index l, the root 0.  The thread that
 // makes a node has both children's boxes and its index and writes the 64-byte record once.
 //
-// Almost all of that happens inside a block: it starts from kAggBlock consecutive leaves,
-// and nodes whose keys lie in the block meet through shared memory.  What is left when no
-// thread of the block can go on -- the O(log kAggBlock) nodes that wait for a neighbour
-// block -- is written to mailboxes in global memory, and a second kernel takes it up from
-// there with one warp per block of the first (both sides' data written before an atomic on
-// the split's flag; the second arrival reads the other side's).  No thread waits for
-// another one.  In one kernel, each block's few climbing threads held its registers and
+// Almost all of that happens inside a block: it starts from kAggBlock consecutive leaves and
+// goes in rounds over the list of subtrees made so far.  A split whose delta is larger than
+// those at the outer ends of its two subtrees is their parent's, so every such pair becomes
+// a node and the list is compacted; no round needs more than its neighbours' entries.  What
+// is left when no pair of the block can go on -- the O(log kAggBlock) nodes that wait for a
+// neighbour block -- is written to mailboxes in global memory, and a second kernel takes it
+// up from there with one warp per block of the first (both sides' data written before an
+// atomic on the split's flag; the second arrival reads the other side's).  No thread waits
+// for another one.  In one kernel, each block's few climbing threads held its registers and
 // shared memory through a chain of fences and atomics: 1,151 us for 8.4 M triangles.
 //
-// Measured on 8,388,608 triangles (heightfield 2048^2): in-place rebuild 1.76 -> 1.11 ms;
-// a refit (these two kernels and a memset of the flags) 0.67 ms.  Bound by the load/store
-// pipe (56 %: the triangle gather, 112 B of stores per triangle, the mail in shared memory)
-// and by the divergence of the climb (9 of 32 lanes, issue slots 44 %).
+// Measured on 8,388,608 triangles (heightfield 2048^2): a refit (these two kernels, the quads
+// and a memset of the flags) 854 us, of which the first kernel 406 us at 41 % of the DRAM
+// bandwidth.  With each leaf's thread climbing through atomics on shared flags (9 of 32
+// lanes at work, against 23) and gathering its triangle alone it was 511 us.  Bound now by
+// the barriers of the rounds and by the load/store pipe (64 %).  Rounds inside each warp
+// first save barriers but lose the lanes (refit 964 us); blocks of 128 and 512 leaves
+// 911 and 872 us.
 #pragma once
 
 #include "lbvh_device.cuh"
@@ -30,7 +35,7 @@
 
 namespace gbrt {
 
-constexpr int kAggBlock = 512;
+constexpr int kAggBlock = 256;
 
 // One side's data at a split: the child's box, the end of its key range away from the
 // split, and its height.
@@ -68,25 +73,6 @@ struct agg_args
     uint32_t* root_height;   // the root's height (segmented: the largest by atomicMax)
     uint32_t* status;
 };
-
-// A 44-byte triangle at a 4-byte aligned address as five 64-bit loads and one 32-bit one
-// (the words before or after the 8-byte aligned ones): half the load instructions, and
-// every one of them touches another line per lane when the triangles are gathered.
-__device__ __forceinline__ tri_in load_tri_gather(gbrt_triangle const* __restrict__ tris, uint64_t i)
-{
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(tris + i);
-    const bool odd = (reinterpret_cast<uintptr_t>(w) & 4u) != 0;
-    const uint2* p = reinterpret_cast<const uint2*>(w + (odd ? 1 : 0));
-    const uint2 v0 = __ldg(p), v1 = __ldg(p + 1), v2 = __ldg(p + 2), v3 = __ldg(p + 3), v4 = __ldg(p + 4);
-    const uint32_t s = __ldg(w + (odd ? 0 : 10));
-    tri_in t;
-    t.geom_id = odd ? s : v0.x;
-    t.prim_id = odd ? v0.x : v0.y;
-    t.v1 = { __uint_as_float(odd ? v0.y : v1.x), __uint_as_float(odd ? v1.x : v1.y), __uint_as_float(odd ? v1.y : v2.x) };
-    t.e1 = { __uint_as_float(odd ? v2.x : v2.y), __uint_as_float(odd ? v2.y : v3.x), __uint_as_float(odd ? v3.x : v3.y) };
-    t.e2 = { __uint_as_float(odd ? v3.y : v4.x), __uint_as_float(odd ? v4.x : v4.y), __uint_as_float(odd ? v4.y : s) };
-    return t;
-}
 
 __device__ __forceinline__ agg_mail pack_mail(box3 const& b, int far_end, int height)
 {
@@ -142,92 +128,169 @@ __device__ __forceinline__ void agg_make_node(agg_args const& a, int lo, int inn
     }
 }
 
+constexpr int kTriWords = sizeof(gbrt_triangle) / 4;
+// Resident blocks the registers must allow (40, a spilled word in the segmented form): five
+// 898 us per refit, eight 891.
+constexpr int kAggMinBlocks = 6;
+
 template <bool Segmented>
-__global__ void __launch_bounds__(kAggBlock) agg_in_blocks(agg_args a)
+__global__ void __launch_bounds__(kAggBlock, kAggMinBlocks) agg_in_blocks(agg_args a)
 {
-    // split kk of the block is the one between its leaves b0 + kk - 1 and b0 + kk; kk = 0 and
-    // kAggBlock are the block's ends
-    // (mail halves as separate arrays: neighbouring lanes' accesses hit different banks)
-    __shared__ float4 mail_a[2][kAggBlock + 1], mail_b[2][kAggBlock + 1];
-    __shared__ uint32_t flags[kAggBlock + 1];
-    __shared__ int delta[kAggBlock + 1];
-    __shared__ uint32_t waiting;
+    // The subtrees made so far, in key order: entry t of a list is the t-th one's first leaf
+    // in the block | (delta at its left end + 1) << 16, and one more entry for the block's end.
+    // A subtree's box and height stand at its first leaf's element (halves as separate
+    // arrays: neighbouring lanes' accesses hit different banks).
+    __shared__ uint32_t list[2][kAggBlock + 1];
+    __shared__ float4 box_a[kAggBlock], box_b[kAggBlock];
+    __shared__ int seg_lo[Segmented ? kAggBlock : 1], seg_inner[Segmented ? kAggBlock : 1];
+    __shared__ uint32_t tri_words[kAggBlock / 32][32 * kTriWords];
+    __shared__ uint32_t kept[kAggBlock / 32];
+    __shared__ uint32_t left_over, waiting;
 
     const int n = int(a.n);
     const int b0 = int(blockIdx.x) * kAggBlock;
-    const int tid = int(threadIdx.x);
+    const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
+    const uint32_t full = 0xFFFFFFFFu, lanes_below = (1u << lane) - 1u;
     const int j = b0 + tid;
-    int lo = 0, hi = n, inner_base = 0;
-    bool active = j < n;
-    if (Segmented && active)
-    {
-        const uint32_t s = upper_segment(a.offsets, a.num_scenes, uint32_t(j));
-        lo = int(__ldg(&a.offsets[s]));
-        hi = int(__ldg(&a.offsets[s + 1]));
-        inner_base = int(__ldg(&a.inner_offsets[s]));
-    }
-    for (int k = tid; k <= kAggBlock; k += kAggBlock) flags[k] = 0;
+    const bool active = j < n;
+    uint32_t m = uint32_t(n - b0 < kAggBlock ? n - b0 : kAggBlock);
+    uint32_t id = 0;
     if (active)
     {
-        if (tid == 0) delta[0] = neighbour_delta(a.codes, j - 1, lo, hi);
-        delta[tid + 1] = neighbour_delta(a.codes, j, lo, hi);
-    }
+        int lo = 0, hi = n;
+        if (Segmented)
+        {
+            const uint32_t s = upper_segment(a.offsets, a.num_scenes, uint32_t(j));
+            lo = int(__ldg(&a.offsets[s]));
+            hi = int(__ldg(&a.offsets[s + 1]));
+            seg_lo[tid] = lo;
+            seg_inner[tid] = int(__ldg(&a.inner_offsets[s]));
+        }
+        if (tid == 0) list[0][0] = uint32_t(neighbour_delta(a.codes, j - 1, lo, hi) + 1) << 16;
+        list[0][tid + 1] = uint32_t(tid + 1) | uint32_t(neighbour_delta(a.codes, j, lo, hi) + 1) << 16;
 
-    box3 box;
-    if (active)
-    {
-        uint32_t id = __ldg(&a.sorted_ids[j]);
+        id = __ldg(&a.sorted_ids[j]);
         if (id >= a.n)
         {
             atomicOr(a.status, kStatusBadIndex);
             id = 0;
         }
-        const tri_in t = load_tri_gather(a.tris_in, id);
-        float4* o = reinterpret_cast<float4*>(a.tris_out + j);
-        o[0] = make_float4(t.v1.x, t.v1.y, t.v1.z, __uint_as_float(t.prim_id));
-        o[1] = make_float4(t.e1.x, t.e1.y, t.e1.z, __uint_as_float(t.geom_id));
-        o[2] = make_float4(t.e2.x, t.e2.y, t.e2.z, __uint_as_float(kLastInLeaf));
-        box = tri_box(t);
     }
-    __syncthreads();
-
-    // inside the block
-    if (active && hi - lo > 1)
+    // The warp's triangles word by word, consecutive lanes on one triangle, and out again as
+    // records: an access touches the lines of three triangles, not of 32.
+    uint32_t* words = tri_words[warp];
+    const uint32_t* in = reinterpret_cast<const uint32_t*>(a.tris_in);
+#pragma unroll
+    for (int k = 0; k < kTriWords; ++k)
     {
-        int l = j, r = j, height = 0;
-        for (;;)
-        {
-            const int dl = delta[l - b0], dr = delta[r - b0 + 1];
-            const bool left = dr > dl;
-            const int kk = left ? r - b0 + 1 : l - b0;
-            const agg_mail mine = pack_mail(box, left ? l : r, height);
-            mail_a[left ? 0 : 1][kk] = mine.a;
-            mail_b[left ? 0 : 1][kk] = mine.b;
-            __threadfence_block();
-            if (atomicOr(&flags[kk], left ? 1u : 2u) == 0) break;   // the other side goes on
-            __threadfence_block();
-            const agg_mail other = { mail_a[left ? 1 : 0][kk], mail_b[left ? 1 : 0][kk] };
-            const agg_mail lm = left ? mine : other, rm = left ? other : mine;
-            const int m = b0 + kk - 1;
-            l = __float_as_int(lm.b.z);
-            r = __float_as_int(rm.b.z);
-            const int pl = delta[l - b0], pr = delta[r - b0 + 1];
-            const bool root = pl < 0 && pr < 0;
-            agg_make_node<Segmented>(a, lo, inner_base, l, r, m, root, pr > pl, lm, rm, box, height);
-            if (root) break;
-        }
+        const int w = 32 * k + lane, t = w / kTriWords;
+        words[w] = __ldg(&in[uint64_t(__shfl_sync(full, id, t)) * kTriWords + (w - kTriWords * t)]);
+    }
+    __syncwarp();
+    {
+        const float* w = reinterpret_cast<const float*>(words + kTriWords * lane);
+        const tri_in t = { { w[2], w[3], w[4] }, { w[5], w[6], w[7] }, { w[8], w[9], w[10] }, 0, 0 };
+        const agg_mail mine = pack_mail(tri_box(t), 0, 0);
+        box_a[tid] = mine.a;
+        box_b[tid] = mine.b;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+        const int q = 32 * k + lane, t = q / 3, part = q - 3 * t;
+        const float* w = reinterpret_cast<const float*>(words + kTriWords * t);
+        const float* v = w + 2 + 3 * part;
+        if (j - lane + t < n)
+            reinterpret_cast<float4*>(a.tris_out + (j - lane))[q] =
+                make_float4(v[0], v[1], v[2], part == 2 ? __uint_as_float(kLastInLeaf) : w[1 - part]);
     }
     if (tid == 0) waiting = 0;
     __syncthreads();
 
-    // the nodes that wait at a split for a node that leaves the block
-    for (int kk = tid; kk <= kAggBlock; kk += kAggBlock)
+    // One round on list `cur`: where the delta between two subtrees is larger than at their
+    // outer ends, they are the children of one node.  Returns whether subtree t stays on
+    // the list (a right child does not), its entry in e1.
+    auto round = [&](int cur, int t, uint32_t& e1) -> bool {
+        if (t >= int(m)) return false;
+        const uint32_t* e = list[cur] + t;
+        e1 = e[0];
+        const uint32_t e2 = e[1];
+        const uint32_t d1 = e1 >> 16, d2 = e2 >> 16;   // + 1: 0 is no common prefix
+        if (t > 0 && d1 > d2 && d1 > e[-1] >> 16) return false;
+        if (t + 1 < int(m) && d2 > d1)
+        {
+            const uint32_t e3 = e[2], d3 = e3 >> 16;
+            if (d2 > d3)
+            {
+                const int l = int(e1 & 0xFFFFu), mid = int(e2 & 0xFFFFu), r = int(e3 & 0xFFFFu) - 1;
+                agg_mail lm = { box_a[l], box_b[l] }, rm = { box_a[mid], box_b[mid] };
+                const int lo = Segmented ? seg_lo[l] : 0, inner_base = Segmented ? seg_inner[l] : 0;
+                box3 box;
+                int height;
+                agg_make_node<Segmented>(a, lo, inner_base, b0 + l, b0 + r, b0 + mid - 1, d1 == 0 && d3 == 0, d3 > d1, lm,
+                                         rm, box, height);
+                const agg_mail made = pack_mail(box, 0, height);
+                box_a[l] = made.a;
+                box_b[l] = made.b;
+            }
+        }
+        return true;
+    };
+    int cur = 0;
+    bool more = true;
+    while (more && m > 32)
     {
-        const uint32_t f = flags[kk];
-        if (f != 1u && f != 2u) continue;
-        const int side = f == 1u ? 0 : 1, m = b0 + kk - 1;
-        a.slots[m].side[side] = { mail_a[side][kk], mail_b[side][kk] };
-        a.waiting[uint64_t(blockIdx.x) * (kAggBlock + 1) + atomicAdd(&waiting, 1u)] = uint32_t(m) << 1 | uint32_t(side);
+        uint32_t e1 = 0;
+        const bool stays = round(cur, tid, e1);
+        const uint32_t mask = __ballot_sync(full, stays);
+        if (lane == 0) kept[warp] = __popc(mask);
+        __syncthreads();
+        const uint32_t of_lane = lane < kAggBlock / 32 ? kept[lane] : 0u;
+        const uint32_t all = __reduce_add_sync(full, of_lane);
+        const uint32_t at = __reduce_add_sync(full, lane < warp ? of_lane : 0u) + __popc(mask & lanes_below);
+        if (stays) list[cur ^ 1][at] = e1;
+        if (tid == 0) list[cur ^ 1][all] = list[cur][m];
+        more = all != m;
+        m = all;
+        cur ^= 1;
+        __syncthreads();
+    }
+    if (warp == 0)
+    {
+        while (more)
+        {
+            uint32_t e1 = 0;
+            const bool stays = round(cur, lane, e1);
+            const uint32_t mask = __ballot_sync(full, stays);
+            const uint32_t all = __popc(mask);
+            if (stays) list[cur ^ 1][__popc(mask & lanes_below)] = e1;
+            if (lane == 0) list[cur ^ 1][all] = list[cur][m];
+            more = all != m;
+            m = all;
+            cur ^= 1;
+            __syncwarp();
+        }
+        if (lane == 0) left_over = m | uint32_t(cur) << 16;
+    }
+    __syncthreads();
+
+    // what is left and not a root waits at a split for a node that leaves the block
+    m = left_over & 0xFFFFu;
+    if (uint32_t(tid) < m)
+    {
+        const uint32_t* e = list[left_over >> 16] + tid;
+        const uint32_t d1 = e[0] >> 16, d2 = e[1] >> 16;
+        if (d1 != 0 || d2 != 0)
+        {
+            const bool left = d2 > d1;
+            const int l = int(e[0] & 0xFFFFu), end = int(e[1] & 0xFFFFu);
+            const int split = b0 + (left ? end : l) - 1;
+            agg_mail mail = { box_a[l], box_b[l] };
+            mail.b.z = __int_as_float(left ? b0 + l : b0 + end - 1);
+            a.slots[split].side[left ? 0 : 1] = mail;
+            a.waiting[uint64_t(blockIdx.x) * (kAggBlock + 1) + atomicAdd(&waiting, 1u)] =
+                uint32_t(split) << 1 | uint32_t(left ? 0 : 1);
+        }
     }
     __syncthreads();
     if (tid == 0) a.num_waiting[blockIdx.x] = waiting;
