@@ -22,12 +22,12 @@
 // shared memory through a chain of fences and atomics: 1,151 us for 8.4 M triangles.
 //
 // Measured on 8,388,608 triangles (heightfield 2048^2): a refit (these two kernels, the quads
-// and a memset of the flags) 854 us, of which the first kernel 406 us at 41 % of the DRAM
+// and a memset of the flags) 799 us, of which the first kernel 406 us at 41 % of the DRAM
 // bandwidth.  With each leaf's thread climbing through atomics on shared flags (9 of 32
 // lanes at work, against 23) and gathering its triangle alone it was 511 us.  Bound now by
 // the barriers of the rounds and by the load/store pipe (64 %).  Rounds inside each warp
-// first save barriers but lose the lanes (refit 964 us); blocks of 128 and 512 leaves
-// 911 and 872 us.
+// first save barriers but lose the lanes (refit 854 -> 964 us); blocks of 128 and 512
+// leaves 911 and 872 us.
 #pragma once
 
 #include "lbvh_device.cuh"
@@ -38,11 +38,11 @@ namespace gbrt {
 constexpr int kAggBlock = 256;
 
 // One side's data at a split: the child's box, the end of its key range away from the
-// split, and its height.
+// split, its height, and between blocks the delta (+ 1) at the far end.
 struct __align__(16) agg_mail
 {
     float4 a;   // lo.x, lo.y, lo.z, hi.x
-    float4 b;   // hi.y, hi.z, far end, height (the last two as bits)
+    float4 b;   // hi.y, hi.z, far end, height | far delta << 8 (the last two as bits)
 };
 // Per split and scene-wide split position: left and right child.  n of these.
 struct agg_slot
@@ -109,7 +109,7 @@ __device__ __forceinline__ void agg_make_node(agg_args const& a, int lo, int inn
                                               int& height)
 {
     const int index = inner_base + (root ? 0 : (is_left ? r : l) - lo);
-    height = max(__float_as_int(lm.b.w), __float_as_int(rm.b.w)) + 1;
+    height = max(__float_as_int(lm.b.w) & 0xFF, __float_as_int(rm.b.w) & 0xFF) + 1;
     const int cl = l == m ? ~m : inner_base + (m - lo);
     const int cr = m + 1 == r ? ~r : inner_base + (m + 1 - lo);
     // xy0, xy1 | z01, link: two 256-bit stores
@@ -287,6 +287,7 @@ __global__ void __launch_bounds__(kAggBlock, kAggMinBlocks) agg_in_blocks(agg_ar
             const int split = b0 + (left ? end : l) - 1;
             agg_mail mail = { box_a[l], box_b[l] };
             mail.b.z = __int_as_float(left ? b0 + l : b0 + end - 1);
+            mail.b.w = __int_as_float(__float_as_int(mail.b.w) | int(left ? d1 : d2) << 8);
             a.slots[split].side[left ? 0 : 1] = mail;
             a.waiting[uint64_t(blockIdx.x) * (kAggBlock + 1) + atomicAdd(&waiting, 1u)] =
                 uint32_t(split) << 1 | uint32_t(left ? 0 : 1);
@@ -298,6 +299,10 @@ __global__ void __launch_bounds__(kAggBlock, kAggMinBlocks) agg_in_blocks(agg_ar
 
 constexpr int kAggTopBlock = 128;
 
+// Bound by the chain of dependent memory accesses of a step, so a step is two of them: the
+// atomic, which is also the fence, and the other side's mail, which carries the delta at
+// its far end.  With fences around the atomic and the deltas from the codes a refit of
+// 5,003 triangles took 58.8 us, now 49.9; of 1,000,000 174 -> 153 us.
 template <bool Segmented>
 __global__ void __launch_bounds__(kAggTopBlock) agg_across_blocks(agg_args a, uint32_t num_blocks)
 {
@@ -309,33 +314,35 @@ __global__ void __launch_bounds__(kAggTopBlock) agg_across_blocks(agg_args a, ui
         const uint32_t w = a.waiting[uint64_t(block) * (kAggBlock + 1) + i];
         int m = int(w >> 1);
         bool left = !(w & 1u);
-        int lo = 0, hi = int(a.n), inner_base = 0;
+        int lo = 0, inner_base = 0;
         if (Segmented)
         {
             const uint32_t s = upper_segment(a.offsets, a.num_scenes, uint32_t(left ? m : m + 1));
             lo = int(__ldg(&a.offsets[s]));
-            hi = int(__ldg(&a.offsets[s + 1]));
             inner_base = int(__ldg(&a.inner_offsets[s]));
         }
-        // (the mail written by the kernel before needs no fence)
         for (;;)
         {
             agg_slot* slot = a.slots + m;
-            if (atomicOr(&a.flags[m], left ? 1u : 2u) == 0) break;   // the other side goes on
-            __threadfence();
+            // releases this side's mail (the kernel before wrote the first), acquires the other's
+            uint32_t seen;
+            asm volatile("atom.acq_rel.gpu.global.or.b32 %0, [%1], %2;"
+                         : "=r"(seen)
+                         : "l"(&a.flags[m]), "r"(left ? 1u : 2u)
+                         : "memory");
+            if (seen == 0) break;   // the other side goes on
             const agg_mail lm = { __ldcg(&slot->side[0].a), __ldcg(&slot->side[0].b) };
             const agg_mail rm = { __ldcg(&slot->side[1].a), __ldcg(&slot->side[1].b) };
             const int l = __float_as_int(lm.b.z), r = __float_as_int(rm.b.z);
-            const int pl = neighbour_delta(a.codes, l - 1, lo, hi), pr = neighbour_delta(a.codes, r, lo, hi);
-            const bool root = pl < 0 && pr < 0;
+            const int pl = __float_as_int(lm.b.w) >> 8, pr = __float_as_int(rm.b.w) >> 8;   // + 1
+            const bool root = pl == 0 && pr == 0;
             left = pr > pl;
             box3 b;
             int height;
             agg_make_node<Segmented>(a, lo, inner_base, l, r, m, root, left, lm, rm, b, height);
             if (root) break;
             m = left ? r : l - 1;
-            a.slots[m].side[left ? 0 : 1] = pack_mail(b, left ? l : r, height);
-            __threadfence();
+            a.slots[m].side[left ? 0 : 1] = pack_mail(b, left ? l : r, height | (left ? pl : pr) << 8);
         }
     }
 }
