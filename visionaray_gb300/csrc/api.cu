@@ -41,14 +41,16 @@ gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
 
 // cudaMalloc and cudaFree of a tree's arrays took 1.2 of the 2.4 ms of building a tree of
 // 8.4 M triangles and destroying it, and half of the time at a few thousand triangles.
-// They come from a memory pool of the context instead.  It keeps at most kPoolKeep bytes
+// They come from a memory pool of the context instead, except for its first tree, often its
+// only one, which would wait for the pool to be made (a context's first build of 5,003
+// triangles 374 us with the pool, 266 without; of 8.4 M 3.22 and 2.58 ms).  The pool keeps at most kPoolKeep bytes
 // (whatever is above goes back to the system when the device next synchronises) and is
 // destroyed with the context; trees that outlive it keep their memory until they are
 // destroyed.  The pool itself is safe for trees destroyed by other threads.
 gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
 {
     if (bvh->arena || n == 0) return GBRT_OK;
-    if (!ctx->pool)
+    if (!ctx->pool && ctx->built_tree)
     {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
@@ -62,7 +64,12 @@ gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
     const size_t nodes = up(size_t(n - 1) * sizeof(bvh2_node)), tris = up(size_t(n) * sizeof(tri48)),
                  words = up(size_t(n) * 4), quads = up(size_t(n) * sizeof(quad_node));
     void* p = nullptr;
-    GBRT_CUDA(ctx, cudaMallocFromPoolAsync(&p, nodes + quads + tris + 2 * words, ctx->pool, ctx->stream));
+    const size_t bytes = nodes + quads + tris + 2 * words;
+    if (ctx->pool)
+        GBRT_CUDA(ctx, cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream));
+    else
+        GBRT_CUDA(ctx, cudaMalloc(&p, bytes));
+    ctx->built_tree = true;
     char* base = static_cast<char*>(p);
     bvh->arena = p;
     bvh->nodes = n > 1 ? reinterpret_cast<bvh2_node*>(base) : nullptr;

@@ -42,9 +42,10 @@ struct gbrt_context
     uint32_t* d_status = nullptr;     // one word of status bits
 
     // Device memory of the trees this context builds: a pool that keeps up to kPoolKeep
-    // bytes of freed trees for the next ones (api.cu, alloc_tree), made at the first build.
+    // bytes of freed trees for the next ones (api.cu, alloc_tree), made at the second build.
     static constexpr uint64_t kPoolKeep = 4ull << 30;
     cudaMemPool_t pool = nullptr;
+    bool built_tree = false;
     // What a build reports to the host, written by its last kernels straight into mapped
     // pinned memory: one synchronisation and no copies at the end of a build.
     gbrt::build_result* h_result = nullptr;
