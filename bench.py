@@ -46,11 +46,11 @@ N_NODE_AO, N_TRI_AO = 65.19375747, 6.29761556             # B_ray = 2436.5 bytes
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, mean of two
 # launches each in one ncu capture of the full-size workload with the default ray
 # order and the shipped kernel build).
-TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.705e9 + 0.201e9, 2.642e9 + 0.542e9
+TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.971e9 + 0.129e9, 3.686e9 + 0.717e9
 # L1 <-> L2 bytes per launch of the same kernels (lts__t_sectors_srcunit_tex_op_read.sum
 # + lts__t_sectors_srcunit_tex_op_write.sum, 32-byte sectors; one single-pass ncu
 # capture of the full-size workload).
-L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (336.27e6 + 45.39e6) * 32, (878.37e6 + 37.64e6) * 32
+L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (201.90e6 + 4.19e6) * 32, (675.85e6 + 31.08e6) * 32
 
 
 # Algorithmic bytes per path-traced sample, B_sample = sum of B_ray over the sample's
@@ -551,7 +551,7 @@ def run_batch(vg, ctx, steps, plain_steps, rprint, num_scenes=512, max_tris=1_00
            "images_bit_identical": identical, "image_mean": round(mean, 5)}
     peak, kind = measured_hbm_peak()
     res["roofline"] = roofline_of(samples, frame_ms * 1e-3, B_SAMPLE_BATCH, peak, f"{kind} hbm_gbs",
-                                  "the persistent frame kernel (batch_pt) alone")
+                                  "the frame alone (its wavefront kernels, or batch_pt)")
     if cpu and world == 1 and (num_scenes, max_tris) == (512, 1_000_000):
         res["cpu_baseline"] = batch_cpu_baseline(tris_host, offsets, cams, params, mats)
     batch.close()
@@ -611,7 +611,7 @@ def run_adjoint(ctx, steps, rprint, flags=0, builder="ploc", cpu=False):
         "forward": roofline_of(samples, r["fwd_ms"] * 1e-3, B_SAMPLE_INVERSE, l2, "L2 measured in this run (best of copy, in-place add, sum)",
                                "forward frame (gbrt_pathtrace_forward)", bound="l2"),
         "backward": roofline_of(samples, r["bwd_ms"] * 1e-3, B_SAMPLE_INVERSE, l2, "L2 measured in this run (best of copy, in-place add, sum)",
-                                "path-replay kernel (replays the forward's segments)", bound="l2")}
+                                "backward pass (replays the forward's segments, then sweeps)", bound="l2")}
     if cpu:
         from visionaray_gb300 import scenes
         tris, mats, lights = scenes.box_scene(n_blobs=204, subdiv=1, seed=1)
@@ -781,7 +781,9 @@ def run_ours(args):
                      "launches_timed": len(kms)}
     d = per["closest"]
     default_cfg = (args.grid, args.origins, args.trace_flags) == (GRID, ORIGINS, 1)
-    roofline = {"bound": "hbm", "kernel": ("trace_rays_permuted<0, 0>" if args.trace_flags & 1 else "trace_rays<0, 0>"),
+    # (sorted or not, GPU-built trees are traced through their quad nodes)
+    kernel = "trace_quads<0>" if args.trace_flags & ~1 == 0 else "trace_rays_permuted<0, ...>"
+    roofline = {"bound": "hbm", "kernel": kernel,
                 "achieved": d["achieved_gbs"], "peak": peak, "unit": "GB/s",
                 "frac": round(d["achieved_gbs"] / peak, 4),
                 "traffic": TRAFFIC_CLOSEST if default_cfg else None,
@@ -789,7 +791,8 @@ def run_ours(args):
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "b_ray": round(b_ray(N_NODE_CLOSEST, N_TRI_CLOSEST), 1),
                 "timing": "CUDA events around the traversal kernel on its stream, mean over the timed launches",
-                "limiter": "latency of dependent node fetches under divergence (ncu: DRAM ~14 % of peak at full size)"}
+                "limiter": "load/store wavefronts and issue slots of divergent node visits (ncu: DRAM ~24 % of "
+                           "peak at full size)"}
     # the pure-I/O floor (48 B per ray: the ray in, the hit out) and the DRAM bandwidth
     # the launch actually drew (its ncu traffic over its event time)
     io_gbs = d["rays"] * 48 / (d["kernel_ms_per_launch"] * 1e-3) / 1e9

@@ -217,7 +217,7 @@ gbrt_status gbrt_bvh_refit(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const
  * the device.  No counterpart in visionaray (its builder always allocates,
  * detail/bvh/lbvh.h:693-834).  Same tree as gbrt_bvh_build_lbvh + gbrt_bvh_export_bvh2:
  * d_nodes receives 2n-1 nodes, d_indices n indices (device buffers of the caller).
- * All temporaries live in one fixed device array of this library (about 10 MB, held
+ * All temporaries live in one fixed device array of this library (about 14 MB, held
  * by every GPU that loads it until exit), so n is limited to 65,536 triangles
  * (GBRT_ERR_TOO_LARGE beyond).  Calls share that array: consecutive calls on a stream
  * are independent, calls that overlap on the GPU race.  The first call on a device

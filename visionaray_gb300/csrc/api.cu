@@ -43,10 +43,10 @@ gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
 // 8.4 M triangles and destroying it, and half of the time at a few thousand triangles.
 // They come from a memory pool of the context instead, except for its first tree, often its
 // only one, which would wait for the pool to be made (a context's first build of 5,003
-// triangles 374 us with the pool, 266 without; of 8.4 M 3.22 and 2.58 ms).  The pool keeps at most kPoolKeep bytes
-// (whatever is above goes back to the system when the device next synchronises) and is
-// destroyed with the context; trees that outlive it keep their memory until they are
-// destroyed.  The pool itself is safe for trees destroyed by other threads.
+// triangles 374 us with the pool, 266 without; of 8.4 M 3.22 and 2.58 ms).  The pool keeps
+// at most kPoolKeep bytes (whatever is above goes back to the system when the device next
+// synchronises) and is destroyed with the context; trees that outlive it keep their memory
+// until they are destroyed.  The pool itself is safe for trees destroyed by other threads.
 gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
 {
     if (bvh->arena || n == 0) return GBRT_OK;
