@@ -87,21 +87,20 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) bp_trace_quads(bat
     __shared__ int stack_mem[kQuadStack * kQuadBlock];
     const bool closest = extend != 0 && blockIdx.y == 0;
     const uint32_t n = closest ? fb.counts[2 * bounce] : fb.counts[2 * bounce - 1];
-    const uint32_t span = quad_span(n, resident);
-    const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
-    if (first >= n) return;
-    const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
+    const quad_work work = quad_share(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5), n, resident,
+                                      fb.taken + (closest ? 2 * bounce : 2 * bounce - 1));
+    if (work.next >= work.end) return;
     auto index = [](uint32_t k) { return k; };
     if (closest)
         quad_trace<false, true, kQuadPathSteps>(
-            stack_mem, v, bad, fb.rays[q], n, next, end, status,
+            stack_mem, v, bad, fb.rays[q], n, work, status,
             [&](uint32_t j) { return a.frames[a.scene[fb.path[q][j]]].root; }, index,
             [&](uint32_t j, trace_result const& h) {
                 fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
             });
     else
         quad_trace<true, true, kQuadPathSteps>(
-            stack_mem, v, bad, fb.shadow_rays, n, next, end, status,
+            stack_mem, v, bad, fb.shadow_rays, n, work, status,
             [&](uint32_t j) { return a.frames[a.scene[fb.shadow_path[j]]].root; }, index,
             [&](uint32_t j, trace_result const& h) { finish_shadow(fb, j, bounce - 1, h.tri >= 0); });
 }
@@ -291,14 +290,14 @@ gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, c
             fb.samples = std::min(ps.samples, b->max_spp - smp);
             const uint32_t n = pixels * fb.samples, blocks = (n + kBlock - 1) / kBlock;
             const uint32_t shade_blocks = std::min(blocks, uint32_t(ctx->num_sms) * kShadeMinBlocks * 4);
-            const uint32_t grid = (quad_max_warps(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+            const uint32_t grid = (std::min(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
             auto trace = [&](int q, uint32_t bounce, bool extend, bool shadow) -> gbrt_status {
                 bp_trace_quads<<<dim3(grid, extend && shadow ? 2 : 1), kQuadBlock, 0, s>>>(
                     a, fb, q, bounce, extend ? 1u : 0u, v, bad, resident, ctx->d_status);
                 GBRT_LAUNCH_CHECK(ctx, "bp_trace_quads");
                 return GBRT_OK;
             };
-            GBRT_CUDA(ctx, cudaMemsetAsync(fb.counts, 0, size_t(num_counts) * 4, s));
+            GBRT_CUDA(ctx, cudaMemsetAsync(fb.counts, 0, size_t(num_counts) * 8, s));
             bp_raygen<<<blocks, kBlock, 0, s>>>(a, fb, n);
             GBRT_LAUNCH_CHECK(ctx, "bp_raygen");
             int q = 0;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t n
                                                     camera_basis cam)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    for (uint32_t k = i; k < num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
+    for (uint32_t k = i; k < 2 * num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
     if (i >= n) return;
     const uint2 ps = path_sample(fb, i);
     v3 d = primary_dir(cam, width, height, frame, ps.x, ps.y);
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t n
 // The traversal of one bounce over the quad nodes: the closest hits of its ray queue
 // (blocks of row 0 when extend is set) and the shadow rays of the bounce before (the other
 // row).  Both queues' lengths are on the device; the grid holds the most warps that any
-// length takes, each warp finds its span from the length.
+// length takes, each warp finds its share from the length.
 __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(frame_buffers fb, int q, uint32_t bounce,
                                                                              uint32_t extend, bvh_view v,
                                                                              uint32_t resident,
@@ -92,19 +92,18 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(fra
     __shared__ int stack_mem[kQuadStack * kQuadBlock];
     const bool closest = extend != 0 && blockIdx.y == 0;
     const uint32_t n = closest ? fb.counts[2 * bounce] : fb.counts[2 * bounce - 1];
-    const uint32_t span = quad_span(n, resident);
-    const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
-    if (first >= n) return;
-    const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
+    const quad_work work = quad_share(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5), n, resident,
+                                      fb.taken + (closest ? 2 * bounce : 2 * bounce - 1));
+    if (work.next >= work.end) return;
     auto index = [](uint32_t k) { return k; };
     auto root = [&](uint32_t) { return v.root; };
     if (closest)
-        quad_trace<false, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.rays[q], n, next, end, status, root, index,
+        quad_trace<false, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.rays[q], n, work, status, root, index,
                                 [&](uint32_t j, trace_result const& h) {
                                     fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
                                 });
     else
-        quad_trace<true, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.shadow_rays, n, next, end, status, root, index,
+        quad_trace<true, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.shadow_rays, n, work, status, root, index,
                                [&](uint32_t j, trace_result const& h) {
                                    finish_shadow(fb, j, bounce - 1, h.tri >= 0);
                                });
@@ -1154,7 +1153,7 @@ gbrt_status with_tracer(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_pt_p
         const uint32_t resident = uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32);
         auto trace = [&](frame_buffers const& fb, int q, uint32_t b, uint32_t n, bool extend,
                          bool shadow) -> gbrt_status {
-            const uint32_t grid = (quad_max_warps(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+            const uint32_t grid = (std::min(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
             pt_trace_quads<<<dim3(grid, extend && shadow ? 2 : 1), kQuadBlock, 0, s>>>(fb, q, b, extend ? 1u : 0u, v,
                                                                                        resident, ctx->d_status);
             GBRT_LAUNCH_CHECK(ctx, "pt_trace_quads");

@@ -9,9 +9,9 @@
 //     the visits (and half the wavefronts);
 //   - every round runs the leaf tests of the lanes that stand at a leaf, then advances each
 //     busy lane by two or three nodes, so no lane waits for a whole descent;
-//   - a warp owns a span of rays and refills its idle lanes from it.
+//   - a warp refills its idle lanes from its rays, and takes more of them when they run out.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 2.10 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.31 ms.  What
+// query 3.36 -> 1.81 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.17 ms.  What
 // bounds it now (a bounce of a 1920 x 1080 path-traced frame): the load/store pipe's
 // wavefronts (80 %), two per lane and node, then issue slots (72 %).
 //
@@ -65,9 +65,10 @@ constexpr int kQuadPathSteps = 2;
 // 65,536 triangles 65 us one per warp, 87 us four per warp).  Beyond that, lanes that
 // advance together pay more than warps (16,384 rays: 88 us sixteen per warp, 100 three per
 // warp; 65,536: 104 us 32 per warp, 132 twelve): about 3/4 of the resident warps, at least
-// half to fully occupied ones.  Long queries go in up to 2 1/4 waves of spans of 128 to
-// 256, which the block scheduler balances (1,048,576 secondary rays: 637 us at 128, 684 at
-// 64, 687 at 256; 4.2 M: 2.60 ms at 128, 2.49 at 256).
+// half to fully occupied ones.  Where no counter is there to share long queries by
+// (quad_share), they go in up to 2 1/4 waves of spans of 128 to 256, which the block
+// scheduler balances (1,048,576 secondary rays: 637 us at 128, 684 at 64, 687 at 256; 4.2 M:
+// 2.60 ms at 128, 2.49 at 256).
 __host__ __device__ __forceinline__ uint32_t quad_span(uint32_t n, uint32_t resident)
 {
     if (n <= resident) return 1;
@@ -83,12 +84,41 @@ __host__ __device__ __forceinline__ uint32_t quad_span(uint32_t n, uint32_t resi
     return many < 128 ? 128 : (many > 256 ? 256 : many);
 }
 
-// The most warps that any ray count up to n takes at quad_span of that count.
-__host__ __forceinline__ uint32_t quad_max_warps(uint32_t n, uint32_t resident)
+// Rays that a warp takes at a time off a shared counter when there are more than kQuadChunk
+// for each resident warp: a warp that got long rays takes fewer, and the launch ends
+// together.  Against fixed spans: 400,000 sorted secondary rays 378 -> 351 us, 1,000,000 636
+// -> 549, 4,194,304 2,096 -> 1,810; camera rays 640^2 200 -> 163, 1024^2 320 -> 281, 2048^2
+// 1,022 -> 1,037; high-definition frame 44.3 -> 41.5 ms, batch of scenes 8.83 -> 7.70.  48
+// and 64 at a time are up to 5 % slower at a few hundred thousand rays, 1 % faster on ambient
+// occlusion; 128 slower.
+constexpr uint32_t kQuadChunk = 32;
+
+// A warp's rays: next .. end - 1 first, then, unless shared is 0, chunks below `shared`
+// (the number of rays) from `first` + what the counter says.
+struct quad_work
 {
-    const uint64_t long_spans = uint64_t(n) / 256 + 1, waves = uint64_t(resident) * 9 / 4 + 1;
-    const uint64_t cap = long_spans > waves ? long_spans : waves;
-    return uint32_t(n < cap ? n : cap);
+    uint32_t next, end, shared, first;
+    uint32_t* taken;
+};
+
+__host__ __device__ __forceinline__ bool quad_shared(uint32_t n, uint32_t resident)
+{
+    return n > resident * kQuadChunk && n < 0xF0000000u;   // chunks past the end do not wrap
+}
+
+// The work of one warp (empty: next >= end).  taken: a zeroed counter, or null.
+__device__ __forceinline__ quad_work quad_share(uint32_t warp, uint32_t n, uint32_t resident, uint32_t* taken)
+{
+    if (taken && quad_shared(n, resident))
+    {
+        if (warp >= resident) return { 0, 0, 0, 0, nullptr };
+        return { warp * kQuadChunk, (warp + 1) * kQuadChunk, n, resident * kQuadChunk, taken };
+    }
+    const uint32_t span = quad_span(n, resident);
+    const uint64_t first = uint64_t(warp) * span;
+    if (first >= n) return { 0, 0, 0, 0, nullptr };
+    const uint32_t next = uint32_t(first);
+    return { next, n - next < span ? n : next + span, 0, 0, nullptr };
 }
 
 __device__ __forceinline__ float max3f(float a, float b, float c)
@@ -129,18 +159,18 @@ __device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d)
            (ax >= low || ax == 0.0f) && (ay >= low || ay == 0.0f) && (az >= low || az == 0.0f);
 }
 
-// Traces the rays index(next .. end - 1) of `rays` with the calling warp (every lane must
-// call it with the same next and end) and calls done(ray, result) for each, in any order
+// Traces the rays index(k) of `rays` for the k of `work` with the calling warp (every lane
+// must call it with the same work) and calls done(ray, result) for each, in any order
 // and from any lane.  index(k) below n is a ray, root(ray) the link its walk starts from.
 // stack_mem: kQuadStack * kQuadBlock shared words of the block.  bad: null when the host
 // knows the quads valid, else their validity word (the last record's org[0]): when it is
 // set every ray takes the pair loop.
 template <bool AnyHit, bool NearFirst, int Steps, class Root, class Index, class Done>
 __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, const float* __restrict__ bad,
-                                           const gbrt_ray* __restrict__ rays, uint32_t n, uint32_t next,
-                                           const uint32_t end, uint32_t* __restrict__ status, Root root, Index index,
-                                           Done done)
+                                           const gbrt_ray* __restrict__ rays, uint32_t n, quad_work work,
+                                           uint32_t* __restrict__ status, Root root, Index index, Done done)
 {
+    uint32_t next = work.next, end = work.end;
     constexpr int kDeep = INT32_MAX;   // best_tri of a ray that the pair loop answers
     const uint32_t full = 0xFFFFFFFFu, none = 0xFFFFFFFFu;
     const uint32_t lane_bit = 1u << (threadIdx.x & 31u);
@@ -242,6 +272,15 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
         const bool leaf = uint32_t(~node) < uint32_t(v.num_tris);
         const uint32_t leaves = __ballot_sync(full, leaf);
         const uint32_t busy = __ballot_sync(full, leaf || uint32_t(node) < uint32_t(v.num_inner));
+        if (next >= end && end < work.shared && 32 - __popc(busy) >= kQuadRefill)
+        {
+            // end == shared once the rays are out
+            uint32_t taken = 0;
+            if (lane_bit == 1u) taken = atomicAdd(work.taken, kQuadChunk);
+            taken = __shfl_sync(full, taken, 0);
+            next = min(work.first + taken, work.shared);
+            end = min(next + kQuadChunk, work.shared);
+        }
         if (busy == 0 || (next < end && 32 - __popc(busy) >= kQuadRefill))
         {
             if (!(busy & lane_bit))

@@ -88,21 +88,20 @@ __global__ void __launch_bounds__(kTraceBlock, AnyHit ? kMinBlocksAny : kMinBloc
         make_uint4(prim, __float_as_uint(h.t), __float_as_uint(h.u), __float_as_uint(h.v));
 }
 
-// The ray queries over the quad nodes: warp w of the grid traces the span [w span, (w + 1)
-// span) of the rays, in the order perm if there is one.
+// The ray queries over the quad nodes, in the order perm if there is one.  taken: the zeroed
+// counter that long queries are shared by, or null.
 template <bool AnyHit>
 __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_view v, const gbrt_ray* __restrict__ rays,
-                                                                          uint32_t n, uint32_t span,
+                                                                          uint32_t n, uint32_t resident, uint32_t* taken,
                                                                           const uint32_t* __restrict__ perm,
                                                                           gbrt_hit* __restrict__ hits,
                                                                           uint32_t* __restrict__ status)
 {
     __shared__ int stack_mem[kQuadStack * kQuadBlock];
-    const uint64_t first = uint64_t(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5)) * span;
-    if (first >= n) return;
-    const uint32_t next = uint32_t(first), end = n - next < span ? n : next + span;
+    const quad_work work = quad_share(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5), n, resident, taken);
+    if (work.next >= work.end) return;
     quad_trace<AnyHit, !AnyHit, kQuadQuerySteps>(
-        stack_mem, v, nullptr, rays, n, next, end, status, [&](uint32_t) { return v.root; },
+        stack_mem, v, nullptr, rays, n, work, status, [&](uint32_t) { return v.root; },
         [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
         [&](uint32_t j, trace_result const& h) {
             const uint32_t prim = h.tri >= 0 ? __float_as_uint(ldg4(&v.tris[h.tri].t0).w) : GBRT_NO_HIT;
@@ -350,11 +349,23 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
     // of one triangle and trees whose boxes the quads do not cover
     const bool quads = bvh->quads_ok && !wide && !compressed && !wide8 && !persistent;
     auto launch_quads = [&](const uint32_t* order) -> gbrt_status {
-        const uint32_t span = quad_span(n, uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32));
-        const uint32_t grid = (uint32_t((uint64_t(n) + span - 1) / span) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
+        const uint32_t resident = uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32);
+        uint32_t* taken = nullptr;
+        uint32_t warps = resident;
+        if (have_scratch && quad_shared(n, resident))
+        {
+            taken = static_cast<uint32_t*>(scratch);
+            GBRT_CUDA(ctx, cudaMemsetAsync(taken, 0, 4, stream));
+        }
+        else
+        {
+            const uint32_t span = quad_span(n, resident);
+            warps = uint32_t((uint64_t(n) + span - 1) / span);
+        }
+        const uint32_t grid = (warps + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
         kernel_timer timer(ctx, stream);
         auto kernel = any_hit ? trace_quads<true> : trace_quads<false>;
-        kernel<<<grid, kQuadBlock, 0, stream>>>(v, d_rays, n, span, order, d_hits, ctx->d_status);
+        kernel<<<grid, kQuadBlock, 0, stream>>>(v, d_rays, n, resident, taken, order, d_hits, ctx->d_status);
         GBRT_LAUNCH_CHECK(ctx, "trace_quads");
         return GBRT_OK;
     };

@@ -28,6 +28,7 @@ struct frame_buffers
     uint2* rng_flags;   // draw counter, flags
     float4* sum;
     uint32_t* counts;   // per bounce: its ray queue's length, its shadow queue's
+    uint32_t* taken;    // per queue: rays taken by warps beyond their first (quad_share)
     // path p of the pass is sample first_sample + p % samples of pixel first_pixel + p / samples
     uint32_t first_pixel, samples, first_sample;
     // the adjoint's replay: per bounce and path a vertex_rec in kRecWords float4
@@ -138,7 +139,7 @@ inline size_t layout_frame_buffers(uint32_t npix, uint32_t n, uint32_t num_count
     const size_t key = sort ? size_t(n) * 4 : 0;
     size_t sizes[] = { size_t(n) * 32, size_t(n) * 32, size_t(n) * 4, size_t(n) * 4, size_t(n) * 16,
                        size_t(n) * 32, size_t(n) * 4,  size_t(n) * 16, size_t(n) * 16, size_t(n) * 16,
-                       size_t(n) * 8,  size_t(npix) * 16, size_t(num_counts) * 4, key, key, key,
+                       size_t(n) * 8,  size_t(npix) * 16, size_t(num_counts) * 8, key, key, key,
                        key, sort ? radix_sort_scratch_bytes(n) : 0,
                        size_t(n) * record_bounces * kRecWords * 16, record_bounces ? size_t(n) * 4 : 0 };
     constexpr int kParts = int(sizeof(sizes) / sizeof(sizes[0]));
@@ -165,6 +166,7 @@ inline size_t layout_frame_buffers(uint32_t npix, uint32_t n, uint32_t num_count
     fb.rng_flags = static_cast<uint2*>(ptr[10]);
     fb.sum = static_cast<float4*>(ptr[11]);
     fb.counts = static_cast<uint32_t*>(ptr[12]);
+    fb.taken = fb.counts + num_counts;
     fb.keys = static_cast<uint32_t*>(ptr[13]);
     fb.vals = static_cast<uint32_t*>(ptr[14]);
     fb.keys_alt = static_cast<uint32_t*>(ptr[15]);
