@@ -46,11 +46,11 @@ N_NODE_AO, N_TRI_AO = 65.19375747, 6.29761556             # B_ray = 2436.5 bytes
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, mean of two
 # launches each in one ncu capture of the full-size workload with the default ray
 # order and the shipped kernel build).
-TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.971e9 + 0.129e9, 3.686e9 + 0.717e9
+TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.177e9 + 0.127e9, 2.417e9 + 0.544e9
 # L1 <-> L2 bytes per launch of the same kernels (lts__t_sectors_srcunit_tex_op_read.sum
 # + lts__t_sectors_srcunit_tex_op_write.sum, 32-byte sectors; one single-pass ncu
 # capture of the full-size workload).
-L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (201.90e6 + 4.19e6) * 32, (675.85e6 + 31.08e6) * 32
+L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (195.53e6 + 4.19e6) * 32, (737.45e6 + 31.39e6) * 32
 
 
 # Algorithmic bytes per path-traced sample, B_sample = sum of B_ray over the sample's
@@ -791,7 +791,7 @@ def run_ours(args):
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "b_ray": round(b_ray(N_NODE_CLOSEST, N_TRI_CLOSEST), 1),
                 "timing": "CUDA events around the traversal kernel on its stream, mean over the timed launches",
-                "limiter": "load/store wavefronts and issue slots of divergent node visits (ncu: DRAM ~24 % of "
+                "limiter": "load/store wavefronts and issue slots of divergent node visits (ncu: DRAM ~21 % of "
                            "peak at full size)"}
     # the pure-I/O floor (48 B per ray: the ray in, the hit out) and the DRAM bandwidth
     # the launch actually drew (its ncu traffic over its event time)
