@@ -11,7 +11,7 @@
 //     busy lane by two or three nodes, so no lane waits for a whole descent;
 //   - a warp refills its idle lanes from its rays, and takes more of them when they run out.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 1.81 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.17 ms.  What
+// query 3.36 -> 1.73 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.10 ms.  What
 // bounds it now (a bounce of a 1920 x 1080 path-traced frame): the load/store pipe's
 // wavefronts (80 %), two per lane and node, then issue slots (72 %).
 //
@@ -47,15 +47,17 @@ namespace gbrt {
 constexpr int kQuadBlock = 128;
 constexpr int kQuadStack = 32;
 // Resident blocks the register allocation must allow: 9 (36 warps, 56 registers, no
-// spills).  Heightfield closest hit 2.10 ms; 2.18 at 10 blocks (48 registers, spilling).
+// spills).  Heightfield closest hit 1.79 ms; 1.86 at 8 blocks; with fixed spans 2.10, 2.18 at
+// 10 blocks (48 registers, spilling).
 constexpr int kQuadMinBlocks = 9;
-// Idle lanes of a warp that trigger a refill (6 and 10 within 1 %, 4 and 12 slower).
+// Idle lanes of a warp that trigger a refill (6 and 11 within 1 %, 4 up to 3 % slower).
 constexpr int kQuadRefill = 8;
 // Node steps per round, after the leaf tests of the lanes that stand at one (waiting for
 // several such lanes costs more than it saves: any 44.4 ms per high-definition frame, two
-// 44.6, three 44.9).  Ray queries take three (heightfield closest hit 2.15 ms at two, 2.10 at
-// three, 2.09 at four; 8.4 M ambient-occlusion rays 2.35, 2.31, 2.33), the path tracer two
-// (three: high-definition frame 44.4 -> 44.1 ms, forward and backward 32.3 -> 33.0).
+// 44.6, three 44.9).  Ray queries take three (heightfield closest hit 1.84 ms at two, 1.79 at
+// three, 1.78 at four; 8.4 M ambient-occlusion rays 2.20, 2.16, 2.18), the path tracer two
+// (three: high-definition frame 41.4 -> 41.5 ms, forward and backward 31.4 -> 32.2, batch of
+// scenes 7.72 -> 7.63).
 constexpr int kQuadQuerySteps = 3;
 constexpr int kQuadPathSteps = 2;
 
