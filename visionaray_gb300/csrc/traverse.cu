@@ -280,11 +280,17 @@ __global__ void __launch_bounds__(kTraceBlock) trace_rays_dynamic(bvh_view v, co
 // pass: cells of 2 bits per axis, any hit 1 bit and the octant.  24 / 21 bits (three passes)
 // against 15 (two) and 6: 4.2 M secondary rays over 8.4 M triangles 1,794, 1,759, 1,726 us;
 // 8.4 M ambient-occlusion rays 2,164, 2,112, 2,098; 200,000 secondary rays 272, 249, 242;
-// 2.1 M uniform rays into 4 M random triangles 1,583, 1,533, 1,508 (unsorted 2,030).
+// 2.1 M uniform rays into 4 M random triangles 1,583, 1,533, 1,508 (unsorted 2,030).  Of
+// many any-hit rays a fine cell holds enough for a whole warp: above kQuadManyRays they
+// have 4 bits per axis and the octant, two passes (8.4 M triangles: 33.6 M rays 8.88 -> 8.35
+// ms, 16.8 M 4.59 -> 4.30, 4.2 M 1.263 -> 1.268; 2.1 M triangles: 16.8 M rays 4.06 -> 4.05,
+// 8.4 M 2.10 -> 2.12).
 constexpr int kCellBitsClosest = 8;
 constexpr int kCellBitsAny = 6;
 constexpr int kQuadCellBitsClosest = 2;
 constexpr int kQuadCellBitsAny = 1;
+constexpr int kQuadCellBitsAnyMany = 4;
+constexpr uint32_t kQuadManyRays = 1u << 23;
 
 // The sort key of each ray (above): cell_bits per axis, then the octant if asked.
 __global__ void __launch_bounds__(kTraceBlock) ray_origin_keys(const gbrt_ray* __restrict__ rays, uint32_t n,
@@ -388,7 +394,8 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
         uint32_t* vals_alt = reinterpret_cast<uint32_t*>(base + 3 * w);
         float3 lo = make_float3(bvh->lo[0], bvh->lo[1], bvh->lo[2]);
         float ext[3] = { bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2] };
-        const int cell_bits = quads ? (any_hit ? kQuadCellBitsAny : kQuadCellBitsClosest)
+        const int any_bits = n > kQuadManyRays ? kQuadCellBitsAnyMany : kQuadCellBitsAny;
+        const int cell_bits = quads ? (any_hit ? any_bits : kQuadCellBitsClosest)
                                     : (any_hit ? kCellBitsAny : kCellBitsClosest);
         const float cells = float(1 << cell_bits);
         float3 scale = make_float3(ext[0] > 0.0f ? cells / ext[0] : 0.0f, ext[1] > 0.0f ? cells / ext[1] : 0.0f,
