@@ -46,11 +46,11 @@ N_NODE_AO, N_TRI_AO = 65.19375747, 6.29761556             # B_ray = 2436.5 bytes
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, mean of two
 # launches each in one ncu capture of the full-size workload with the default ray
 # order and the shipped kernel build).
-TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.177e9 + 0.127e9, 2.417e9 + 0.544e9
+TRAFFIC_CLOSEST, TRAFFIC_ANY = 2.265e9 + 0.127e9, 2.420e9 + 0.544e9
 # L1 <-> L2 bytes per launch of the same kernels (lts__t_sectors_srcunit_tex_op_read.sum
 # + lts__t_sectors_srcunit_tex_op_write.sum, 32-byte sectors; one single-pass ncu
 # capture of the full-size workload).
-L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (195.53e6 + 4.19e6) * 32, (737.45e6 + 31.39e6) * 32
+L2_TRAFFIC_CLOSEST, L2_TRAFFIC_ANY = (254.94e6 + 4.18e6) * 32, (806.15e6 + 31.38e6) * 32
 
 
 # Algorithmic bytes per path-traced sample, B_sample = sum of B_ray over the sample's
