@@ -2,7 +2,8 @@
 time: at and around the line where that starts (32 rays for each of the resident warps, 36
 per multiprocessor), one ray more, a partial last chunk and several chunks per warp, sorted
 and in input order, every ray gets the node pairs' answer, byte for byte, and the hits past
-the last ray stay untouched."""
+the last ray stay untouched; any-hit queries likewise on both sides of 2^23 rays, where the
+keys of their order change."""
 import numpy as np
 import pytest
 import torch
@@ -37,3 +38,19 @@ def test_shared_queries_equal_pairs(extra, sort):
         query(d, pairs, out=want[:n])
         ctx.synchronize()
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("n", [1 << 23, (1 << 23) + 1])
+def test_the_finer_order_of_many_any_hit_rays(n):
+    ctx = vg.Context(0)
+    ctx.set_trace_flags(vg.Context.TRACE_SORT_RAYS)
+    tris = scenes.soup(500, seed=4, offset=0.05)
+    bvh = vg.lbvh_builder(ctx).build(vg.as_device_bytes(tris))
+    nodes, idx = bvh.export_bvh2()
+    pairs = vg.IndexBVH.upload(nodes, idx, tris, ctx)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rays = torch.rand((n, 8), generator=g, device="cuda") - 0.5
+    rays[:, :3] += 0.5
+    rays[:, 6], rays[:, 7] = 0.0, 3e38
+    assert torch.equal(vg.any_hit(rays, bvh).view(torch.int32), vg.any_hit(rays, pairs).view(torch.int32))
+    ctx.synchronize()
