@@ -35,8 +35,6 @@
 
 namespace gbrt {
 
-constexpr int kAggBlock = 256;
-
 // One side's data at a split: the child's box, the end of its key range away from the
 // split, its height, and between blocks the delta (+ 1) at the far end.
 struct __align__(16) agg_mail
@@ -49,6 +47,7 @@ struct agg_slot
 {
     agg_mail side[2];
 };
+static_assert(sizeof(agg_slot) == 64, "lbvh_scratch_layout_for counts 64 bytes per slot");
 
 struct agg_args
 {
@@ -88,10 +87,6 @@ __device__ __forceinline__ int neighbour_delta(const uint32_t* __restrict__ code
     const uint32_t x = __ldg(&codes[j]) ^ __ldg(&codes[j + 1]);
     return x == 0 ? 32 + __clz(uint32_t(j - lo) ^ uint32_t(j + 1 - lo)) : __clz(x);
 }
-
-// Words of agg_args::waiting and num_waiting for n leaves.
-constexpr uint64_t agg_blocks(uint64_t n) { return (n + kAggBlock - 1) / kAggBlock; }
-constexpr uint64_t agg_waiting_words(uint64_t n) { return agg_blocks(n) * (kAggBlock + 2); }
 
 __device__ __forceinline__ void store8(void* p, float a, float b, float c, float d, float e, float f, float g, float h)
 {

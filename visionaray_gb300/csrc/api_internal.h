@@ -314,6 +314,12 @@ struct lbvh_scratch_layout
 
 constexpr size_t scratch_align(size_t v) { return (v + 255) & ~size_t(255); }
 
+// Leaves of a block of the bottom-up build (agglomerate.cuh), its blocks for n leaves, and
+// the words of agg_args::waiting and num_waiting: one home for every scratch layout.
+constexpr int kAggBlock = 256;
+constexpr uint64_t agg_blocks(uint64_t n) { return (n + kAggBlock - 1) / kAggBlock; }
+constexpr uint64_t agg_waiting_words(uint64_t n) { return agg_blocks(n) * (kAggBlock + 2); }
+
 constexpr lbvh_scratch_layout lbvh_scratch_layout_for(uint32_t n)
 {
     lbvh_scratch_layout l{};
@@ -324,7 +330,7 @@ constexpr lbvh_scratch_layout lbvh_scratch_layout_for(uint32_t n)
     l.keys_alt = o;    o = scratch_align(o + size_t(n) * 4);
     l.vals_alt = o;    o = scratch_align(o + size_t(n) * 4);
     l.flags = o;       o = scratch_align(o + size_t(n) * 4);
-    l.waiting = o;     o = scratch_align(o + (size_t(n) / 512 + 1) * 514 * 4);   // agg_waiting_words
+    l.waiting = o;     o = scratch_align(o + size_t(agg_waiting_words(n)) * 4);
     l.slots = o;       o = scratch_align(o + size_t(n) * 64);   // agg_slot (agglomerate.cuh)
     l.nodes = o;       o = scratch_align(o + size_t(n) * 64);
     l.tris = o;        o = scratch_align(o + size_t(n) * 48);
