@@ -352,10 +352,12 @@ gbrt_status build_lbvh_in_scratch(gbrt_context* ctx, gbrt_triangle const* d_tris
                                   size_t scratch_bytes, gbrt_bvh_node* d_nodes, uint32_t* d_indices);
 
 // quads.cu: the quad nodes of num_inner > 0 node pairs on `stream` (quads holds num_inner + 1
-// records, the last one's org[0] cleared before); enqueue only.  host_bad (may be null): a
-// word that is set if the tree must not be traversed through them.
-gbrt_status make_quads(gbrt_context* ctx, bvh2_node const* nodes, uint32_t num_inner, quad_node* quads,
-                       uint32_t* host_bad, cudaStream_t stream);
+// records, the last one's org[0] cleared before); enqueue only.  The pairs are one tree's with
+// the root pair `root`, or, with roots non-null, those of num_scenes trees, tree s's from its
+// root pair roots[s] on (num_scenes + 1 entries).  host_bad (may be null): a word that is set if
+// the tree must not be traversed through them.
+gbrt_status make_quads(gbrt_context* ctx, bvh2_node const* nodes, uint32_t num_inner, uint32_t const* roots,
+                       uint32_t num_scenes, uint32_t root, quad_node* quads, uint32_t* host_bad, cudaStream_t stream);
 
 // radix_sort.cu: stable LSD sort of (key, value) pairs by the low `key_bits` bits.
 // Result lands in (keys, values); keys_alt/values_alt are same-sized scratch.  With

@@ -252,7 +252,8 @@ gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, c
     if (force_quads || b->quads_gen != b->build_gen)
     {
         GBRT_CUDA(ctx, cudaMemsetAsync(b->quads + b->total_inner, 0, sizeof(quad_node), s));
-        gbrt_status st = make_quads(ctx, b->nodes, b->total_inner, b->quads, nullptr, s);
+        gbrt_status st = make_quads(ctx, b->nodes, b->total_inner, b->d_inner_offsets, b->num_scenes, 0, b->quads,
+                                    nullptr, s);
         if (st != GBRT_OK) return st;
         b->quads_gen = b->build_gen;
     }

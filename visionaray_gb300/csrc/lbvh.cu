@@ -657,7 +657,8 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
         st = agglomerate<false>(ctx, args, s);
         if (st != GBRT_OK) return st;
         ctx->h_result->quads_bad = 0;
-        st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+        st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
+                        &result->quads_bad, s);
         if (st != GBRT_OK) return st;
         report_build<<<1, 1, 0, s>>>(bvh->nodes, root_height, result);
         GBRT_LAUNCH_CHECK(ctx, "report_build");
@@ -799,7 +800,8 @@ gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_
     if (st != GBRT_OK) return st;
     GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
     ctx->h_result->quads_bad = 0;
-    st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+    st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
+                    &result->quads_bad, s);
     if (st != GBRT_OK) return st;
     report_build<<<1, 1, 0, s>>>(bvh->nodes + (bvh->root > 0 ? bvh->root : 0), nullptr, result);
     GBRT_LAUNCH_CHECK(ctx, "report_build");

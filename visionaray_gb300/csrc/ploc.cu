@@ -556,7 +556,8 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     if (n > 1)
     {
         GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
-        st = make_quads(ctx, bvh->nodes, bvh->num_inner, bvh->quads, &result->quads_bad, s);
+        st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
+                        &result->quads_bad, s);
         if (st != GBRT_OK) return st;
     }
     GBRT_CUDA(ctx, cudaStreamSynchronize(s));

@@ -149,16 +149,30 @@ __device__ __forceinline__ bool leaf_box_hit(f3 o, f3 id, float tmin, float tmax
     return fminf(tmax, fminf(fmaxf(lx, hx), fminf(fmaxf(ly, hy), fmaxf(lz, hz)))) >= tn;
 }
 
-// Whether the quads' conservative arithmetic covers a ray: components finite and
-// moderate, each direction component zero or not below 2^-40 of the largest.  Within
-// these bounds 1 / d clamped to 2^64 and the products with it stay normal floats.
-__device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d)
+// The reciprocal of a zero direction component.  The pair loop takes FLT_MAX, with which an
+// axis is entered at -inf and left at inf for any origin between its planes; here the
+// distances have to stay finite, and quad_ray_ok sees to it that they are still beyond
+// those of the other axes.
+constexpr float kQuadZeroRcp = 7.555786372591432e22f;   // 2^76
+__device__ __forceinline__ float quad_rcp(float d) { return d != 0.0f ? __frcp_rn(d) : kQuadZeroRcp; }
+
+// Whether the quads' conservative arithmetic covers a ray that starts from node `root`:
+// components finite and moderate, each direction component zero or not below 2^-40 of the
+// largest.  What overflows within these bounds becomes an infinity or a NaN that leaves its
+// axis unbounded.  With a zero component, an origin between the planes of that axis is
+// inside them by the margin of a step, at least 2^-6.5 cell * 2^76 as a distance; cells are
+// at least 2^-40 of the tree's largest coordinate M (quads.cu), so that is above 2^29.4 M,
+// and the distances along the largest component d are at most (M + |o|) / d: not more than
+// 2^28.1 M for an origin within 2^14 M and d above 2^-14.
+__device__ __forceinline__ bool quad_ray_ok(f3 o, f3 d, bvh_view const& v, int root)
 {
     const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     const float md = fmaxf(fmaxf(ax, ay), az), low = md * 9.094947017729282e-13f;
     const float mo = fabsf(o.x) + fabsf(o.y) + fabsf(o.z);
-    return md >= 9.094947017729282e-13f && md <= 1.099511627776e12f && mo <= 1.152921504606847e18f &&
-           (ax >= low || ax == 0.0f) && (ay >= low || ay == 0.0f) && (az >= low || az == 0.0f);
+    const bool ok = md >= 9.094947017729282e-13f && md <= 1.099511627776e12f && mo <= 1.152921504606847e18f &&
+                    (ax >= low || ax == 0.0f) && (ay >= low || ay == 0.0f) && (az >= low || az == 0.0f);
+    if (uint32_t(root) >= uint32_t(v.num_inner) || (ax != 0.0f && ay != 0.0f && az != 0.0f)) return ok;
+    return ok && md >= 6.103515625e-05f && mo <= 16384.0f * tree_reach(v.nodes + root);
 }
 
 // Traces the rays index(k) of `rays` for the k of `work` with the calling warp (every lane
@@ -326,18 +340,17 @@ __device__ __forceinline__ void quad_trace(int* stack_mem, bvh_view const& v, co
                     {
                         const float4 r0 = ldg4(&rays[ray]);
                         const float4 r1 = ldg4(reinterpret_cast<const float4*>(&rays[ray]) + 1);
-                        const float big = 1.8446744073709552e19f;   // 2^64
                         o = { r0.x, r0.y, r0.z };
                         d = { r0.w, r1.x, r1.y };
-                        id = { fminf(fmaxf(safe_rcp(d.x), -big), big), fminf(fmaxf(safe_rcp(d.y), -big), big),
-                               fminf(fmaxf(safe_rcp(d.z), -big), big) };
+                        id = { quad_rcp(d.x), quad_rcp(d.y), quad_rcp(d.z) };
                         tmin = r1.z;
                         limit = tmax = r1.w;
                         best_t = second_t = FLT_MAX;
                         top = col;
                         asm volatile("st.shared.b32 [%0], %1;" ::"r"(top), "r"(kEmptyLink) : "memory");
-                        const bool ok = quad_ray_ok(o, d) && !(bad && *bad != 0.0f);
-                        node = ok ? root(ray) : kEmptyLink;
+                        const int start = root(ray);
+                        const bool ok = quad_ray_ok(o, d, v, start) && !(bad && *bad != 0.0f);
+                        node = ok ? start : kEmptyLink;
                         best_tri = ok ? -1 : kDeep;
                     }
                     else

@@ -15,8 +15,7 @@
 // the root meets fewer: which ones those are is not known bottom-up, and the pass is bound
 // by HBM traffic either way (64 B read and 64 B written per pair).
 
-#include "api_internal.h"
-#include "device_math.cuh"
+#include "traverse_core.cuh"
 
 namespace gbrt {
 namespace {
@@ -54,13 +53,16 @@ __device__ __forceinline__ float open_area(slot const& s, uint32_t num_inner)
     return uint32_t(s.link) < num_inner ? fminf(fmaxf(area, 0.0f), FLT_MAX) : -1.0f;
 }
 
+// roots: null, or the first node pairs of num_scenes trees (batches); root: the only tree's.
 __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __restrict__ nodes, uint32_t num_inner,
-                                                          quad_node* __restrict__ quads,
+                                                          const uint32_t* __restrict__ roots, uint32_t num_scenes,
+                                                          uint32_t root, quad_node* __restrict__ quads,
                                                           uint32_t* __restrict__ host_bad)
 {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= num_inner) return;
     const bvh2_node p = nodes[i];
+    const float reach = tree_reach(nodes + (roots ? __ldg(&roots[upper_segment(roots, num_scenes, i)]) : root));
     // named values: an array indexed by the choice goes to local memory (0.28 -> 0.70 ms for
     // 8.4 M triangles)
     slot s0 = child(p, 0), s1 = child(p, 1), s2 = s1, s3;
@@ -101,9 +103,12 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
     {
         // cell: the smallest power of two that covers the box with 252 of them and is at
         // least 2^-20 of its largest coordinate, so that org = low corner - cell is below
-        // the corner by about a cell after rounding and every plane below stays in 0..255
+        // the corner by about a cell after rounding and every plane below stays in 0..255;
+        // at least 2^-40 of the tree's largest coordinate for rays along the planes
+        // (quad_ray_ok)
         const float far_coord = fmaxf(fabsf(blo[a]), fabsf(bhi[a]));
         float t = fmaxf(__fdiv_ru(__fsub_ru(bhi[a], blo[a]), 252.0f), far_coord * 9.5367431640625e-07f);
+        t = fmaxf(t, reach * 9.094947017729282e-13f);
         t = fminf(fmaxf(t, 8.271806125530277e-25f), kQuadMaxCoord);   // 2^-80
         const int e = int((__float_as_uint(t) + 0x7FFFFFu) >> 23) - 127;
         const float cell = __int_as_float((e + 127) << 23);
@@ -142,10 +147,11 @@ __global__ void __launch_bounds__(kBlock) make_quad_nodes(const bvh2_node* __res
 
 } // namespace
 
-gbrt_status make_quads(gbrt_context* ctx, bvh2_node const* nodes, uint32_t num_inner, quad_node* quads,
-                       uint32_t* host_bad, cudaStream_t stream)
+gbrt_status make_quads(gbrt_context* ctx, bvh2_node const* nodes, uint32_t num_inner, uint32_t const* roots,
+                       uint32_t num_scenes, uint32_t root, quad_node* quads, uint32_t* host_bad, cudaStream_t stream)
 {
-    make_quad_nodes<<<(num_inner + kBlock - 1) / kBlock, kBlock, 0, stream>>>(nodes, num_inner, quads, host_bad);
+    make_quad_nodes<<<(num_inner + kBlock - 1) / kBlock, kBlock, 0, stream>>>(nodes, num_inner, roots, num_scenes, root,
+                                                                            quads, host_bad);
     GBRT_LAUNCH_CHECK(ctx, "make_quad_nodes");
     return GBRT_OK;
 }

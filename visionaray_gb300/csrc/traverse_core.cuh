@@ -437,6 +437,14 @@ __device__ __forceinline__ uint32_t upper_segment(const uint32_t* __restrict__ o
     return lo;
 }
 
+// The largest coordinate (absolute) of the boxes of a node pair; of a root's, of its tree.
+__device__ __forceinline__ float tree_reach(const bvh2_node* __restrict__ root)
+{
+    const float4 a = ldg4(&root->xy0), b = ldg4(&root->xy1), c = ldg4(&root->z01);
+    auto largest = [](float4 q) { return fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))); };
+    return fmaxf(largest(a), fmaxf(largest(b), largest(c)));
+}
+
 // Everything a query needs from a BVH handle, passed to kernels by value.
 struct bvh_view
 {
