@@ -119,7 +119,8 @@ int         gbrt_abi_version(void);
 #define GBRT_TRACE_WIDE_NODES 2u
 /* Persistent traversal: a grid that just fills the GPU, whose warps refill idle lanes
  * with new rays from an atomic counter instead of idling until their slowest ray ends
- * (node pairs only; hits identical bit for bit).                                     */
+ * (node pairs only; hits identical bit for bit, but for rays in the plane of a triangle:
+ * gbrt_trace_closest_hit).                                                           */
 #define GBRT_TRACE_PERSISTENT 4u
 /* With this flag set when gbrt_bvh_build_lbvh runs, the 4-wide nodes are also stored
  * quantised to 64 bytes in the layout of visionaray's bvh_compressed_node<4> (bvh.h:
@@ -238,7 +239,12 @@ gbrt_status gbrt_bvh_morton_codes(gbrt_context* ctx, gbrt_bvh const* bvh, uint32
  * (detail/traverse_linear.inl:192-225 -> detail/bvh/intersect.inl:41-357 with the
  * ray/triangle test of math/intersect.h:176-229).  A hit is accepted iff the
  * triangle test hits with tmin <= t <= tmax and t strictly below the best t so far
- * (update_if.h:68-107).                                                            */
+ * (update_if.h:68-107).
+ * Trees built on the GPU are traversed through nodes of four children.  The hits equal
+ * those over the node pairs (GBRT_TRACE_PERSISTENT, uploaded trees, the megakernel) bit
+ * for bit, but for one case: where a ray runs in the plane of a triangle to within
+ * rounding, the computed t of that triangle can lie anywhere along the ray, and whether it
+ * is met before a hit in front of it hides it depends on the order of the nodes.       */
 gbrt_status gbrt_trace_closest_hit(gbrt_context* ctx, gbrt_bvh const* bvh,
                                    gbrt_ray const* d_rays, uint32_t n, gbrt_hit* d_hits);
 
@@ -382,8 +388,8 @@ typedef struct gbrt_pt_params
 #define GBRT_PT_NO_RUSSIAN_ROULETTE 2u
 /* Scheduling only: one thread per pixel runs all its samples and bounces (one launch
  * per frame, shadow rays traced in-thread) instead of the wavefront passes.  Same
- * arithmetic and random numbers: the images are identical bit for bit.  About 2x
- * slower than the wavefront on the box and inverse-rendering workloads (GB300).     */
+ * arithmetic and random numbers: the images are identical bit for bit (but for rays in
+ * the plane of a triangle, gbrt_trace_closest_hit).  About 2x slower than the wavefront on the box and inverse-rendering workloads (GB300).     */
 #define GBRT_PT_MEGAKERNEL 4u
 /* Scheduling only: each bounce's ray and shadow queues are ordered by the Morton cell
  * of their origins before they are traced (images identical bit for bit).  Slower on

@@ -2,7 +2,8 @@
 their arithmetic is at its limits (the tree traced as built, and uploaded again from its
 export, which traverses the pairs only): rays with zero direction components among
 triangles far thinner than their distance, from near and far, along directions of any
-length."""
+length; rays in the plane of a surface that is turned against the axes, whose hits are
+rounding errors."""
 import numpy as np
 import pytest
 
@@ -107,3 +108,41 @@ def test_scenes_of_different_size_in_a_batch():
         images.append(batch.pathtrace(batch.new_images()).clone())
     batch.ctx.synchronize()
     assert torch.equal(images[0].view(torch.int32), images[1].view(torch.int32))
+
+
+def turned_plane(k, seed, noise):
+    """k x k squares (two triangles each) in a plane turned at random, vertices off by noise."""
+    rng = np.random.default_rng(seed)
+    x, y = np.meshgrid(np.arange(k + 1), np.arange(k + 1), indexing="ij")
+    g = np.stack([x, y, np.zeros_like(x)], 2) / k @ np.linalg.qr(rng.normal(size=(3, 3)))[0].T
+    g = (g + rng.normal(size=g.shape) * noise).astype(np.float32)
+    a, b, c, d = g[:-1, :-1], g[1:, :-1], g[1:, 1:], g[:-1, 1:]
+    t = np.zeros(2 * k * k, vg.TRIANGLE)
+    for h, (p, q, r) in enumerate(((a, b, d), (c, d, b))):
+        t["v1"][h::2], t["e1"][h::2] = p.reshape(-1, 3), (q - p).reshape(-1, 3)
+        t["e2"][h::2] = (r - p).reshape(-1, 3)
+    t["prim_id"] = np.arange(len(t))
+    return t
+
+
+@pytest.mark.parametrize("builder", ["lbvh", "ploc"])
+@pytest.mark.parametrize("noise", [0.0, 1e-8, 1e-7])
+@pytest.mark.parametrize("k", [16, 64])
+def test_rays_in_a_turned_plane(k, noise, builder):
+    """Rays between two points of the plane, from the first one and from outside."""
+    n = 400_000
+    t = turned_plane(k, 3, noise)
+    rng = np.random.default_rng(k)
+
+    def points():
+        s = t[rng.integers(0, len(t), n)]
+        w = rng.dirichlet((1, 1, 1), n)
+        return s["v1"].astype(float) + s["e1"] * w[:, 1:2] + s["e2"] * w[:, 2:3]
+
+    p, q = points(), points()
+    d = (q - p) / np.linalg.norm(q - p, axis=1, keepdims=True)
+    r = np.zeros(n, vg.RAY)
+    r["ori"], r["dir"], r["tmax"] = p, d, FLT_MAX
+    r["ori"][::2] -= 2.0 * d[::2].astype(np.float32)
+    want = assert_quads_equal_pairs(t, r, builder)
+    assert (want["prim_id"] != 0xFFFFFFFF).sum() > n // 2

@@ -55,15 +55,16 @@ struct tri_hit
 {
     bool hit;
     float t, u, v;
+    float det;   // the determinant; set whether or not there is a hit
 };
 
 // Ray / triangle test of visionaray math/intersect.h:176-229: two-sided, rejects only
 // a zero determinant, barycentric bounds b1 in [0,1], b2 >= 0, b1 + b2 <= 1.
 __device__ __forceinline__ tri_hit intersect_triangle(f3 ori, f3 dir, f3 v1, f3 e1, f3 e2)
 {
-    tri_hit r{ false, -1.0f, 0.0f, 0.0f };
     f3 s1 = cross_rn(dir, e2);
     float div = dot_rn(s1, e1);
+    tri_hit r{ false, -1.0f, 0.0f, 0.0f, div };
     if (!(div != 0.0f)) return r;
     float inv_div = __frcp_rn(div);
     f3 d = sub_rn(ori, v1);
