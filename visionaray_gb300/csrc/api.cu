@@ -566,11 +566,13 @@ static gbrt_status trace_device(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray
     if (!aligned16(d_rays) || !aligned16(d_hits))
         return fail(ctx, GBRT_ERR_INVALID_ARG, "trace: ray and hit buffers must be 16-byte aligned");
     device_guard g(ctx->device);
-    if (ctx->trace_flags & (GBRT_TRACE_SORT_RAYS | GBRT_TRACE_PERSISTENT))
-    {
-        gbrt_status s2 = ensure_trace_scratch(ctx, n);
-        if (s2 != GBRT_OK) return s2;
-    }
+    // A query in input order keeps nothing in the context: queries on several streams in turn
+    // (gbrt_context_set_stream) may overlap, and a captured one stays valid when a later query
+    // needs a larger scratch.
+    if (!(ctx->trace_flags & (GBRT_TRACE_SORT_RAYS | GBRT_TRACE_PERSISTENT)))
+        return trace(ctx, bvh, d_rays, n, d_hits, any_hit, ctx->stream, nullptr, 0);
+    gbrt_status s2 = ensure_trace_scratch(ctx, n);
+    if (s2 != GBRT_OK) return s2;
     return trace(ctx, bvh, d_rays, n, d_hits, any_hit, ctx->stream, ctx->trace_scratch, ctx->trace_scratch_bytes);
 }
 

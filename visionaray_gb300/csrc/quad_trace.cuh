@@ -105,10 +105,12 @@ __host__ __device__ __forceinline__ uint32_t quad_span(uint32_t n, uint32_t resi
 // Rays that a warp takes at a time off a shared counter when there are more than kQuadChunk
 // for each resident warp: a warp that got long rays takes fewer, and the launch ends
 // together.  Against fixed spans: 400,000 sorted secondary rays 378 -> 351 us, 1,000,000 636
-// -> 549, 4,194,304 2,096 -> 1,810; camera rays 640^2 200 -> 163, 1024^2 320 -> 281, 2048^2
-// 1,022 -> 1,037; high-definition frame 44.3 -> 41.5 ms, batch of scenes 8.83 -> 7.70.  48
-// and 64 at a time are up to 5 % slower at a few hundred thousand rays, 1 % faster on ambient
-// occlusion; 128 slower.
+// -> 549, 4,194,304 2,096 -> 1,810; high-definition frame 44.3 -> 41.5 ms, batch of scenes
+// 8.83 -> 7.70.  48 and 64 at a time are up to 5 % slower at a few hundred thousand rays, 1 %
+// faster on ambient occlusion; 128 slower.  The counter is part of the memory that sorted
+// queries, host-buffer queries, frames and batches have; a device query in input order has
+// none (trace_device in api.cu) and keeps the spans (with a counter camera rays would take
+// 163 us for 200 at 640^2, 281 for 320 at 1024^2, 1,037 for 1,022 at 2048^2).
 constexpr uint32_t kQuadChunk = 32;
 
 // A warp's rays: next .. end - 1 first, then, unless shared is 0, chunks below `shared`
