@@ -487,8 +487,9 @@ gbrt_status gbrt_pathtrace_forward(gbrt_context* ctx, gbrt_pt_scene const* scene
  * ADDED to; zero them first).  Each (pixel, sample) path is re-traced from its random
  * numbers -- the same shading code as the forward frame, so the same path -- and its
  * vertices swept backwards; nothing of the forward frame is stored.  Paths are replayed in
- * passes whose state and vertex records take at most about 3 GB of context-owned memory.
- * Gradients are accumulated with warp-reduced FP32 atomics.  Geometry, visibility and
+ * passes whose state and vertex records take at most about 3 GB (less where the device has
+ * less), allocated and freed in stream order: the call can be captured in a graph and may
+ * overlap other calls on other streams.  Gradients are accumulated with warp-reduced FP32 atomics.  Geometry, visibility and
  * roulette decisions are not differentiated.  num_bounces <= 16.  A scene over
  * instances (gbrt_pt_scene_create_instanced) replays through the same two-level tree;
  * a slot's gradient sums the vertices of every instance that uses the slot.      */

@@ -98,3 +98,96 @@ def test_host_queries_in_input_order_share_their_rays(soup_tree, extra):
     want = vg.closest_hit(rays, bvh).cpu().numpy()
     got = vg.closest_hit(rays.cpu().numpy().view(vg.RAY).reshape(-1), bvh)
     assert got.tobytes() == want.tobytes()
+
+
+class Box:
+    """A path-traced box with per-slot parameters."""
+
+    def __init__(self, width, height):
+        tris, mats, lights = scenes.box_scene(n_blobs=3, subdiv=3, seed=4)
+        self.ctx = vg.Context(0)
+        self.bvh = vg.lbvh_builder(self.ctx).build(vg.as_device_bytes(tris))
+        self.scene = vg.PTScene(self.bvh, mats, lights)
+        self.width, self.height = width, height
+        rng = np.random.default_rng(1)
+        self.albedo = torch.from_numpy(rng.uniform(0.3, 0.7, (len(mats), 3)).astype(np.float32)).cuda()
+        self.emission = torch.from_numpy(np.ascontiguousarray(mats["color"])).cuda()
+        self.adjoint = torch.from_numpy(rng.uniform(-1, 1, (height, width, 4)).astype(np.float32)).cuda()
+        self.ctx.synchronize()
+
+    def params(self, spp, depth, flags=0):
+        return scenes.pt_params(self.width, self.height, spp, num_bounces=depth, frame_id=3, flags=flags,
+                                ambient=(0.1, 0.2, 0.3))
+
+    def frame(self, spp, depth, flags=0, out=None):
+        out = torch.zeros((self.height, self.width, 4), device="cuda") if out is None else out
+        return vg.pathtrace_frame(self.scene, scenes.box_camera(), self.params(spp, depth, flags), out)
+
+    def backward(self, spp, depth, grads=None):
+        grads = grads or (torch.zeros_like(self.albedo), torch.zeros_like(self.emission))
+        return vg.pathtrace_backward(self.scene, scenes.box_camera(), self.params(spp, depth, 3), self.albedo,
+                                     self.emission, self.adjoint, *grads)
+
+
+def assert_close(got, want, scale=1.0):
+    """FP32 atomics: the sums' rounding depends on the order (relative L2 1e-4)."""
+    for g, w in zip(got, want):
+        w = scale * w.double()
+        assert float((g.double() - w).norm()) <= 1e-4 * float(w.norm())
+
+
+def test_a_first_backward_call_can_be_captured():
+    box = Box(64, 48)
+    grads = torch.zeros_like(box.albedo), torch.zeros_like(box.emission)
+    graph = capture(box.ctx, lambda: box.backward(5, 6, grads))
+    want = box.backward(5, 6)
+    box.frame(16, 8)             # the context's own buffers come and go
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert_close(grads, want, 3.0)
+    box.ctx.synchronize()
+
+
+def test_backward_calls_overlap_frames_and_each_other():
+    box = Box(256, 200)
+    image = box.frame(8, 5).clone()
+    want = box.backward(8, 5)
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    images = [torch.zeros_like(image) for _ in range(6)]
+    grads = [(torch.zeros_like(box.albedo), torch.zeros_like(box.emission)) for _ in range(2)]
+    torch.cuda.synchronize()
+    for k in range(6):
+        with on_stream(box.ctx, streams[0]):
+            box.frame(8, 5, out=images[k])
+        for j in range(2):
+            with on_stream(box.ctx, streams[1 + j]):
+                box.backward(8, 5, grads[j])
+    torch.cuda.synchronize()
+    for got in images:
+        assert torch.equal(got.view(torch.int32), image.view(torch.int32))
+    for got in grads:
+        assert_close(got, want, 6.0)
+    box.ctx.synchronize()
+
+
+@contextlib.contextmanager
+def little_memory(free_bytes):
+    """Leaves about free_bytes of the device's memory to others."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(max(1, torch.cuda.mem_get_info()[0] - free_bytes), dtype=torch.uint8, device="cuda")
+    yield
+    torch.cuda.synchronize()
+    del hog
+    torch.cuda.empty_cache()
+
+
+def test_a_backward_call_with_little_memory():
+    box = Box(512, 512)
+    box.backward(1, 1)
+    grads = torch.zeros_like(box.albedo), torch.zeros_like(box.emission)
+    with little_memory(1 << 30):   # the passes would take 2.9 GB
+        box.backward(16, 6, grads)
+    assert_close(grads, box.backward(16, 6))
+    box.ctx.synchronize()

@@ -39,6 +39,19 @@ gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
     return GBRT_OK;
 }
 
+gbrt_status ensure_pool(gbrt_context* ctx)
+{
+    if (ctx->pool) return GBRT_OK;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    GBRT_CUDA(ctx, cudaMemPoolCreate(&ctx->pool, &props));
+    uint64_t keep = gbrt_context::kPoolKeep;
+    GBRT_CUDA(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    return GBRT_OK;
+}
+
 // cudaMalloc and cudaFree of a tree's arrays took 1.2 of the 2.4 ms of building a tree of
 // 8.4 M triangles and destroying it, and half of the time at a few thousand triangles.
 // They come from a memory pool of the context instead, except for its first tree, often its
@@ -50,15 +63,10 @@ gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
 gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
 {
     if (bvh->arena || n == 0) return GBRT_OK;
-    if (!ctx->pool && ctx->built_tree)
+    if (ctx->built_tree)
     {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = ctx->device;
-        GBRT_CUDA(ctx, cudaMemPoolCreate(&ctx->pool, &props));
-        uint64_t keep = gbrt_context::kPoolKeep;
-        GBRT_CUDA(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        gbrt_status st = ensure_pool(ctx);
+        if (st != GBRT_OK) return st;
     }
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t nodes = up(size_t(n - 1) * sizeof(bvh2_node)), tris = up(size_t(n) * sizeof(tri48)),

@@ -41,8 +41,9 @@ struct gbrt_context
 
     uint32_t* d_status = nullptr;     // one word of status bits
 
-    // Device memory of the trees this context builds: a pool that keeps up to kPoolKeep
-    // bytes of freed trees for the next ones (api.cu, alloc_tree), made at the second build.
+    // Device memory of the trees this context builds and of its backward passes: a pool that
+    // keeps up to kPoolKeep freed bytes for the next ones (api.cu, alloc_tree; pathtrace.cu,
+    // replay_memory), made at the second build or the first backward pass.
     static constexpr uint64_t kPoolKeep = 4ull << 30;
     cudaMemPool_t pool = nullptr;
     bool built_tree = false;
@@ -271,6 +272,15 @@ struct device_guard
     }
 };
 
+// Whether work on `stream` is being captured into a graph.
+inline bool is_capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status == cudaStreamCaptureStatusActive;
+    cudaGetLastError();   // the legacy stream while another one is captured
+    return false;
+}
+
 // Sets ctx->last_error and returns `st`.
 gbrt_status fail(gbrt_context* ctx, gbrt_status st, std::string const& what);
 // Maps a CUDA error to a status, recording `where`.
@@ -278,6 +288,8 @@ gbrt_status check_cuda(gbrt_context* ctx, cudaError_t err, const char* where);
 // The arrays of a tree of n > 0 triangles (nothing to do if it has them already): one
 // allocation from the context's pool.
 gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n);
+// Makes the context's memory pool, if it has none.
+gbrt_status ensure_pool(gbrt_context* ctx);
 // The host and device address of the context's build_result (allocated once).
 gbrt_status ensure_result(gbrt_context* ctx, build_result** device);
 // Grows the context scratch to at least `bytes`.

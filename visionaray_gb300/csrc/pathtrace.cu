@@ -624,9 +624,9 @@ uint32_t pass_samples(uint32_t npix, uint32_t spp)
 
 // The context's buffers of a pass (layout_frame_buffers).
 gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint32_t num_counts, bool sort,
-                              uint32_t record_bounces, frame_buffers& fb)
+                              frame_buffers& fb)
 {
-    const size_t total = layout_frame_buffers(npix, n, num_counts, sort, record_bounces, nullptr, fb);
+    const size_t total = layout_frame_buffers(npix, n, num_counts, sort, 0, nullptr, fb);
     if (ctx->pt_scratch_bytes < total)
     {
         if (ctx->pt_scratch)
@@ -639,7 +639,7 @@ gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint
         GBRT_CUDA(ctx, cudaMalloc(&ctx->pt_scratch, total));
         ctx->pt_scratch_bytes = total;
     }
-    layout_frame_buffers(npix, n, num_counts, sort, record_bounces, ctx->pt_scratch, fb);
+    layout_frame_buffers(npix, n, num_counts, sort, 0, ctx->pt_scratch, fb);
     return GBRT_OK;
 }
 
@@ -1059,7 +1059,7 @@ gbrt_status render_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
     const uint32_t samples = pass_samples(npix, p.spp);
     const uint32_t num_counts = 2 * (p.num_bounces + 1);
     frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, npix, npix * samples, num_counts, sort, 0, fb);
+    gbrt_status st = frame_buffers_for(ctx, npix, npix * samples, num_counts, sort, fb);
     if (st != GBRT_OK) return st;
     for (uint32_t smp = 0; smp < p.spp; smp += fb.samples)
     {
@@ -1075,8 +1075,47 @@ gbrt_status render_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
     return GBRT_OK;
 }
 
-// Bytes of vertex records that a backward pass may hold (its paths: at most kPassPaths).
+// Bytes of vertex records that a backward pass may hold (its paths: at most kPassPaths), and
+// the paths of a pass below which an allocation that fails is an error.
 constexpr uint64_t kRecordBytes = 2ull << 30;
+constexpr uint64_t kLeastPaths = 4096;
+
+// The memory of a backward call's passes, allocated and freed in stream order: a call shares
+// none with others, so it may overlap any call on another stream, and in a captured graph it
+// is the graph's own.  In a capture it comes from the device's pool, otherwise from the
+// context's, which keeps it for the next call.
+struct replay_memory
+{
+    void* base = nullptr;
+    cudaStream_t stream;
+
+    explicit replay_memory(cudaStream_t s) : stream(s) {}
+    replay_memory(replay_memory const&) = delete;
+    replay_memory& operator=(replay_memory const&) = delete;
+    ~replay_memory()
+    {
+        if (base) cudaFreeAsync(base, stream);
+    }
+    gbrt_status allocate(gbrt_context* ctx, size_t bytes, bool& out_of_memory)
+    {
+        cudaError_t e = cudaSuccess;
+        if (is_capturing(stream))
+        {
+            e = cudaMallocAsync(&base, bytes, stream);
+        }
+        else
+        {
+            gbrt_status st = ensure_pool(ctx);
+            if (st != GBRT_OK) return st;
+            e = cudaMallocFromPoolAsync(&base, bytes, ctx->pool, stream);
+        }
+        out_of_memory = e == cudaErrorMemoryAllocation;
+        if (e == cudaSuccess) return GBRT_OK;
+        base = nullptr;
+        if (out_of_memory) cudaGetLastError();
+        return check_cuda(ctx, e, "replay memory");
+    }
+};
 
 // Path-replay backpropagation in passes of a range of pixels and samples: each pass replayed
 // by the frame's stages with records, then swept.
@@ -1088,13 +1127,21 @@ gbrt_status replay_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
 {
     if (p.num_bounces == 0) return GBRT_OK;   // paths without vertices
     const uint32_t npix = p.width * p.height;
-    const uint64_t most = std::min(kPassPaths, kRecordBytes / (uint64_t(p.num_bounces) * kRecWords * 16));
-    const uint32_t pixels = uint32_t(std::min<uint64_t>(npix, most));
-    const uint32_t samples = uint32_t(std::min<uint64_t>(p.spp, most / pixels));
     const uint32_t num_counts = 2 * (p.num_bounces + 1);
     frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, 0, pixels * samples, num_counts, sort, p.num_bounces, fb);
-    if (st != GBRT_OK) return st;
+    replay_memory memory(ctx->stream);
+    uint32_t pixels = 0, samples = 0;
+    for (uint64_t most = std::min(kPassPaths, kRecordBytes / (uint64_t(p.num_bounces) * kRecWords * 16));; most /= 2)
+    {
+        pixels = uint32_t(std::min<uint64_t>(npix, most));
+        samples = uint32_t(std::min<uint64_t>(p.spp, most / pixels));
+        bool out_of_memory = false;
+        gbrt_status st = memory.allocate(
+            ctx, layout_frame_buffers(0, pixels * samples, num_counts, sort, p.num_bounces, nullptr, fb), out_of_memory);
+        if (st == GBRT_OK) break;
+        if (!out_of_memory || most < 2 * kLeastPaths) return st;
+    }
+    layout_frame_buffers(0, pixels * samples, num_counts, sort, p.num_bounces, memory.base, fb);
     for (uint32_t smp = 0; smp < p.spp; smp += samples)
     {
         fb.first_sample = smp;
@@ -1103,7 +1150,7 @@ gbrt_status replay_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
         {
             fb.first_pixel = px;
             const uint32_t n = std::min(pixels, npix - px) * fb.samples;
-            st = run_pass(ctx, scene, cam, p, sp, is, false, fb, n, num_counts, trace);
+            gbrt_status st = run_pass(ctx, scene, cam, p, sp, is, false, fb, n, num_counts, trace);
             if (st != GBRT_OK) return st;
             pt_sweep<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
                 fb, n, p.num_bounces, 1.0f / float(p.spp), sp, reinterpret_cast<const float4*>(d_image_adjoint),
