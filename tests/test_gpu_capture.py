@@ -8,6 +8,7 @@ import torch
 
 import visionaray_gb300 as vg
 from visionaray_gb300 import scenes
+from visionaray_gb300.types import PT_SORT_QUEUES
 
 pytestmark = pytest.mark.gpu
 
@@ -24,7 +25,7 @@ def capture(ctx, call):
     """A graph of what call() enqueues on the context's stream."""
     torch.cuda.synchronize()
     graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
-    with torch.cuda.graph(graph, stream=stream), on_stream(ctx, stream):
+    with on_stream(ctx, stream), torch.cuda.graph(graph, stream=stream):
         call()
     return graph
 
@@ -190,4 +191,40 @@ def test_a_backward_call_with_little_memory():
     with little_memory(1 << 30):   # the passes would take 2.9 GB
         box.backward(16, 6, grads)
     assert_close(grads, box.backward(16, 6))
+    box.ctx.synchronize()
+
+
+@pytest.mark.parametrize("spp,depth,flags", [(1, 4, 0), (9, 4, 0), (1, 60, 0), (3, 4, PT_SORT_QUEUES)])
+def test_a_frame_is_captured_after_another_of_its_size(spp, depth, flags):
+    """Whatever its samples, bounces and queue order; the graph stays valid when later
+    frames need larger buffers, captured or not."""
+    box = Box(96, 70)
+    box.frame(1, 4)
+    out = torch.zeros((box.height, box.width, 4), device="cuda")
+    graph = capture(box.ctx, lambda: box.frame(spp, depth, flags, out))
+    want = box.frame(spp, depth, flags).clone()
+    box.frame(300, 2)
+    other = Box(96, 70)
+    for k in range(3):
+        out.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+        more = torch.zeros_like(out)
+        second = capture(box.ctx, lambda: box.frame(400 + k, 2, 0, more))
+        second.replay()
+        assert torch.equal(more.view(torch.int32), other.frame(400 + k, 2).view(torch.int32))
+    box.ctx.synchronize()
+
+
+def test_a_frame_with_little_memory():
+    box, other = Box(1024, 513), Box(1024, 513)
+    want = other.frame(9, 3).clone()
+    other.ctx.synchronize()
+    got = [torch.zeros_like(want) for _ in range(2)]
+    with little_memory(300 << 20):   # the passes would take 500 MB
+        for image in got:
+            box.frame(9, 3, out=image)
+    for image in got:
+        assert torch.equal(image.view(torch.int32), want.view(torch.int32))
     box.ctx.synchronize()

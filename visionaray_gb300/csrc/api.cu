@@ -308,6 +308,7 @@ gbrt_status gbrt_context_destroy(gbrt_context* ctx)
         cudaFree(ctx->trace_scratch);
         cudaFree(ctx->scratch);
         cudaFree(ctx->pt_scratch);
+        for (void* p : ctx->pt_retired) cudaFree(p);
         cudaFree(ctx->d_trig);
         cudaFree(ctx->d_status);
     }

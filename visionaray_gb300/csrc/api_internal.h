@@ -66,6 +66,10 @@ struct gbrt_context
     // Path-tracer wavefront state (grown on demand, freed with the context).
     void* pt_scratch = nullptr;
     size_t pt_scratch_bytes = 0;
+    // Whether a captured frame uses pt_scratch: it is then kept in pt_retired, for the
+    // graph's replays, when a larger one takes its place (each at least twice as large).
+    bool pt_captured = false;
+    std::vector<void*> pt_retired;
     // The path tracer's sample angles: cos and sin (rounded once from double) of
     // 2 pi u for each of the 2^24 values u = k / 2^24 a random draw takes (float2 per
     // k, 128 MB), filled once by ensure_trig_table (pathtrace.cu).

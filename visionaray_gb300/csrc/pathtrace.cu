@@ -65,11 +65,11 @@ constexpr int kShadeMinBlocks = 8;
 // Jittered primary rays (detail/sched_common.h:209-233: jitter x drawn before y) through
 // the pinhole camera (detail/pinhole_camera.inl:103-120), and the pass's queue lengths.
 __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t n, uint32_t width,
-                                                    uint32_t height, uint32_t frame, uint32_t num_counts,
+                                                    uint32_t height, uint32_t frame, uint64_t num_counts,
                                                     camera_basis cam)
 {
     uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    for (uint32_t k = i; k < 2 * num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
+    for (uint64_t k = i; k < 2 * num_counts; k += gridDim.x * kBlock) fb.counts[k] = k == 0 ? n : 0;
     if (i >= n) return;
     const uint2 ps = path_sample(fb, i);
     v3 d = primary_dir(cam, width, height, frame, ps.x, ps.y);
@@ -622,24 +622,60 @@ uint32_t pass_samples(uint32_t npix, uint32_t spp)
     return uint32_t((spp + passes - 1) / passes);
 }
 
-// The context's buffers of a pass (layout_frame_buffers).
-gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t n, uint32_t num_counts, bool sort,
+// A frame's queue lengths for num_bounces bounces: a ray and a shadow queue of each.
+uint64_t queue_counts(uint32_t num_bounces) { return 2 * (uint64_t(num_bounces) + 1); }
+
+// Queue lengths that pt_scratch always has room for, so that its size does not depend on the
+// bounces of an ordinary frame (64 KB).
+constexpr uint64_t kMinCounts = 8192;
+
+// The context's buffers of a frame's passes of `samples` samples per pixel.  pt_scratch is
+// made as large as the passes ask for and never smaller than a pass of one sample, sorted or
+// not, takes, which is all a frame needs: where there is no room for more -- in a capture,
+// which must not allocate, or where the device has none -- samples is lowered.  So after a
+// frame of some size, any frame of that size can be captured.
+gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t num_bounces, bool sort, uint32_t& samples,
                               frame_buffers& fb)
 {
-    const size_t total = layout_frame_buffers(npix, n, num_counts, sort, 0, nullptr, fb);
-    if (ctx->pt_scratch_bytes < total)
+    const uint64_t counts = queue_counts(num_bounces);
+    auto bytes_for = [&](uint32_t smp) { return layout_frame_buffers(npix, npix * smp, counts, sort, 0, nullptr, fb); };
+    const size_t least = layout_frame_buffers(npix, npix, std::max(counts, kMinCounts), true, 0, nullptr, fb);
+    const bool capturing = is_capturing(ctx->stream);
+    if (ctx->pt_scratch_bytes < std::max(bytes_for(samples), least) &&
+        !(capturing && ctx->pt_scratch_bytes >= bytes_for(1)))
     {
+        // frames in flight may still use the old buffers, captured frames may be replayed
+        const size_t kept = ctx->pt_captured ? ctx->pt_scratch_bytes : 0;
         if (ctx->pt_scratch)
         {
             GBRT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            GBRT_CUDA(ctx, cudaFree(ctx->pt_scratch));
+            if (kept)
+                ctx->pt_retired.push_back(ctx->pt_scratch);
+            else
+                GBRT_CUDA(ctx, cudaFree(ctx->pt_scratch));
             ctx->pt_scratch = nullptr;
             ctx->pt_scratch_bytes = 0;
+            ctx->pt_captured = false;
         }
-        GBRT_CUDA(ctx, cudaMalloc(&ctx->pt_scratch, total));
-        ctx->pt_scratch_bytes = total;
+        for (size_t twice = 2 * kept;;)
+        {
+            const size_t bytes = std::max(std::max(bytes_for(samples), least), twice);
+            const cudaError_t e = cudaMalloc(&ctx->pt_scratch, bytes);
+            if (e == cudaSuccess)
+            {
+                ctx->pt_scratch_bytes = bytes;
+                break;
+            }
+            ctx->pt_scratch = nullptr;
+            if (e != cudaErrorMemoryAllocation || (samples == 1 && !twice)) return check_cuda(ctx, e, "path buffers");
+            cudaGetLastError();
+            if (!twice) samples = (samples + 1) / 2;
+            twice = 0;
+        }
     }
-    layout_frame_buffers(npix, n, num_counts, sort, 0, ctx->pt_scratch, fb);
+    while (samples > 1 && bytes_for(samples) > ctx->pt_scratch_bytes) samples = (samples + 1) / 2;
+    ctx->pt_captured |= capturing;
+    layout_frame_buffers(npix, npix * samples, counts, sort, 0, ctx->pt_scratch, fb);
     return GBRT_OK;
 }
 
@@ -1025,14 +1061,14 @@ shade_kernel pick_shade(gbrt_pt_scene const* scene, bool record)
 template <class Trace>
 gbrt_status run_pass(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_basis const& cam, gbrt_pt_params const& p,
                      shade_params sp, inst_shade const& is, bool empty, frame_buffers const& fb, uint32_t n,
-                     uint32_t num_counts, Trace const& trace)
+                     Trace const& trace)
 {
     cudaStream_t s = ctx->stream;
     const uint32_t blocks = (n + kBlock - 1) / kBlock;
     const uint32_t shade_blocks = std::min(blocks, uint32_t(ctx->num_sms) * kShadeMinBlocks * 4);
     const shade_kernel shade = pick_shade(scene, fb.rec != nullptr);
     const bool lights = scene->num_lights > 0;
-    pt_raygen<<<blocks, kBlock, 0, s>>>(fb, n, p.width, p.height, p.frame_id, num_counts, cam);
+    pt_raygen<<<blocks, kBlock, 0, s>>>(fb, n, p.width, p.height, p.frame_id, queue_counts(p.num_bounces), cam);
     GBRT_LAUNCH_CHECK(ctx, "pt_raygen");
     int q = 0;
     for (uint32_t b = 0; b < p.num_bounces && !empty; ++b)
@@ -1056,16 +1092,15 @@ gbrt_status render_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
                           float4 bg, float* d_accum, float* d_color, Trace const& trace)
 {
     const uint32_t npix = p.width * p.height;
-    const uint32_t samples = pass_samples(npix, p.spp);
-    const uint32_t num_counts = 2 * (p.num_bounces + 1);
+    uint32_t samples = pass_samples(npix, p.spp);
     frame_buffers fb;
-    gbrt_status st = frame_buffers_for(ctx, npix, npix * samples, num_counts, sort, fb);
+    gbrt_status st = frame_buffers_for(ctx, npix, p.num_bounces, sort, samples, fb);
     if (st != GBRT_OK) return st;
     for (uint32_t smp = 0; smp < p.spp; smp += fb.samples)
     {
         fb.first_sample = smp;
         fb.samples = std::min(samples, p.spp - smp);
-        st = run_pass(ctx, scene, cam, p, sp, is, empty, fb, npix * fb.samples, num_counts, trace);
+        st = run_pass(ctx, scene, cam, p, sp, is, empty, fb, npix * fb.samples, trace);
         if (st != GBRT_OK) return st;
         pt_accumulate<<<(npix + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
             fb, npix, smp + fb.samples >= p.spp ? 1u : 0u, bg, float(p.spp), p.sfactor, p.dfactor,
@@ -1127,7 +1162,7 @@ gbrt_status replay_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
 {
     if (p.num_bounces == 0) return GBRT_OK;   // paths without vertices
     const uint32_t npix = p.width * p.height;
-    const uint32_t num_counts = 2 * (p.num_bounces + 1);
+    const uint64_t num_counts = queue_counts(p.num_bounces);
     frame_buffers fb;
     replay_memory memory(ctx->stream);
     uint32_t pixels = 0, samples = 0;
@@ -1150,7 +1185,7 @@ gbrt_status replay_passes(gbrt_context* ctx, gbrt_pt_scene const* scene, camera_
         {
             fb.first_pixel = px;
             const uint32_t n = std::min(pixels, npix - px) * fb.samples;
-            gbrt_status st = run_pass(ctx, scene, cam, p, sp, is, false, fb, n, num_counts, trace);
+            gbrt_status st = run_pass(ctx, scene, cam, p, sp, is, false, fb, n, trace);
             if (st != GBRT_OK) return st;
             pt_sweep<<<(n + kBlock - 1) / kBlock, kBlock, 0, ctx->stream>>>(
                 fb, n, p.num_bounces, 1.0f / float(p.spp), sp, reinterpret_cast<const float4*>(d_image_adjoint),

@@ -133,7 +133,7 @@ inline size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 // The buffers of a pass of n paths over npix pixels with num_counts queue lengths; sort: with
 // the queue order's keys; record_bounces: with the vertex records of that many bounces.
 // Returns their bytes; with base non-null sets fb to them.
-inline size_t layout_frame_buffers(uint32_t npix, uint32_t n, uint32_t num_counts, bool sort, uint32_t record_bounces,
+inline size_t layout_frame_buffers(uint32_t npix, uint32_t n, uint64_t num_counts, bool sort, uint32_t record_bounces,
                                    void* base, frame_buffers& fb)
 {
     const size_t key = sort ? size_t(n) * 4 : 0;
