@@ -617,9 +617,11 @@ gbrt_status gbrt_batch_height(gbrt_context* ctx, gbrt_batch const* batch, uint32
  * equals the one gbrt_pathtrace_frame renders with its camera, params and lights).  With
  * the full 64-entry stack, width 2 and no sorting (the default) the frame goes through the
  * queues of the wavefront renderer, all scenes' paths together, and the block and tile of
- * the launch shape do not matter; otherwise through a single persistent launch whose warps
- * take tiles of pixels of any scene from one atomic work queue.  d_images: RGBA32F, 16-byte aligned,
- * scene s at pixel offset sum_{t<s} width_t * height_t.  Enqueue only.              */
+ * the launch shape do not matter; otherwise, where the device has no room for the queues
+ * (up to 1 GB, kept by the batch) and when the caller captures the frame in a graph, through
+ * a single persistent launch whose warps take tiles of pixels of any scene from one atomic
+ * work queue.  d_images: RGBA32F, 16-byte aligned, scene s at pixel offset
+ * sum_{t<s} width_t * height_t.  Enqueue only.                                      */
 gbrt_status gbrt_batch_pathtrace(gbrt_context* ctx, gbrt_batch* batch, float* d_images);
 
 /* The lights of each scene of a batch (make_kernel_params' light list per scene,

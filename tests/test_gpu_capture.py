@@ -8,7 +8,7 @@ import torch
 
 import visionaray_gb300 as vg
 from visionaray_gb300 import scenes
-from visionaray_gb300.types import PT_SORT_QUEUES
+from visionaray_gb300.types import CAMERA, MATERIAL, MATTE, PT_PARAMS, PT_SORT_QUEUES
 
 pytestmark = pytest.mark.gpu
 
@@ -228,3 +228,48 @@ def test_a_frame_with_little_memory():
     for image in got:
         assert torch.equal(image.view(torch.int32), want.view(torch.int32))
     box.ctx.synchronize()
+
+
+def make_batch(side, spp, depth, scenes_n=2):
+    parts = [scenes.soup(500 + 300 * k, seed=k, offset=0.05) for k in range(scenes_n)]
+    batch = vg.Batch(np.concatenate([[0], np.cumsum([len(t) for t in parts])]), vg.Context(0))
+    set_frames(batch, scenes_n, side, spp, depth)
+    batch.build(vg.as_device_bytes(np.concatenate(parts)))
+    batch.ctx.synchronize()
+    return batch
+
+
+def set_frames(batch, scenes_n, side, spp, depth):
+    cams, params = np.zeros(scenes_n, CAMERA), np.zeros(scenes_n, PT_PARAMS)
+    for k in range(scenes_n):
+        cams[k] = scenes.box_camera((0.5, 0.5, 2.0), (0.5, 0.5, 0.5), (0.0, 1.0, 0.0), 50.0)
+        params[k] = scenes.pt_params(side, side, spp, num_bounces=depth, frame_id=1, ambient=(1.0, 1.0, 1.0))
+    mats = np.zeros(1, MATERIAL)
+    mats["kind"], mats["color"], mats["scale"] = MATTE, 0.7, 1.0
+    batch.set_frames(cams, params, mats)
+
+
+def test_a_first_batch_frame_can_be_captured():
+    """And its graph renders whatever frames are set later, as the frame itself does."""
+    batch = make_batch(32, 2, 3)
+    out = batch.new_images()
+    graph = capture(batch.ctx, lambda: batch.pathtrace(out))
+    for spp, depth in ((2, 3), (40, 5), (1, 1)):
+        set_frames(batch, 2, 32, spp, depth)
+        want = batch.pathtrace(batch.new_images())
+        out.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+    batch.ctx.synchronize()
+
+
+def test_a_batch_frame_with_little_memory():
+    batch, other = make_batch(1024, 2, 3), make_batch(1024, 2, 3)
+    want, got = other.pathtrace(other.new_images()), batch.new_images()
+    other.ctx.synchronize()
+    with little_memory(300 << 20):   # the passes would take 800 MB
+        batch.pathtrace(got)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert torch.equal(batch.pathtrace(batch.new_images()).view(torch.int32), want.view(torch.int32))
+    batch.ctx.synchronize()

@@ -411,12 +411,12 @@ gbrt_status batch_collapse(gbrt_context* ctx, gbrt_batch* b, uint32_t width, cud
 // it (the wide collapse, the pixel order); force_collapse re-collapses even when the
 // last build's collapse at this width is current.
 gbrt_status batch_frame_stage(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t stream,
-                              bool force_collapse);
+                              bool force_collapse, bool wavefront);
 // batch_wf.cu: whether the launch's frames go through the wavefront renderer, its buffers
-// (allocated outside a capture), and the frame (enqueue only; force_quads re-makes the quad
-// nodes even when the last build's are current).
+// (outside a capture; false if the device has no room for them), and the frame (enqueue only;
+// force_quads re-makes the quad nodes even when the last build's are current).
 bool batch_wavefront_applies(gbrt_batch const* b);
-gbrt_status ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b);
+bool ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b);
 gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t s, bool force_quads);
 
 } // namespace gbrt

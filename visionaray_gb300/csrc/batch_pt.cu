@@ -122,23 +122,26 @@ gbrt_status ensure_batch_sort(gbrt_context* ctx, gbrt_batch* b)
     return GBRT_OK;
 }
 
-// What the current launch shape needs allocated before a frame (never during a capture).
-gbrt_status ensure_batch_extras(gbrt_context* ctx, gbrt_batch* b)
+// What the current launch shape needs allocated before a frame (never during a capture), and
+// whether the frame goes through the wavefront renderer: where its memory is not to be had,
+// and for a frame that the caller captures, the persistent kernel needs none.
+gbrt_status ensure_batch_extras(gbrt_context* ctx, gbrt_batch* b, bool& wavefront)
 {
+    wavefront = false;
     if (b->launch.width != 2)
     {
         gbrt_status st = ensure_batch_wide(ctx, b);
         if (st != GBRT_OK) return st;
     }
     if (b->launch.sort) return ensure_batch_sort(ctx, b);
-    if (batch_wavefront_applies(b)) return ensure_batch_wavefront(ctx, b);
+    wavefront = batch_wavefront_applies(b) && !is_capturing(ctx->stream) && ensure_batch_wavefront(ctx, b);
     return GBRT_OK;
 }
 
 } // namespace
 
 gbrt_status batch_frame_stage(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t stream,
-                              bool force_collapse)
+                              bool force_collapse, bool wavefront)
 {
     if (b->frames_set != b->num_scenes) return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: frames not set");
     if (!d_images || (reinterpret_cast<uintptr_t>(d_images) & 15u))
@@ -149,7 +152,7 @@ gbrt_status batch_frame_stage(gbrt_context* ctx, gbrt_batch* b, float* d_images,
         return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: wide nodes not allocated");
     if (b->launch.sort && (!b->sort_buf || b->sort_capacity < b->total_pixels))
         return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: sort buffers not allocated");
-    if (batch_wavefront_applies(b))
+    if (wavefront)
     {
         if (!ctx->d_trig) return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: frames not set on this context");
         return batch_wavefront(ctx, b, d_images, stream, force_collapse);
@@ -364,9 +367,10 @@ extern "C" gbrt_status gbrt_batch_pathtrace(gbrt_context* ctx, gbrt_batch* batch
     if (!ctx) return GBRT_ERR_INVALID_ARG;
     if (!batch) return fail(ctx, GBRT_ERR_INVALID_ARG, "batch_pathtrace: null batch");
     device_guard g(ctx->device);
-    gbrt_status st = ensure_batch_extras(ctx, batch);
+    bool wavefront = false;
+    gbrt_status st = ensure_batch_extras(ctx, batch, wavefront);
     if (st != GBRT_OK) return st;
-    return batch_frame_stage(ctx, batch, d_images, ctx->stream, false);
+    return batch_frame_stage(ctx, batch, d_images, ctx->stream, false, wavefront);
 }
 
 extern "C" gbrt_status gbrt_batch_run_graph(gbrt_context* ctx, gbrt_batch* batch, gbrt_triangle const* d_tris,
@@ -386,12 +390,13 @@ extern "C" gbrt_status gbrt_batch_run_graph(gbrt_context* ctx, gbrt_batch* batch
         }
         if (!batch->capture_stream)
             GBRT_CUDA(ctx, cudaStreamCreateWithFlags(&batch->capture_stream, cudaStreamNonBlocking));
-        gbrt_status est = ensure_batch_extras(ctx, batch);   // nothing allocates inside the capture
+        bool wavefront = false;
+        gbrt_status est = ensure_batch_extras(ctx, batch, wavefront);   // nothing allocates inside the capture
         if (est != GBRT_OK) return est;
         const uint64_t before = ctx->launches;
         GBRT_CUDA(ctx, cudaStreamBeginCapture(batch->capture_stream, cudaStreamCaptureModeThreadLocal));
         gbrt_status st = batch_build(ctx, batch, d_tris, batch->capture_stream);
-        if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, batch->capture_stream, true);
+        if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, batch->capture_stream, true, wavefront);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(batch->capture_stream, &graph);
         const uint64_t captured = ctx->launches - before;
@@ -446,12 +451,13 @@ extern "C" gbrt_status gbrt_batch_autotune(gbrt_context* ctx, gbrt_batch* batch,
     auto try_launch = [&](gbrt_batch_launch const& l) {
         if (result != GBRT_OK) return;
         batch->launch = l;
-        gbrt_status st = ensure_batch_extras(ctx, batch);
-        if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, ctx->stream, true);   // warm-up
+        bool wavefront = false;
+        gbrt_status st = ensure_batch_extras(ctx, batch, wavefront);
+        if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, ctx->stream, true, wavefront);   // warm-up
         for (uint32_t r = 0; st == GBRT_OK && r < reps; ++r)
         {
             if (r == 0 && cudaEventRecord(ev[0], ctx->stream) != cudaSuccess) st = GBRT_ERR_CUDA;
-            if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, ctx->stream, true);
+            if (st == GBRT_OK) st = batch_frame_stage(ctx, batch, d_images, ctx->stream, true, wavefront);
         }
         float ms = 0.0f;
         if (st == GBRT_OK && (cudaEventRecord(ev[1], ctx->stream) != cudaSuccess ||

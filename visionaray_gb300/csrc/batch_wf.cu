@@ -13,7 +13,9 @@
 //
 // Used for launches on the node pairs, unsorted, with the full 64-entry stack (a shorter
 // one reports trees it does not hold, which the quads' walk would not).  Enqueue only: the
-// buffers belong to the batch, so a captured frame stays valid whatever the context does.
+// buffers belong to the batch, so its captured frame stays valid whatever the context does.
+// A frame that the caller captures goes through the persistent kernel: its replays must
+// allow later calls to change the frames, and to need larger buffers.
 
 #include "batch_pt.cuh"
 #include "wavefront.cuh"
@@ -225,24 +227,30 @@ bool batch_wavefront_applies(gbrt_batch const* b)
            b->total_pixels > 0 && b->total_inner > 0;
 }
 
-gbrt_status ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b)
+bool ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b)
 {
-    if (!b->quads) GBRT_CUDA(ctx, cudaMalloc(&b->quads, (size_t(b->total_inner) + 1) * sizeof(quad_node)));
+    auto allocate = [](auto** p, size_t bytes) {
+        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+        *p = nullptr;
+        cudaGetLastError();
+        return false;
+    };
+    if (!b->quads && !allocate(&b->quads, (size_t(b->total_inner) + 1) * sizeof(quad_node))) return false;
     const pass_shape ps = shape_of(b);
     const uint32_t n = ps.pixels * ps.samples;
     frame_buffers fb;
     const size_t bytes = layout_frame_buffers(ps.pixels, n, 2 * (b->max_bounces + 1), false, 0, nullptr, fb) +
                          2 * align256(size_t(n) * 4);
-    if (b->path_bytes >= bytes) return GBRT_OK;
+    if (b->path_bytes >= bytes) return true;
     // frames in flight may still use the old buffers
-    GBRT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (b->path_buf && cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
     cudaFree(b->path_buf);
     b->path_buf = nullptr;
     b->path_bytes = 0;
     b->graph_dirty = true;
-    GBRT_CUDA(ctx, cudaMalloc(&b->path_buf, bytes));
+    if (!allocate(&b->path_buf, bytes)) return false;
     b->path_bytes = bytes;
-    return GBRT_OK;
+    return true;
 }
 
 gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, cudaStream_t s, bool force_quads)
