@@ -263,7 +263,8 @@ gbrt_status batch_wavefront(gbrt_context* ctx, gbrt_batch* b, float* d_images, c
         gbrt_status st = make_quads(ctx, b->nodes, b->total_inner, b->d_inner_offsets, b->num_scenes, 0, b->quads,
                                     nullptr, s);
         if (st != GBRT_OK) return st;
-        b->quads_gen = b->build_gen;
+        // only captured here: a graph that fails to come about has made none
+        if (!is_capturing(s)) b->quads_gen = b->build_gen;
     }
     const pass_shape ps = shape_of(b);
     const uint32_t num_counts = 2 * (b->max_bounces + 1);
