@@ -615,7 +615,8 @@ gbrt_status gbrt_batch_height(gbrt_context* ctx, gbrt_batch const* batch, uint32
 
 /* One frame of every scene (the same shading as gbrt_pathtrace_frame, so scene s's image
  * equals the one gbrt_pathtrace_frame renders with its camera, params and lights).  With
- * the full 64-entry stack, width 2 and no sorting (the default) the frame goes through the
+ * the full 64-entry stack, width 2 and no sorting (the default), scenes of more than a few
+ * hundred triangles and not too many bounces for the paths the frame goes through the
  * queues of the wavefront renderer, all scenes' paths together, and the block and tile of
  * the launch shape do not matter; otherwise, where the device has no room for the queues
  * (up to 1 GB, kept by the batch) and when the caller captures the frame in a graph, through

@@ -12,8 +12,9 @@
 // quad nodes of the 9.6 M triangles.
 //
 // Used for launches on the node pairs, unsorted, with the full 64-entry stack (a shorter
-// one reports trees it does not hold, which the quads' walk would not).  Enqueue only: the
-// buffers belong to the batch, so its captured frame stays valid whatever the context does.
+// one reports trees it does not hold, which the quads' walk would not), where it is the
+// faster one (batch_wavefront_applies).  Enqueue only: the buffers belong to the
+// batch, so its captured frame stays valid whatever the context does.
 // A frame that the caller captures goes through the persistent kernel: its replays must
 // allow later calls to change the frames, and to need larger buffers.
 
@@ -221,10 +222,30 @@ pass_shape shape_of(gbrt_batch const* b)
 
 } // namespace
 
+// Where the persistent kernel is the faster one (measured against it, ms wavefront and
+// persistent, one sample unless stated):
+//   - Every bounce is two launches for all paths, however few are left (6 us when none is),
+//     where the persistent kernel's threads end with their paths, but take a pixel's samples
+//     one after the other.  Trees of 2,000 triangles in the open: 65,536 pixels 0.31 and 0.31
+//     at 8 bounces, 0.39 and 0.32 at 16, 2.4 and 0.30 at 256; 1,048,576 pixels 0.84 and 0.92 at
+//     16, 1.01 and 0.92 at 32; 4,194,304 pixels 2.27 and 2.86 at 32, 4.55 and 2.85 at 256;
+//     4,096 pixels of 256 samples at 8 bounces 0.76 and 40.8.
+//   - Small trees are not worth the queues' traffic.  4,194,304 pixels, 1, 2 and 3 bounces:
+//     34 triangles (room with a blob) 0.50, 1.01, 1.61 and 0.26, 0.45, 0.71; 734 triangles 0.60,
+//     1.25, 1.93 and 0.34, 0.90, 1.91; 20,494 triangles 0.90, 1.84, 2.77 and 0.79, 2.42, 4.60;
+//     2,000 triangles in the open 1.02 and 1.23 at one bounce.  65,536 pixels, which do not fill
+//     the GPU: 34 triangles 0.04, 0.06, 0.08 and 0.02, 0.04, 0.06; 200 in the open 0.048 and
+//     0.071 at one bounce.
 bool batch_wavefront_applies(gbrt_batch const* b)
 {
-    return b->launch.width == 2 && b->launch.sort == 0 && b->launch.stack == uint32_t(kStackSize) &&
-           b->total_pixels > 0 && b->total_inner > 0;
+    if (b->launch.width != 2 || b->launch.sort != 0 || b->launch.stack != uint32_t(kStackSize) || b->total_pixels == 0 ||
+        b->total_inner == 0)
+        return false;
+    const pass_shape ps = shape_of(b);
+    if (b->max_bounces > 8ull * ps.samples + uint64_t(ps.pixels) * ps.samples / (1u << 17)) return false;
+    uint32_t least_triangles = b->max_bounces <= 1 ? 2048 : b->max_bounces == 2 ? 1024 : 256;
+    if (ps.pixels < (1u << 19)) least_triangles = ps.samples >= 4 ? 0 : 128;
+    return b->total / b->num_scenes >= least_triangles;
 }
 
 bool ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b)
