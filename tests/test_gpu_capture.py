@@ -273,3 +273,38 @@ def test_a_batch_frame_with_little_memory():
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     assert torch.equal(batch.pathtrace(batch.new_images()).view(torch.int32), want.view(torch.int32))
     batch.ctx.synchronize()
+
+
+def test_captured_queries_and_frames_over_a_rebuilt_tree():
+    """Replays after rebuilds and refits, among them one with triangles beyond what the quad
+    nodes cover, give what the calls give then."""
+    tris, mats, lights = scenes.box_scene(n_blobs=3, subdiv=3, seed=4)
+    ctx = vg.Context(0)
+    bvh = vg.lbvh_builder(ctx).build(vg.as_device_bytes(tris))
+    scene = vg.PTScene(bvh, mats, lights)
+    rays = random_rays(20000, 6)
+    params = scenes.pt_params(48, 36, 1, num_bounces=4, frame_id=3)
+    hits, image = torch.zeros((20000, 4), device="cuda"), torch.zeros((36, 48, 4), device="cuda")
+    vg.pathtrace_frame(scene, scenes.box_camera(), params, image)
+
+    def calls(hits, image):
+        vg.closest_hit(rays, bvh, out=hits)
+        vg.pathtrace_frame(scene, scenes.box_camera(), params, image)
+
+    graph = capture(ctx, lambda: calls(hits, image))
+    far = tris.copy()
+    far["v1"][::40] = 3e38
+    moved = tris.copy()
+    moved["v1"] += np.float32(0.01)
+    for geometry in (tris, far, moved):
+        for change in (bvh.rebuild, bvh.refit):
+            change(vg.as_device_bytes(geometry))
+            want = torch.zeros_like(hits), torch.zeros_like(image)
+            calls(*want)
+            hits.fill_(-1.0)
+            image.fill_(-1.0)
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(hits.view(torch.int32), want[0].view(torch.int32))
+            assert torch.equal(image.view(torch.int32), want[1].view(torch.int32))
+    ctx.synchronize()

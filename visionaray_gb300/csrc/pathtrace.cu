@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kBlock) pt_raygen(frame_buffers fb, uint32_t n
 // length takes, each warp finds its share from the length.
 __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(frame_buffers fb, int q, uint32_t bounce,
                                                                              uint32_t extend, bvh_view v,
-                                                                             uint32_t resident,
+                                                                             const float* bad, uint32_t resident,
                                                                              uint32_t* __restrict__ status)
 {
     __shared__ int stack_mem[kQuadStack * kQuadBlock];
@@ -98,12 +98,12 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) pt_trace_quads(fra
     auto index = [](uint32_t k) { return k; };
     auto root = [&](uint32_t) { return v.root; };
     if (closest)
-        quad_trace<false, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.rays[q], n, work, status, root, index,
+        quad_trace<false, true, kQuadPathSteps>(stack_mem, v, bad, fb.rays[q], n, work, status, root, index,
                                 [&](uint32_t j, trace_result const& h) {
                                     fb.hits[j] = make_uint4(uint32_t(h.tri), __float_as_uint(h.t), 0u, 0u);
                                 });
     else
-        quad_trace<true, true, kQuadPathSteps>(stack_mem, v, nullptr, fb.shadow_rays, n, work, status, root, index,
+        quad_trace<true, true, kQuadPathSteps>(stack_mem, v, bad, fb.shadow_rays, n, work, status, root, index,
                                [&](uint32_t j, trace_result const& h) {
                                    finish_shadow(fb, j, bounce - 1, h.tri >= 0);
                                });
@@ -1233,11 +1233,12 @@ gbrt_status with_tracer(gbrt_context* ctx, gbrt_pt_scene const* scene, gbrt_pt_p
     if (bvh->quads_ok && !wide && !sort)
     {
         const uint32_t resident = uint32_t(ctx->num_sms) * kQuadMinBlocks * (kQuadBlock / 32);
+        const float* bad = quads_validity(bvh, s);
         auto trace = [&](frame_buffers const& fb, int q, uint32_t b, uint32_t n, bool extend,
                          bool shadow) -> gbrt_status {
             const uint32_t grid = (std::min(n, resident) + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
             pt_trace_quads<<<dim3(grid, extend && shadow ? 2 : 1), kQuadBlock, 0, s>>>(fb, q, b, extend ? 1u : 0u, v,
-                                                                                       resident, ctx->d_status);
+                                                                                       bad, resident, ctx->d_status);
             GBRT_LAUNCH_CHECK(ctx, "pt_trace_quads");
             return GBRT_OK;
         };

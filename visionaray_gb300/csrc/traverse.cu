@@ -89,10 +89,12 @@ __global__ void __launch_bounds__(kTraceBlock, AnyHit ? kMinBlocksAny : kMinBloc
 }
 
 // The ray queries over the quad nodes, in the order perm if there is one.  taken: the zeroed
-// counter that long queries are shared by, or null.
+// counter that long queries are shared by, or null.  bad: the quads' validity word for a
+// captured query, whose replays see the trees of later builds; null for one that runs now.
 template <bool AnyHit>
 __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_view v, const gbrt_ray* __restrict__ rays,
                                                                           uint32_t n, uint32_t resident, uint32_t* taken,
+                                                                          const float* bad,
                                                                           const uint32_t* __restrict__ perm,
                                                                           gbrt_hit* __restrict__ hits,
                                                                           uint32_t* __restrict__ status)
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(kQuadBlock, kQuadMinBlocks) trace_quads(bvh_vi
     const quad_work work = quad_share(blockIdx.x * (kQuadBlock / 32) + (threadIdx.x >> 5), n, resident, taken);
     if (work.next >= work.end) return;
     quad_trace<AnyHit, !AnyHit, kQuadQuerySteps>(
-        stack_mem, v, nullptr, rays, n, work, status, [&](uint32_t) { return v.root; },
+        stack_mem, v, bad, rays, n, work, status, [&](uint32_t) { return v.root; },
         [&](uint32_t k) { return perm ? __ldg(&perm[k]) : k; },
         [&](uint32_t j, trace_result const& h) {
             const uint32_t prim = h.tri >= 0 ? __float_as_uint(ldg4(&v.tris[h.tri].t0).w) : GBRT_NO_HIT;
@@ -379,7 +381,8 @@ gbrt_status trace(gbrt_context* ctx, gbrt_bvh const* bvh, gbrt_ray const* d_rays
         const uint32_t grid = (warps + kQuadBlock / 32 - 1) / (kQuadBlock / 32);
         kernel_timer timer(ctx, stream);
         auto kernel = any_hit ? trace_quads<true> : trace_quads<false>;
-        kernel<<<grid, kQuadBlock, 0, stream>>>(v, d_rays, n, resident, taken, order, d_hits, ctx->d_status);
+        kernel<<<grid, kQuadBlock, 0, stream>>>(v, d_rays, n, resident, taken, quads_validity(bvh, stream), order, d_hits,
+                                                ctx->d_status);
         GBRT_LAUNCH_CHECK(ctx, "trace_quads");
         return GBRT_OK;
     };

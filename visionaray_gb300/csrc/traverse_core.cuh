@@ -463,6 +463,13 @@ inline bvh_view view_of(gbrt_bvh const* b)
              int32_t(b->num_nodes4), int32_t(b->num_prims), int32_t(b->num_nodes8) };
 }
 
+// The validity word of a tree's quads where a kernel has to look at it: in work that is
+// captured now and replayed over whatever a rebuild or a refit has put into the tree.
+inline const float* quads_validity(gbrt_bvh const* b, cudaStream_t stream)
+{
+    return is_capturing(stream) ? &b->quads[b->num_inner].org[0] : nullptr;
+}
+
 // Wide: the 4-wide nodes (present for trees with inner nodes built by the LBVH builder).
 template <bool AnyHit, bool Wide>
 __device__ __forceinline__ trace_result traverse_view(bvh_view const& v, f3 o, f3 d, float tmin, float tmax,
