@@ -308,3 +308,45 @@ def test_captured_queries_and_frames_over_a_rebuilt_tree():
             assert torch.equal(hits.view(torch.int32), want[0].view(torch.int32))
             assert torch.equal(image.view(torch.int32), want[1].view(torch.int32))
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("trees", [1, 2])
+def test_a_tree_is_destroyed_during_a_relaxed_capture(trees):
+    """A context's first tree and a later one: the capture goes on."""
+    ctx = vg.Context(0)
+    tris = vg.as_device_bytes(scenes.soup(5000, seed=1))
+    built = [vg.lbvh_builder(ctx).build(tris) for _ in range(trees)]
+    x = torch.zeros(64, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        x.add_(1)
+        built[-1].close()
+        x.add_(1)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 2.0
+
+
+def test_a_destroyed_tree_is_not_reused_under_queued_queries():
+    """Trees built into the memory of one whose queries are still queued."""
+    ctx = vg.Context(0)
+    tris = [scenes.soup(50000, seed=k, offset=0.05) for k in range(2)]
+    d = [vg.as_device_bytes(t) for t in tris]
+    keep = vg.lbvh_builder(ctx).build(d[0])
+    rays = random_rays(400_000, 8)
+    want = vg.closest_hit(rays, keep)
+    out = [torch.zeros_like(want) for _ in range(4)]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for k in range(4):
+        tree = vg.lbvh_builder(ctx).build(d[0])
+        with on_stream(ctx, side):
+            for _ in range(20):
+                vg.closest_hit(rays, tree, out=out[k])
+        tree.close()
+        vg.lbvh_builder(ctx).build(d[1]).close()
+    torch.cuda.synchronize()
+    for got in out:
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    ctx.synchronize()

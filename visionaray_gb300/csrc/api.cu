@@ -78,6 +78,7 @@ gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
     else
         GBRT_CUDA(ctx, cudaMalloc(&p, bytes));
     ctx->built_tree = true;
+    bvh->pooled = ctx->pool != nullptr;
     char* base = static_cast<char*>(p);
     bvh->arena = p;
     bvh->nodes = n > 1 ? reinterpret_cast<bvh2_node*>(base) : nullptr;
@@ -109,8 +110,14 @@ void free_bvh_arrays(gbrt_bvh* b)
     free_wide_nodes(b);
     if (b->arena)
     {
-        // what cudaFree does for memory of its own: no queued work reads the arrays any more
-        cudaDeviceSynchronize();
+        // cudaFree waits until no queued work reads memory of its own, but not for a pool's.
+        // So a small block of its own is freed first: unlike cudaDeviceSynchronize that is
+        // allowed while a stream is captured in relaxed mode.
+        void* block = nullptr;
+        if (b->pooled && cudaMalloc(&block, 256) == cudaSuccess)
+            cudaFree(block);
+        else if (b->pooled)
+            cudaDeviceSynchronize();
         cudaFree(b->arena);
         b->arena = nullptr;
     }

@@ -134,6 +134,7 @@ struct gbrt_bvh
     // GPU-built trees: one allocation that holds nodes, quads, tris, sorted_codes and
     // sorted_ids; null for uploaded trees, which own nodes and tris themselves
     void* arena = nullptr;
+    bool pooled = false;         // the arena is from the context's pool
     gbrt::bvh2_node* nodes = nullptr;
     gbrt::tri48* tris = nullptr; // leaf order
     // LBVH only: sorted Morton codes and, per sorted position, the input index.
