@@ -1,5 +1,6 @@
-"""Calls on several streams and in captured graphs: what a call enqueues does not depend on
-what the context's other calls do to its memory later or at the same time."""
+"""Calls on several streams, in captured graphs and with little memory: what a call enqueues
+does not depend on what the context's other calls do to its memory later or at the same
+time, and the memory that a context keeps to be faster is not asked for where there is none."""
 import contextlib
 
 import numpy as np
@@ -350,3 +351,44 @@ def test_a_destroyed_tree_is_not_reused_under_queued_queries():
     for got in out:
         assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     ctx.synchronize()
+
+
+def test_a_tree_with_little_memory():
+    """A tree without its quad nodes: built, rebuilt and refitted, traced as with them."""
+    ctx = vg.Context(0)
+    tris = scenes.heightfield(707, seed=1)
+    d, rays = vg.as_device_bytes(tris), random_rays(100_000, 9)
+    rays[:, 1] += 0.5
+    rays[:, 4] = -0.5
+    first = vg.lbvh_builder(ctx).build(d)
+    want = vg.closest_hit(rays, first)
+    nodes, idx = first.export_bvh2()
+    first.close()
+    with little_memory(150 << 20):   # the tree takes 184 MB, 120 without the quads
+        tree = vg.lbvh_builder(ctx).build(d)
+        got = [vg.closest_hit(rays, tree)]
+        tree.rebuild(d)
+        got.append(vg.closest_hit(rays, tree))
+        tree.refit(d)
+        got.append(vg.closest_hit(rays, tree))
+    for hits in got:
+        assert torch.equal(hits.view(torch.int32), want.view(torch.int32))
+    again, indices = tree.export_bvh2()
+    assert again.tobytes() == nodes.tobytes() and indices.tobytes() == idx.tobytes()
+    assert int((want.view(torch.int32)[:, 0] != -1).sum()) > 10_000
+    ctx.synchronize()
+
+
+def test_what_the_pool_keeps_is_given_back():
+    """A sorted query's scratch (134 MB) fits once the pool's freed trees are given back."""
+    ctx = vg.Context(0)
+    d, rays = vg.as_device_bytes(scenes.heightfield(707, seed=1)), random_rays(8_000_000, 9)
+    keep = vg.lbvh_builder(ctx).build(d)
+    want = vg.closest_hit(rays, keep)
+    out = torch.zeros_like(want)
+    vg.lbvh_builder(ctx).build(d).close()
+    with little_memory(50 << 20):
+        ctx.set_trace_flags(vg.Context.TRACE_SORT_RAYS)
+        vg.closest_hit(rays, keep, out=out)
+        ctx.synchronize()
+    assert torch.equal(out.view(torch.int32), want.view(torch.int32))

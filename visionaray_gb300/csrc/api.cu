@@ -22,6 +22,20 @@ gbrt_status check_cuda(gbrt_context* ctx, cudaError_t err, const char* where)
     return fail(ctx, err == cudaErrorMemoryAllocation ? GBRT_ERR_OUT_OF_MEMORY : GBRT_ERR_CUDA, msg);
 }
 
+cudaError_t device_malloc(gbrt_context* ctx, void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->pool)
+    {
+        cudaGetLastError();
+        e = cudaStreamSynchronize(ctx->stream);   // what it has freed is the pool's by then
+        if (e == cudaSuccess) e = cudaMemPoolTrimTo(ctx->pool, 0);
+        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
 {
     if (ctx->scratch_bytes >= bytes) return GBRT_OK;
@@ -34,7 +48,7 @@ gbrt_status ensure_scratch(gbrt_context* ctx, size_t bytes)
         ctx->scratch_bytes = 0;
     }
     size_t grow = std::max(bytes, size_t(1) << 20);
-    GBRT_CUDA(ctx, cudaMalloc(&ctx->scratch, grow));
+    GBRT_CUDA(ctx, device_malloc(ctx, &ctx->scratch, grow));
     ctx->scratch_bytes = grow;
     return GBRT_OK;
 }
@@ -70,20 +84,29 @@ gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n)
     }
     auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
     const size_t nodes = up(size_t(n - 1) * sizeof(bvh2_node)), tris = up(size_t(n) * sizeof(tri48)),
-                 words = up(size_t(n) * 4), quads = up(size_t(n) * sizeof(quad_node));
+                 words = up(size_t(n) * 4);
+    size_t quads = up(size_t(n) * sizeof(quad_node));
     void* p = nullptr;
-    const size_t bytes = nodes + quads + tris + 2 * words;
-    if (ctx->pool)
-        GBRT_CUDA(ctx, cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream));
-    else
-        GBRT_CUDA(ctx, cudaMalloc(&p, bytes));
+    auto allocate = [&]() {
+        const size_t bytes = nodes + quads + tris + 2 * words;
+        return ctx->pool ? cudaMallocFromPoolAsync(&p, bytes, ctx->pool, ctx->stream) : device_malloc(ctx, &p, bytes);
+    };
+    cudaError_t e = allocate();
+    if (e == cudaErrorMemoryAllocation)
+    {
+        // without the quads: queries go through the node pairs
+        cudaGetLastError();
+        quads = 0;
+        e = allocate();
+    }
+    if (e != cudaSuccess) return check_cuda(ctx, e, "tree");
     ctx->built_tree = true;
     bvh->pooled = ctx->pool != nullptr;
     char* base = static_cast<char*>(p);
     bvh->arena = p;
     bvh->nodes = n > 1 ? reinterpret_cast<bvh2_node*>(base) : nullptr;
     base += nodes;
-    bvh->quads = n > 1 ? reinterpret_cast<quad_node*>(base) : nullptr;
+    bvh->quads = n > 1 && quads ? reinterpret_cast<quad_node*>(base) : nullptr;
     base += quads;
     bvh->tris = reinterpret_cast<tri48*>(base);
     bvh->sorted_codes = reinterpret_cast<uint32_t*>(base + tris);
@@ -144,7 +167,7 @@ gbrt_status ensure_trace_scratch(gbrt_context* ctx, uint32_t n)
         ctx->trace_scratch = nullptr;
         ctx->trace_scratch_bytes = 0;
     }
-    GBRT_CUDA(ctx, cudaMalloc(&ctx->trace_scratch, bytes));
+    GBRT_CUDA(ctx, device_malloc(ctx, &ctx->trace_scratch, bytes));
     ctx->trace_scratch_bytes = bytes;
     return GBRT_OK;
 }
@@ -166,9 +189,9 @@ gbrt_status ensure_slots(gbrt_context* ctx, size_t rays_per_slot)
     {
         if (!ctx->slot_stream[k]) GBRT_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->slot_stream[k], cudaStreamNonBlocking));
         if (!ctx->slot_done[k]) GBRT_CUDA(ctx, cudaEventCreateWithFlags(&ctx->slot_done[k], cudaEventDisableTiming));
-        GBRT_CUDA(ctx, cudaMalloc(&ctx->slot_rays[k], rays_per_slot * sizeof(gbrt_ray)));
-        GBRT_CUDA(ctx, cudaMalloc(&ctx->slot_hits[k], rays_per_slot * sizeof(gbrt_hit)));
-        GBRT_CUDA(ctx, cudaMalloc(&ctx->slot_trace_scratch[k], trace_scratch_bytes(uint32_t(rays_per_slot))));
+        GBRT_CUDA(ctx, device_malloc(ctx, &ctx->slot_rays[k], rays_per_slot * sizeof(gbrt_ray)));
+        GBRT_CUDA(ctx, device_malloc(ctx, &ctx->slot_hits[k], rays_per_slot * sizeof(gbrt_hit)));
+        GBRT_CUDA(ctx, device_malloc(ctx, &ctx->slot_trace_scratch[k], trace_scratch_bytes(uint32_t(rays_per_slot))));
     }
     ctx->slot_capacity = rays_per_slot;
     ctx->slot_trace_scratch_bytes = trace_scratch_bytes(uint32_t(rays_per_slot));

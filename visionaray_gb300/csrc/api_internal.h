@@ -293,6 +293,8 @@ gbrt_status check_cuda(gbrt_context* ctx, cudaError_t err, const char* where);
 // The arrays of a tree of n > 0 triangles (nothing to do if it has them already): one
 // allocation from the context's pool.
 gbrt_status alloc_tree(gbrt_context* ctx, gbrt_bvh* bvh, uint32_t n);
+// cudaMalloc; where the device has no room, what the context's pool keeps is given back first.
+cudaError_t device_malloc(gbrt_context* ctx, void** p, size_t bytes);
 // Makes the context's memory pool, if it has none.
 gbrt_status ensure_pool(gbrt_context* ctx);
 // The host and device address of the context's build_result (allocated once).

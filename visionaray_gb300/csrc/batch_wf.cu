@@ -250,13 +250,17 @@ bool batch_wavefront_applies(gbrt_batch const* b)
 
 bool ensure_batch_wavefront(gbrt_context* ctx, gbrt_batch* b)
 {
-    auto allocate = [](auto** p, size_t bytes) {
-        if (cudaMalloc(p, bytes) == cudaSuccess) return true;
-        *p = nullptr;
+    auto allocate = [&](void** p, size_t bytes) {
+        if (device_malloc(ctx, p, bytes) == cudaSuccess) return true;
         cudaGetLastError();
         return false;
     };
-    if (!b->quads && !allocate(&b->quads, (size_t(b->total_inner) + 1) * sizeof(quad_node))) return false;
+    if (!b->quads)
+    {
+        void* quads = nullptr;
+        if (!allocate(&quads, (size_t(b->total_inner) + 1) * sizeof(quad_node))) return false;
+        b->quads = static_cast<quad_node*>(quads);
+    }
     const pass_shape ps = shape_of(b);
     const uint32_t n = ps.pixels * ps.samples;
     frame_buffers fb;

@@ -657,15 +657,16 @@ gbrt_status build_lbvh(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
         st = agglomerate<false>(ctx, args, s);
         if (st != GBRT_OK) return st;
         ctx->h_result->quads_bad = 0;
-        st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
-                        &result->quads_bad, s);
+        if (bvh->quads)
+            st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
+                            &result->quads_bad, s);
         if (st != GBRT_OK) return st;
         report_build<<<1, 1, 0, s>>>(bvh->nodes, root_height, result);
         GBRT_LAUNCH_CHECK(ctx, "report_build");
         GBRT_CUDA(ctx, cudaStreamSynchronize(s));
         const uint32_t h = ctx->h_result->height;
         bvh->height = h;
-        bvh->quads_ok = ctx->h_result->quads_bad == 0;
+        bvh->quads_ok = bvh->quads && ctx->h_result->quads_bad == 0;
         set_scene_box(bvh, *ctx->h_result);
 
         // collapse into wide nodes (on request), one level per launch; the pair tree has
@@ -798,15 +799,18 @@ gbrt_status refit_lbvh(gbrt_context* ctx, gbrt_bvh* bvh, gbrt_triangle const* d_
     build_result* result = nullptr;
     gbrt_status st = ensure_result(ctx, &result);
     if (st != GBRT_OK) return st;
-    GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
     ctx->h_result->quads_bad = 0;
-    st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
-                    &result->quads_bad, s);
+    if (bvh->quads)
+    {
+        GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
+        st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
+                        &result->quads_bad, s);
+    }
     if (st != GBRT_OK) return st;
     report_build<<<1, 1, 0, s>>>(bvh->nodes + (bvh->root > 0 ? bvh->root : 0), nullptr, result);
     GBRT_LAUNCH_CHECK(ctx, "report_build");
     GBRT_CUDA(ctx, cudaStreamSynchronize(s));
-    bvh->quads_ok = ctx->h_result->quads_bad == 0;
+    bvh->quads_ok = bvh->quads && ctx->h_result->quads_bad == 0;
     set_scene_box(bvh, *ctx->h_result);
     return GBRT_OK;
 }

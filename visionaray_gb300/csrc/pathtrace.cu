@@ -660,7 +660,7 @@ gbrt_status frame_buffers_for(gbrt_context* ctx, uint32_t npix, uint32_t num_bou
         for (size_t twice = 2 * kept;;)
         {
             const size_t bytes = std::max(std::max(bytes_for(samples), least), twice);
-            const cudaError_t e = cudaMalloc(&ctx->pt_scratch, bytes);
+            const cudaError_t e = device_malloc(ctx, &ctx->pt_scratch, bytes);
             if (e == cudaSuccess)
             {
                 ctx->pt_scratch_bytes = bytes;

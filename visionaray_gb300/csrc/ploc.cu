@@ -553,7 +553,7 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     ploc_tail<<<1, kTailThreads, kTailBytes, s>>>(lo[iter & 1], hi[iter & 1], state + (iter & 1), bvh->num_inner,
                                                   bvh->nodes, result, ctx->d_status);
     GBRT_LAUNCH_CHECK(ctx, "ploc_tail");
-    if (n > 1)
+    if (bvh->quads)
     {
         GBRT_CUDA(ctx, cudaMemsetAsync(bvh->quads + bvh->num_inner, 0, sizeof(quad_node), s));
         st = make_quads(ctx, bvh->nodes, bvh->num_inner, nullptr, 0, uint32_t(bvh->root), bvh->quads,
@@ -565,7 +565,7 @@ gbrt_status build_ploc(gbrt_context* ctx, gbrt_triangle const* d_tris, uint32_t 
     if (r.stuck) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: inconsistent merge step");
     if (r.made != n - 1) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: wrong node count");
     if (r.root != bvh->root) return fail(ctx, GBRT_ERR_CUDA, "PLOC build: unexpected root");
-    bvh->quads_ok = n > 1 && r.quads_bad == 0;
+    bvh->quads_ok = bvh->quads && r.quads_bad == 0;
     bvh->height = r.height;
     for (int a = 0; a < 3; ++a)
     {
