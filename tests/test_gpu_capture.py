@@ -392,3 +392,26 @@ def test_what_the_pool_keeps_is_given_back():
         vg.closest_hit(rays, keep, out=out)
         ctx.synchronize()
     assert torch.equal(out.view(torch.int32), want.view(torch.int32))
+
+
+def test_frames_after_a_replayed_graph():
+    """A frame on the stream after a replay renders the replay's trees, which quad nodes made
+    before it do not hold."""
+    parts = [scenes.soup(800, seed=k, offset=0.05) for k in range(2)]
+    batch = vg.Batch(np.array([0, 800]), vg.Context(0))
+    set_frames(batch, 1, 32, 1, 3)
+    d = [vg.as_device_bytes(t) for t in parts]
+    want = []
+    for k in range(2):
+        batch.build(d[k])
+        want.append(batch.pathtrace(batch.new_images()).clone())
+    images = batch.new_images()
+    batch.run_graph(d[0], images)
+    assert torch.equal(images, want[0])
+    batch.build(d[1])
+    assert torch.equal(batch.pathtrace(batch.new_images()), want[1])
+    batch.run_graph(d[0], images)
+    assert torch.equal(images, want[0])
+    assert torch.equal(batch.pathtrace(batch.new_images()), want[0])
+    assert not torch.equal(want[0], want[1])
+    batch.ctx.synchronize()

@@ -256,6 +256,7 @@ struct gbrt_batch
     cudaGraphExec_t graph = nullptr;
     uint64_t graph_launches = 0;    // kernels per replay
     bool graph_dirty = true;
+    bool graph_quads = false;       // whether it makes the quad nodes
     const void* graph_tris = nullptr;
     void* graph_images = nullptr;
 };

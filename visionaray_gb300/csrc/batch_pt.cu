@@ -416,8 +416,10 @@ extern "C" gbrt_status gbrt_batch_run_graph(gbrt_context* ctx, gbrt_batch* batch
         batch->graph_tris = d_tris;
         batch->graph_images = d_images;
         batch->graph_dirty = false;
+        batch->graph_quads = wavefront;
     }
     GBRT_CUDA(ctx, cudaGraphLaunch(batch->graph, ctx->stream));
+    batch->quads_gen = batch->graph_quads ? batch->build_gen : 0;   // the replay's trees
     ctx->launches += batch->graph_launches;
     return GBRT_OK;
 }
