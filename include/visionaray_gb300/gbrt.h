@@ -96,7 +96,11 @@ typedef struct gbrt_tlas    gbrt_tlas;
 /* Binds a context to CUDA device `device` and stream `stream` (a cudaStream_t, or
  * NULL for the legacy default stream).  No visionaray counterpart: visionaray's
  * builders and schedulers take the stream per call (detail/cuda_sched.h:39,
- * detail/bvh/lbvh.h:669-679); the context carries it once instead.               */
+ * detail/bvh/lbvh.h:669-679); the context carries it once instead.
+ * A context keeps device memory for its next calls until it is destroyed: scratch of the
+ * largest build and the largest sorted query, the buffers of its largest frame (up to about
+ * 1 GB, less where the device has less), and a pool of up to 4 GiB of destroyed trees and
+ * finished backward passes, which is given back when its own allocations fail.       */
 gbrt_status gbrt_context_create(int device, void* stream, gbrt_context** out);
 gbrt_status gbrt_context_destroy(gbrt_context* ctx);
 gbrt_status gbrt_context_set_stream(gbrt_context* ctx, void* stream);
@@ -389,7 +393,8 @@ typedef struct gbrt_pt_params
 /* Scheduling only: one thread per pixel runs all its samples and bounces (one launch
  * per frame, shadow rays traced in-thread) instead of the wavefront passes.  Same
  * arithmetic and random numbers: the images are identical bit for bit (but for rays in
- * the plane of a triangle, gbrt_trace_closest_hit).  About 2x slower than the wavefront on the box and inverse-rendering workloads (GB300).     */
+ * the plane of a triangle, gbrt_trace_closest_hit).  About 2x slower than the wavefront
+ * on the box and inverse-rendering workloads (GB300).                                */
 #define GBRT_PT_MEGAKERNEL 4u
 /* Scheduling only: each bounce's ray and shadow queues are ordered by the Morton cell
  * of their origins before they are traced (images identical bit for bit).  Slower on
@@ -489,8 +494,8 @@ gbrt_status gbrt_pathtrace_forward(gbrt_context* ctx, gbrt_pt_scene const* scene
  * vertices swept backwards; nothing of the forward frame is stored.  Paths are replayed in
  * passes whose state and vertex records take at most about 3 GB (less where the device has
  * less), allocated and freed in stream order: the call can be captured in a graph and may
- * overlap other calls on other streams.  Gradients are accumulated with warp-reduced FP32 atomics.  Geometry, visibility and
- * roulette decisions are not differentiated.  num_bounces <= 16.  A scene over
+ * overlap other calls on other streams.  Gradients are accumulated with warp-reduced FP32
+ * atomics.  Geometry, visibility and roulette decisions are not differentiated.  num_bounces <= 16.  A scene over
  * instances (gbrt_pt_scene_create_instanced) replays through the same two-level tree;
  * a slot's gradient sums the vertices of every instance that uses the slot.      */
 gbrt_status gbrt_pathtrace_backward(gbrt_context* ctx, gbrt_pt_scene const* scene,

@@ -8,7 +8,7 @@
 // scene's root, shading with that scene's constants, shadow rays.  The arithmetic and the
 // random numbers are the persistent kernel's, so the images are equal bit for bit.
 // Measured: 64 scenes of 1 k to 1 M triangles, 6.7 M one-sample pixels of 3 bounces: frame
-// 10.1 ms in the persistent kernel (launch {128, 32, 64, BLOCKS}), 8.3 here, 0.28 of them the
+// 10.1 ms in the persistent kernel (launch {128, 32, 64, BLOCKS}), 6.6 here, 0.32 of them the
 // quad nodes of the 9.6 M triangles.
 //
 // Used for launches on the node pairs, unsorted, with the full 64-entry stack (a shorter

@@ -11,7 +11,7 @@
 //     busy lane by two or three nodes, so no lane waits for a whole descent;
 //   - a warp refills its idle lanes from its rays, and takes more of them when they run out.
 // Measured, heightfield 2048^2 with 4,194,304 sorted secondary rays: 19 lanes active, the
-// query 3.36 -> 1.73 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.10 ms.  What
+// query 3.36 -> 1.78 ms; 8.4 M ambient-occlusion rays over 1024^2: 3.63 -> 2.15 ms.  What
 // bounds it now (a bounce of a 1920 x 1080 path-traced frame): the load/store pipe's
 // wavefronts (80 %), two per lane and node, then issue slots (72 %).
 //
